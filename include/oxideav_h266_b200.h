@@ -533,10 +533,10 @@ int h266_chain_plan_create_ex(h266_ctx *ctx, const h266_picture *pic, const h266
 int h266_chain_plan_device_sideinfo(const h266_chain_plan *plan);
 /* Which deblocking side information a picture gets (host only, no context,
  * no device): 0 built on the host (the crate's walk, src/deblock.rs:630-983);
- * 1 built on the device, no two edge footprints can overlap (luma CUs and
- * transform blocks of at least 8 samples, no sub-block grids, 4:2:0 or 4:0:0:
- * the grid-mode tile kernel when SAO or ALF runs); 2 built on the device with
- * footprints that may chain, other chroma formats (the grid-mode strip
+ * 1 built on the device, no edge segment writes samples another of its pass
+ * uses (no transform edges beside the sub-block grid of their CU, 4:2:0 or
+ * 4:0:0: the grid-mode tile kernel when SAO or ALF runs); 2 built on the device
+ * with segments that may chain, other chroma formats (the grid-mode strip
  * kernels).  Negative: an H266_ERR_* code for invalid arguments. */
 int h266_sideinfo_mode(const h266_picture *pic, const h266_in_loop_filter_args *args);
 /* Executes n plans on n device pictures (pics[i] with plans[i]; sizes may

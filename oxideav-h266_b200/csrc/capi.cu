@@ -736,7 +736,7 @@ struct DbSide {
   uint32_t n_comp[2] = {0, 0};
   uint32_t band_off[2][3] = {{0, 0, 0}, {0, 0, 0}};
   uint32_t n_bands[2][3] = {{0, 0, 0}, {0, 0, 0}};
-  bool tiles_ok = false;
+  bool tiles_ok = false, tiles_grid8 = false;
   uint32_t tiles_x = 0, tiles_y = 0;
   uint32_t tb_off[2][3] = {{0, 0, 0}, {0, 0, 0}};
   // side information built on the device: the walk's inputs (pointers are
@@ -759,6 +759,7 @@ void stage_deblock(const DeblockPlan &pl, std::vector<uint8_t> &b, Staged &st, D
     }
   }
   db.tiles_ok = pl.tiles_ok;
+  db.tiles_grid8 = pl.tiles_grid8;
   db.tiles_x = pl.tiles_x;
   db.tiles_y = pl.tiles_y;
   if (pl.tiles_ok) {
@@ -838,7 +839,7 @@ int run_deblock(h266_ctx *ctx, cudaStream_t stream, const uint8_t *base, const S
     Prof pf(ctx, stream, H266_PROF_DEBLOCK);
     return launch_deblock_tiles(stream, src, dst, lut, bd, v, h,
                                 reinterpret_cast<const uint32_t *>(base + st.tile_bounds), db.tb_off, db.n_bands,
-                                db.tiles_x, db.tiles_y, &ctx->launches);
+                                db.tiles_x, db.tiles_y, db.tiles_grid8, &ctx->launches);
   }
   if (!ctx->force_global_deblock && deblock_strips_fit(dst)) {
     Prof pf(ctx, stream, H266_PROF_DEBLOCK);
@@ -983,8 +984,9 @@ int prepare_chain(Prep &pr, const h266_picture &pic, const h266_in_loop_filter_a
   in.n_rows = a.n_clip_rows;
   H266_TRY(build_pass2(pic, in, pr.h));
   pr.blob.clear();
+  bool grid8 = false;
   const int mode = allow_device ? device_walk_mode(pic, a.cus, a.n_cus, a.chroma_cus, a.n_chroma_cus, a.deblock,
-                                                   a.chroma_format_idc)
+                                                   a.chroma_format_idc, &grid8)
                                 : 0;
   if (mode) {
     Blob blob{pr.blob};
@@ -993,6 +995,7 @@ int prepare_chain(Prep &pr, const h266_picture &pic, const h266_in_loop_filter_a
     db.dw_tiles = mode == 1 && (pr.h.do_sao || pr.h.do_alf);
     db.dw.tile_lists = mode == 1;  // the walk lists each tile's cells (within the lists' caps in mode 1)
     db.dw.tiles_consume = db.dw_tiles;
+    db.dw.grid8 = grid8;
     db.dw_sep = a.chroma_cus != nullptr;
     db.dw_mv = a.mv_grid && a.mv_grid->cells && a.mv_grid->cells_w * a.mv_grid->cells_h;
     DeviceWalkIn &w = db.dw;
@@ -1010,7 +1013,6 @@ int prepare_chain(Prep &pr, const h266_picture &pic, const h266_in_loop_filter_a
     w.cw = (int)pic.cb.width;
     w.ch = (int)pic.cb.height;
     // the CU lists packed: every CU's head, the tails of CUs with a TU map or a TB split
-    w.max_cu_dim = 4;
     const h266_deblock_cu *lists[2] = {a.cus, a.chroma_cus};
     const uint64_t counts[2] = {a.n_cus, db.dw_sep ? a.n_chroma_cus : 0};
     thread_local std::vector<CuTail> tails;
@@ -1054,9 +1056,6 @@ int prepare_chain(Prep &pr, const h266_picture &pic, const h266_in_loop_filter_a
         } else {
           std::memcpy(heads + i * kCuHeadBytes, &c, kCuHeadBytes);
         }
-        // only sub-block grids, TB splits and 64-sample TU tiling put edges inside a CU
-        if (c.has_num_sb || c.has_tb_split || (c.has_tu64 && std::max(c.w, c.h) > 64))
-          w.max_cu_dim = std::max(w.max_cu_dim, std::max(c.w, c.h));
         if (c.has_tu64 || c.has_tb_split) {
           CuTail t;
           t.index = (uint32_t)i;
@@ -2676,8 +2675,9 @@ int check_plan_batch(h266_ctx *ctx, uint32_t n, h266_chain_plan *const *plans, h
 // Queues a batch of chain executions on `stream` with its parameter tables in
 // `bb`: the device walks of the pictures that derive their side information
 // on the device (three launches for all of them), one tile-deblocking launch
-// and one SAO/ALF launch per kernel variant over every picture's tiles, and
-// per picture whatever the batched kernels do not take.
+// per region size over every picture's tiles, the strip kernels' two launches
+// over every other picture, one SAO/ALF launch per kernel variant, and per
+// picture whatever the batched kernels do not take.
 // `upload`: the stream that carries the parameter table's upload (the
 // end-to-end pipeline's upload stream, so that the table is copied in issue
 // order with the planes instead of competing with them); `stream` by default.
@@ -2687,24 +2687,47 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
   if (!n) return H266_OK;
   H266_TRY(bb.init());
   struct Run {
-    bool tile, packed;
+    bool tile, strips, packed;
     int variant;
   };
   std::vector<Run> runs(n);
-  std::vector<uint8_t> tile_params, walk_items;
-  std::vector<uint32_t> tile_first(1, 0), walk_first[3] = {{0}, {0}, {0}};  // clear, CU map, walk CTAs
+  std::vector<uint8_t> tile_params[2], walk_items;  // tiles: by region, [1] for edges on the 8x8 grid
+  std::vector<uint32_t> tile_first[2] = {{0}, {0}}, walk_first[3] = {{0}, {0}, {0}};  // clear, CU map, walk CTAs
   WalkBatchCounts walk_total;
   const size_t wis = walk_batch_item_size();
   std::vector<Pass2Args> p2[kPass2Variants];
   std::vector<uint32_t> p2_first[kPass2Variants];
-  const size_t tps = deblock_tile_params_size();
+  const size_t tps = deblock_tile_params_size(), sps = strip_params_size();
+  std::vector<uint8_t> strip_params[2];  // rows, columns
+  std::vector<uint32_t> strip_first[2] = {{0}, {0}};
+  StripCounts strip_total;
+  auto add_strips = [&] {
+    for (std::vector<uint8_t> &p : strip_params) p.resize(p.size() + sps);
+    return std::make_pair(strip_params[0].data() + strip_params[0].size() - sps,
+                          strip_params[1].data() + strip_params[1].size() - sps);
+  };
+  auto count_strips = [&](const StripCounts &c) {
+    strip_total.rows += c.rows;
+    strip_total.cols += c.cols;
+    strip_total.smem_rows = std::max(strip_total.smem_rows, c.smem_rows);
+    strip_total.smem_cols = std::max(strip_total.smem_cols, c.smem_cols);
+    strip_first[0].push_back(strip_total.rows);
+    strip_first[1].push_back(strip_total.cols);
+  };
   for (uint32_t i = 0; i < n; ++i) {
     BatchItem &it = items[i];
     Run &r = runs[i];
     const uint8_t *base = it.st.base;
     r.tile = it.pass2 && (it.db.device_walk ? it.db.dw_tiles : it.db.tiles_ok) && !ctx->force_global_deblock &&
              !ctx->force_strip_deblock;
-    if (r.tile && it.db.device_walk) {  // the side information is derived on the device first, batched
+    const DPlane *dst = it.pass2 ? it.S : it.P;
+    // pictures filtered in place and listed twice run one after the other
+    const bool twice = !it.pass2 && std::count_if(items.begin(), items.end(), [&](const BatchItem &o) {
+                                      return !o.pass2 && o.P[0].s == it.P[0].s;
+                                    }) > 1;
+    r.strips = !r.tile && !twice && (it.db.device_walk || (!ctx->force_global_deblock && deblock_strips_fit(dst)));
+    if (it.db.device_walk && !twice) {  // the side information is derived on the device first, batched
+      if (!it.walk) return set_error(H266_ERR_INVALID_ARGUMENT, "device-built side information without walk scratch");
       DeviceWalkOut g;
       WalkBatchCounts c;
       walk_items.resize(walk_items.size() + wis);
@@ -2713,23 +2736,39 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
       walk_first[0].push_back(walk_first[0].back() + c.clear_ctas);
       walk_first[1].push_back(walk_first[1].back() + c.grid_ctas);
       walk_first[2].push_back(walk_first[2].back() + c.walk_ctas);
-      walk_total.offsets = std::max(walk_total.offsets, c.offsets);
-      tile_params.resize(tile_params.size() + tps);
-      const uint32_t tc =
-          fill_deblock_tile_params_grid(tile_params.data() + tile_params.size() - tps, it.P, it.S, it.lut, it.bd, g);
-      tile_first.push_back(tile_first.back() + tc);
-    } else if (r.tile) {
+      if (r.tile) {
+        std::vector<uint8_t> &tp = tile_params[it.db.dw.grid8];
+        std::vector<uint32_t> &tf = tile_first[it.db.dw.grid8];
+        tp.resize(tp.size() + tps);
+        tf.push_back(tf.back() +
+                     fill_deblock_tile_params_grid(tp.data() + tp.size() - tps, it.P, it.S, it.lut, it.bd, g));
+      } else {
+        auto [rows, cols] = add_strips();
+        StripCounts sc;
+        H266_TRY(fill_strip_params_grid(rows, cols, it.P, dst, it.lut, it.bd, g, sc));
+        count_strips(sc);
+      }
+    } else if (r.tile || r.strips) {
       const StripSide v{reinterpret_cast<const EdgeSeg *>(base + it.st.seg[0]),
                         reinterpret_cast<const uint32_t *>(base + it.st.comp[0]),
                         reinterpret_cast<const uint32_t *>(base + it.st.band[0])};
       const StripSide h{reinterpret_cast<const EdgeSeg *>(base + it.st.seg[1]),
                         reinterpret_cast<const uint32_t *>(base + it.st.comp[1]),
                         reinterpret_cast<const uint32_t *>(base + it.st.band[1])};
-      tile_params.resize(tile_params.size() + tps);
-      const uint32_t c = fill_deblock_tile_params(tile_params.data() + tile_params.size() - tps, it.P, it.S, it.lut,
-                                                  it.bd, v, h, reinterpret_cast<const uint32_t *>(base + it.st.tile_bounds),
-                                                  it.db.tb_off, it.db.n_bands, it.db.tiles_x, it.db.tiles_y);
-      tile_first.push_back(tile_first.back() + c);
+      if (r.strips) {
+        auto [rows, cols] = add_strips();
+        StripCounts sc;
+        fill_strip_params(rows, cols, it.P, dst, it.lut, it.bd, v, h, it.db.band_off, it.db.n_bands, sc);
+        count_strips(sc);
+      } else {
+        std::vector<uint8_t> &tp = tile_params[it.db.tiles_grid8];
+        std::vector<uint32_t> &tf = tile_first[it.db.tiles_grid8];
+        tp.resize(tp.size() + tps);
+        tf.push_back(tf.back() + fill_deblock_tile_params(
+                                     tp.data() + tp.size() - tps, it.P, it.S, it.lut, it.bd, v, h,
+                                     reinterpret_cast<const uint32_t *>(base + it.st.tile_bounds), it.db.tb_off,
+                                     it.db.n_bands, it.db.tiles_x, it.db.tiles_y, it.db.tiles_grid8));
+      }
     }
     r.packed = it.pass2 && it.packed && !ctx->force_scalar;
     r.variant = -1;
@@ -2748,8 +2787,16 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
   std::vector<uint8_t> &b = bb.blob;
   b.clear();
   Blob blob{b};
-  const size_t off_tp = blob.put(tile_params.data(), tile_params.size());
-  const size_t off_tf = blob.put(tile_first.data(), tile_first.size() * sizeof(uint32_t));
+  size_t off_tp[2], off_tf[2];
+  for (int k = 0; k < 2; ++k) {
+    off_tp[k] = blob.put(tile_params[k].data(), tile_params[k].size());
+    off_tf[k] = blob.put(tile_first[k].data(), tile_first[k].size() * sizeof(uint32_t));
+  }
+  size_t off_sp[2], off_sf[2];
+  for (int k = 0; k < 2; ++k) {
+    off_sp[k] = blob.put(strip_params[k].data(), strip_params[k].size());
+    off_sf[k] = blob.put(strip_first[k].data(), strip_first[k].size() * sizeof(uint32_t));
+  }
   const size_t off_wi = blob.put(walk_items.data(), walk_items.size());
   size_t off_wf[3];
   for (int k = 0; k < 3; ++k) off_wf[k] = blob.put(walk_first[k].data(), walk_first[k].size() * sizeof(uint32_t));
@@ -2773,13 +2820,7 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
   H266_CUDA(cudaEventRecord(bb.staged, ups));
   if (ups != stream) H266_CUDA(cudaStreamWaitEvent(stream, bb.staged, 0));
   const uint8_t *dside = bb.side.as<uint8_t>();
-  // deblocking: per picture where the tile kernel does not apply, then the batched walks and tiles
-  for (uint32_t i = 0; i < n; ++i) {
-    BatchItem &it = items[i];
-    if (runs[i].tile) continue;
-    if (it.pass2) H266_TRY(run_deblock(ctx, stream, it.st.base, it.st, it.db, it.P, it.S, it.lut, it.bd, it.walk));
-    else H266_TRY(run_deblock(ctx, stream, it.st.base, it.st, it.db, it.P, it.P, it.lut, it.bd, it.walk));
-  }
+  // deblocking: the batched walks, per picture where only global memory takes the planes, then the batched strips and tiles
   if (walk_first[0].size() > 1) {
     walk_total.clear_ctas = walk_first[0].back();
     walk_total.grid_ctas = walk_first[1].back();
@@ -2790,10 +2831,23 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
                                reinterpret_cast<const uint32_t *>(dside + off_wf[2]), (int)walk_first[0].size() - 1,
                                walk_total, &ctx->launches));
   }
-  if (tile_first.size() > 1) {
+  for (uint32_t i = 0; i < n; ++i) {
+    BatchItem &it = items[i];
+    if (runs[i].tile || runs[i].strips) continue;
+    H266_TRY(run_deblock(ctx, stream, it.st.base, it.st, it.db, it.P, it.pass2 ? it.S : it.P, it.lut, it.bd, it.walk));
+  }
+  if (strip_first[0].size() > 1) {
     Prof pf(ctx, stream, H266_PROF_DEBLOCK);
-    H266_TRY(launch_deblock_tiles_batch(stream, dside + off_tp, reinterpret_cast<const uint32_t *>(dside + off_tf),
-                                        (int)tile_first.size() - 1, tile_first.back(), &ctx->launches));
+    H266_TRY(launch_strips_batch(stream, dside + off_sp[0], reinterpret_cast<const uint32_t *>(dside + off_sf[0]),
+                                 dside + off_sp[1], reinterpret_cast<const uint32_t *>(dside + off_sf[1]),
+                                 (int)strip_first[0].size() - 1, strip_total, &ctx->launches));
+  }
+  for (int k = 0; k < 2; ++k) {
+    if (tile_first[k].size() < 2) continue;
+    Prof pf(ctx, stream, H266_PROF_DEBLOCK);
+    H266_TRY(launch_deblock_tiles_batch(stream, k != 0, dside + off_tp[k],
+                                        reinterpret_cast<const uint32_t *>(dside + off_tf[k]),
+                                        (int)tile_first[k].size() - 1, tile_first[k].back(), &ctx->launches));
   }
   // SAO / ALF: per picture where the packed kernel does not apply, then one launch per variant
   for (uint32_t i = 0; i < n; ++i) {

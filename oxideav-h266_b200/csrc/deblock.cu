@@ -6,12 +6,9 @@
 // samples, so it is done up front here and produces an explicit segment list.
 // Segments are then grouped into components: two segments of the same pass
 // and plane that lie on the same 4-line (luma) or 2-line (chroma) band and
-// whose sample footprints overlap along the edge normal are in one component.
-// A segment's footprint is [pos - R(mflP), pos + R(mflQ)) with R(m) = 4 for
-// m <= 3 and m + 1 otherwise: every sample the decision or the filters of
-// src/deblock.rs:1224-2075 read or write lies inside it.  Segments of
-// different components therefore touch disjoint samples and commute; inside
-// a component the segments keep the reference's processing order.  The
+// one of which writes samples that the other uses are in one component
+// (seg_span).  Segments of different components therefore commute; inside a
+// component the segments keep the reference's processing order.  The
 // vertical pass runs to completion before the horizontal one, as in
 // apply_deblocking_clipped (src/deblock.rs:540-615).
 //
@@ -19,6 +16,7 @@
 // reference's clamped reads and bounds-checked Clip1 writes on global memory.
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cstring>
 #include <memory>
 #include <numeric>
@@ -363,18 +361,14 @@ H266_HD inline void walk_segment(const h266_deblock_cu *cus_, const Grid &grid, 
 
 // deblock_cu_dir (src/deblock.rs:707-983) for CU `idx`: every edge segment it
 // owns, in the reference's order, passed to `emit`.
-#pragma nv_exec_check_disable
-// `only_off` >= 0 restricts the walk to the edge at that offset inside the CU
-// (the device runs one thread per offset).
 template <class Grid, class Mv, class Emit>
-H266_HD void walk_cu(const h266_deblock_cu *cus_, const Grid &grid, const PlaneCfg &pc, bool vert, const Mv &mv,
-                     const uint32_t *nf, uint64_t n_nf, size_t idx, Emit &emit, int only_off = -1) {
+void walk_cu(const h266_deblock_cu *cus_, const Grid &grid, const PlaneCfg &pc, bool vert, const Mv &mv,
+             const uint32_t *nf, uint64_t n_nf, size_t idx, Emit &emit) {
   const h266_deblock_cu &cu = cus_[idx];
   const CuWalkGeo g = cu_walk_geo(cu, pc, vert, nf, n_nf);
   if (g.off_grid) return;
   Cu q_geo{cu};
-  for (uint32_t off = only_off >= 0 ? (uint32_t)only_off : 0; off < g.n_cb; off += g.step) {
-    if (only_off >= 0 && off != (uint32_t)only_off) break;
+  for (uint32_t off = 0; off < g.n_cb; off += g.step) {
     const bool is_tb = off == 0 ? g.filter_edge : q_geo.tb_boundary(off, vert, g.chroma);
     const bool is_sb = !g.chroma && off % g.sb == 0 && off / g.sb <= g.last_sb && (off > 0 || g.filter_edge);
     if (!is_tb && !is_sb) continue;
@@ -395,21 +389,66 @@ void Walker::walk(const PlaneCfg &pc, bool vert, const MvGrid &mv, const uint32_
   for (size_t idx = 0; idx < n_; ++idx) walk_cu(cus_, *this, pc, vert, mv, nf, n_nf, idx, emit);
 }
 
-inline int reach(int m) { return m <= 3 ? 4 : m + 1; }
-__device__ __forceinline__ int reach_d(int m) { return m <= 3 ? 4 : m + 1; }
+// The samples a segment's side reads and writes, counted from the edge.  A luma
+// side of maxFilterLength m (`other`: the far side's) writes m samples (one at
+// least) and its decision and filters use m + 1 of them, three at least
+// (src/deblock.rs:1224-1776): p0..p2 always, p3 only where the strong filter is
+// open (both lengths above 2) or the far side is long, which also makes a short
+// side 3.  Chroma uses 4 and writes 3 (src/deblock.rs:1803-2075).  The filters
+// load more samples than they use, so two segments depend on each other only
+// where one writes what the other uses: edges 4 apart (maxFilterLength 1 on
+// both sides) and 8 apart (3) do not, as the standard means them not to.
+H266_HD inline int reach_w(int m, int other, bool chroma) {
+  return chroma ? 3 : std::max(other > 3 ? std::max(m, 3) : m, 1);
+}
+H266_HD inline int reach_r(int m, int other, bool chroma) {
+  const int w = reach_w(m, other, chroma);
+  return w <= 2 ? 3 : w + 1;
+}
+struct SegSpan {  // along the edge normal: [ws, we) written, [rs, re) used
+  int ws, we, rs, re;
+};
+#ifndef __CUDA_ARCH__
+// seg_span's distances by the segment's length byte, for the host's lists of 10^5 segments.
+struct ReachTable {
+  int8_t d[2][256][4];  // [chroma]: write P, write Q, use P, use Q
+  ReachTable() {
+    for (int c = 0; c < 2; ++c)
+      for (int m = 0; m < 256; ++m) {
+        const int mp = m >> 4, mq = m & 15;
+        d[c][m][0] = (int8_t)reach_w(mp, mq, c != 0);
+        d[c][m][1] = (int8_t)reach_w(mq, mp, c != 0);
+        d[c][m][2] = (int8_t)reach_r(mp, mq, c != 0);
+        d[c][m][3] = (int8_t)reach_r(mq, mp, c != 0);
+      }
+  }
+};
+const ReachTable kReach;
+#endif
+H266_HD inline SegSpan seg_span(const EdgeSeg &s) {
+  const int pos = (s.flags & 1) ? s.x : s.y;
+  const bool c = s.plane != 0;
+#ifndef __CUDA_ARCH__
+  const int8_t *t = kReach.d[c][s.mfl];
+  return SegSpan{pos - t[0], pos + t[1], pos - t[2], pos + t[3]};
+#endif
+  const int mp = s.mfl >> 4, mq = s.mfl & 15;
+  return SegSpan{pos - reach_w(mp, mq, c), pos + reach_w(mq, mp, c), pos - reach_r(mp, mq, c), pos + reach_r(mq, mp, c)};
+}
 
 // Groups one (pass, plane) segment list into components and appends them.
-// Components come out band by band, by footprint start inside a band, with
-// their members in emission (reference) order.  Segments are bucketed by band
-// in emission order; decode order visits the CUs crossing a band from its low
+// Components come out band by band, by position inside a band, with their
+// members in emission (reference) order.  Segments are bucketed by band in
+// emission order; decode order visits the CUs crossing a band from its low
 // end to its high end (z-scan inside a CTB, raster / tile order between CTBs),
-// so a bucket is normally sorted by footprint start already and the pass is
-// linear.  A bucket that is not (CU lists in an unusual order) is sorted, and
-// its components' members are put back in emission order.
+// so a bucket is normally sorted by position already and the pass is linear.
+// A bucket that is not (CU lists in an unusual order) is sorted, and its
+// components' members are put back in emission order.  A component ends where
+// nothing before writes what anything after uses, nor the other way round.
 struct GroupScratch {
-  struct Item {  // a segment with its footprint and emission index, bucketed by band
+  struct Item {  // a segment with its position and emission index, bucketed by band
     EdgeSeg s;
-    int32_t start, end;
+    int32_t pos;
     uint32_t i;
   };
   std::vector<uint32_t> head;
@@ -438,8 +477,7 @@ void group(const std::vector<Emitted> &segs, std::vector<EdgeSeg> &dst, std::vec
       const EdgeSeg &s = segs[i].s;
       const bool vert = s.flags & 1;
       const int pos = vert ? s.x : s.y;
-      g.items[cur[vert ? s.y : s.x]++] =
-          GroupScratch::Item{s, pos - reach(s.mfl >> 4), pos + reach(s.mfl & 15), (uint32_t)i};
+      g.items[cur[vert ? s.y : s.x]++] = GroupScratch::Item{s, pos, (uint32_t)i};
     }
     for (size_t b = g.head.size() - 1; b > 0; --b) g.head[b] = g.head[b - 1];  // cursor[b] ended at start[b + 1]
     g.head[0] = 0;
@@ -449,19 +487,28 @@ void group(const std::vector<Emitted> &segs, std::vector<EdgeSeg> &dst, std::vec
   EdgeSeg *out = dst.data() + d0;
   size_t o = 0;
   uint32_t longest = max_len;
-  auto by_start = [](const GroupScratch::Item &a, const GroupScratch::Item &b) { return a.start < b.start; };
+  auto by_pos = [](const GroupScratch::Item &a, const GroupScratch::Item &b) { return a.pos < b.pos; };
   for (size_t b = 0; b + 1 < g.head.size(); ++b) {
     GroupScratch::Item *lo = g.items.data() + g.head[b], *hi = g.items.data() + g.head[b + 1];
     if (lo == hi) continue;
-    const bool sorted = std::is_sorted(lo, hi, by_start);
-    if (!sorted) std::stable_sort(lo, hi, by_start);  // ties keep emission order
+    const bool sorted = std::is_sorted(lo, hi, by_pos);
+    if (!sorted) std::stable_sort(lo, hi, by_pos);  // ties keep emission order
+    int32_t we = INT32_MIN, re = INT32_MIN;  // furthest write and use so far
     for (GroupScratch::Item *i = lo; i < hi;) {
-      GroupScratch::Item *j = i + 1;
-      int32_t e = i->end;
-      while (j < hi && j->start < e) {
-        e = std::max(e, j->end);
+      GroupScratch::Item *j = i;
+      bool meets;  // something from j on writes what something before uses, or the other way round
+      do {
+        const SegSpan f = seg_span(j->s);
+        we = std::max(we, f.we);
+        re = std::max(re, f.re);
+        const int32_t far = j->pos + 16;  // a side reaches at most 8 samples
         ++j;
-      }
+        meets = false;
+        for (const GroupScratch::Item *k = j; k < hi && k->pos < far && !meets; ++k) {
+          const SegSpan q = seg_span(k->s);
+          meets = we > q.rs || re > q.ws;
+        }
+      } while (meets);
       comp.push_back((uint32_t)(d0 + o));
       if (sorted || j - i == 1) {
         for (GroupScratch::Item *t = i; t < j; ++t) out[o++] = t->s;
@@ -504,23 +551,18 @@ void index_bands(const h266_picture &pic, DeblockPlan &plan) {
   }
 }
 
-// Fills the component ranges of the tile kernel.  A vertical-pass component
-// runs in every tile whose columns its footprint reaches and whose rows
-// widened by the halo hold its band (the horizontal pass of those rows reads
-// its output); a horizontal-pass component runs in the tile holding its band
-// whose rows its footprint reaches.  Footprints are clipped to the plane, so
-// components touching no sample of it are in no range.
-void index_tiles(const h266_picture &pic, uint32_t cfi, DeblockPlan &plan) {
-  plan.tiles_ok = false;
+// Fills the component ranges of the tile kernel for regions widened by `hx`
+// columns and `hy` rows of luma (kTileHaloXC / kTileHaloYC of chroma); false
+// when the regions are too small for the plan.  A vertical-pass component runs
+// in every tile whose columns it writes and whose rows widened by the halo
+// hold its band (the horizontal pass of those rows uses its output); a
+// horizontal-pass component runs in the tile holding its band whose rows it
+// writes.  Everything a listed component uses must lie in the region, and what
+// it uses is written by no component outside it (components of a band touch
+// each other's samples nowhere).
+bool index_tiles_halo(const h266_picture &pic, DeblockPlan &plan, int hx, int hy) {
   const int T = kDeblockTile;
   const int w = (int)pic.luma.width, h = (int)pic.luma.height;
-  plan.tiles_x = (uint32_t)((w + T - 1) / T);
-  plan.tiles_y = (uint32_t)((h + T - 1) / T);
-  const bool chroma = (uint64_t)pic.cb.width * pic.cb.height != 0 || (uint64_t)pic.cr.width * pic.cr.height != 0;
-  if (cfi > 1 || (cfi == 0 && chroma)) return;
-  if (chroma && (pic.cb.width != (pic.luma.width + 1) / 2 || pic.cb.height != (pic.luma.height + 1) / 2 ||
-                 pic.cr.width != pic.cb.width || pic.cr.height != pic.cb.height))
-    return;
   const int tiles_x = (int)plan.tiles_x, tiles_y = (int)plan.tiles_y;
   std::vector<uint32_t> &tb = plan.tile_bounds;
   tb.clear();
@@ -535,47 +577,47 @@ void index_tiles(const h266_picture &pic, uint32_t cfi, DeblockPlan &plan) {
       plan.tb_off[d][p] = (uint32_t)tb.size();
       const uint32_t nb = plan.n_bands[d][p];
       if (!nb) continue;
-      const int tp = p ? T / 2 : T, halo = p ? kDeblockHaloC : kDeblockHaloY, unit = p ? 2 : 4;
+      const int tp = p ? T / 2 : T, unit = p ? 2 : 4;
+      const int halo = d == 0 ? (p ? kTileHaloXC : hx) : (p ? kTileHaloYC : hy);  // along the edge normal
+      const int rows = p ? kTileHaloYC : hy;  // vertical pass: rows around the tile whose bands run
       const int along = d == 0 ? (p ? (int)pic.cb.width : w) : (p ? (int)pic.cb.height : h);
-      const int n_t = d == 0 ? tiles_x : tiles_y;  // tiles along the footprint axis
+      const int n_t = d == 0 ? tiles_x : tiles_y;  // tiles along the edge normal
       const uint32_t *bf = plan.band_first[d].data() + plan.band_off[d][p];
       const size_t base = tb.size();
       tb.resize(base + (size_t)nb * n_t * 2);
-      thread_local std::vector<int32_t> fs, fe;  // clipped footprints of one band's components
+      thread_local std::vector<SegSpan> sp;  // spans of one band's components, inside the plane
       for (uint32_t b = 0; b < nb; ++b) {
         const uint32_t c0 = bf[b], c1 = bf[b + 1];
-        fs.resize(c1 - c0);
-        fe.resize(c1 - c0);
+        sp.resize(c1 - c0);
         for (uint32_t c = c0; c < c1; ++c) {
-          const EdgeSeg &f = segs[comp[c]];
-          const int pos = (f.flags & 1) ? f.x : f.y;
-          int s = pos - reach(f.mfl >> 4), e = pos + reach(f.mfl & 15);
+          SegSpan f = seg_span(segs[comp[c]]);
           for (uint32_t i = comp[c] + 1; i < comp[c + 1]; ++i) {
-            const EdgeSeg &g = segs[i];
-            const int q = (g.flags & 1) ? g.x : g.y;
-            s = std::min(s, q - reach(g.mfl >> 4));
-            e = std::max(e, q + reach(g.mfl & 15));
+            const SegSpan g = seg_span(segs[i]);
+            f.ws = std::min(f.ws, g.ws);
+            f.we = std::max(f.we, g.we);
+            f.rs = std::min(f.rs, g.rs);
+            f.re = std::max(f.re, g.re);
           }
-          if (e - s > halo) return;  // longer than the halo: strip kernels
-          fs[c - c0] = std::max(s, 0);
-          fe[c - c0] = std::min(e, along);
+          sp[c - c0] = SegSpan{std::max(f.ws, 0), std::min(f.we, along), std::max(f.rs, 0), std::min(f.re, along)};
         }
         uint32_t lo = c0, hi = c0;
         for (int t = 0; t < n_t; ++t) {
           const int t0 = t * tp, t1 = std::min((t + 1) * tp, along);
-          while (lo < c1 && fe[lo - c0] <= t0) ++lo;
+          while (lo < c1 && sp[lo - c0].we <= t0) ++lo;
           if (hi < lo) hi = lo;
-          while (hi < c1 && fs[hi - c0] < t1) ++hi;
+          while (hi < c1 && sp[hi - c0].ws < t1) ++hi;
           tb[base + ((size_t)b * n_t + t) * 2] = lo;
           tb[base + ((size_t)b * n_t + t) * 2 + 1] = hi;
+          // components of a band are in order, so their use starts and ends are too
+          if (lo < hi && (sp[lo - c0].rs < t0 - halo || sp[hi - 1 - c0].re > (t + 1) * tp + halo)) return false;
           // count the segments of the tiles that take this band's range (the
-          // tile kernel stages them in shared lists of kTileListY / kTileListC)
+          // tile kernel stages them in shared lists)
           const uint32_t n = comp[hi] - comp[lo];
           if (!n) continue;
           if (d == 0) {
             const int band = (int)b * unit;
-            const int ty0 = band - halo < 0 ? 0 : (band - halo) / tp;
-            const int ty1 = std::min(tiles_y - 1, (band + unit + halo - 1) / tp);
+            const int ty0 = band - rows < 0 ? 0 : (band - rows) / tp;
+            const int ty1 = std::min(tiles_y - 1, (band + unit + rows - 1) / tp);
             for (int ty = ty0; ty <= ty1; ++ty) load[((size_t)ty * tiles_x + t) * 3 + p] += n;
           } else {
             const int tx = (int)b * unit / tp;
@@ -585,9 +627,26 @@ void index_tiles(const h266_picture &pic, uint32_t cfi, DeblockPlan &plan) {
       }
     }
     for (size_t k = 0; k < load.size(); ++k)
-      if (load[k] > (uint32_t)(k % 3 ? kTileListC : kTileListY)) return;
+      if (load[k] > tile_list_cap(hx == kTileHaloX8, d, (int)(k % 3))) return false;
   }
-  plan.tiles_ok = true;
+  return true;
+}
+
+// The tile kernel's component ranges: the regions of edges on the 8x8 grid
+// where they do, else the wider ones.
+void index_tiles(const h266_picture &pic, uint32_t cfi, DeblockPlan &plan) {
+  plan.tiles_ok = false;
+  const int T = kDeblockTile;
+  const int w = (int)pic.luma.width, h = (int)pic.luma.height;
+  plan.tiles_x = (uint32_t)((w + T - 1) / T);
+  plan.tiles_y = (uint32_t)((h + T - 1) / T);
+  const bool chroma = (uint64_t)pic.cb.width * pic.cb.height != 0 || (uint64_t)pic.cr.width * pic.cr.height != 0;
+  if (cfi > 1 || (cfi == 0 && chroma)) return;
+  if (chroma && (pic.cb.width != (pic.luma.width + 1) / 2 || pic.cb.height != (pic.luma.height + 1) / 2 ||
+                 pic.cr.width != pic.cb.width || pic.cr.height != pic.cb.height))
+    return;
+  plan.tiles_grid8 = index_tiles_halo(pic, plan, kTileHaloX8, kTileHaloY8);
+  plan.tiles_ok = plan.tiles_grid8 || index_tiles_halo(pic, plan, kTileHaloX4, kTileHaloY4);
 }
 
 }  // namespace
@@ -1018,13 +1077,7 @@ struct ClampLine {
     else P.wr(qx, qy + d, v, maxv);
   }
 };
-template <int SN>
 struct RawLine {
-  uint16_t *q;  // q0 of the line
-  __host__ __device__ __forceinline__ int rd(int d) const { return q[d * SN]; }
-  __host__ __device__ __forceinline__ void wr(int d, int v, int maxv) const { q[d * SN] = (uint16_t)min(max(v, 0), maxv); }
-};
-struct RawLineDyn {
   uint16_t *q;
   int sn;
   __host__ __device__ __forceinline__ int rd(int d) const { return q[d * sn]; }
@@ -1038,151 +1091,59 @@ __host__ __device__ __forceinline__ void load_luma_line(const Line &L, int s[16]
   for (int d = -8; d < 8; ++d) s[8 + d] = L.rd(d);
 }
 
-// The decision terms of one luma line (§8.8.3.6.2, src/deblock.rs:1224-1410).
-struct LumaStats {
-  int dp, dq, sp, sq, spq;  // |p2-2p1+p0|, |q2-2q1+q0|, |p3-p0|, |q0-q3|, |p0-q0|
-  int dpx, dqx;             // |p5-2p4+p3|, |q5-2q4+q3|
-  int sp7, sq7;             // |p7-p6-p5+p4|, |q4-q5-q6+q7|
-  int pmd, qmd;             // |p3-p(mflP)|, |q3-q(mflQ)| for mfl 5 / 7
-};
-
-__host__ __device__ __forceinline__ LumaStats luma_stats(const EdgeSeg &e, const int s[16]) {
-#define PL(i) s[7 - (i)]
-#define QL(j) s[8 + (j)]
-  const int mp = e.mfl >> 4, mq = e.mfl & 15;
-  LumaStats t;
-  t.dp = abs(PL(2) - 2 * PL(1) + PL(0));
-  t.dq = abs(QL(2) - 2 * QL(1) + QL(0));
-  t.sp = abs(PL(3) - PL(0));
-  t.sq = abs(QL(0) - QL(3));
-  t.spq = abs(PL(0) - QL(0));
-  t.dpx = abs(PL(5) - 2 * PL(4) + PL(3));
-  t.dqx = abs(QL(5) - 2 * QL(4) + QL(3));
-  t.sp7 = abs(PL(7) - PL(6) - PL(5) + PL(4));
-  t.sq7 = abs(QL(4) - QL(5) - QL(6) + QL(7));
-  t.pmd = abs(PL(3) - (mp == 7 ? PL(7) : (mp == 5 ? PL(5) : PL(3))));
-  t.qmd = abs(QL(3) - (mq == 7 ? QL(7) : (mq == 5 ? QL(5) : QL(3))));
-#undef PL
-#undef QL
-  return t;
-}
-
+// The outcome of a luma segment's decision (§8.8.3.6.2, src/deblock.rs:1224-1410).
 struct LumaDecision {
-  int mode;  // 0: no filtering (dE = 0), 1: long filter, 2: short filter
   int mp, mq;
   bool strong, dep, deq;
 };
 
-// The segment's decision from the terms of lines 0 (a) and 3 (b).
-__host__ __device__ __forceinline__ LumaDecision luma_decide(const EdgeSeg &e, const LumaStats &a,
-                                                             const LumaStats &b) {
-  const int tc = e.tc, beta = e.beta;
-  LumaDecision dc;
-  dc.mp = e.mfl >> 4;
-  dc.mq = e.mfl & 15;
-  dc.strong = dc.dep = dc.deq = false;
-  const int tc_gate = (5 * tc + 1) >> 1;
-  const bool p_large = dc.mp > 3 && !(e.flags & 2);
-  const bool q_large = dc.mq > 3;
-  if (p_large || q_large) {
-    int dp0l = a.dp, dp3l = b.dp, dq0l = a.dq, dq3l = b.dq;
-    if (p_large) {
-      dp0l = (a.dp + a.dpx + 1) >> 1;
-      dp3l = (b.dp + b.dpx + 1) >> 1;
-    } else {
-      dc.mp = 3;
+// The long filter of one luma line (samples s) with lengths mp, mq.
+template <class Line>
+__device__ __forceinline__ void luma_long_line(const Line &L, const EdgeSeg &e, int mp, int mq, const int s[16],
+                                               int maxv) {
+  const int tc = e.tc;
+  const bool plt_p = e.flags & 4, plt_q = e.flags & 8;
+  int p[8], q[8];  // entries beyond mflP / mflQ are zero as in the reference's arrays
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    p[i] = i <= mp ? s[7 - i] : 0;
+    q[i] = i <= mq ? s[8 + i] : 0;
+  }
+  int mid;  // refMiddle, eqs. 1389-1394
+  if (mp == 5 && mq == 5)
+    mid = (p[4] + p[3] + 2 * (p[2] + p[1] + p[0] + q[0] + q[1] + q[2]) + q[3] + q[4] + 8) >> 4;
+  else if (mp == mq)
+    mid = (p[6] + p[5] + p[4] + p[3] + p[2] + p[1] + 2 * (p[0] + q[0]) + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] +
+           8) >> 4;
+  else if ((mp == 7 && mq == 5) || (mp == 5 && mq == 7))
+    mid = (p[5] + p[4] + p[3] + p[2] + 2 * (p[1] + p[0] + q[0] + q[1]) + q[2] + q[3] + q[4] + q[5] + 8) >> 4;
+  else if ((mp == 5 && mq == 3) || (mp == 3 && mq == 5))
+    mid = (p[3] + p[2] + p[1] + p[0] + q[0] + q[1] + q[2] + q[3] + 4) >> 3;
+  else if (mp == 3 && mq == 7)
+    mid = (2 * (p[2] + p[1] + p[0] + q[0]) + p[0] + p[1] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + 8) >> 4;
+  else
+    mid = (p[6] + p[5] + p[4] + p[3] + p[2] + p[1] + 2 * (q[2] + q[1] + q[0] + p[0]) + q[0] + q[1] + 8) >> 4;
+  const int rp = mp == 7 ? (p[7] + p[6] + 1) >> 1 : (mp == 5 ? (p[5] + p[4] + 1) >> 1 : (p[3] + p[2] + 1) >> 1);
+  const int rq = mq == 7 ? (q[7] + q[6] + 1) >> 1 : (mq == 5 ? (q[5] + q[4] + 1) >> 1 : (q[3] + q[2] + 1) >> 1);
+#pragma unroll
+  for (int i = 0; i < 7; ++i) {
+    if (i < mp && !plt_p) {
+      const int f = long_f(mp, i), lim = (tc * long_t(mp, i)) >> 1;
+      L.wr(-i - 1, clampd((mid * f + rp * (64 - f) + 32) >> 6, p[i] - lim, p[i] + lim), maxv);
     }
-    if (q_large) {
-      dq0l = (a.dq + a.dqx + 1) >> 1;
-      dq3l = (b.dq + b.dqx + 1) >> 1;
-    }
-    int sp0l = a.sp, sp3l = b.sp, sq0l = a.sq, sq3l = b.sq;
-    if (dc.mp == 7) {
-      sp0l += a.sp7;
-      sp3l += b.sp7;
-    }
-    if (dc.mq == 7) {
-      sq0l += a.sq7;
-      sq3l += b.sq7;
-    }
-    if ((dp0l + dq0l) + (dp3l + dq3l) < beta) {
-      const int t1 = (3 * beta) >> 5, t2 = beta >> 4;
-      int spl0 = sp0l, sql0 = sq0l, spl3 = sp3l, sql3 = sq3l;
-      if (p_large) {
-        spl0 = (spl0 + a.pmd + 1) >> 1;
-        spl3 = (spl3 + b.pmd + 1) >> 1;
-      }
-      if (q_large) {
-        sql0 = (sql0 + a.qmd + 1) >> 1;
-        sql3 = (sql3 + b.qmd + 1) >> 1;
-      }
-      if (2 * (dp0l + dq0l) < t2 && spl0 + sql0 < t1 && a.spq < tc_gate && 2 * (dp3l + dq3l) < t2 &&
-          spl3 + sql3 < t1 && b.spq < tc_gate) {
-        dc.mode = 1;
-        return dc;
-      }
+    if (i < mq && !plt_q) {
+      const int f = long_f(mq, i), lim = (tc * long_t(mq, i)) >> 1;
+      L.wr(i, clampd((mid * f + rq * (64 - f) + 32) >> 6, q[i] - lim, q[i] + lim), maxv);
     }
   }
-  if (a.dp + a.dq + b.dp + b.dq >= beta) {
-    dc.mode = 0;  // dE = 0
-    return dc;
-  }
-  dc.mode = 2;
-  if (dc.mp > 2 && dc.mq > 2) {
-    const int t1 = beta >> 3, t2 = beta >> 2;
-    dc.strong = 2 * (a.dp + a.dq) < t2 && a.sp + a.sq < t1 && a.spq < tc_gate && 2 * (b.dp + b.dq) < t2 &&
-                b.sp + b.sq < t1 && b.spq < tc_gate;
-  }
-  if (dc.strong) dc.mp = dc.mq = 3;
-  const int side_gate = (beta + (beta >> 1)) >> 3;
-  dc.dep = dc.mp > 1 && dc.mq > 1 && a.dp + b.dp < side_gate;
-  dc.deq = dc.mp > 1 && dc.mq > 1 && a.dq + b.dq < side_gate;
-  return dc;
 }
 
-// Filters one luma line (samples s) of a segment after its decision.
+// The short filters (strong or weak) of one luma line.
 template <class Line>
-__host__ __device__ __forceinline__ void luma_filter_line(const Line &L, const EdgeSeg &e, const LumaDecision &dc,
-                                                          const int s[16], int maxv) {
-  const int tc = e.tc, mp = dc.mp, mq = dc.mq;
+__device__ __forceinline__ void luma_short_line(const Line &L, const EdgeSeg &e, const LumaDecision &dc,
+                                                const int s[16], int maxv) {
+  const int tc = e.tc;
   const bool plt_p = e.flags & 4, plt_q = e.flags & 8;
-  if (dc.mode == 1) {
-    int p[8], q[8];  // entries beyond mflP / mflQ are zero as in the reference's arrays
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      p[i] = i <= mp ? s[7 - i] : 0;
-      q[i] = i <= mq ? s[8 + i] : 0;
-    }
-    int mid;  // refMiddle, eqs. 1389-1394
-    if (mp == 5 && mq == 5)
-      mid = (p[4] + p[3] + 2 * (p[2] + p[1] + p[0] + q[0] + q[1] + q[2]) + q[3] + q[4] + 8) >> 4;
-    else if (mp == mq)
-      mid = (p[6] + p[5] + p[4] + p[3] + p[2] + p[1] + 2 * (p[0] + q[0]) + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] +
-             8) >> 4;
-    else if ((mp == 7 && mq == 5) || (mp == 5 && mq == 7))
-      mid = (p[5] + p[4] + p[3] + p[2] + 2 * (p[1] + p[0] + q[0] + q[1]) + q[2] + q[3] + q[4] + q[5] + 8) >> 4;
-    else if ((mp == 5 && mq == 3) || (mp == 3 && mq == 5))
-      mid = (p[3] + p[2] + p[1] + p[0] + q[0] + q[1] + q[2] + q[3] + 4) >> 3;
-    else if (mp == 3 && mq == 7)
-      mid = (2 * (p[2] + p[1] + p[0] + q[0]) + p[0] + p[1] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + 8) >> 4;
-    else
-      mid = (p[6] + p[5] + p[4] + p[3] + p[2] + p[1] + 2 * (q[2] + q[1] + q[0] + p[0]) + q[0] + q[1] + 8) >> 4;
-    const int rp = mp == 7 ? (p[7] + p[6] + 1) >> 1 : (mp == 5 ? (p[5] + p[4] + 1) >> 1 : (p[3] + p[2] + 1) >> 1);
-    const int rq = mq == 7 ? (q[7] + q[6] + 1) >> 1 : (mq == 5 ? (q[5] + q[4] + 1) >> 1 : (q[3] + q[2] + 1) >> 1);
-#pragma unroll
-    for (int i = 0; i < 7; ++i) {
-      if (i < mp && !plt_p) {
-        const int f = long_f(mp, i), lim = (tc * long_t(mp, i)) >> 1;
-        L.wr(-i - 1, clampd((mid * f + rp * (64 - f) + 32) >> 6, p[i] - lim, p[i] + lim), maxv);
-      }
-      if (i < mq && !plt_q) {
-        const int f = long_f(mq, i), lim = (tc * long_t(mq, i)) >> 1;
-        L.wr(i, clampd((mid * f + rq * (64 - f) + 32) >> 6, q[i] - lim, q[i] + lim), maxv);
-      }
-    }
-    return;
-  }
-  if (dc.mode == 0) return;
   const int p3 = s[4], p2 = s[5], p1 = s[6], p0 = s[7], q0 = s[8], q1 = s[9], q2 = s[10], q3 = s[11];
   int np = 0, nq = 0;
   int op0 = 0, op1 = 0, op2 = 0, oq0 = 0, oq1 = 0, oq2 = 0;
@@ -1219,6 +1180,76 @@ __host__ __device__ __forceinline__ void luma_filter_line(const Line &L, const E
     if (i < np) L.wr(-i - 1, op[i], maxv);
     if (i < nq) L.wr(i, oq[i], maxv);
   }
+}
+
+// One luma segment by the 4 lanes of a group (lanes base .. base + 3 of the
+// warp, a line each), the decision of src/deblock.rs:1224-1410: every lane
+// forms its line's sums and whether its line passes each filter's conditions,
+// and lanes 0 and 3 pass those on -- three words, the conditions in the top
+// bits of the first (|p2 - 2 p1 + p0| stays below 2^18).  LONG: one side is
+// longer than 3 (is_long); without it only the 4 samples on each side are read
+// and none of the long terms formed.
+__device__ __forceinline__ bool is_long(const EdgeSeg &e) { return (e.mfl >> 4) > 3 || (e.mfl & 15) > 3; }
+
+template <bool LONG, class Line>
+__device__ __forceinline__ void luma_lines(const Line &L, const EdgeSeg &e, int maxv, int base, unsigned mask) {
+  int s[16];
+  if (LONG) {
+    load_luma_line(L, s);
+  } else {
+#pragma unroll
+    for (int d = -4; d < 4; ++d) s[8 + d] = L.rd(d);
+  }
+#define PL(i) s[7 - (i)]
+#define QL(j) s[8 + (j)]
+  const int tc = e.tc, beta = e.beta;
+  int mp = e.mfl >> 4, mq = e.mfl & 15;
+  const int tc_gate = (5 * tc + 1) >> 1;
+  const int dp = abs(PL(2) - 2 * PL(1) + PL(0)), dq = abs(QL(2) - 2 * QL(1) + QL(0));
+  const int sp = abs(PL(3) - PL(0)), sq = abs(QL(0) - QL(3));
+  const bool gate = abs(PL(0) - QL(0)) < tc_gate;
+  uint32_t w = (uint32_t)dp;
+  if (gate && 2 * (dp + dq) < (beta >> 2) && sp + sq < (beta >> 3)) w |= 1u << 30;
+  if (LONG) {
+    const bool p_large = mp > 3 && !(e.flags & 2), q_large = mq > 3;
+    bool long_ok = false;
+    if (p_large || q_large) {  // the same for the whole group
+      if (!p_large) mp = 3;
+      int dpl = dp, dql = dq, spl = sp, sql = sq;
+      if (mp == 7) spl += abs(PL(7) - PL(6) - PL(5) + PL(4));
+      if (mq == 7) sql += abs(QL(4) - QL(5) - QL(6) + QL(7));
+      if (p_large) {
+        dpl = (dp + abs(PL(5) - 2 * PL(4) + PL(3)) + 1) >> 1;
+        spl = (spl + abs(PL(3) - (mp == 7 ? PL(7) : (mp == 5 ? PL(5) : PL(3)))) + 1) >> 1;
+      }
+      if (q_large) {
+        dql = (dq + abs(QL(5) - 2 * QL(4) + QL(3)) + 1) >> 1;
+        sql = (sql + abs(QL(3) - (mq == 7 ? QL(7) : (mq == 5 ? QL(5) : QL(3)))) + 1) >> 1;
+      }
+      const bool ok = gate && 2 * (dpl + dql) < (beta >> 4) && spl + sql < ((3 * beta) >> 5);
+      const uint32_t v = (uint32_t)(dpl + dql) | (ok ? 1u << 31 : 0u);
+      const uint32_t v0 = __shfl_sync(mask, v, base), v3 = __shfl_sync(mask, v, base + 3);
+      long_ok = (v0 & v3) >> 31 && (int)((v0 & 0x7FFFFFFFu) + (v3 & 0x7FFFFFFFu)) < beta;
+    }
+    if (long_ok) {
+      luma_long_line(L, e, mp, mq, s, maxv);
+      return;
+    }
+  }
+#undef PL
+#undef QL
+  const uint32_t w0 = __shfl_sync(mask, w, base), w3 = __shfl_sync(mask, w, base + 3);
+  const int dqs = __shfl_sync(mask, dq, base) + __shfl_sync(mask, dq, base + 3);
+  const int dps = (int)((w0 & 0x3FFFFFFFu) + (w3 & 0x3FFFFFFFu));
+  if (dps + dqs >= beta) return;  // dE = 0
+  LumaDecision dc;
+  dc.strong = mp > 2 && mq > 2 && ((w0 & w3) >> 30) != 0;
+  dc.mp = dc.strong ? 3 : mp;
+  dc.mq = dc.strong ? 3 : mq;
+  const int side_gate = (beta + (beta >> 1)) >> 3;
+  dc.dep = dc.mp > 1 && dc.mq > 1 && dps < side_gate;
+  dc.deq = dc.mp > 1 && dc.mq > 1 && dqs < side_gate;
+  luma_short_line(L, e, dc, s, maxv);
 }
 
 // Samples of a chroma line: s[4 + d], d in [-4, 3].
@@ -1346,21 +1377,11 @@ __device__ __forceinline__ int plane_of(const StripParams &a, int &bid) {
 
 // One segment by a group of G lanes (G = 4 luma lines, 2 chroma lines); lane
 // k of the group owns line k.  `base` is the group's first lane in the warp.
-// PITCH is the window's row pitch when it is a compile-time constant (0:
-// v.ld), used for direct access along columns.
 template <int G, class Line>
 __device__ __forceinline__ void segment_lines(const Line &L, const EdgeSeg &e, int maxv, int base, unsigned mask) {
   if (G == 4) {
-    int s[16];
-    load_luma_line(L, s);
-    const LumaStats t = luma_stats(e, s);
-    LumaStats a, b;  // lines 0 and 3
-#define XCHG(f)                       \
-  a.f = __shfl_sync(mask, t.f, base); \
-  b.f = __shfl_sync(mask, t.f, base + 3);
-    XCHG(dp) XCHG(dq) XCHG(sp) XCHG(sq) XCHG(spq) XCHG(dpx) XCHG(dqx) XCHG(sp7) XCHG(sq7) XCHG(pmd) XCHG(qmd)
-#undef XCHG
-    luma_filter_line(L, e, luma_decide(e, a, b), s, maxv);
+    if (is_long(e)) luma_lines<true>(L, e, maxv, base, mask);
+    else luma_lines<false>(L, e, maxv, base, mask);
   } else {
     int s[8];
     load_chroma_line(L, s);
@@ -1370,23 +1391,31 @@ __device__ __forceinline__ void segment_lines(const Line &L, const EdgeSeg &e, i
   }
 }
 
-template <int G, int PITCH>
+// Segments whose samples leave the window (at the plane's edges), out of line:
+// few take it, and its copies of the filters would crowd the others' code out
+// of the instruction caches.
+template <int G>
+__device__ __noinline__ void segment_clamped(SharedView v, EdgeSeg e, int maxv, int k, int base, unsigned mask) {
+  const bool vert = e.flags & 1;
+  const int qx = vert ? e.x : e.x + k, qy = vert ? e.y + k : e.y;
+  segment_lines<G>(ClampLine<SharedView>{v, qx, qy, vert}, e, maxv, base, mask);
+}
+
+// One code path for both passes, with the step between samples as a number.
+template <int G>
 __device__ __forceinline__ void segment_group(const SharedView &v, const EdgeSeg &e, int maxv, int k, int base,
                                               unsigned mask) {
   const bool vert = e.flags & 1;
   constexpr int R = G == 4 ? 8 : 4;  // samples read on each side of the edge
-  const int qx = vert ? e.x : e.x + k, qy = vert ? e.y + k : e.y;
   // the segment's samples: R on each side across G lines
   const int x0 = vert ? e.x - R : e.x, x1 = vert ? e.x + R : e.x + G;
   const int y0 = vert ? e.y : e.y - R, y1 = vert ? e.y + G : e.y + R;
   const bool inside = x0 >= v.ox && y0 >= v.oy && x1 <= v.ox + v.ww && y1 <= v.oy + v.wh;
   if (inside) {  // uniform over the group: the window lies inside the plane, no clamping
-    uint16_t *q = v.s + (qy - v.oy) * v.ld + (qx - v.ox);
-    if (vert) segment_lines<G>(RawLine<1>{q}, e, maxv, base, mask);
-    else if (PITCH > 0) segment_lines<G>(RawLine<(PITCH > 0 ? PITCH : 1)>{q}, e, maxv, base, mask);
-    else segment_lines<G>(RawLineDyn{q, v.ld}, e, maxv, base, mask);
+    const int sn = vert ? 1 : v.ld, sl = vert ? v.ld : 1;
+    segment_lines<G>(RawLine{v.s + (e.y - v.oy) * v.ld + (e.x - v.ox) + k * sl, sn}, e, maxv, base, mask);
   } else {
-    segment_lines<G>(ClampLine<SharedView>{v, qx, qy, vert}, e, maxv, base, mask);
+    segment_clamped<G>(v, e, maxv, k, base, mask);
   }
 }
 
@@ -1394,7 +1423,7 @@ __device__ __forceinline__ void segment_group(const SharedView &v, const EdgeSeg
 // of a group walk the same segments; after each segment the group
 // synchronises, as the next segment may read samples another lane wrote
 // (a line clamped onto another at the plane edge).
-template <int G, int PITCH>
+template <int G>
 __device__ __forceinline__ void run_components(const StripParams &a, const SharedView &v, uint32_t c0, uint32_t c1) {
   const int lane = threadIdx.x & 31, k = lane % G, base = lane - k;
   const unsigned mask = ((1u << G) - 1) << base;
@@ -1402,76 +1431,101 @@ __device__ __forceinline__ void run_components(const StripParams &a, const Share
   for (uint32_t c = c0 + threadIdx.x / G; c < c1; c += groups) {
     const uint32_t e = a.comp[c + 1];
     for (uint32_t i = a.comp[c]; i < e; ++i) {
-      segment_group<G, PITCH>(v, a.segs[i], a.maxv, k, base, mask);
+      segment_group<G>(v, a.segs[i], a.maxv, k, base, mask);
       __syncwarp(mask);
     }
   }
 }
 
-// Grid mode: does the cell at slot s, whose footprint starts at `start`,
-// continue a run -- does an earlier footprint of the band end past `start`?
-// Footprints [pos - R(mflP), pos + R(mflQ)) reach at most 8 samples and
-// cells are 4 (luma) or 8 (chroma) samples apart, so only the 3 cells before
-// s can reach it.
-__device__ __forceinline__ bool continues_run(const EdgeSeg *cells, uint32_t s, int start) {
-  for (uint32_t t = s > 3 ? s - 3 : 0; t < s; ++t) {
-    const EdgeSeg f = cells[t];
-    if (f.bs && ((f.flags & 1) ? f.x : f.y) + reach_d(f.mfl & 15) > start) return true;
+// Grid mode: does a run of cells start at slot s of the band -- does no cell
+// before s write what one from s on uses, nor the other way round?  Cells are 4
+// (luma) or 8 (chroma) samples apart and a segment reaches at most 8, so only
+// the 3 cells before s and the 3 from s on can meet.
+__device__ __forceinline__ bool run_starts(const EdgeSeg *cells, uint32_t s, uint32_t ns) {
+  int we = INT_MIN, re = INT_MIN, ws = INT_MAX, rs = INT_MAX;
+#pragma unroll
+  for (int k = 1; k <= 3; ++k) {
+    if (s < (uint32_t)k) break;
+    const EdgeSeg f = cells[s - k];
+    if (!f.bs) continue;
+    const SegSpan x = seg_span(f);
+    we = max(we, x.we);
+    re = max(re, x.re);
   }
-  return false;
+  if (we == INT_MIN) return true;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (s + k >= ns) break;
+    const EdgeSeg f = cells[s + k];
+    if (!f.bs) continue;
+    const SegSpan x = seg_span(f);
+    ws = min(ws, x.ws);
+    rs = min(rs, x.rs);
+  }
+  return we <= rs && re <= ws;
 }
 
-// Grid mode: the runs of bands [0, nb) of cell grid g (ns cells per band), one
-// lane group per run.  A run is a maximal sequence of occupied cells, in
-// position order, each starting before the furthest footprint end of the
-// cells before it: the host grouping's components, whose members come in
-// position order when every row and column of the CU map is in decode order
-// (checked on the host before the walk runs on the device).  Footprint starts
-// never decrease along a band (spacing 4, reach 4..8), so a run ends at the
-// first occupied cell that does not start inside it, and that cell lies
-// within 3 cells of the run's last member or not at all.
-template <int G, int PITCH>
+// Grid mode: the runs of bands [0, nb) of cell grid g (ns cells per band).  A
+// run is a maximal sequence of occupied cells without such a start inside: the
+// host grouping's components, whose members come in position order when every
+// row and column of the CU map is in decode order (checked on the host before
+// the walk runs on the device).  A cell more than 3 slots after the run's last
+// one starts another.  The CTA lists the run starts of kRunChunk slots with a
+// thread per slot, then a lane group takes a run at a time: most slots are
+// empty, and scanning them by lane groups took most of the kernels' time.
+constexpr uint32_t kRunChunk = 1024;
+
+template <int G>
 __device__ __forceinline__ void run_cell_runs(const StripParams &a, const SharedView &v, const EdgeSeg *g, uint32_t ns,
                                               uint32_t nb) {
+  __shared__ uint16_t s_list[kRunChunk];
+  __shared__ uint32_t s_n, s_next;
   const int lane = threadIdx.x & 31, k = lane % G, base = lane - k;
   const unsigned mask = ((1u << G) - 1) << base;
-  const uint32_t groups = blockDim.x / G, total = ns * nb;
-  for (uint32_t i = threadIdx.x / G; i < total; i += groups) {
-    const uint32_t b = i / ns, s = i - b * ns;
-    const EdgeSeg *cells = g + (size_t)b * ns;
-    EdgeSeg e = cells[s];
-    if (!e.bs) continue;
-    const bool vert = e.flags & 1;
-    int pos = vert ? e.x : e.y;
-    if (continues_run(cells, s, pos - reach_d(e.mfl >> 4))) continue;  // not the first of its run
-    int end = pos + reach_d(e.mfl & 15);
-    uint32_t cur = s;
-    for (;;) {
-      segment_group<G, PITCH>(v, e, a.maxv, k, base, mask);
-      __syncwarp(mask);
-      uint32_t nx = cur + 1;
-      bool found = false;
-      for (; nx < ns && nx <= cur + 3; ++nx) {
-        e = cells[nx];
-        if (e.bs) {
-          found = true;
-          break;
-        }
-      }
-      if (!found) break;
-      pos = vert ? e.x : e.y;
-      if (pos - reach_d(e.mfl >> 4) >= end) break;
-      end = max(end, pos + reach_d(e.mfl & 15));
-      cur = nx;
+  const uint32_t total = ns * nb;
+  for (uint32_t c0 = 0; c0 < total; c0 += kRunChunk) {
+    if (threadIdx.x == 0) s_n = s_next = 0;
+    __syncthreads();
+    for (uint32_t i = c0 + threadIdx.x; i < min(total, c0 + kRunChunk); i += blockDim.x) {
+      const uint32_t b = i / ns, s = i - b * ns;
+      const EdgeSeg *cells = g + (size_t)b * ns;
+      if (cells[s].bs && run_starts(cells, s, ns)) s_list[atomicAdd(&s_n, 1u)] = (uint16_t)(i - c0);
     }
+    __syncthreads();
+    const uint32_t n = s_n;
+    for (;;) {
+      uint32_t t = 0;
+      if (k == 0) t = atomicAdd(&s_next, 1u);
+      t = __shfl_sync(mask, t, base);
+      if (t >= n) break;
+      const uint32_t i = c0 + s_list[t], b = i / ns;
+      const EdgeSeg *cells = g + (size_t)b * ns;
+      uint32_t cur = i - b * ns;
+      EdgeSeg e = cells[cur];
+      for (;;) {
+        segment_group<G>(v, e, a.maxv, k, base, mask);
+        __syncwarp(mask);
+        uint32_t nx = cur + 1;
+        bool found = false;
+        for (; nx < ns && nx <= cur + 3; ++nx) {
+          e = cells[nx];
+          if (e.bs) {
+            found = true;
+            break;
+          }
+        }
+        if (!found || run_starts(cells, nx, ns)) break;
+        cur = nx;
+      }
+    }
+    __syncthreads();  // the list is free again
   }
 }
 
 // Vertical pass: one CTA per band of rows, all planes in one grid.  Loads the
 // rows from src (luma through the LMCS LUT), filters, stores them to dst.
-__global__ void __launch_bounds__(128) k_deblock_rows(StripParams a) {
+__device__ __forceinline__ void deblock_rows_cta(const StripParams &a, int band) {
   extern __shared__ __align__(16) uint16_t sm[];
-  int band = blockIdx.x;
   const int plane = plane_of(a, band);
   const DPlane src = a.src[plane], dst = a.dst[plane];
   const int unit = plane ? 2 : 4;
@@ -1500,13 +1554,13 @@ __global__ void __launch_bounds__(128) k_deblock_rows(StripParams a) {
   if (a.grid_mode) {
     if ((uint32_t)band < a.grid_bands[plane]) {
       const EdgeSeg *g = a.grid[plane] + (size_t)band * a.grid_slots[plane];
-      if (plane == 0) run_cell_runs<4, 0>(a, view, g, a.grid_slots[plane], 1);
-      else run_cell_runs<2, 0>(a, view, g, a.grid_slots[plane], 1);
+      if (plane == 0) run_cell_runs<4>(a, view, g, a.grid_slots[plane], 1);
+      else run_cell_runs<2>(a, view, g, a.grid_slots[plane], 1);
     }
   } else {
     const uint32_t *bf = a.band_first + a.band_off[plane];
-    if (plane == 0) run_components<4, 0>(a, view, bf[band], bf[band + 1]);
-    else run_components<2, 0>(a, view, bf[band], bf[band + 1]);
+    if (plane == 0) run_components<4>(a, view, bf[band], bf[band + 1]);
+    else run_components<2>(a, view, bf[band], bf[band + 1]);
   }
   __syncthreads();
   const int nvo = vec_ok(dst) ? w / 8 : 0;
@@ -1523,9 +1577,8 @@ __global__ void __launch_bounds__(128) k_deblock_rows(StripParams a) {
 }
 
 // Horizontal pass: one CTA per 8-column strip (full plane height), in place.
-__global__ void __launch_bounds__(128, 8) k_deblock_cols(StripParams a) {
+__device__ __forceinline__ void deblock_cols_cta(const StripParams &a, int strip) {
   extern __shared__ __align__(16) uint16_t sm[];
-  int strip = blockIdx.x;
   const int plane = plane_of(a, strip);
   const DPlane p = a.dst[plane];
   const int unit = plane ? 2 : 4;
@@ -1550,15 +1603,15 @@ __global__ void __launch_bounds__(128, 8) k_deblock_cols(StripParams a) {
     const uint32_t b0 = min((uint32_t)(x0 / unit), nb), b1 = min((uint32_t)((x0 + kStripCols) / unit), nb);
     if (b1 > b0) {
       const EdgeSeg *g = a.grid[plane] + (size_t)b0 * a.grid_slots[plane];
-      if (plane == 0) run_cell_runs<4, kStripCols>(a, view, g, a.grid_slots[plane], b1 - b0);
-      else run_cell_runs<2, kStripCols>(a, view, g, a.grid_slots[plane], b1 - b0);
+      if (plane == 0) run_cell_runs<4>(a, view, g, a.grid_slots[plane], b1 - b0);
+      else run_cell_runs<2>(a, view, g, a.grid_slots[plane], b1 - b0);
     }
   } else {
     const uint32_t *bf = a.band_first + a.band_off[plane];
     const uint32_t nb = a.n_bands[plane];
     const uint32_t b0 = min((uint32_t)(x0 / unit), nb), b1 = min((uint32_t)((x0 + kStripCols) / unit), nb);
-    if (plane == 0) run_components<4, kStripCols>(a, view, bf[b0], bf[b1]);
-    else run_components<2, kStripCols>(a, view, bf[b0], bf[b1]);
+    if (plane == 0) run_components<4>(a, view, bf[b0], bf[b1]);
+    else run_components<2>(a, view, bf[b0], bf[b1]);
   }
   __syncthreads();
   if (vec) {
@@ -1575,6 +1628,43 @@ __global__ void __launch_bounds__(128, 8) k_deblock_cols(StripParams a) {
   }
 }
 
+__global__ void __launch_bounds__(128, 8) k_deblock_rows(const __grid_constant__ StripParams a) {
+  deblock_rows_cta(a, blockIdx.x);
+}
+__global__ void __launch_bounds__(128, 8) k_deblock_cols(const __grid_constant__ StripParams a) {
+  deblock_cols_cta(a, blockIdx.x);
+}
+
+// Many pictures in one grid: CTAs [first[i], first[i + 1]) are picture i's
+// bands (or strips), whose parameters are params[i].
+__device__ __forceinline__ int strip_picture(const StripParams *__restrict__ params,
+                                             const uint32_t *__restrict__ first, int n, StripParams &s) {
+  int lo = 0, hi = n;  // first[lo] <= blockIdx.x < first[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (first[mid] <= blockIdx.x) lo = mid;
+    else hi = mid;
+  }
+  static_assert(sizeof(StripParams) % 4 == 0, "word copy");
+  const uint32_t *src = reinterpret_cast<const uint32_t *>(params + lo);
+  uint32_t *dst = reinterpret_cast<uint32_t *>(&s);
+  for (int i = threadIdx.x; i < (int)(sizeof(StripParams) / 4); i += blockDim.x) dst[i] = src[i];
+  __syncthreads();
+  return (int)(blockIdx.x - first[lo]);
+}
+__global__ void __launch_bounds__(128, 8) k_deblock_rows_batch(const StripParams *__restrict__ params,
+                                                               const uint32_t *__restrict__ first, int n) {
+  __shared__ StripParams s;
+  const int cta = strip_picture(params, first, n, s);
+  deblock_rows_cta(s, cta);
+}
+__global__ void __launch_bounds__(128, 8) k_deblock_cols_batch(const StripParams *__restrict__ params,
+                                                               const uint32_t *__restrict__ first, int n) {
+  __shared__ StripParams s;
+  const int cta = strip_picture(params, first, n, s);
+  deblock_cols_cta(s, cta);
+}
+
 // ------------------------------------------------------------ tile kernel
 // One CTA per 64x64 luma tile and its 32x32 chroma tiles.  The tile's region
 // -- the tile widened by the halo -- is staged once by TMA box loads (luma
@@ -1586,12 +1676,27 @@ __global__ void __launch_bounds__(128, 8) k_deblock_cols(StripParams a) {
 // output.  Components span at most the halo (checked on the host, or by
 // construction for the device walk's pictures), so every clamped read of a
 // listed component stays inside the region.
+//
+// Two regions (G8).  Edges on the 8x8 luma grid that write in the tile lie at
+// most on its borders and use 8 samples beyond them, so 8 rows and columns of
+// halo hold everything; edges on the 4x4 grid can lie 4 samples outside and
+// reach 12, with columns rounded up to 16 (the TMA box starts on 16 bytes).
+// Chroma edges are on the 8x8 chroma grid in both and use 4 samples.  Against
+// one region of 16 (chroma 8) rows and columns for both, the G8 region has
+// 0.68 of the samples to copy and map and 5/6 of the row bands in its vertical
+// pass.
 constexpr int kTileThreads = 256;
-constexpr int kRegionY = kDeblockTile + 2 * kDeblockHaloY;      // 96
-constexpr int kRegionC = kDeblockTile / 2 + 2 * kDeblockHaloC;  // 48
-constexpr int kPitchY = kRegionY + 8;                           // smem row pitch, samples
-constexpr int kPitchC = kRegionC + 8;
-constexpr size_t kTileSmem = (size_t)(kRegionY * kPitchY + 2 * kRegionC * kPitchC) * 2;
+template <bool G8>
+struct TileGeo {
+  static constexpr int HX = G8 ? kTileHaloX8 : kTileHaloX4, HY = G8 ? kTileHaloY8 : kTileHaloY4;
+  static constexpr int RW = kDeblockTile + 2 * HX, RH = kDeblockTile + 2 * HY;
+  static constexpr int RWC = kDeblockTile / 2 + 2 * kTileHaloXC, RHC = kDeblockTile / 2 + 2 * kTileHaloYC;
+  static constexpr int PY = RW + 8, PC = RWC + 8;  // smem row pitches (and TMA box widths), samples
+  // region offsets in samples: TMA destinations on 128 bytes
+  static constexpr int OFF1 = (RH * PY + 63) / 64 * 64, OFF2 = OFF1 + (RHC * PC + 63) / 64 * 64;
+  static constexpr size_t SMEM = (size_t)(OFF2 + RHC * PC) * 2;
+  __device__ static constexpr int off(int p) { return p == 0 ? 0 : (p == 1 ? OFF1 : OFF2); }
+};
 
 struct TileParams {
   DPlane src[3], dst[3];
@@ -1611,9 +1716,9 @@ struct TileParams {
   const EdgeSeg *grid[2][3];
   uint32_t grid_slots[2][3];
   const uint32_t *grid_count;       // cells per (tile, pass, plane), listed by the walk
-  const uint32_t *grid_list[2][3];  // their grid indices, kTileListY / kTileListC per tile
-  // The regions staged by the TMA unit: one box per plane, kPitch wide and
-  // kRegion high, at the tile's origin less the halo (tma 0: vector loads).
+  const uint32_t *grid_list[2][3];  // their grid indices, tile_list_cap() per tile
+  // The regions staged by the TMA unit: one box per plane, a row pitch wide
+  // and the region high, at the tile's origin less the halo (tma 0: vector loads).
   int tma;
   CUtensorMap tmap[3];
 };
@@ -1667,15 +1772,17 @@ __device__ __forceinline__ void store_window(const uint16_t *sm, int pitch, cons
 // plane p), by one warp.
 // The staged window of plane p of tile (tx, ty): the tile widened by the
 // halo, clipped to the plane.  Recomputed where needed rather than kept live.
+template <bool G8>
 __device__ __forceinline__ SharedView tile_view(const TileParams &a, uint16_t *sm, int p, int tx, int ty) {
+  using Geo = TileGeo<G8>;
   const DPlane &src = a.src[p];
-  const int tp = p ? kDeblockTile / 2 : kDeblockTile, halo = p ? kDeblockHaloC : kDeblockHaloY;
-  const int pitch = p ? kPitchC : kPitchY;
-  uint16_t *box = p == 0 ? sm : sm + kRegionY * kPitchY + (p - 1) * kRegionC * kPitchC;
-  const int rx = tx * tp - halo, ry = ty * tp - halo;  // the box's origin, before clipping to the plane
+  const int tp = p ? kDeblockTile / 2 : kDeblockTile, hx = p ? kTileHaloXC : Geo::HX, hy = p ? kTileHaloYC : Geo::HY;
+  const int pitch = p ? Geo::PC : Geo::PY;
+  const int rx = tx * tp - hx, ry = ty * tp - hy;  // the box's origin, before clipping to the plane
   const int ox = max(rx, 0), oy = max(ry, 0);
-  const int ww = min(tx * tp + tp + halo, src.w) - ox, wh = min(ty * tp + tp + halo, src.h) - oy;
-  return SharedView{box + (oy - ry) * pitch + (ox - rx), pitch, ox, oy, max(ww, 0), max(wh, 0), src.w, src.h};
+  const int ww = min(tx * tp + tp + hx, src.w) - ox, wh = min(ty * tp + tp + hy, src.h) - oy;
+  return SharedView{sm + Geo::off(p) + (oy - ry) * pitch + (ox - rx), pitch, ox, oy, max(ww, 0), max(wh, 0), src.w,
+                    src.h};
 }
 
 // An EdgeSeg moved as three 32-bit words (every array of them here starts on
@@ -1705,9 +1812,11 @@ __device__ __forceinline__ void seg_copy(EdgeSeg *dst, const EdgeSeg *src) {
 // the filters run: their segments one component after another and each
 // component's first segment (start[n] ends the last one), so the filter
 // phase reads no global memory.
+// `order` lists the components with the short-filter ones first, so that the
+// 8 luma components of a warp task seldom mix both kinds.
 struct TileStage {
   EdgeSeg *seg;
-  uint16_t *start;
+  uint16_t *start, *order;
   uint32_t cap;
 };
 
@@ -1726,10 +1835,11 @@ __device__ __forceinline__ int band_of(const uint32_t *prefix, uint32_t x) {
 // component and segment in the staged arrays, then the warp stages every
 // component start and segment.  `band` is the warp's scratch (4 x 33).  The
 // host keeps every tile's segment count within the caps.
+template <bool G8>
 __device__ __forceinline__ uint32_t stage_host(const TileParams &a, int d, int p, int tx, int ty, const TileStage &st,
                                                uint32_t (*band)[kTileBands + 1]) {
   const int lane = threadIdx.x & 31;
-  const int tp = p ? kDeblockTile / 2 : kDeblockTile, halo = p ? kDeblockHaloC : kDeblockHaloY, unit = p ? 2 : 4;
+  const int tp = p ? kDeblockTile / 2 : kDeblockTile, halo = p ? kTileHaloYC : TileGeo<G8>::HY, unit = p ? 2 : 4;
   const int nb = (int)a.n_bands[d][p];
   int b0, b1, n_t, t;
   if (d == 0) {  // row bands of the tile's rows widened by the halo
@@ -1799,17 +1909,41 @@ __device__ __forceinline__ uint32_t stage_grid(const TileParams &a, int d, int p
   return n;
 }
 
+// Puts the luma components' order into st.order: those without a long segment
+// first, both kinds in their own order.  By one warp, after staging.
+__device__ __forceinline__ void stage_order(const TileStage &st, uint32_t n) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  uint32_t shorts = 0, longs = 0;
+  for (uint32_t j0 = 0; j0 < n; j0 += 32) {
+    const uint32_t j = j0 + lane;
+    bool in = j < n, lg = false;
+    if (in)
+      for (uint32_t i = st.start[j]; i < st.start[j + 1]; ++i) lg = lg || is_long(st.seg[i]);
+    const unsigned ms = __ballot_sync(0xFFFFFFFFu, in && !lg), ml = __ballot_sync(0xFFFFFFFFu, in && lg);
+    const unsigned below = (1u << lane) - 1;
+    if (in) st.order[lg ? n - 1 - (longs + __popc(ml & below)) : shorts + __popc(ms & below)] = (uint16_t)j;
+    shorts += __popc(ms);
+    longs += __popc(ml);
+  }
+}
+
+template <bool G8>
 struct TileShared {
-  alignas(16) EdgeSeg seg_y[2][kTileListY];
-  alignas(16) EdgeSeg seg_c[2][2][kTileListC];
-  uint16_t start_y[2][kTileListY + 1], start_c[2][2][kTileListC + 1];
+  static constexpr uint32_t CV = tile_list_cap(G8, 0, 0), CH = tile_list_cap(G8, 1, 0);
+  static constexpr uint32_t CC = tile_list_cap(G8, 0, 1);
+  alignas(16) EdgeSeg seg_v[CV];
+  alignas(16) EdgeSeg seg_h[CH];
+  alignas(16) EdgeSeg seg_c[2][2][CC];
+  uint16_t start_v[CV + 1], start_h[CH + 1], start_c[2][2][CC + 1];
+  uint16_t order_v[CV], order_h[CH];
   uint32_t band[6][4][kTileBands + 1];  // stage_host scratch per (pass, plane)
   uint32_t n_comp[2][3];
   uint32_t task[2];                   // the passes' next warp task
   alignas(8) unsigned long long bar;  // completion of the TMA region copies
   __device__ TileStage stage(int d, int p) {
-    return p == 0 ? TileStage{seg_y[d], start_y[d], (uint32_t)kTileListY}
-                  : TileStage{seg_c[d][p - 1], start_c[d][p - 1], (uint32_t)kTileListC};
+    if (p) return TileStage{seg_c[d][p - 1], start_c[d][p - 1], nullptr, CC};
+    return d ? TileStage{seg_h, start_h, order_h, CH} : TileStage{seg_v, start_v, order_v, CV};
   }
 };
 
@@ -1818,12 +1952,15 @@ struct TileShared {
 // chroma components (groups of 2), so no plane waits for another; warps take
 // tasks from a shared counter, so a warp with long components does not hold
 // the others at the pass's barrier.
-__device__ __forceinline__ void run_tile_pass(const TileParams &a, uint16_t *sm, TileShared &ts, int tx, int ty,
+template <bool G8>
+__device__ __forceinline__ void run_tile_pass(const TileParams &a, uint16_t *sm, TileShared<G8> &ts, int tx, int ty,
                                               int d) {
+  using Geo = TileGeo<G8>;
   const int lane = threadIdx.x & 31;
   const uint32_t n0 = ts.n_comp[d][0], n1 = ts.n_comp[d][1], n2 = ts.n_comp[d][2];
   const uint32_t tasks0 = (n0 + 7) / 8, tasks1 = (n1 + 15) / 16, tasks2 = (n2 + 15) / 16;
   const uint32_t total = tasks0 + tasks1 + tasks2;
+  const TileStage sy = ts.stage(d, 0);
   for (;;) {
     uint32_t t = 0;
     if (lane == 0) t = atomicAdd(&ts.task[d], 1u);
@@ -1832,12 +1969,13 @@ __device__ __forceinline__ void run_tile_pass(const TileParams &a, uint16_t *sm,
     if (t < tasks0) {
       const int k = lane & 3, base = lane - k;
       const unsigned mask = 0xFu << base;
-      const uint32_t j = t * 8 + (lane >> 2);
-      if (j < n0) {
-        const SharedView v = tile_view(a, sm, 0, tx, ty);
-        const uint32_t e = ts.start_y[d][j + 1];
-        for (uint32_t i = ts.start_y[d][j]; i < e; ++i) {
-          segment_group<4, kPitchY>(v, seg_get(&ts.seg_y[d][i]), a.maxv, k, base, mask);
+      // the long components (the list's end) first: they take longest
+      const uint32_t at = (tasks0 - 1 - t) * 8 + (lane >> 2);
+      if (at < n0) {
+        const SharedView v = tile_view<G8>(a, sm, 0, tx, ty);
+        const uint32_t j = sy.order[at], e = sy.start[j + 1];
+        for (uint32_t i = sy.start[j]; i < e; ++i) {
+          segment_group<4>(v, seg_get(sy.seg + i), a.maxv, k, base, mask);
           __syncwarp(mask);
         }
       }
@@ -1849,10 +1987,10 @@ __device__ __forceinline__ void run_tile_pass(const TileParams &a, uint16_t *sm,
       const unsigned mask = 0x3u << base;
       const uint32_t j = tt * 16 + (lane >> 1);
       if (j < (cr ? n2 : n1)) {
-        const SharedView v = tile_view(a, sm, cr ? 2 : 1, tx, ty);
+        const SharedView v = tile_view<G8>(a, sm, cr ? 2 : 1, tx, ty);
         const uint32_t e = ts.start_c[d][c][j + 1];
         for (uint32_t i = ts.start_c[d][c][j]; i < e; ++i) {
-          segment_group<2, kPitchC>(v, seg_get(&ts.seg_c[d][c][i]), a.maxv, k, base, mask);
+          segment_group<2>(v, seg_get(&ts.seg_c[d][c][i]), a.maxv, k, base, mask);
           __syncwarp(mask);
         }
       }
@@ -1862,10 +2000,12 @@ __device__ __forceinline__ void run_tile_pass(const TileParams &a, uint16_t *sm,
 
 // Tile t of the picture whose parameters are `a` (`g`: the same parameters in
 // global or parameter memory, for the tensor maps).
+template <bool G8>
 __device__ __forceinline__ void deblock_tile(const TileParams &a, const TileParams *g, int t) {
+  using Geo = TileGeo<G8>;
   extern __shared__ __align__(128) uint16_t sm_tile[];  // TMA destinations: 128-byte aligned
   uint16_t *sm = sm_tile;
-  __shared__ TileShared ts;
+  __shared__ TileShared<G8> ts;
   const int tx = t % (int)a.tiles_x, ty = t / (int)a.tiles_x;
   const int warp = threadIdx.x >> 5;
   // Thread 0 starts the TMA copies of the planes' regions; meanwhile warps
@@ -1878,39 +2018,41 @@ __device__ __forceinline__ void deblock_tile(const TileParams &a, const TilePara
       uint32_t bytes = 0;
 #pragma unroll
       for (int p = 0; p < 3; ++p)
-        if (a.src[p].w > 0 && a.src[p].h > 0) bytes += (p ? kRegionC * kPitchC : kRegionY * kPitchY) * 2;
+        if (a.src[p].w > 0 && a.src[p].h > 0) bytes += (p ? Geo::RHC * Geo::PC : Geo::RH * Geo::PY) * 2;
       tile_dev::mbar_expect_tx(&ts.bar, bytes);
 #pragma unroll
       for (int p = 0; p < 3; ++p) {
         if (a.src[p].w <= 0 || a.src[p].h <= 0) continue;
-        const int tp = p ? kDeblockTile / 2 : kDeblockTile, halo = p ? kDeblockHaloC : kDeblockHaloY;
-        uint16_t *box = p == 0 ? sm : sm + kRegionY * kPitchY + (p - 1) * kRegionC * kPitchC;
+        const int tp = p ? kDeblockTile / 2 : kDeblockTile;
+        const int hx = p ? kTileHaloXC : Geo::HX, hy = p ? kTileHaloYC : Geo::HY;
         tile_dev::tmap_acquire(&g->tmap[p]);
-        tile_dev::tma_load_2d(box, &g->tmap[p], tx * tp - halo, ty * tp - halo, &ts.bar);
+        tile_dev::tma_load_2d(sm + Geo::off(p), &g->tmap[p], tx * tp - hx, ty * tp - hy, &ts.bar);
       }
     }
   }
   if (warp < 6) {
     const int d = warp / 3, p = warp % 3;
-    const uint32_t n = a.grid_mode ? stage_grid(a, d, p, t, ts.stage(d, p))
-                                   : stage_host(a, d, p, tx, ty, ts.stage(d, p), ts.band[warp]);
+    const TileStage st = ts.stage(d, p);
+    const uint32_t n = a.grid_mode ? stage_grid(a, d, p, t, st) : stage_host<G8>(a, d, p, tx, ty, st, ts.band[warp]);
+    if (p == 0) stage_order(st, n);
     if ((threadIdx.x & 31) == 0) ts.n_comp[d][p] = n;
   }
   if (!a.tma) {
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
-      const SharedView v = tile_view(a, sm, p, tx, ty);
+      const SharedView v = tile_view<G8>(a, sm, p, tx, ty);
       if (v.ww > 0 && v.wh > 0) load_window(v.s, v.ld, a.src[p], v.ox, v.oy, v.ww, v.wh, p == 0 ? a.lut : nullptr);
     }
     __syncthreads();
   } else {
     __syncthreads();  // the barrier's initialisation and the staged components
     bool ok = tile_dev::mbar_wait_bounded(&ts.bar, 0);
-    if (ok && a.lut) {  // luma through the LMCS LUT, in place (the whole box: samples outside the plane are never read)
+    if (ok && a.lut) {  // luma through the LMCS LUT, in place (the whole region: samples outside the plane are never read)
       uint32_t *w = reinterpret_cast<uint32_t *>(sm);
-      for (int i = threadIdx.x; i < kRegionY * kPitchY / 2; i += blockDim.x) {
-        const uint32_t u = w[i];
-        w[i] = (uint32_t)a.lut[u & 0xFFFF] | (uint32_t)a.lut[u >> 16] << 16;
+      for (int i = threadIdx.x; i < Geo::RH * (Geo::RW / 2); i += blockDim.x) {
+        const int r = i / (Geo::RW / 2), c = i - r * (Geo::RW / 2) + r * (Geo::PY / 2);
+        const uint32_t u = w[c];
+        w[c] = (uint32_t)a.lut[u & 0xFFFF] | (uint32_t)a.lut[u >> 16] << 16;
       }
     }
     ok = __syncthreads_and(ok);
@@ -1922,26 +2064,28 @@ __device__ __forceinline__ void deblock_tile(const TileParams &a, const TilePara
       return;
     }
   }
-#pragma unroll
+#pragma unroll 1
   for (int d = 0; d < 2; ++d) {
-    run_tile_pass(a, sm, ts, tx, ty, d);
+    run_tile_pass<G8>(a, sm, ts, tx, ty, d);
     __syncthreads();
   }
 #pragma unroll
   for (int p = 0; p < 3; ++p) {
-    const SharedView v = tile_view(a, sm, p, tx, ty);
+    const SharedView v = tile_view<G8>(a, sm, p, tx, ty);
     const int tp = p ? kDeblockTile / 2 : kDeblockTile, x0 = tx * tp, y0 = ty * tp;
     const int iw = min(x0 + tp, a.dst[p].w) - x0, ih = min(y0 + tp, a.dst[p].h) - y0;
     if (iw > 0 && ih > 0 && v.ww > 0 && v.wh > 0) store_window(v.s, v.ld, a.dst[p], v.ox, v.oy, x0, y0, iw, ih);
   }
 }
 
+template <bool G8>
 __global__ void __launch_bounds__(kTileThreads, 4) k_deblock_tiles(const __grid_constant__ TileParams a) {
-  deblock_tile(a, &a, blockIdx.x);
+  deblock_tile<G8>(a, &a, blockIdx.x);
 }
 
 // Many pictures in one grid: CTAs [first[i], first[i + 1]) are the tiles of
 // picture i, whose parameters are params[i].
+template <bool G8>
 __global__ void __launch_bounds__(kTileThreads, 4) k_deblock_tiles_batch(const TileParams *__restrict__ params,
                                                                          const uint32_t *__restrict__ first, int n) {
   __shared__ TileParams s_params;  // the picture's parameters, read once per CTA
@@ -1956,7 +2100,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) k_deblock_tiles_batch(const T
   uint32_t *dst = reinterpret_cast<uint32_t *>(&s_params);
   for (int i = threadIdx.x; i < (int)(sizeof(TileParams) / 4); i += blockDim.x) dst[i] = src[i];
   __syncthreads();
-  deblock_tile(s_params, params + lo, (int)(blockIdx.x - first[lo]));
+  deblock_tile<G8>(s_params, params + lo, (int)(blockIdx.x - first[lo]));
 }
 
 size_t rows_smem(const DPlane &p) { return (size_t)4 * row_pitch(p.w) * 2; }
@@ -1972,117 +2116,131 @@ bool deblock_strips_fit(const DPlane planes[3]) {
   return true;
 }
 
-int launch_deblock_strips(cudaStream_t st, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
-                          int bit_depth, const StripSide &v, const StripSide &h, const uint32_t band_off[2][3],
-                          const uint32_t n_bands[2][3], uint64_t *launches) {
-  StripParams a;
-  std::memset(&a, 0, sizeof a);
-  size_t smem_rows = 0, smem_cols = 0;
-  uint32_t ctas_rows = 0, ctas_cols = 0;
-  uint32_t strips[3];
+size_t strip_params_size() { return sizeof(StripParams); }
+
+namespace {
+
+// What both forms of the strip kernels' parameters share: planes, CTA counts
+// (a row band of `rows[i]` per plane, a strip per kStripCols columns) and
+// shared memory.
+void strip_geometry(const DPlane src[3], const DPlane dst[3], const uint16_t *lut, int bit_depth,
+                    const uint32_t rows[3], StripParams &v, StripParams &h, StripCounts &c) {
+  std::memset(&v, 0, sizeof v);
+  std::memset(&h, 0, sizeof h);
+  c = StripCounts{};
   for (int i = 0; i < 3; ++i) {
-    a.src[i] = src[i];
-    a.dst[i] = dst[i];
-    const bool empty = (int64_t)src[i].w * src[i].h == 0;
-    strips[i] = empty ? 0 : (uint32_t)((src[i].w + kStripCols - 1) / kStripCols);
-    if (!empty) {
-      smem_rows = std::max(smem_rows, rows_smem(src[i]));
-      smem_cols = std::max(smem_cols, cols_smem(src[i]));
+    v.src[i] = h.src[i] = src[i];
+    v.dst[i] = h.dst[i] = dst[i];
+    if ((int64_t)src[i].w * src[i].h == 0) continue;
+    v.ctas[i] = rows[i];
+    h.ctas[i] = (uint32_t)((src[i].w + kStripCols - 1) / kStripCols);
+    c.smem_rows = std::max(c.smem_rows, rows_smem(src[i]));
+    c.smem_cols = std::max(c.smem_cols, cols_smem(src[i]));
+    c.rows += v.ctas[i];
+    c.cols += h.ctas[i];
+  }
+  v.lut = lut;
+  v.maxv = h.maxv = (1 << bit_depth) - 1;
+}
+
+}  // namespace
+
+void fill_strip_params(void *rows, void *cols, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
+                       int bit_depth, const StripSide &v, const StripSide &h, const uint32_t band_off[2][3],
+                       const uint32_t n_bands[2][3], StripCounts &c) {
+  StripParams p[2];
+  strip_geometry(src, dst, lut, bit_depth, n_bands[0], p[0], p[1], c);
+  const StripSide *side[2] = {&v, &h};
+  for (int d = 0; d < 2; ++d) {
+    p[d].segs = side[d]->segs;
+    p[d].comp = side[d]->comp;
+    p[d].band_first = side[d]->band_first;
+    for (int i = 0; i < 3; ++i) {
+      p[d].band_off[i] = band_off[d][i];
+      p[d].n_bands[i] = n_bands[d][i];
     }
-    ctas_rows += empty ? 0 : n_bands[0][i];
-    ctas_cols += strips[i];
   }
-  a.lut = lut;
-  a.maxv = (1 << bit_depth) - 1;
-  // vertical pass
-  a.segs = v.segs;
-  a.comp = v.comp;
-  a.band_first = v.band_first;
-  for (int i = 0; i < 3; ++i) {
-    a.band_off[i] = band_off[0][i];
-    a.n_bands[i] = n_bands[0][i];
-    a.ctas[i] = (int64_t)src[i].w * src[i].h ? n_bands[0][i] : 0;
+  std::memcpy(rows, &p[0], sizeof p[0]);
+  std::memcpy(cols, &p[1], sizeof p[1]);
+}
+
+// On the device walk's cell grids.  Row bands follow the plane sizes, so
+// planes without segments (chroma of a 4:0:0 walk) are still copied.
+int fill_strip_params_grid(void *rows, void *cols, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
+                           int bit_depth, const DeviceWalkOut &g, StripCounts &c) {
+  StripParams p[2];
+  uint32_t bands[3];
+  for (int i = 0; i < 3; ++i) bands[i] = (uint32_t)((src[i].h + (i ? 1 : 3)) / (i ? 2 : 4));
+  strip_geometry(src, dst, lut, bit_depth, bands, p[0], p[1], c);
+  if (c.smem_rows > (size_t)kMaxStripSmem || c.smem_cols > (size_t)kMaxStripSmem)
+    return set_error(H266_ERR_UNSUPPORTED, "deblock: planes too large for the strip kernels");
+  for (int d = 0; d < 2; ++d) {
+    p[d].grid_mode = 1;
+    for (int i = 0; i < 3; ++i) {
+      p[d].grid[i] = g.grid[d][i];
+      p[d].grid_slots[i] = g.slots[d][i];
+      p[d].grid_bands[i] = g.bands[d][i];
+    }
   }
-  if (ctas_rows) {
-    if (smem_rows > 48 * 1024)
-      H266_CUDA(cudaFuncSetAttribute(k_deblock_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows));
-    k_deblock_rows<<<ctas_rows, 128, smem_rows, st>>>(a);
+  std::memcpy(rows, &p[0], sizeof p[0]);
+  std::memcpy(cols, &p[1], sizeof p[1]);
+  return H266_OK;
+}
+
+namespace {
+template <class K>
+int strip_smem(K kern, size_t bytes) {
+  if (bytes > 40 * 1024)  // above the default limit with the kernels' static shared memory
+    H266_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  return H266_OK;
+}
+
+int launch_strips_single(cudaStream_t st, const StripParams &v, const StripParams &h, const StripCounts &c,
+                         uint64_t *launches) {
+  if (c.rows) {
+    H266_TRY(strip_smem(k_deblock_rows, c.smem_rows));
+    k_deblock_rows<<<c.rows, 128, c.smem_rows, st>>>(v);
     H266_CUDA(cudaGetLastError());
     ++*launches;
   }
-  // horizontal pass, in place on dst
-  a.segs = h.segs;
-  a.comp = h.comp;
-  a.band_first = h.band_first;
-  a.lut = nullptr;
-  for (int i = 0; i < 3; ++i) {
-    a.band_off[i] = band_off[1][i];
-    a.n_bands[i] = n_bands[1][i];
-    a.ctas[i] = strips[i];
-  }
-  if (ctas_cols) {
-    if (smem_cols > 48 * 1024)
-      H266_CUDA(cudaFuncSetAttribute(k_deblock_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols));
-    k_deblock_cols<<<ctas_cols, 128, smem_cols, st>>>(a);
+  if (c.cols) {
+    H266_TRY(strip_smem(k_deblock_cols, c.smem_cols));
+    k_deblock_cols<<<c.cols, 128, c.smem_cols, st>>>(h);
     H266_CUDA(cudaGetLastError());
     ++*launches;
   }
   return H266_OK;
 }
+}  // namespace
 
-// Strip kernels on the device walk's cell grids: a CTA per row band of each
-// plane (vertical pass, src -> dst), then per 8-column strip (horizontal pass,
-// in place on dst).  Row bands follow the plane sizes, so planes without
-// segments (chroma of a 4:0:0 walk) are still copied.
+int launch_deblock_strips(cudaStream_t st, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
+                          int bit_depth, const StripSide &v, const StripSide &h, const uint32_t band_off[2][3],
+                          const uint32_t n_bands[2][3], uint64_t *launches) {
+  StripParams rows, cols;
+  StripCounts c;
+  fill_strip_params(&rows, &cols, src, dst, lut, bit_depth, v, h, band_off, n_bands, c);
+  return launch_strips_single(st, rows, cols, c, launches);
+}
+
 int launch_deblock_strips_grid(cudaStream_t st, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
                                int bit_depth, const DeviceWalkOut &g, uint64_t *launches) {
-  StripParams a;
-  std::memset(&a, 0, sizeof a);
-  a.grid_mode = 1;
-  size_t smem_rows = 0, smem_cols = 0;
-  uint32_t ctas_rows = 0, ctas_cols = 0, rows[3], strips[3];
-  for (int i = 0; i < 3; ++i) {
-    a.src[i] = src[i];
-    a.dst[i] = dst[i];
-    const bool empty = (int64_t)src[i].w * src[i].h == 0;
-    const int unit = i ? 2 : 4;
-    rows[i] = empty ? 0 : (uint32_t)((src[i].h + unit - 1) / unit);
-    strips[i] = empty ? 0 : (uint32_t)((src[i].w + kStripCols - 1) / kStripCols);
-    if (!empty) {
-      smem_rows = std::max(smem_rows, rows_smem(src[i]));
-      smem_cols = std::max(smem_cols, cols_smem(src[i]));
-    }
-    ctas_rows += rows[i];
-    ctas_cols += strips[i];
-  }
-  if (smem_rows > (size_t)kMaxStripSmem || smem_cols > (size_t)kMaxStripSmem)
-    return set_error(H266_ERR_UNSUPPORTED, "deblock: planes too large for the strip kernels");
-  a.lut = lut;
-  a.maxv = (1 << bit_depth) - 1;
-  for (int i = 0; i < 3; ++i) {
-    a.grid[i] = g.grid[0][i];
-    a.grid_slots[i] = g.slots[0][i];
-    a.grid_bands[i] = g.bands[0][i];
-    a.ctas[i] = rows[i];
-  }
-  if (ctas_rows) {
-    if (smem_rows > 48 * 1024)
-      H266_CUDA(cudaFuncSetAttribute(k_deblock_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows));
-    k_deblock_rows<<<ctas_rows, 128, smem_rows, st>>>(a);
+  StripParams rows, cols;
+  StripCounts c;
+  H266_TRY(fill_strip_params_grid(&rows, &cols, src, dst, lut, bit_depth, g, c));
+  return launch_strips_single(st, rows, cols, c, launches);
+}
+
+int launch_strips_batch(cudaStream_t st, const void *d_rows, const uint32_t *d_first_rows, const void *d_cols,
+                        const uint32_t *d_first_cols, int n, const StripCounts &c, uint64_t *launches) {
+  if (c.rows) {
+    H266_TRY(strip_smem(k_deblock_rows_batch, c.smem_rows));
+    k_deblock_rows_batch<<<c.rows, 128, c.smem_rows, st>>>(static_cast<const StripParams *>(d_rows), d_first_rows, n);
     H266_CUDA(cudaGetLastError());
     ++*launches;
   }
-  a.lut = nullptr;
-  for (int i = 0; i < 3; ++i) {
-    a.grid[i] = g.grid[1][i];
-    a.grid_slots[i] = g.slots[1][i];
-    a.grid_bands[i] = g.bands[1][i];
-    a.ctas[i] = strips[i];
-  }
-  if (ctas_cols) {
-    if (smem_cols > 48 * 1024)
-      H266_CUDA(cudaFuncSetAttribute(k_deblock_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cols));
-    k_deblock_cols<<<ctas_cols, 128, smem_cols, st>>>(a);
+  if (c.cols) {
+    H266_TRY(strip_smem(k_deblock_cols_batch, c.smem_cols));
+    k_deblock_cols_batch<<<c.cols, 128, c.smem_cols, st>>>(static_cast<const StripParams *>(d_cols), d_first_cols, n);
     H266_CUDA(cudaGetLastError());
     ++*launches;
   }
@@ -2100,9 +2258,14 @@ int prepare_tile_kernels() {
   H266_CUDA(cudaGetDevice(&dev));
   const uint64_t bit = 1ull << (dev & 63);
   if (done.load(std::memory_order_relaxed) & bit) return H266_OK;
-  for (const void *k : {reinterpret_cast<const void *>(k_deblock_tiles), reinterpret_cast<const void *>(k_deblock_tiles_batch)}) {
-    H266_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem));
-    H266_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  const std::pair<const void *, size_t> kernels[] = {
+      {reinterpret_cast<const void *>(k_deblock_tiles<true>), TileGeo<true>::SMEM},
+      {reinterpret_cast<const void *>(k_deblock_tiles_batch<true>), TileGeo<true>::SMEM},
+      {reinterpret_cast<const void *>(k_deblock_tiles<false>), TileGeo<false>::SMEM},
+      {reinterpret_cast<const void *>(k_deblock_tiles_batch<false>), TileGeo<false>::SMEM}};
+  for (const auto &k : kernels) {
+    H266_CUDA(cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.second));
+    H266_CUDA(cudaFuncSetAttribute(k.first, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   }
   done.fetch_or(bit);
   return H266_OK;
@@ -2120,19 +2283,30 @@ int deblock_wait_timeouts(uint32_t *count) {
 namespace {
 // The tensor maps of the tile kernel's region boxes (a.tma 0 when a plane
 // cannot be described: unaligned base or stride).
-void tile_tma_maps(TileParams &a) {
+template <bool G8>
+bool tile_maps(TileParams &a) {
+  using Geo = TileGeo<G8>;
   bool ok = true;
   for (int p = 0; p < 3 && ok; ++p)
     if (a.src[p].w > 0 && a.src[p].h > 0)
-      ok = encode_plane_map(&a.tmap[p], a.src[p], p ? kPitchC : kPitchY, p ? kRegionC : kRegionY);
-  a.tma = ok ? 1 : 0;
+      ok = encode_plane_map(&a.tmap[p], a.src[p], p ? Geo::PC : Geo::PY, p ? Geo::RHC : Geo::RH);
+  return ok;
+}
+void tile_tma_maps(TileParams &a, bool grid8) { a.tma = grid8 ? tile_maps<true>(a) : tile_maps<false>(a); }
+
+int launch_tiles(cudaStream_t st, const TileParams &a, bool grid8, uint32_t n) {
+  H266_TRY(prepare_tile_kernels());
+  if (grid8) k_deblock_tiles<true><<<n, kTileThreads, TileGeo<true>::SMEM, st>>>(a);
+  else k_deblock_tiles<false><<<n, kTileThreads, TileGeo<false>::SMEM, st>>>(a);
+  H266_CUDA(cudaGetLastError());
+  return H266_OK;
 }
 }  // namespace
 
 uint32_t fill_deblock_tile_params(void *out, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
                                   int bit_depth, const StripSide &v, const StripSide &h, const uint32_t *tile_bounds,
                                   const uint32_t tb_off[2][3], const uint32_t n_bands[2][3], uint32_t tiles_x,
-                                  uint32_t tiles_y) {
+                                  uint32_t tiles_y, bool grid8) {
   TileParams a;
   std::memset(&a, 0, sizeof a);
   for (int i = 0; i < 3; ++i) {
@@ -2152,7 +2326,7 @@ uint32_t fill_deblock_tile_params(void *out, const DPlane src[3], const DPlane d
   a.tiles_x = tiles_x;
   a.tiles_y = tiles_y;
   a.maxv = (1 << bit_depth) - 1;
-  tile_tma_maps(a);
+  tile_tma_maps(a, grid8);
   std::memcpy(out, &a, sizeof a);
   return tiles_x * tiles_y;
 }
@@ -2160,23 +2334,23 @@ uint32_t fill_deblock_tile_params(void *out, const DPlane src[3], const DPlane d
 int launch_deblock_tiles(cudaStream_t st, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
                          int bit_depth, const StripSide &v, const StripSide &h, const uint32_t *tile_bounds,
                          const uint32_t tb_off[2][3], const uint32_t n_bands[2][3], uint32_t tiles_x,
-                         uint32_t tiles_y, uint64_t *launches) {
+                         uint32_t tiles_y, bool grid8, uint64_t *launches) {
   TileParams a;
   const uint32_t n = fill_deblock_tile_params(&a, src, dst, lut, bit_depth, v, h, tile_bounds, tb_off, n_bands,
-                                              tiles_x, tiles_y);
+                                              tiles_x, tiles_y, grid8);
   if (!n) return H266_OK;
-  H266_TRY(prepare_tile_kernels());
-  k_deblock_tiles<<<n, kTileThreads, kTileSmem, st>>>(a);
-  H266_CUDA(cudaGetLastError());
+  H266_TRY(launch_tiles(st, a, grid8, n));
   ++*launches;
   return H266_OK;
 }
 
-int launch_deblock_tiles_batch(cudaStream_t st, const void *d_params, const uint32_t *d_first, int n, uint32_t ctas,
-                               uint64_t *launches) {
+int launch_deblock_tiles_batch(cudaStream_t st, bool grid8, const void *d_params, const uint32_t *d_first, int n,
+                               uint32_t ctas, uint64_t *launches) {
   if (!ctas || n <= 0) return H266_OK;
   H266_TRY(prepare_tile_kernels());
-  k_deblock_tiles_batch<<<ctas, kTileThreads, kTileSmem, st>>>(static_cast<const TileParams *>(d_params), d_first, n);
+  const TileParams *params = static_cast<const TileParams *>(d_params);
+  if (grid8) k_deblock_tiles_batch<true><<<ctas, kTileThreads, TileGeo<true>::SMEM, st>>>(params, d_first, n);
+  else k_deblock_tiles_batch<false><<<ctas, kTileThreads, TileGeo<false>::SMEM, st>>>(params, d_first, n);
   H266_CUDA(cudaGetLastError());
   ++*launches;
   return H266_OK;
@@ -2203,16 +2377,23 @@ int launch_deblock(cudaStream_t st, const DPlane planes[3], int bit_depth, const
 // ===================================================================== device-built side information
 int device_walk_mode(const h266_picture &pic, const h266_deblock_cu *cus, uint64_t n_cus,
                      const h266_deblock_cu *chroma_cus, uint64_t n_chroma, const h266_deblock_params &params,
-                     uint32_t cfi) {
+                     uint32_t cfi, bool *grid8) {
+  if (grid8) *grid8 = false;
   if (params.disabled || params.bit_depth < 8 || params.bit_depth > 16 || params.ctb_log2_size_y > 16) return 0;
   if (cfi > 3) return 0;
   const int w = (int)pic.luma.width, h = (int)pic.luma.height;
   if (w <= 0 || h <= 0) return 0;
   const bool chroma = (uint64_t)pic.cb.width * pic.cb.height != 0 || (uint64_t)pic.cr.width * pic.cr.height != 0;
   if (n_cus > (uint64_t)INT32_MAX || n_chroma > (uint64_t)INT32_MAX) return 0;
-  // The tile kernel's condition: no two segments' footprints overlap, every
-  // one inside a cell of the tile halo -- luma CUs and transform blocks at
-  // least 8 samples, no sub-block edges, 4:2:0 or 4:0:0.
+  // The tile kernel's condition: no segment writes what another of its pass
+  // uses (seg_span), 4:2:0 or 4:0:0.  Transform edges never do: an edge next to
+  // a transform block of 4 samples has maxFilterLength 1 (3 samples used), of
+  // 8 to 28 at most 3 (4 used), of 32 or more at most 7 (8 used), so an edge
+  // uses no more than the block on either side of it.  Sub-block edges lie 8 or
+  // more apart with at most 3, 2 next to a CU or transform edge 8 away (at most
+  // 5); only a transform edge off the sub-block grid, which keeps its full
+  // length, comes closer to one.  On the 8x8 grid the smaller regions do.
+  bool on8 = true;
   bool no_chains = cfi <= 1 && !(cfi == 0 && chroma);
   if (chroma && (pic.cb.width != (pic.luma.width + 1) / 2 || pic.cb.height != (pic.luma.height + 1) / 2 ||
                  pic.cr.width != pic.cb.width || pic.cr.height != pic.cb.height))
@@ -2238,22 +2419,42 @@ int device_walk_mode(const h266_picture &pic, const h266_deblock_cu *cus, uint64
   for (int l = 0; l < 2; ++l) {
     if (!lists[l]) continue;
     bits.assign((size_t)words * ch4, 0);
-    bool chains = false;  // 4-sample edges, sub-block edges or narrow transform blocks in this list
+    bool chains = false;  // luma segments of this list may use what others write
+    bool narrow = false;  // luma edges less than 8 apart, or sub-block edges
     for (uint64_t i = 0; i < counts[l]; ++i) {
       const h266_deblock_cu &c = lists[l][i];
       if ((c.x | c.y | c.w | c.h) & 3 || c.w == 0 || c.h == 0) return 0;
       if ((uint64_t)c.x + c.w > (uint64_t)w || (uint64_t)c.y + c.h > (uint64_t)h) return 0;
       if (c.has_tb_split && (c.tb_split.n_bounds < 1 || c.tb_split.n_bounds > 3)) return 0;
-      if (c.w < 8 || c.h < 8 || c.has_num_sb) chains = true;
-      if (c.has_tb_split) {
-        const uint32_t dim = c.tb_split.vertical ? c.w : c.h;
-        uint32_t prev = 0;
-        for (int k = 0; k < c.tb_split.n_bounds; ++k) {
-          const uint32_t b = c.tb_split.bounds[k];
-          if (b < prev + 8) chains = true;
-          prev = b;
+      if (l == 0) {  // chroma edges are 8 chroma samples apart and use 4
+        if ((c.x | c.y | c.w | c.h) & 7) on8 = false;
+        narrow = narrow || c.w < 8 || c.h < 8 || c.has_num_sb;
+        // the edges inside the CU: vertical, horizontal
+        const int dirs = c.has_num_sb || c.has_tb_split || c.has_tu64 ? 2 : 0;
+        for (int dir = 0; dir < dirs; ++dir) {
+          const uint32_t dim = dir == 0 ? c.w : c.h;
+          // sub-block edges at the multiples k * sb, k <= last_sb (cu_walk_geo)
+          const uint32_t nsb = c.has_num_sb ? std::max(dir == 0 ? c.num_sb_x : c.num_sb_y, 1u) : 1u;
+          const uint32_t sb = std::max(8u, dim / nsb), last_sb = std::min(std::max(dim / 8, 1u) - 1, nsb - 1);
+          if (last_sb && (sb & 7)) on8 = false;
+          auto tb_edge = [&](uint32_t b) {
+            if (b & 7) on8 = false;
+            if (last_sb && (b % sb || b / sb > last_sb)) chains = true;
+          };
+          if (c.has_tu64 && dim > 64) {
+            for (uint32_t b = 64; b < dim; b += 64) tb_edge(b);
+          } else if (c.has_tb_split && (c.tb_split.vertical != 0) == (dir == 0)) {
+            uint32_t prev = 0;
+            for (int k = 0; k < c.tb_split.n_bounds; ++k) {
+              const uint32_t b = c.tb_split.bounds[k];
+              if (b <= prev || b >= dim || (b & 3)) chains = true;  // not a partition of the CU on the 4x4 grid
+              else tb_edge(b);
+              narrow = narrow || b < prev + 8;
+              prev = b;
+            }
+            narrow = narrow || dim < prev + 8;
+          }
         }
-        if (dim < prev + 8) chains = true;
       }
       const uint32_t x0 = c.x / 4, x1 = (c.x + c.w) / 4;
       for (uint32_t y = c.y / 4; y < (c.y + c.h) / 4; ++y) {
@@ -2268,9 +2469,9 @@ int device_walk_mode(const h266_picture &pic, const h266_deblock_cu *cus, uint64
       }
     }
     if (chains) no_chains = false;
-    // Only luma footprints chain (chroma edges are 8 chroma samples apart and
-    // reach 4), so only the luma list's order matters.
-    if (l != 0 || !chains) continue;
+    // Chains run in position order, which is the reference's where the list is
+    // in decode order; lists with narrow edges out of it stay on the host.
+    if (!chains && !narrow) continue;
     map.assign((size_t)cw4 * ch4, -1);
     for (uint64_t i = 0; i < counts[l]; ++i) {
       const h266_deblock_cu &c = lists[l][i];
@@ -2291,6 +2492,7 @@ int device_walk_mode(const h266_picture &pic, const h266_deblock_cu *cus, uint64
       }
     }
   }
+  if (grid8) *grid8 = on8;
   return no_chains ? 1 : 2;
 }
 
@@ -2338,22 +2540,22 @@ struct WalkParams {
   uint32_t slots[2][3], bands[2][3];
   // Per-tile lists for the grid-mode tile kernel (null when the strip kernels
   // consume the grids): tile_count[tile * 6 + pass * 3 + plane] cells, listed
-  // at tile_list[pass][plane][tile * cap], cap kTileListY (luma) or
-  // kTileListC (chroma).
+  // at tile_list[pass][plane][tile * cap], cap tile_list_cap().
   uint32_t *tile_count;
   uint32_t *tile_list[2][3];
   uint32_t tiles_x, tiles_y;
+  int grid8;  // the tile kernel's region: 0 the wider one
   int pw[3], ph[3];
 };
 
 // A segment into its grid cell and, for the tile kernel, into the list of
-// every tile it runs in: a vertical-pass segment in the tiles whose columns
-// its footprint reaches and whose rows widened by the halo hold its band, a
-// horizontal-pass segment in the tile holding its band whose rows its
-// footprint reaches (the host's index_tiles rule).  A picture the tile kernel
-// takes has no two footprints overlapping and edges at least 8 samples apart,
-// so a tile's list holds at most 24 bands x 12 luma (16 x 12 horizontal) or
-// 24 x 6 chroma cells, within the caps.
+// every tile it runs in: a vertical-pass segment in the tiles whose columns it
+// writes and whose rows widened by the halo hold its band, a horizontal-pass
+// segment in the tile holding its band whose rows it writes (the host's
+// index_tiles_halo rule).  A segment writes at most 7 samples, so a tile's
+// band lists edges from 4 before its first to 4 after its last sample: on the
+// 8x8 grid 9 of them, on the 4x4 grid 19, in 20 (22) bands of the vertical and
+// 16 of the horizontal pass; chroma 5 in 20 and 16 bands.  All within the caps.
 struct GridEmit {
   const WalkParams *a;
   int d, p;
@@ -2366,9 +2568,11 @@ struct GridEmit {
     const uint32_t cell = band * slots + pos;
     a->grid[d][p][cell] = s;
     if (!a->tile_count) return;
-    const int tp = p ? kDeblockTile / 2 : kDeblockTile, halo = p ? kDeblockHaloC : kDeblockHaloY;
-    const int along = vert ? a->pw[p] : a->ph[p], q = vert ? s.x : s.y, bc = vert ? s.y : s.x;
-    const int fs = max(q - reach_d(s.mfl >> 4), 0), fe = min(q + reach_d(s.mfl & 15), along);
+    const int tp = p ? kDeblockTile / 2 : kDeblockTile;
+    const int halo = p ? kTileHaloYC : (a->grid8 ? kTileHaloY8 : kTileHaloY4);
+    const int along = vert ? a->pw[p] : a->ph[p], bc = vert ? s.y : s.x;
+    const SegSpan f = seg_span(s);
+    const int fs = max(f.ws, 0), fe = min(f.we, along);
     if (fs >= fe) return;  // touches no sample of the plane
     int x0, x1, y0, y1;    // tile columns and rows
     if (vert) {
@@ -2383,7 +2587,7 @@ struct GridEmit {
     }
     x1 = min(x1, (int)a->tiles_x - 1);
     y1 = min(y1, (int)a->tiles_y - 1);
-    const uint32_t cap = p ? kTileListC : kTileListY;
+    const uint32_t cap = tile_list_cap(a->grid8, d, p);
     for (int ty = y0; ty <= y1; ++ty)
       for (int tx = x0; tx <= x1; ++tx) {
         const uint32_t t = (uint32_t)ty * a->tiles_x + tx;
@@ -2482,27 +2686,126 @@ __global__ void k_cu_grid(const __grid_constant__ WalkParams a, int list) {
   if (i < unpack_items(a, list)) unpack_item(a, list, i);
 }
 
-// The edge walk of one CU for one (plane, pass) list (blockIdx.y = plane * 2 +
-// pass) at one edge offset (blockIdx.z: offset / step; offsets beyond the CU
-// return at once).
-__global__ void __launch_bounds__(128) k_walk(const __grid_constant__ WalkParams a) {
-  const int l = blockIdx.y, plane = l / 2, d = l % 2;
-  const int list = plane ? 1 : 0;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n[list]) return;
-  const h266_deblock_cu &cu = a.cus[list][i];
-  const uint32_t step = plane ? 8 * (d == 0 ? a.cfg[plane].sub_w : a.cfg[plane].sub_h) : 4;
-  const uint32_t off = blockIdx.z * step;
-  if (off >= (d == 0 ? cu.w : cu.h)) return;
+// The edge walk of 32 consecutive CUs (from `base`) of one (plane, pass) list,
+// by `split` warps of the CTA: every warp counts the segments of its lanes'
+// CUs -- all edges of a CU, its own (offset 0) and those inside it -- and the
+// warps take the group's segments one per lane, so lanes stay busy whatever
+// the CU sizes, and no lane walks more than its share of the dependent loads
+// (CU map, P-side CU record, motion) that bound the walk.  One thread per CU
+// (and edge offset) took 59 us on one 1080p picture of 5300 CUs and 70 us on a
+// multi-type-tree one of 12000.
+// Edges inside a CU are found 32 offsets at a time (a bit per offset), so a CU
+// of any size works.  `pre` and `mask` are the warp's scratch, 32 words each.
+__device__ __forceinline__ void walk_group(const WalkParams &a, int l, uint32_t base, int part, int split,
+                                           uint32_t *pre, uint32_t *mask) {
+  const int plane = l / 2, d = l % 2, list = plane ? 1 : 0, lane = threadIdx.x & 31;
+  const bool vert = d == 0;
+  const h266_deblock_cu *cus = a.cus[list];
   const DevCuGrid grid{a.cu_grid[list], a.cw4, a.ch4};
   const GridEmit emit{&a, d, plane};
-  if (plane == 0 && a.has_mv && a.mv_per_cu) {
-    const CuMotion mv{&a.mv, a.mv_per_cu, DevCuGrid{a.cu_grid[0], a.cw4, a.ch4}};
-    walk_cu(a.cus[list], grid, a.cfg[plane], d == 0, mv, a.nf[d], a.n_nf[d], i, emit, (int)off);
-  } else {
-    const MvGrid mv{plane == 0 && a.has_mv ? &a.mv : nullptr};
-    walk_cu(a.cus[list], grid, a.cfg[plane], d == 0, mv, a.nf[d], a.n_nf[d], i, emit, (int)off);
+  auto with_mv = [&](auto &&f) {
+    if (plane == 0 && a.has_mv && a.mv_per_cu) f(CuMotion{&a.mv, a.mv_per_cu, DevCuGrid{a.cu_grid[0], a.cw4, a.ch4}});
+    else f(MvGrid{plane == 0 && a.has_mv ? &a.mv : nullptr});
+  };
+  const uint32_t i = base + lane;
+  bool walks = false;  // the CU has edges of this list
+  uint32_t n_off = 0, along = 0;
+  CuWalkGeo mine{};
+  if (i < a.n[list]) {
+    const h266_deblock_cu &cu = cus[i];
+    mine = cu_walk_geo(cu, a.cfg[plane], vert, a.nf[d], a.n_nf[d]);
+    walks = !mine.off_grid;
+    // only sub-block grids, TB splits and 64-sample TU tiling put edges inside a CU
+    const bool inner = cu.has_num_sb || cu.has_tb_split || (cu.has_tu64 && mine.n_cb > 64);
+    n_off = !walks ? 0 : (inner ? (mine.n_cb + mine.step - 1) / mine.step : 1);
+    along = (mine.n_other + mine.seg - 1) / mine.seg;
   }
+  // f(lane whose CU holds the segment, the segment's index in that CU) for this part's share of the group's segments
+  auto each = [&](uint32_t nseg, auto &&f) {
+    uint32_t incl = nseg;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    pre[lane] = incl - nseg;
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    __syncwarp();
+    for (uint32_t t = part * 32 + lane; t < total; t += split * 32) {
+      const int j = band_of(pre, t);
+      f(j, t - pre[j]);
+    }
+    __syncwarp();  // pre and mask are free again
+  };
+  const uint32_t max_off = __reduce_max_sync(0xFFFFFFFFu, n_off);
+  if (max_off <= 1) {  // only the CUs' own edges (124 against 140 us per 16 1080p pictures by the general loop)
+    each(walks && mine.filter_edge ? along : 0, [&](int j, uint32_t r) {
+      const size_t idx = base + j;
+      const CuWalkGeo g = cu_walk_geo(cus[idx], a.cfg[plane], vert, a.nf[d], a.n_nf[d]);
+      with_mv([&](const auto &mv) {
+        WalkMemo memo;
+        walk_segment(cus, grid, a.cfg[plane], vert, mv, idx, g, 0, g.filter_edge, !g.chroma && g.filter_edge, r * g.seg,
+                     emit, memo);
+      });
+    });
+    return;
+  }
+  for (uint32_t o0 = 0; o0 < max_off; o0 += 32) {
+    uint32_t m = 0;  // bit k: the offset (o0 + k) * step is an edge of the CU
+    if (walks) {
+      const Cu geo{cus[i]};
+      const uint32_t hi = min(n_off, o0 + 32);
+      for (uint32_t o = o0; o < hi; ++o) {
+        const uint32_t off = o * mine.step;
+        const bool is_tb = o == 0 ? mine.filter_edge : geo.tb_boundary(off, vert, mine.chroma);
+        const bool is_sb =
+            !mine.chroma && off % mine.sb == 0 && off / mine.sb <= mine.last_sb && (o > 0 || mine.filter_edge);
+        if (is_tb || is_sb) m |= 1u << (o - o0);
+      }
+    }
+    mask[lane] = m;
+    each((uint32_t)__popc(m) * along, [&](int j, uint32_t r) {
+      const size_t idx = base + j;
+      const CuWalkGeo g = cu_walk_geo(cus[idx], a.cfg[plane], vert, a.nf[d], a.n_nf[d]);
+      const uint32_t n_along = (g.n_other + g.seg - 1) / g.seg;
+      uint32_t e = r / n_along, bits = mask[j];
+      const uint32_t k = (r - e * n_along) * g.seg;
+      for (; e; --e) bits &= bits - 1;
+      const uint32_t off = (o0 + (uint32_t)__ffs(bits) - 1) * g.step;
+      const bool is_tb = off == 0 ? g.filter_edge : Cu{cus[idx]}.tb_boundary(off, vert, g.chroma);
+      const bool is_sb = !g.chroma && off % g.sb == 0 && off / g.sb <= g.last_sb && (off > 0 || g.filter_edge);
+      with_mv([&](const auto &mv) {
+        WalkMemo memo;
+        walk_segment(cus, grid, a.cfg[plane], vert, mv, idx, g, off, is_tb, is_sb, k, emit, memo);
+      });
+    });
+  }
+}
+
+constexpr int kWalkThreads = 128;
+
+// The walk's CTAs of list l: a group of 32 CUs per warp of the CTA, each
+// group's segments shared by the gridDim.z CTAs of the same x.
+__device__ __forceinline__ void walk_cta(const WalkParams &a, int l, uint32_t b) {
+  __shared__ uint32_t s_pre[kWalkThreads / 32][32], s_mask[kWalkThreads / 32][32];
+  const int warp = threadIdx.x >> 5;
+  const uint32_t base = b * kWalkThreads + warp * 32;
+  if (base >= a.n[l >= 2 ? 1 : 0]) return;  // uniform per warp
+  walk_group(a, l, base, blockIdx.z, gridDim.z, s_pre[warp], s_mask[warp]);
+}
+
+// CTAs per 32-CU group: several while the groups alone leave the SMs short of
+// warps to cover the walk's dependent loads (one 1080p picture of 5300 CUs has
+// 1000 groups over its six lists, 1.7 per scheduler); one for batches that
+// have the warps, as every CTA of a group counts its CUs again.
+uint32_t walk_split(uint32_t ctas) {
+  const uint32_t warps = ctas * 6 * (kWalkThreads / 32), want = 148 * 32;
+  return warps >= want ? 1 : std::min(4u, want / std::max(warps, 1u) + 1);
+}
+
+// One picture's walk: blockIdx.y = plane * 2 + pass.
+__global__ void __launch_bounds__(kWalkThreads) k_walk(const __grid_constant__ WalkParams a) {
+  walk_cta(a, blockIdx.y, blockIdx.x);
 }
 
 size_t align_up(size_t n) { return (n + 255) & ~(size_t)255; }
@@ -2554,7 +2857,7 @@ WalkLayout walk_layout(const DeviceWalkIn &in) {
   for (int d = 0; d < 2; ++d)
     for (int p = 0; p < 3; ++p) {
       L.tile_list[d][p] = off;
-      off += align_up(tiles * (p ? kTileListC : kTileListY) * sizeof(uint32_t));
+      off += align_up(tiles * tile_list_cap(in.grid8, d, p) * sizeof(uint32_t));
     }
   L.total = off;
   return L;
@@ -2618,6 +2921,8 @@ void fill_walk(const DeviceWalkIn &in, uint8_t *scratch, WalkParams &a, DeviceWa
   out.tiles_y = (uint32_t)((in.h + kDeblockTile - 1) / kDeblockTile);
   a.tile_count = in.tile_lists ? reinterpret_cast<uint32_t *>(scratch + L.tile_count) : nullptr;
   out.tile_count = a.tile_count;
+  a.grid8 = in.grid8;
+  out.grid8 = in.grid8;
   a.tiles_x = out.tiles_x;
   a.tiles_y = out.tiles_y;
   a.pw[0] = in.w;
@@ -2646,11 +2951,9 @@ int launch_device_walk(cudaStream_t st, const DeviceWalkIn &in, uint8_t *scratch
     ++*launches;
   }
   const uint32_t nmax = std::max(a.n[0], a.n[1]);
-  // offsets per CU: at most max dimension / 4 (luma; chroma has fewer)
-  uint32_t max_dim = 4;
-  max_dim = std::max(max_dim, in.max_cu_dim);
   if (nmax) {
-    k_walk<<<dim3((nmax + 127) / 128, lists, (max_dim + 3) / 4), 128, 0, st>>>(a);
+    const uint32_t ctas = (nmax + kWalkThreads - 1) / kWalkThreads;
+    k_walk<<<dim3(ctas, lists, walk_split(ctas)), kWalkThreads, 0, st>>>(a);
     H266_CUDA(cudaGetLastError());
     ++*launches;
   }
@@ -2662,7 +2965,7 @@ int launch_device_walk(cudaStream_t st, const DeviceWalkIn &in, uint8_t *scratch
 // The walks of many pictures in three launches: the clearing of every
 // picture's CU maps (-1) and segment grids (bS 0), the CU maps, and the edge
 // walk.  Per picture a WalkBatchItem (parameters, clear extents, the walk's
-// list count and offsets); CTAs find their picture by binary search over
+// list count); CTAs find their picture by binary search over
 // per-launch prefix tables of CTA counts.
 struct WalkBatchItem {
   WalkParams p;
@@ -2708,9 +3011,9 @@ __global__ void __launch_bounds__(128) k_cu_grid_batch(const WalkBatchItem *__re
   if (i < unpack_items(a, list)) unpack_item(a, list, i);
 }
 
-// blockIdx.y = plane * 2 + pass, blockIdx.z = edge offset / step, as k_walk.
-__global__ void __launch_bounds__(128) k_walk_batch(const WalkBatchItem *__restrict__ items,
-                                                    const uint32_t *__restrict__ first, int n) {
+// blockIdx.y = plane * 2 + pass, as k_walk.
+__global__ void __launch_bounds__(kWalkThreads) k_walk_batch(const WalkBatchItem *__restrict__ items,
+                                                             const uint32_t *__restrict__ first, int n) {
   __shared__ WalkParams s;
   const int p = batch_pick(first, n, blockIdx.x);
   if (blockIdx.y >= items[p].lists) return;  // uniform per CTA
@@ -2719,59 +3022,7 @@ __global__ void __launch_bounds__(128) k_walk_batch(const WalkBatchItem *__restr
   uint32_t *dst = reinterpret_cast<uint32_t *>(&s);
   for (int i = threadIdx.x; i < (int)(sizeof(WalkParams) / 4); i += blockDim.x) dst[i] = src[i];
   __syncthreads();
-  const WalkParams &a = s;
-  const int l = blockIdx.y, plane = l / 2, d = l % 2;
-  const int list = plane ? 1 : 0;
-  const bool vert = d == 0;
-  const DevCuGrid grid{a.cu_grid[list], a.cw4, a.ch4};
-  const GridEmit emit{&a, d, plane};
-  auto with_mv = [&](auto &&f) {
-    if (plane == 0 && a.has_mv && a.mv_per_cu) f(CuMotion{&a.mv, a.mv_per_cu, DevCuGrid{a.cu_grid[0], a.cw4, a.ch4}});
-    else f(MvGrid{plane == 0 && a.has_mv ? &a.mv : nullptr});
-  };
-  if (blockIdx.z == 0) {
-    // The CUs' own edges (offset 0), packed: lane j of a warp counts the
-    // segments of CU base + j's edge, and the warp walks all 32 CUs'
-    // segments one per lane per round, so lanes stay busy whatever the CU
-    // sizes (no memo across segments: the same values, recomputed).
-    __shared__ uint32_t s_pre[4][32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t base = (blockIdx.x - first[p]) * blockDim.x + warp * 32, i = base + lane;
-    uint32_t nseg = 0;
-    if (i < a.n[list]) {
-      const CuWalkGeo g = cu_walk_geo(a.cus[list][i], a.cfg[plane], vert, a.nf[d], a.n_nf[d]);
-      if (!g.off_grid && g.filter_edge) nseg = (g.n_other + g.seg - 1) / g.seg;
-    }
-    uint32_t incl = nseg;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    s_pre[warp][lane] = incl - nseg;
-    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    __syncwarp();
-    for (uint32_t t = lane; t < total; t += 32) {
-      const int j = band_of(s_pre[warp], t);  // the lane whose CU holds segment t
-      const size_t idx = base + j;
-      const CuWalkGeo g = cu_walk_geo(a.cus[list][idx], a.cfg[plane], vert, a.nf[d], a.n_nf[d]);
-      const uint32_t k = (t - s_pre[warp][j]) * g.seg;
-      with_mv([&](const auto &mv) {
-        WalkMemo memo;
-        walk_segment(a.cus[list], grid, a.cfg[plane], vert, mv, idx, g, 0, g.filter_edge, !g.chroma && g.filter_edge,
-                     k, emit, memo);
-      });
-    }
-    return;
-  }
-  // edges inside a CU (blockIdx.z = offset / step): one thread per CU
-  const uint32_t i = (blockIdx.x - first[p]) * blockDim.x + threadIdx.x;
-  if (i >= a.n[list]) return;
-  const h266_deblock_cu &cu = a.cus[list][i];
-  const uint32_t step = plane ? 8 * (vert ? a.cfg[plane].sub_w : a.cfg[plane].sub_h) : 4;
-  const uint32_t off = blockIdx.z * step;
-  if (off >= (vert ? cu.w : cu.h)) return;
-  with_mv([&](const auto &mv) { walk_cu(a.cus[list], grid, a.cfg[plane], vert, mv, a.nf[d], a.n_nf[d], i, emit, (int)off); });
+  walk_cta(s, blockIdx.y, blockIdx.x - first[p]);
 }
 
 }  // namespace
@@ -2792,7 +3043,6 @@ void fill_walk_batch_item(void *out, const DeviceWalkIn &in, uint8_t *scratch, D
   c.clear_ctas = (it.ff_vec + it.zero_vec + kClearVecPerCta - 1) / kClearVecPerCta;
   c.grid_ctas = (unpack_items(it.p, 0) + 127) / 128 + (it.cu_lists == 2 ? (unpack_items(it.p, 1) + 127) / 128 : 0);
   c.walk_ctas = (std::max(it.p.n[0], it.p.n[1]) + 127) / 128;
-  c.offsets = (std::max<uint32_t>(4, in.max_cu_dim) + 3) / 4;
   std::memcpy(out, &it, sizeof it);
 }
 
@@ -2812,7 +3062,7 @@ int launch_walk_batch(cudaStream_t st, const void *d_items, const uint32_t *d_fi
     ++*launches;
   }
   if (total.walk_ctas) {
-    k_walk_batch<<<dim3(total.walk_ctas, 6, total.offsets), 128, 0, st>>>(items, d_first_walk, n);
+    k_walk_batch<<<dim3(total.walk_ctas, 6, walk_split(total.walk_ctas)), kWalkThreads, 0, st>>>(items, d_first_walk, n);
     H266_CUDA(cudaGetLastError());
     ++*launches;
   }
@@ -2839,7 +3089,7 @@ uint32_t fill_deblock_tile_params_grid(void *out, const DPlane src[3], const DPl
   a.tiles_x = g.tiles_x;
   a.tiles_y = g.tiles_y;
   a.maxv = (1 << bit_depth) - 1;
-  tile_tma_maps(a);
+  tile_tma_maps(a, g.grid8);
   std::memcpy(out, &a, sizeof a);
   return g.tiles_x * g.tiles_y;
 }
@@ -2847,29 +3097,9 @@ uint32_t fill_deblock_tile_params_grid(void *out, const DPlane src[3], const DPl
 int launch_deblock_tiles_grid(cudaStream_t st, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
                               int bit_depth, const DeviceWalkOut &g, uint64_t *launches) {
   TileParams a;
-  std::memset(&a, 0, sizeof a);
-  for (int i = 0; i < 3; ++i) {
-    a.src[i] = src[i];
-    a.dst[i] = dst[i];
-    for (int d = 0; d < 2; ++d) {
-      a.n_bands[d][i] = g.bands[d][i];
-      a.grid[d][i] = g.grid[d][i];
-      a.grid_slots[d][i] = g.slots[d][i];
-      a.grid_list[d][i] = g.tile_list[d][i];
-    }
-  }
-  a.grid_count = g.tile_count;
-  a.grid_mode = 1;
-  a.lut = lut;
-  a.tiles_x = g.tiles_x;
-  a.tiles_y = g.tiles_y;
-  a.maxv = (1 << bit_depth) - 1;
-  tile_tma_maps(a);
-  const uint64_t n = (uint64_t)g.tiles_x * g.tiles_y;
+  const uint32_t n = fill_deblock_tile_params_grid(&a, src, dst, lut, bit_depth, g);
   if (!n) return H266_OK;
-  H266_TRY(prepare_tile_kernels());
-  k_deblock_tiles<<<(unsigned)n, kTileThreads, kTileSmem, st>>>(a);
-  H266_CUDA(cudaGetLastError());
+  H266_TRY(launch_tiles(st, a, g.grid8, n));
   ++*launches;
   return H266_OK;
 }

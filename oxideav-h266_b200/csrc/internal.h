@@ -130,20 +130,29 @@ struct DeblockPlan {
   // vertical pass tile_bounds[tb_off[0][p] + (band * tiles_x + tx) * 2] and the
   // next entry are the first and end component of the band reaching tile
   // column tx; for the horizontal pass the same with (column band * tiles_y +
-  // ty).  tiles_ok is false when a component spans more than the tile halo, a
+  // ty).  tiles_ok is false when a component uses more than the tile halo, a
   // tile would list more components than the kernel's shared list holds, or
   // the chroma format is not 4:2:0 / 4:0:0; the strip kernels run then.
   bool tiles_ok = false;
+  bool tiles_grid8 = false;  // the ranges fit the smaller regions
   uint32_t tiles_x = 0, tiles_y = 0;
   std::vector<uint32_t> tile_bounds;
   uint32_t tb_off[2][3] = {{0, 0, 0}, {0, 0, 0}};
 };
 
-constexpr int kDeblockTile = 64;      // luma tile edge of the tile kernel
-constexpr int kDeblockHaloY = 16;     // luma halo (a component's footprint is at most 16 samples)
-constexpr int kDeblockHaloC = 8;      // chroma halo (footprints of at most 8 samples)
-constexpr int kTileListY = 320;       // shared list entries per pass: luma components of a tile
-constexpr int kTileListC = 176;       // chroma components of a tile, per plane
+constexpr int kDeblockTile = 64;  // luma tile edge of the tile kernel
+// Halo of the tile kernel's regions, in samples: luma with every edge on the
+// 8x8 grid, luma with edges on the 4x4 grid, chroma.
+constexpr int kTileHaloX8 = 8, kTileHaloY8 = 8, kTileHaloX4 = 16, kTileHaloY4 = 12;
+constexpr int kTileHaloXC = 8, kTileHaloYC = 4;
+// Shared list entries of pass d (0 vertical, 1 horizontal) and plane p: the
+// segments of a tile's components.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr uint32_t tile_list_cap(bool grid8, int d, int p) {
+  return p ? 128u : (grid8 ? (d ? 192u : 256u) : (d ? 320u : 432u));
+}
 
 int build_deblock_plan(const h266_picture &pic, const h266_deblock_cu *cus, uint64_t n_cus,
                        const h266_deblock_cu *chroma_cus, uint64_t n_chroma, const h266_deblock_mv_grid *mv,
@@ -169,7 +178,7 @@ int launch_deblock_strips(cudaStream_t st, const DPlane src[3], const DPlane dst
 int launch_deblock_tiles(cudaStream_t st, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
                          int bit_depth, const StripSide &v, const StripSide &h, const uint32_t *tile_bounds,
                          const uint32_t tb_off[2][3], const uint32_t n_bands[2][3], uint32_t tiles_x,
-                         uint32_t tiles_y, uint64_t *launches);
+                         uint32_t tiles_y, bool grid8, uint64_t *launches);
 // Batched tile kernel: fill_deblock_tile_params writes one picture's kernel
 // parameters (deblock_tile_params_size() bytes) to `out` and returns its CTA
 // count; CTAs [first[i], first[i + 1]) of the batched launch are picture i's.
@@ -177,23 +186,24 @@ size_t deblock_tile_params_size();
 uint32_t fill_deblock_tile_params(void *out, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
                                   int bit_depth, const StripSide &v, const StripSide &h, const uint32_t *tile_bounds,
                                   const uint32_t tb_off[2][3], const uint32_t n_bands[2][3], uint32_t tiles_x,
-                                  uint32_t tiles_y);
-int launch_deblock_tiles_batch(cudaStream_t st, const void *d_params, const uint32_t *d_first, int n, uint32_t ctas,
-                               uint64_t *launches);
+                                  uint32_t tiles_y, bool grid8);
+int launch_deblock_tiles_batch(cudaStream_t st, bool grid8, const void *d_params, const uint32_t *d_first, int n,
+                               uint32_t ctas, uint64_t *launches);
 // ---------------------------------------------------------------- device-built side information
 // Device-built side information: the edge walk runs on the device from the
 // CU lists and the motion grid and writes each segment to a dense per-band
-// cell grid.  device_walk_mode returns 1 when no two segments' footprints can
-// overlap (luma CUs and transform blocks at least 8 samples, no sub-block
-// edges, 4:2:0 or 4:0:0): every cell is a component and the tile kernel scans
-// the grids; 2 when footprints may chain (the strip kernels run each band's
-// runs of cells in position order, which needs the luma CU list in decode
-// order along every row and column of its CU map); 0 when the host must build
+// cell grid.  device_walk_mode returns 1 when no segment can write samples
+// another of its pass uses (4:2:0 or 4:0:0, no transform edges beside the
+// sub-block grid of their CU): every cell is a component and the tile kernel
+// takes the cells the walk lists per tile, with the smaller regions when every
+// luma edge lies on the 8x8 grid (*grid8); 2 when segments may chain (the strip
+// kernels run each band's runs of cells in position order, which needs the luma
+// CU list in decode order along every row and column of its CU map); 0 when the host must build
 // the plan (CUs off the 4x4 grid, outside the picture or overlapping, CU lists
 // out of order, planes too large for the strip kernels, invalid input).
 int device_walk_mode(const h266_picture &pic, const h266_deblock_cu *cus, uint64_t n_cus,
                      const h266_deblock_cu *chroma_cus, uint64_t n_chroma, const h266_deblock_params &params,
-                     uint32_t cfi);
+                     uint32_t cfi, bool *grid8 = nullptr);
 // The CU lists travel to the device packed: per CU its first kCuHeadBytes
 // (position, size, QPs, flags, sub-block counts), and a CuTail (the 64-sample
 // TU map and TB split) only for CUs that have either; with motion by CU, a
@@ -239,8 +249,7 @@ struct DeviceWalkIn {  // device pointers
   h266_deblock_params params;
   uint32_t cfi;
   int w, h, cw, ch;      // luma and chroma plane sizes
-  uint32_t max_cu_dim;   // largest width or height of the CUs with edges inside them (4: none);
-                         // the walk launches offsets 0 .. max_cu_dim - 4 (step 4)
+  bool grid8;            // every luma edge on the 8x8 grid
   bool tile_lists;       // also list each tile's cells for the grid-mode tile kernel
   bool tiles_consume;    // the tile kernel (not the strip kernels) reads the grids: empty cells need no clearing
 };
@@ -249,13 +258,30 @@ struct DeviceWalkOut {
   EdgeSeg *grid[2][3];
   uint32_t slots[2][3], bands[2][3];
   uint32_t tiles_x, tiles_y;
+  bool grid8;
   uint32_t *tile_count;       // with DeviceWalkIn::tile_lists: cells per (tile, pass, plane)
-  uint32_t *tile_list[2][3];  // and their grid indices, kTileListY / kTileListC per tile
+  uint32_t *tile_list[2][3];  // and their grid indices, tile_list_cap() per tile
 };
 int launch_device_walk(cudaStream_t st, const DeviceWalkIn &in, uint8_t *scratch, DeviceWalkOut &out,
                        uint64_t *launches);
 int launch_deblock_tiles_grid(cudaStream_t st, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
                               int bit_depth, const DeviceWalkOut &g, uint64_t *launches);
+// Batched strip kernels: fill_strip_params(_grid) writes one picture's
+// parameters of both passes (strip_params_size() bytes each) and its CTA counts
+// and shared memory; the batch's totals (counts summed, shared memory the
+// largest) go to the launch, whose prefix tables select a CTA's picture.
+struct StripCounts {
+  uint32_t rows = 0, cols = 0;
+  size_t smem_rows = 0, smem_cols = 0;
+};
+size_t strip_params_size();
+void fill_strip_params(void *rows, void *cols, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
+                       int bit_depth, const StripSide &v, const StripSide &h, const uint32_t band_off[2][3],
+                       const uint32_t n_bands[2][3], StripCounts &c);
+int fill_strip_params_grid(void *rows, void *cols, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
+                           int bit_depth, const DeviceWalkOut &g, StripCounts &c);
+int launch_strips_batch(cudaStream_t st, const void *d_rows, const uint32_t *d_first_rows, const void *d_cols,
+                        const uint32_t *d_first_cols, int n, const StripCounts &c, uint64_t *launches);
 int launch_deblock_strips_grid(cudaStream_t st, const DPlane src[3], const DPlane dst[3], const uint16_t *lut,
                                int bit_depth, const DeviceWalkOut &g, uint64_t *launches);
 // Batched device walk: fill_walk_batch_item writes one picture's item
@@ -265,7 +291,7 @@ int launch_deblock_strips_grid(cudaStream_t st, const DPlane src[3], const DPlan
 // the CU maps and walk the edges; the grid-mode tile parameters of each
 // picture then go into a batched tile launch like any other.
 struct WalkBatchCounts {
-  uint32_t clear_ctas = 0, grid_ctas = 0, walk_ctas = 0, offsets = 0;  // offsets: the largest, over the batch
+  uint32_t clear_ctas = 0, grid_ctas = 0, walk_ctas = 0;
 };
 size_t walk_batch_item_size();
 void fill_walk_batch_item(void *out, const DeviceWalkIn &in, uint8_t *scratch, DeviceWalkOut &g, WalkBatchCounts &c);
