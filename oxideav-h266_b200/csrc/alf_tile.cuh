@@ -1,11 +1,26 @@
 // Device helpers shared by the chain's SAO / ALF / CC-ALF tile kernel
 // (sao_alf3.cu) and the encoder's luma ALF trial kernel (sao_alf2.cu).
 //
-// Packed coefficient words (AlfTablesDev::luma_packed / chroma_packed): per
-// tap three words -- the clip value in both 16-bit lanes, its negation in both
-// lanes, and the coefficient as a signed byte in bytes 0 and 3, so that
-// __dp2a_lo(s, f) weights the low lane of a packed pair of tap sums and
-// __dp2a_hi(s, f) the high lane.
+// Packed filters (AlfTablesDev::luma_packed / chroma_packed): two 16-bit clip
+// values c a word (2^14 as 2^14 - 1, the same for samples below 2^14), four
+// coefficients a word, and the accumulator start -sum(2 c f) of the offset form
+// below.  A thread's luma filter is 48 bytes, three 16-byte loads (lanes of a
+// warp read different entries, so each load costs its distinct lines; a word
+// per clip, coefficient and negated clip cost 24 loads from 144 bytes).
+// Expanded for use: c in both 16-bit lanes, and the coefficient as a signed
+// byte in bytes 0 and 3, so that dp2a.lo weights the low lane of a packed pair
+// of tap sums and dp2a.hi the high lane.
+//
+// Offset form of the clipped taps: clip(n - cur, -c, c) + c lies in [0, 2c] and
+// is max(min(n + (c - cur), 2c), 0), one instruction per pair of samples
+// (viaddmin with relu) where the plain form takes two, and two of them add
+// without a carry between the lanes, so the sum is an ordinary add and leaves
+// the ALU pipe (64 lanes a clock, the pass's bound) to the clips; dp2a runs on
+// the FMA pipe.  The 2c that every tap sum carries is in the accumulator
+// start.  c - cur is formed lane-wise by one 32-bit add from
+// 0x8000 - cur (no borrow), which leaves 0x8000 in each lane; the windows hold
+// samples + 0x8000 (kBias) to cancel it.  Samples of 2^14 and above, outside
+// any supported depth, would wrap: tiles that hold one take the plain form.
 #pragma once
 
 #include <initializer_list>
@@ -24,7 +39,7 @@ __device__ __forceinline__ int sgn(int v) { return (v > 0) - (v < 0); }
 // neighbour (the second is its negation), and the rectangle of samples whose
 // two neighbours lie inside the picture and the clip rectangle.  tlo / thi
 // hold the same offsets as a signed-byte table (bytes 0..3 of tlo, then thi)
-// indexed by the band index 0..3 (4 = no offset) or by 4 + sign + sign.
+// indexed by the band index 0..3 (4 = no offset) or by 2 - sign - sign.
 struct SaoLocal {
   int type, band, bd_shift;
   int off[4];   // band offset per band index 0..3 after the band position
@@ -61,9 +76,9 @@ __device__ __forceinline__ void sao_local(SaoLocal &s, const SaoCtbDev &p, int p
   if (p.type == 1) {
     s.tlo = b(p.off[0]) | b(p.off[1]) << 8 | b(p.off[2]) << 16 | b(p.off[3]) << 24;
     s.thi = 0;
-  } else {  // indexed by (sign + 2) + (sign + 2) = 2 + edgeIdx, so the table starts at byte 2
-    s.tlo = b(s.eo[0]) << 16 | b(s.eo[1]) << 24;
-    s.thi = b(s.eo[2]) | b(s.eo[3]) << 8 | b(s.eo[4]) << 16;
+  } else {  // indexed by (1 - sign) + (1 - sign): eo[] backwards
+    s.tlo = b(s.eo[4]) | b(s.eo[3]) << 8 | b(s.eo[2]) << 16 | b(s.eo[1]) << 24;
+    s.thi = b(s.eo[0]);
   }
 }
 
@@ -98,6 +113,45 @@ __device__ __forceinline__ uint32_t clipd(uint32_t n, uint32_t ncur, uint32_t c2
 }
 __device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) { return __viaddmax_s16x2(a, b, 0x80008000u); }
 __device__ __forceinline__ uint32_t neg2(uint32_t a) { return __viaddmax_s16x2(~a, 0x00010001u, 0x80008000u); }
+
+constexpr uint32_t kBias = 0x80008000u;  // the windows' samples are stored with 0x8000 added in each lane
+
+// clip(n - cur, -c, c) + c for both lanes: nb the biased pair, b = c - cur + 0x8000 per lane, c22 = 2c per lane
+__device__ __forceinline__ uint32_t clip_off(uint32_t nb, uint32_t b, uint32_t c22) {
+  return __viaddmin_s16x2_relu(nb, b, c22);
+}
+// acc + the low (high) lane of the unsigned pair s times the signed byte 0 (3) of f
+__device__ __forceinline__ int dp2a_ulo(uint32_t s, uint32_t f, int acc) {
+  int r;
+  asm("dp2a.lo.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(s), "r"(f), "r"(acc));
+  return r;
+}
+__device__ __forceinline__ int dp2a_uhi(uint32_t s, uint32_t f, int acc) {
+  int r;
+  asm("dp2a.hi.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(s), "r"(f), "r"(acc));
+  return r;
+}
+// Clip value k of packed words in both lanes; coefficient k of packed words in bytes 0 and 3.
+__device__ __forceinline__ uint32_t clip_of(const uint32_t *w, int k) {
+  return __byte_perm(w[k / 2], 0u, (k & 1) ? 0x3232 : 0x1010);
+}
+__device__ __forceinline__ uint32_t coef_of(const uint32_t *w, int k) {
+  return __byte_perm(w[k / 4], 0u, 0x0440u + 0x1001u * (k & 3));
+}
+// The expanded clips and coefficients of packed luma entry `e`; returns the accumulator start.
+__device__ __forceinline__ int luma_filter(const uint32_t *e, uint32_t c2[12], uint32_t f[12]) {
+  const uint4 *q = reinterpret_cast<const uint4 *>(e);
+  const uint4 a = __ldg(q), b = __ldg(q + 1), d = __ldg(q + 2);
+  const uint32_t w[10] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, d.x, d.y};
+#pragma unroll
+  for (int k = 0; k < 12; ++k) {
+    c2[k] = clip_of(w, k);
+    f[k] = coef_of(w + 6, k);
+  }
+  return (int)w[9];
+}
+// The clip value as the plain form takes it.
+__device__ __forceinline__ uint32_t plain_clip(uint32_t c2) { return c2 == 0x3FFF3FFFu ? 0x40004000u : c2; }
 
 template <int DX>
 __device__ __forceinline__ void luma_tap(const uint16_t *up, const uint16_t *dn, int c0, const uint32_t ncur[2],
@@ -147,32 +201,35 @@ __device__ __forceinline__ void classify(int sh, int sv, int sd0, int sd1, int a
   t_out = (uint8_t)((kTransposeTable >> ((dir1 * 2 + (dir2 >> 1)) * 2)) & 3);
 }
 
-// Laplacian sums per 2x2 cell of the luma window `sL` (unpadded rows):
-// cell (cx, cy) covers positions (X0 - 2 + 2cx + d, Y0 - 2 + 2cy + d), d = 0, 1.
+// Laplacian sums per 2x2 cell of the luma window `sL`: cell (cx, cy) covers
+// positions (X0 - 2 + 2cx + d, Y0 - 2 + 2cy + d), d = 0, 1.  The horizontal and
+// vertical sums share a word, the diagonal ones another: a sum is at most
+// 4 * (2^14 - 1) below 2^14 (a tile with larger samples classifies its blocks
+// from the window itself).
 template <class S, int NT>
-__device__ __forceinline__ void luma_cells(const uint16_t *sL, uint4 *cell) {
+__device__ __forceinline__ void luma_cells(const uint16_t *sL, uint2 *cell) {
   for (int i = threadIdx.x; i < S::CH * S::CW; i += NT) {
     const int cy = i / S::CW, cx = i - cy * S::CW;
-    uint4 g = make_uint4(0, 0, 0, 0);
+    uint32_t h = 0, v = 0, d0 = 0, d1 = 0;
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
       const int r = 2 * cy + d + 1;  // sL row of the position: y = Y0 - 2 + 2cy + d
       const int c = 2 * cx + d + 2;  // sL col: x = X0 - 2 + 2cx + d
       const uint16_t *row = &sL[r * S::SLP + c];
       const int c2 = 2 * row[0];
-      g.x += abs(c2 - row[-1] - row[1]);
-      g.y += abs(c2 - row[-S::SLP] - row[S::SLP]);
-      g.z += abs(c2 - row[-S::SLP - 1] - row[S::SLP + 1]);
-      g.w += abs(c2 - row[-S::SLP + 1] - row[S::SLP - 1]);
+      h += abs(c2 - row[-1] - row[1]);
+      v += abs(c2 - row[-S::SLP] - row[S::SLP]);
+      d0 += abs(c2 - row[-S::SLP - 1] - row[S::SLP + 1]);
+      d1 += abs(c2 - row[-S::SLP + 1] - row[S::SLP - 1]);
     }
-    cell[i] = g;
+    cell[i] = make_uint2(h + (v << 16), d0 + (d1 << 16));
   }
 }
 
 // Class and transposeIdx of every 4x4 block of a W x TH tile (src/alf.rs:750-1008).
 template <int W, int TH, class S, int NT>
-__device__ __forceinline__ void luma_classes(const uint16_t *sL, const uint4 *cell, uint8_t *cls_f, uint8_t *cls_t,
-                                             int Y0, int y_ctb, int ctb, int ph, int bd) {
+__device__ __forceinline__ void luma_classes(const uint16_t *sL, const uint2 *cell, uint8_t *cls_f, uint8_t *cls_t,
+                                             int Y0, int y_ctb, int ctb, int ph, int bd, bool big) {
   const bool bottom = y_ctb + ctb >= ph;
   const bool carve = !bottom || (ph - y_ctb) > ctb - 4;
   const int vb = y_ctb + ctb - 4;
@@ -180,7 +237,7 @@ __device__ __forceinline__ void luma_classes(const uint16_t *sL, const uint4 *ce
   for (int b = threadIdx.x; b < NB; b += NT) {
     const int bx = b % (W / 4), by = b / (W / 4);
     const int y4 = Y0 + 4 * by - y_ctb;
-    if (y4 == ctb - 8 || y4 == ctb - 4) {  // virtual-boundary rows: windows and padding differ
+    if (big || y4 == ctb - 8 || y4 == ctb - 4) {  // virtual-boundary rows: windows and padding differ
       int min_y = -2, max_y = 5, ac = 2;
       if (y4 == ctb - 8 && carve) { max_y = 3; ac = 3; }
       else if (y4 == ctb - 4 && carve) { min_y = 0; ac = 3; }
@@ -205,18 +262,30 @@ __device__ __forceinline__ void luma_classes(const uint16_t *sL, const uint4 *ce
       }
       classify(sh, sv, sd0, sd1, ac, bd, cls_f[b], cls_t[b]);
     } else {
-      uint4 s = make_uint4(0, 0, 0, 0);
+      uint32_t sh = 0, sv = 0, sd0 = 0, sd1 = 0;
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
+      for (int r = 0; r < 4; ++r) {
+        const uint2 *q = &cell[(2 * by + r) * S::CW + 2 * bx];
+        uint2 g[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint4 g = cell[(2 * by + r) * S::CW + 2 * bx + c];
-          s.x += g.x;
-          s.y += g.y;
-          s.z += g.z;
-          s.w += g.w;
+        for (int c = 0; c < 4; ++c) g[c] = q[c];
+        if (bd <= 12) {  // four cells of 4 * 4095 at most add within their halves
+          const uint32_t x = g[0].x + g[1].x + g[2].x + g[3].x, y = g[0].y + g[1].y + g[2].y + g[3].y;
+          sh += x & 0xFFFF;
+          sv += x >> 16;
+          sd0 += y & 0xFFFF;
+          sd1 += y >> 16;
+        } else {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            sh += g[c].x & 0xFFFF;
+            sv += g[c].x >> 16;
+            sd0 += g[c].y & 0xFFFF;
+            sd1 += g[c].y >> 16;
+          }
         }
-      classify((int)s.x, (int)s.y, (int)s.z, (int)s.w, 2, bd, cls_f[b], cls_t[b]);
+      }
+      classify((int)sh, (int)sv, (int)sd0, (int)sd1, 2, bd, cls_f[b], cls_t[b]);
     }
   }
 }

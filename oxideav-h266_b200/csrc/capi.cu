@@ -500,30 +500,39 @@ const int kTranspose[4][12] = {{0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11},
 bool build_packed(Pass2Host &h, int bd, uint32_t cfi, const h266_alf_aps_data *caps) {
   if (bd > 14 || (cfi != 0 && cfi != 1)) return false;
   auto in8 = [](int v) { return v >= -128 && v <= 127; };
+  // an entry of kLumaEntry words: two 16-bit clip values a word, four coefficient bytes a word, the accumulator start
+  auto put_tap = [](uint32_t *w, int clip_words, int k, int coef, int clip) {
+    const uint32_t c = (uint32_t)std::min(clip, 16383);  // 2^14 never binds below 2^14: doubled clips fit 15 bits
+    w[k / 2] |= c << (16 * (k & 1));
+    w[clip_words + k / 4] |= ((uint32_t)coef & 0xFF) << (8 * (k & 3));
+    return -2 * (int)c * coef;
+  };
   const size_t slots = h.luma_tab.size() / 600;
-  h.luma_packed.assign(slots * 100 * 36, 0);
+  h.luma_packed.assign(slots * 100 * kLumaEntry, 0);
   for (size_t s = 0; s < slots; ++s)
     for (int c = 0; c < 25; ++c)
-      for (int t = 0; t < 4; ++t)
+      for (int t = 0; t < 4; ++t) {
+        uint32_t *w = &h.luma_packed[((s * 100) + c * 4 + t) * kLumaEntry];
+        int start = 0;
         for (int k = 0; k < 12; ++k) {
           const int src = kTranspose[t][k];
-          const int coef = h.luma_tab[s * 600 + c * 12 + src], clip = h.luma_tab[s * 600 + 300 + c * 12 + src];
+          const int coef = h.luma_tab[s * 600 + c * 12 + src];
           if (!in8(coef)) return false;
-          uint32_t *w = &h.luma_packed[((s * 100) + c * 4 + t) * 36 + 3 * k];
-          w[0] = ((uint32_t)clip & 0xFFFF) | ((uint32_t)clip << 16);
-          w[1] = ((uint32_t)(-clip) & 0xFFFF) | ((uint32_t)(-clip) << 16);
-          w[2] = ((uint32_t)coef & 0xFF) | ((uint32_t)coef & 0xFF) << 24;  // dp2a_lo: low lane, dp2a_hi: high lane
+          start += put_tap(w, 6, k, coef, h.luma_tab[s * 600 + 300 + c * 12 + src]);
         }
-  if (caps)
-    for (uint32_t f = 0; f < caps->n_chroma_filters; ++f)
-      for (int k = 0; k < 6; ++k) {
-        const int coef = caps->chroma_coeff[f][k], clip = alf_clip_value(bd, caps->chroma_clip_idx[f][k]);
-        if (!in8(coef)) return false;
-        uint32_t *w = &h.args.tables.chroma_packed[f * 18 + 3 * k];
-        w[0] = ((uint32_t)clip & 0xFFFF) | ((uint32_t)clip << 16);
-        w[1] = ((uint32_t)(-clip) & 0xFFFF) | ((uint32_t)(-clip) << 16);
-        w[2] = ((uint32_t)coef & 0xFF) | ((uint32_t)coef & 0xFF) << 24;
+        w[9] = (uint32_t)start;
       }
+  if (caps)
+    for (uint32_t f = 0; f < caps->n_chroma_filters; ++f) {
+      uint32_t *w = h.args.tables.chroma_packed[f];
+      int start = 0;
+      for (int k = 0; k < 6; ++k) {
+        const int coef = caps->chroma_coeff[f][k];
+        if (!in8(coef)) return false;
+        start += put_tap(w, 3, k, coef, alf_clip_value(bd, caps->chroma_clip_idx[f][k]));
+      }
+      w[5] = (uint32_t)start;
+    }
   // CC-ALF taps are applied as signed-byte dp2a weights
   for (int c = 0; c < 2; ++c)
     for (int f = 0; f < 4; ++f)

@@ -327,6 +327,9 @@ struct CtbDev {      // everything pass 2 needs per CTB
 };
 static_assert(sizeof(CtbDev) == 52, "CtbDev layout");
 
+// Words of a packed luma filter: 6 of clip values, 3 of coefficients, the
+// accumulator start, padding to 16-byte loads.
+constexpr int kLumaEntry = 12;
 struct AlfTablesDev {
   // luma filter sets: slot -> [25 classes][12] coefficients and clip values
   const int32_t *luma_coeff;  // slot s at [s * 600, s * 600 + 300)
@@ -334,9 +337,9 @@ struct AlfTablesDev {
   int32_t chroma_coeff[8][6];
   int32_t chroma_clip[8][6];
   int32_t cc_coeff[2][4][7];  // [cb/cr][filter][tap]
-  // packed-arithmetic form (sao_alf2.cu): per tap three words (c|c<<16, -c|-c<<16, coeff & 0xff)
-  const uint32_t *luma_packed;  // [slot][class * 4 + transposeIdx][12 taps][3], taps pre-permuted
-  uint32_t chroma_packed[8 * 18];  // [alt][6 taps][3]
+  // packed-arithmetic form (alf_tile.cuh), taps pre-permuted
+  const uint32_t *luma_packed;   // [slot][class * 4 + transposeIdx][kLumaEntry]
+  uint32_t chroma_packed[8][8];  // [alt]: 3 words of clip values, 2 of coefficients, the accumulator start
 };
 
 struct Pass2Args {

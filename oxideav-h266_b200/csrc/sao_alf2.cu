@@ -27,7 +27,7 @@ struct TrialSmem {
   static constexpr int SLP = SLW;                         // its row pitch
   static constexpr int CW = W / 2 + 2, CH = TH / 2 + 2;  // 2x2 Laplacian cells
   alignas(16) uint16_t sL[SLH * SLW];
-  alignas(16) uint4 cell[CH * CW];
+  alignas(16) uint2 cell[CH * CW];
   uint8_t cls_f[(TH / 4) * (W / 4)], cls_t[(TH / 4) * (W / 4)];
   alignas(8) unsigned long long sse[kAlfMaxTrials + 1];
 };
@@ -56,19 +56,21 @@ __global__ void __launch_bounds__(NT, 2) k_alf_luma_trials(const __grid_constant
   const int rx0 = max((int)me.rect[0], 0), ry0 = max((int)me.rect[1], 0);
   const int rx1 = min((int)me.rect[2], pw), ry1 = min((int)me.rect[3], ph);
   const DPlane LS = a.src[0];
-  int wide = 0;  // a sample above 2^BitDepth - 1 (outside the picture format): clips may bind for every set
+  int wide = 0, big = 0;  // a sample above 2^BitDepth - 1 (outside the picture format): clips may bind for every set
   for (int i = tid; i < S::SLH * S::SLW; i += NT) {  // clamped into the fetch rectangle (sample(), src/alf.rs:1093-1110)
     const int r = i / S::SLW, c = i - r * S::SLW;
     const int ax = clampd(X0 - 4 + c, rx0, rx1 - 1), ay = clampd(Y0 - 3 + r, ry0, ry1 - 1);
     const uint16_t v = LS.s[(int64_t)ay * LS.stride + ax];
     wide |= v > maxv;
+    big |= v >= 1 << 14;
     sm.sL[i] = v;
   }
   if (tid <= trials) sm.sse[tid] = 0;
   wide = __syncthreads_or(wide);
+  big = __syncthreads_or(big);
   luma_cells<S, NT>(sm.sL, sm.cell);
   __syncthreads();
-  luma_classes<W, TH, S, NT>(sm.sL, sm.cell, sm.cls_f, sm.cls_t, Y0, y_ctb, ctb, ph, bd);
+  luma_classes<W, TH, S, NT>(sm.sL, sm.cell, sm.cls_f, sm.cls_t, Y0, y_ctb, ctb, ph, bd, big != 0);
   __syncthreads();
 
   constexpr int RUNS = TH * W / 4;
@@ -108,17 +110,18 @@ __global__ void __launch_bounds__(NT, 2) k_alf_luma_trials(const __grid_constant
       const int j = 4 * by + (tid % TPB) * RPT + rr;
       luma_sums(sm, j, bx, Y0 + j - y_ctb, ctb, sum[rr], cur[rr], shift[rr]);
     }
-    const uint32_t *tab0 = a.tables.luma_packed + (size_t)cls * 36 + 2;  // coefficient words of trial t at + t * 3600
-    uint32_t fn[12];  // the next trial's coefficients, loaded while the current trial runs
+    // coefficient words of trial t at + t * 100 * kLumaEntry
+    const uint32_t *tab0 = a.tables.luma_packed + (size_t)cls * kLumaEntry + 6;
+    uint32_t fn[3];  // the next trial's coefficients, loaded while the current trial runs
 #pragma unroll
-    for (int k = 0; k < 12; ++k) fn[k] = first > 0 ? __ldg(tab0 + 3 * k) : 0u;
+    for (int k = 0; k < 3; ++k) fn[k] = first > 0 ? __ldg(tab0 + k) : 0u;
     for (int t = 0; t < first; ++t) {
       uint32_t f[12];
 #pragma unroll
-      for (int k = 0; k < 12; ++k) f[k] = fn[k];
+      for (int k = 0; k < 12; ++k) f[k] = coef_of(fn, k);
       if (t + 1 < first) {
 #pragma unroll
-        for (int k = 0; k < 12; ++k) fn[k] = __ldg(tab0 + (size_t)(t + 1) * 3600 + 3 * k);
+        for (int k = 0; k < 3; ++k) fn[k] = __ldg(tab0 + (size_t)(t + 1) * 100 * kLumaEntry + k);
       }
       unsigned long long e = 0;
 #pragma unroll
@@ -149,13 +152,12 @@ __global__ void __launch_bounds__(NT, 2) k_alf_luma_trials(const __grid_constant
     }
   }
   for (int t = first; t < trials; ++t) {
-    const uint32_t *tab = a.tables.luma_packed + ((size_t)t * 100 + cls) * 36;
     uint32_t c2[12], nc2[12], f[12];
+    luma_filter(a.tables.luma_packed + ((size_t)t * 100 + cls) * kLumaEntry, c2, f);
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
-      c2[k] = __ldg(tab + 3 * k);
-      nc2[k] = __ldg(tab + 3 * k + 1);
-      f[k] = __ldg(tab + 3 * k + 2);
+      c2[k] = plain_clip(c2[k]);
+      nc2[k] = neg2(c2[k]);
     }
     unsigned long long e = 0;
 #pragma unroll

@@ -15,15 +15,21 @@
 //     read as 0 and are never used, as every read is clamped into the clip
 //     rectangle) while the CTA resolves the SAO parameters of the 3x3 CTB
 //     neighbourhood;
-//  2. post-SAO windows of all planes: inside the tile's own CTB and clip
-//     rectangle two samples per thread step in packed 16-bit lanes (sign
-//     terms by lane-wise clamps, offsets looked up from a signed-byte table
-//     with one byte permute), the rest sample by sample;
+//  2. post-SAO windows of all planes, four samples per thread step: inside the
+//     tile's own CTB and clip rectangle with one set of parameters, then the
+//     quads of neighbouring CTBs with theirs (branch-free, all types), then
+//     sample by sample only what is clamped or at the edge of the clip
+//     rectangle; signs are one relu clamp per neighbour, offsets come from a
+//     signed-byte table by one byte permute;
 //  3. luma Laplacian sums per 2x2 cell beside the chroma planes' 5x5 ALF and
 //     CC-ALF (a thread per 8 chroma samples of a row, CC-ALF taps as 6 dp2a);
 //  4. luma classes, one 4x4 block per thread;
 //  5. the 7x7 luma diamond, one block per thread with its 12 taps in
 //     registers and each of the 7 rows held as packed words.
+// The ALU pipe (64 lanes a clock: half the issue rate) bounds phases 2, 3 and
+// 5, so the taps are in the offset form of alf_tile.cuh.  16 1080p 10-bit
+// pictures: 389 us (472 with two clamps a tap, pairs instead of quads, border
+// samples one by one and word-per-value filter tables).
 #include <atomic>
 #include <type_traits>
 #include <utility>
@@ -43,6 +49,14 @@ constexpr uint64_t kWaitNs = 20000000;  // 20 ms: a tile gives up on its window 
 // left unfiltered); read and cleared by pass2_wait_timeouts.
 __device__ unsigned int g_wait_timeouts;
 
+// Packed SAO parameters of one CTB and component.
+struct alignas(16) SaoFast {
+  int type;          // 0 copy, 1 band, 2 edge
+  int row, shift_x;  // edge: the first neighbour's row offset in the window and column offset (-1, 0, 1)
+  uint32_t tlo, thi;  // signed-byte offset table
+  uint32_t shift, lane_mask, band_add;  // band: lane index ((c >> shift) - band) & 31
+};
+
 template <int W, int TH>
 struct Smem3 {
   static constexpr int DLW = W + 16, DLH = TH + 8;          // deblocked luma [X0-8, X1+8) x [Y0-4, Y1+4)
@@ -59,7 +73,7 @@ struct Smem3 {
   static constexpr int DC_OFF = (DL_BYTES + 127) & ~127;
   static constexpr int DC_STRIDE = (DC_BYTES + 127) & ~127;
   static constexpr int D_BYTES = DC_OFF + 2 * DC_STRIDE;
-  static constexpr int CELL_BYTES = CH * CW * 16;
+  static constexpr int CELL_BYTES = CH * CW * 8;
   static constexpr int U_BYTES = D_BYTES > CELL_BYTES ? D_BYTES : CELL_BYTES;
   // the deblocked windows (TMA destinations); the Laplacian cells reuse the
   // space once the post-SAO windows exist
@@ -68,11 +82,13 @@ struct Smem3 {
   alignas(16) uint16_t sC[2][SCH * SCP];
   uint8_t cls_f[(TH / 4) * (W / 4)], cls_t[(TH / 4) * (W / 4)];
   SaoLocal sao[3][9];
+  SaoFast fast[3][9];
   alignas(8) unsigned long long bar;
+  int big;  // some window sample is 2^14 or above
   unsigned any_sao;  // bit comp * 9 + n: neighbour n of the 3x3 CTB neighbourhood has SAO for comp
   __device__ uint16_t *dL() { return reinterpret_cast<uint16_t *>(u); }
   __device__ uint16_t *dC(int c) { return reinterpret_cast<uint16_t *>(u + DC_OFF + c * DC_STRIDE); }
-  __device__ uint4 *cell() { return reinterpret_cast<uint4 *>(u); }
+  __device__ uint2 *cell() { return reinterpret_cast<uint2 *>(u); }
 };
 
 // TMA and mbarrier helpers (tma.cuh); waits give up after kWaitNs.
@@ -91,7 +107,7 @@ __device__ __forceinline__ void static_for(F &&f) {
 // ---------------------------------------------------------------- packed helpers
 __device__ __forceinline__ uint32_t ld32(const uint16_t *p) { return *reinterpret_cast<const uint32_t *>(p); }
 __device__ __forceinline__ uint2 ld64(const uint16_t *p) { return *reinterpret_cast<const uint2 *>(p); }
-__device__ __forceinline__ void st32(uint16_t *p, uint32_t v) { *reinterpret_cast<uint32_t *>(p) = v; }
+__device__ __forceinline__ void st64(uint16_t *p, uint2 v) { *reinterpret_cast<uint2 *>(p) = v; }
 
 // Byte permute with sign replication (PTX prmt, default mode: selector bit 3
 // copies the sign bit of the selected byte).
@@ -101,32 +117,18 @@ __device__ __forceinline__ uint32_t prmt(uint32_t lo, uint32_t hi, uint32_t sel)
   return r;
 }
 
-// Selector that turns per-lane byte indices (0..7 in each 16-bit lane) into
-// the two lanes' sign-extended table bytes.
-__device__ __forceinline__ uint32_t lane_sel(uint32_t idx) {
-  const uint32_t t = (idx | (idx >> 8)) & 0x0707u;  // lane 0 index in bits 0-2, lane 1 in bits 8-10
-  return t | (t << 4) | 0x8080u;
+// Offsets of two samples from the signed-byte table, idx their indices (0..7
+// in each 16-bit lane): the indices in the selector's nibbles 0 and 2, the same
+// with the sign-copy bit in nibbles 1 and 3 (the permute reads the low 16 bits).
+__device__ __forceinline__ uint32_t lane_bytes(uint32_t tlo, uint32_t thi, uint32_t idx) {
+  return prmt(tlo, thi, (idx + (idx >> 8)) * 0x11u + 0x8080u);
 }
 
-// Pair (p[0], p[1]) at any sample offset (odd offsets from two aligned words).
-__device__ __forceinline__ uint32_t pair_any(const uint16_t *p, bool odd) {
-  return odd ? __byte_perm(ld32(p - 1), ld32(p + 1), 0x5432) : ld32(p);
-}
-
-// Per-component state of the packed SAO step: the tile's own CTB parameters.
-struct SaoFast {
-  int type;          // 0 copy, 1 band, 2 edge
-  int nb;            // neighbour offset in the window (edge)
-  bool nb_odd;
-  uint32_t tlo, thi;  // signed-byte offset table
-  uint32_t shift, lane_mask, band_add;  // band: lane index ((c >> shift) - band) & 31
-};
-
-__device__ __forceinline__ SaoFast sao_fast(const SaoLocal &p, bool on) {
+__device__ __forceinline__ SaoFast sao_fast(const SaoLocal &p, int pitch) {
   SaoFast f;
-  f.type = on ? p.type : 0;
-  f.nb = p.nb;
-  f.nb_odd = (p.nb & 1) != 0;
+  f.type = p.type;
+  f.row = p.type != 2 || p.nb >= -1 ? 0 : -pitch;
+  f.shift_x = p.type != 2 ? 0 : p.nb - f.row;
   f.tlo = p.tlo;
   f.thi = p.thi;
   f.shift = (uint32_t)p.bd_shift;
@@ -136,81 +138,109 @@ __device__ __forceinline__ SaoFast sao_fast(const SaoLocal &p, bool on) {
   return f;
 }
 
-// SAO of the pair at d (window pointer; both samples inside the CTB, the clip
-// rectangle and the edge-offset availability rectangle), samples below 2^12.
-__device__ __forceinline__ uint32_t sao_pair(const SaoFast &f, const uint16_t *d, uint32_t maxv2) {
-  const uint32_t c = ld32(d);
-  if (f.type == 0) return c;
-  uint32_t off;
-  if (f.type == 2) {
-    const uint32_t a = pair_any(d + f.nb, f.nb_odd), b = pair_any(d - f.nb, f.nb_odd);
-    const uint32_t cb = c | 0x80008000u;
-    // lane-wise sign(c - n) + 2 in [1, 3]; the two add to 2 + sign + sign + 2
-    const uint32_t sa =
-        __viaddmin_s16x2(__viaddmax_s16x2((cb - a) ^ 0x80008000u, 0x00020002u, 0x00010001u), 0u, 0x00030003u);
-    const uint32_t sb =
-        __viaddmin_s16x2(__viaddmax_s16x2((cb - b) ^ 0x80008000u, 0x00020002u, 0x00010001u), 0u, 0x00030003u);
-    off = prmt(f.tlo, f.thi, lane_sel(sa + sb));
-  } else {
-    const uint32_t k = (((c >> f.shift) & f.lane_mask) + f.band_add) & 0x001F001Fu;
-    off = prmt(f.tlo, f.thi, lane_sel(__viaddmin_u16x2(k, 0u, 0x00040004u)));
-  }
-  return __viaddmin_s16x2(__viaddmax_s16x2(c, off, 0u), 0u, maxv2);
+// The same of any CTB and type, without branches, for lanes with parameters of
+// their own (the copy type's table is all zero and its row and column offsets
+// 0): both indices are formed and the type picks one.
+__device__ __forceinline__ uint2 sao_quad_any(const SaoFast &f, const uint16_t *d, uint32_t maxv2) {
+  const uint2 c = ld64(d);
+  const bool left = f.shift_x < 0, right = f.shift_x > 0;
+  const uint32_t sel = f.shift_x ? 0x5432u : 0x3210u;
+  // samples x + h .. x + h + 3: each pair from two neighbouring words
+  const uint16_t *ra = d + f.row, *rb = d - f.row;
+  const uint2 wa = ld64(ra), wb = ld64(rb);
+  const uint32_t xa = ld32(left ? ra - 2 : ra + 4), xb = ld32(left ? rb + 4 : rb - 2);
+  const uint32_t a0 = __byte_perm(left ? xa : wa.x, left ? wa.x : wa.y, sel);
+  const uint32_t a1 = __byte_perm(left ? wa.x : wa.y, left ? wa.y : xa, sel);
+  const uint32_t b0 = __byte_perm(right ? xb : wb.x, right ? wb.x : wb.y, sel);
+  const uint32_t b1 = __byte_perm(right ? wb.x : wb.y, right ? wb.y : xb, sel);
+  const uint32_t n0 = __viaddmax_s16x2(~c.x, 0x00020002u, 0x80008000u);  // 1 - c
+  const uint32_t n1 = __viaddmax_s16x2(~c.y, 0x00020002u, 0x80008000u);
+  const uint32_t e0 = __viaddmin_s16x2_relu(a0, n0, 0x00020002u) + __viaddmin_s16x2_relu(b0, n0, 0x00020002u);
+  const uint32_t e1 = __viaddmin_s16x2_relu(a1, n1, 0x00020002u) + __viaddmin_s16x2_relu(b1, n1, 0x00020002u);
+  const uint32_t k0 = __viaddmin_u16x2((((c.x >> f.shift) & f.lane_mask) + f.band_add) & 0x001F001Fu, 0u, 0x00040004u);
+  const uint32_t k1 = __viaddmin_u16x2((((c.y >> f.shift) & f.lane_mask) + f.band_add) & 0x001F001Fu, 0u, 0x00040004u);
+  const uint32_t v0 = __viaddmin_s16x2_relu(c.x, lane_bytes(f.tlo, f.thi, f.type == 2 ? e0 : k0), maxv2);
+  const uint32_t v1 = __viaddmin_s16x2_relu(c.y, lane_bytes(f.tlo, f.thi, f.type == 2 ? e1 : k1), maxv2);
+  return f.type ? make_uint2(v0, v1) : c;
 }
 
-// A rectangle of window positions: [x0, x0 + 2 * npx) x [y0, y0 + ny) in
-// pairs (fast) or the remaining window samples around it (slow).
+// Samples (x + h .. x + h + 3) of the row at r = &row[x] (8-byte aligned), h in -1, 0, 1.
+__device__ __forceinline__ uint2 quad_shifted(const uint16_t *r, int h) {
+  const uint2 w = ld64(r);
+  if (h == 0) return w;
+  if (h < 0) return make_uint2(__byte_perm(ld32(r - 2), w.x, 0x5432), __byte_perm(w.x, w.y, 0x5432));
+  return make_uint2(__byte_perm(w.x, w.y, 0x5432), __byte_perm(w.y, ld32(r + 4), 0x5432));
+}
+
+// SAO of the 4 samples at d (8-byte aligned window pointer; all inside one CTB,
+// the clip rectangle and the CTB's edge-offset availability rectangle), samples
+// below 2^12.
+__device__ __forceinline__ uint2 sao_quad(const SaoFast &f, const uint16_t *d, uint32_t maxv2) {
+  const uint2 c = ld64(d);
+  if (f.type == 0) return c;
+  uint32_t o0, o1;
+  if (f.type == 2) {
+    const uint2 a = quad_shifted(d + f.row, f.shift_x), b = quad_shifted(d - f.row, -f.shift_x);
+    // lane-wise 1 - sign(c - n) = clip(n - c + 1, 0, 2); the two add to the table index
+    const uint32_t n0 = __viaddmax_s16x2(~c.x, 0x00020002u, 0x80008000u);  // 1 - c
+    const uint32_t n1 = __viaddmax_s16x2(~c.y, 0x00020002u, 0x80008000u);
+    o0 = __viaddmin_s16x2_relu(a.x, n0, 0x00020002u) + __viaddmin_s16x2_relu(b.x, n0, 0x00020002u);
+    o1 = __viaddmin_s16x2_relu(a.y, n1, 0x00020002u) + __viaddmin_s16x2_relu(b.y, n1, 0x00020002u);
+  } else {
+    const uint32_t k0 = (((c.x >> f.shift) & f.lane_mask) + f.band_add) & 0x001F001Fu;
+    const uint32_t k1 = (((c.y >> f.shift) & f.lane_mask) + f.band_add) & 0x001F001Fu;
+    o0 = __viaddmin_u16x2(k0, 0u, 0x00040004u);
+    o1 = __viaddmin_u16x2(k1, 0u, 0x00040004u);
+  }
+  return make_uint2(__viaddmin_s16x2_relu(c.x, lane_bytes(f.tlo, f.thi, o0), maxv2),
+                    __viaddmin_s16x2_relu(c.y, lane_bytes(f.tlo, f.thi, o1), maxv2));
+}
+
+// A rectangle of window quads: columns [x0, x0 + 4 * nq), rows [y0, y0 + ny) of
+// component samples, x0 a multiple of 4.
 struct FastRect {
-  int x0, y0, npx, ny;
-  uint32_t magic;  // floor(i / npx) = umulhi(i, magic) for the indices used (npx > 1)
-  __device__ int row_of(uint32_t i) const { return npx == 1 ? (int)i : (int)__umulhi(i, magic); }
-  __device__ int pairs() const { return npx * ny; }
+  int x0, y0, nq, ny;
+  uint32_t magic;  // floor(i / nq) = umulhi(i, magic) for the indices used (nq > 1)
+  __device__ int row_of(uint32_t i) const { return nq == 1 ? (int)i : (int)__umulhi(i, magic); }
+  __device__ int quads() const { return nq * ny; }
 };
 
 __device__ __forceinline__ FastRect fast_rect(int x0, int x1, int y0, int y1) {
   FastRect r;
-  x0 = (x0 + 1) & ~1;
-  x1 &= ~1;
+  x0 = (x0 + 3) & ~3;
+  x1 &= ~3;
   r.x0 = x0;
   r.y0 = y0;
-  r.npx = x1 > x0 ? (x1 - x0) / 2 : 0;
+  r.nq = x1 > x0 ? (x1 - x0) / 4 : 0;
   r.ny = y1 > y0 ? y1 - y0 : 0;
-  if (!r.npx || !r.ny) r.npx = r.ny = 0;
-  r.magic = r.npx > 1 ? 0xFFFFFFFFu / (uint32_t)r.npx + 1u : 0u;  // 2^32 / 1 does not fit: row_of
+  if (!r.nq || !r.ny) r.nq = r.ny = 0;
+  r.magic = r.nq > 1 ? 0xFFFFFFFFu / (uint32_t)r.nq + 1u : 0u;  // 2^32 / 1 does not fit: row_of
   return r;
 }
 
-// The i-th window sample outside the fast rectangle of a WW x WH window whose
-// origin is (wx0, wy0): rows above, rows below, then the left and right parts
-// of the fast rows.
-__device__ __forceinline__ void slow_pos(int i, int wx0, int wy0, int WW, int WH, const FastRect &f, int &x, int &y) {
+// The i-th window quad outside the fast rectangle of a window WQ quads wide and
+// WH rows high whose origin is (wx0, wy0): rows above, rows below, then the left
+// and right parts of the fast rows.
+__device__ __forceinline__ void rest_pos(int i, int wx0, int wy0, int WQ, int WH, const FastRect &f, int &x, int &y) {
   const int fy0 = f.ny ? f.y0 : wy0, fy1 = f.ny ? f.y0 + f.ny : wy0;
-  const int n_top = WW * (fy0 - wy0), n_bot = WW * (wy0 + WH - fy1);
-  if (i < n_top) {
-    y = wy0 + i / WW;
-    x = wx0 + i % WW;
+  const int n_top = WQ * (fy0 - wy0), n_bot = WQ * (wy0 + WH - fy1);
+  if (i < n_top + n_bot) {
+    const int r = i / WQ;
+    x = wx0 + 4 * (i - r * WQ);
+    y = i < n_top ? wy0 + r : fy1 + r - (fy0 - wy0);
     return;
   }
-  i -= n_top;
-  if (i < n_bot) {
-    y = fy1 + i / WW;
-    x = wx0 + i % WW;
-    return;
-  }
-  i -= n_bot;
-  const int lw = f.x0 - wx0, n_left = lw * f.ny;
-  if (i < n_left) {
-    y = fy0 + i / lw;
-    x = wx0 + i % lw;
-    return;
-  }
-  i -= n_left;
-  const int rw = wx0 + WW - (f.x0 + 2 * f.npx);
-  y = fy0 + i / rw;
-  x = f.x0 + 2 * f.npx + i % rw;
+  i -= n_top + n_bot;
+  const int lq = (f.x0 - wx0) / 4, rq = WQ - lq - f.nq, sq = lq + rq;  // seldom more than one each
+  int r, c;
+  if (sq == 1) { r = i; c = 0; }
+  else if (sq == 2) { r = i >> 1; c = i & 1; }
+  else { r = i / sq; c = i - r * sq; }
+  y = fy0 + r;
+  x = wx0 + 4 * (c < lq ? c : c + f.nq);
 }
 
-__device__ __forceinline__ int slow_count(int WW, int WH, const FastRect &f) { return WW * WH - 2 * f.pairs(); }
+__device__ __forceinline__ int rest_count(int WQ, int WH, const FastRect &f) { return WQ * WH - f.quads(); }
 
 // Rows of packed words around a run of samples: word k covers samples
 // (c0 - 2B + 2k, c0 - 2B + 2k + 1) of the row at p = &row[c0].
@@ -244,6 +274,62 @@ __device__ __forceinline__ void load_words(Words<NW, B> &r, const uint16_t *p, i
     } else {
       r.w[k] = ld32(q + 2 * k);
     }
+  }
+}
+
+// The plain form of the clipped taps for tiles that hold a sample of 2^14 or
+// above, tap by tap (out of line: no picture of a supported depth has any).
+__device__ __forceinline__ uint32_t pair_plain(const uint16_t *p) {
+  return ((uint32_t)p[0] | (uint32_t)p[1] << 16) ^ kBias;
+}
+__device__ __forceinline__ void tap_plain(const uint16_t *up, const uint16_t *dn, uint32_t ncur, uint32_t c2,
+                                          uint32_t f, int acc[2]) {
+  const uint32_t nc2 = neg2(c2);
+  const uint32_t s = add2(clipd(pair_plain(up), ncur, c2, nc2), clipd(pair_plain(dn), ncur, c2, nc2));
+  acc[0] = __dp2a_lo((int)s, (int)f, acc[0]);
+  acc[1] = __dp2a_hi((int)s, (int)f, acc[1]);
+}
+// taps (dx, dy) of the 7x7 and 5x5 diamonds in table order, mirrored taps at (-dx, -dy)
+__constant__ int8_t kLumaTaps[12][2] = {{0, 3}, {1, 2}, {0, 2}, {-1, 2}, {2, 1}, {1, 1},
+                                        {0, 1}, {-1, 1}, {-2, 1}, {3, 0}, {2, 0}, {1, 0}};
+__constant__ int8_t kChromaTaps[6][2] = {{0, 2}, {1, 1}, {0, 1}, {-1, 1}, {2, 0}, {1, 0}};
+
+__device__ __noinline__ void luma_run_plain(const uint16_t *R0, int pitch, int y1, int y2, int y3, int shift,
+                                            const uint32_t *tab, int maxv, int out[4]) {
+  const int ys[4] = {0, y1, y2, y3};
+#pragma unroll 1
+  for (int q = 0; q < 2; ++q) {
+    const uint16_t *R = R0 + 2 * q;
+    const uint32_t cur = pair_plain(R), ncur = neg2(cur);
+    int acc[2] = {0, 0};
+#pragma unroll 1
+    for (int k = 0; k < 12; ++k) {
+      const int o = ys[kLumaTaps[k][1]] * pitch + kLumaTaps[k][0];
+      tap_plain(R + o, R - o, ncur, plain_clip(clip_of(tab, k)), coef_of(tab + 6, k), acc);
+    }
+    const int round = 1 << (shift - 1);
+    out[2 * q] = clampd((int)(cur & 0xFFFF) + ((acc[0] + round) >> shift), 0, maxv);
+    out[2 * q + 1] = clampd((int)(cur >> 16) + ((acc[1] + round) >> shift), 0, maxv);
+  }
+}
+
+template <int SPT>
+__device__ __noinline__ void chroma_run_plain(const uint16_t *R0, int pitch, int y1, int y2, int shift,
+                                              const uint32_t *ct, int maxv, int v[SPT]) {
+  const int ys[3] = {0, y1, y2};
+#pragma unroll 1
+  for (int q = 0; q < SPT / 2; ++q) {
+    const uint16_t *R = R0 + 2 * q;
+    const uint32_t cur = pair_plain(R), ncur = neg2(cur);
+    int acc[2] = {0, 0};
+#pragma unroll 1
+    for (int k = 0; k < 6; ++k) {
+      const int o = ys[kChromaTaps[k][1]] * pitch + kChromaTaps[k][0];
+      tap_plain(R + o, R - o, ncur, plain_clip(clip_of(ct, k)), coef_of(ct + 3, k), acc);
+    }
+    const int round = 1 << (shift - 1);
+    v[2 * q] = clampd((int)(cur & 0xFFFF) + ((acc[0] + round) >> shift), 0, maxv);
+    v[2 * q + 1] = clampd((int)(cur >> 16) + ((acc[1] + round) >> shift), 0, maxv);
   }
 }
 
@@ -307,6 +393,7 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
     for (int c = 0; c < 2; ++c)
       if (chroma_on[c]) tma_load_2d(sm.dC(c), &maps->tmap[1 + c], xc0 - 8, yc0 - 3, &sm.bar);
   }
+  if (tid == 32) sm.big = 0;
   int my_type = 0;
   if (tid < 27) {
     const int comp = tid / 9, n = tid % 9;
@@ -332,6 +419,7 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
       sao_local(s, c.sao[comp], comp ? S::DCW : S::DLW, q0, q1, q2, q3, bd);
       my_type = s.type;
     }
+    sm.fast[comp][n] = sao_fast(s, comp ? S::DCW : S::DLW);
   }
   if (tid < 32) {
     const unsigned m = __ballot_sync(0xFFFFFFFFu, my_type != 0);
@@ -407,61 +495,87 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
     phase ^= 1u;
   }
 
-  // ---- (2) post-SAO windows, clamped into the fetch rectangle
-  const SaoFast fs[3] = {sao_fast(sm.sao[0][4], sao_on[0]), sao_fast(sm.sao[1][4], sao_on[1]),
-                         sao_fast(sm.sao[2][4], sao_on[2])};
+  // ---- (2) post-SAO windows (biased), clamped into the fetch rectangle, 4 samples per step
+  uint32_t seen = 0;  // every sample or'ed together
   {
-    const int nf0 = fr[0].pairs(), nf1 = chroma_on[0] ? fr[1].pairs() : 0, nf2 = chroma_on[1] ? fr[2].pairs() : 0;
+    constexpr int WQL = S::SLW / 4, WQC = S::SCW / 4;
     const uint16_t *dL = sm.dL();
-    for (int i = tid; i < nf0 + nf1 + nf2; i += NT3) {
-      if (i < nf0) {
-        const FastRect &f = fr[0];
-        const int r = f.row_of((uint32_t)i), x = f.x0 + 2 * (i - r * f.npx), y = f.y0 + r;
-        const uint16_t *d = dL + (y - (Y0 - 4)) * S::DLW + (x - (X0 - 8));
-        st32(&sm.sL[(y - (Y0 - 3)) * S::SLP + (x - (X0 - 4))], sao_pair(fs[0], d, maxv2));
-      } else {
-        const int cc = i < nf0 + nf1 ? 0 : 1;
-        const int j = i - nf0 - (cc ? nf1 : 0);
-        const FastRect &f = fr[1 + cc];
-        const int r = f.row_of((uint32_t)j), x = f.x0 + 2 * (j - r * f.npx), y = f.y0 + r;
-        const uint16_t *d = sm.dC(cc) + (y - (yc0 - 3)) * S::DCW + (x - (xc0 - 8));
-        st32(&sm.sC[cc][(y - (yc0 - 2)) * S::SCP + (x - (xc0 - 4))], sao_pair(fs[1 + cc], d, maxv2));
+    auto put = [&](uint16_t *w, uint2 v) {
+      seen |= v.x | v.y;
+      st64(w, make_uint2(v.x ^ kBias, v.y ^ kBias));
+    };
+    {  // the tile's own CTB inside the clip rectangle: one set of parameters
+      const SaoFast f = sm.fast[0][4];
+      const FastRect q = fr[0];
+      for (int i = tid; i < q.quads(); i += NT3) {
+        const int r = q.row_of((uint32_t)i), x = q.x0 + 4 * (i - r * q.nq), y = q.y0 + r;
+        put(&sm.sL[(y - (Y0 - 3)) * S::SLP + (x - (X0 - 4))],
+            sao_quad(f, dL + (y - (Y0 - 4)) * S::DLW + (x - (X0 - 8)), maxv2));
       }
     }
-    // the rest sample by sample: neighbouring CTBs, clamped positions, edges of the clip rectangle
-    const int ns0 = slow_count(S::SLW, S::SLH, fr[0]);
-    const int ns1 = chroma_on[0] ? slow_count(S::SCW, S::SCH, fr[1]) : 0;
-    const int ns2 = chroma_on[1] ? slow_count(S::SCW, S::SCH, fr[2]) : 0;
-    for (int i = tid; i < ns0 + ns1 + ns2; i += NT3) {
-      int x, y;
-      if (i < ns0) {
-        slow_pos(i, X0 - 4, Y0 - 3, S::SLW, S::SLH, fr[0], x, y);
-        const int ax = clampd(x, rx0, rx1 - 1), ay = clampd(y, ry0, ry1 - 1);
-        const uint16_t *d = &dL[(ay - (Y0 - 4)) * S::DLW + ax - (X0 - 8)];
-        int v = *d;
-        if (sao_on[0]) {
-          const SaoLocal &p = sm.sao[0][((ay >> log2) - ry + 1) * 3 + ((ax >> log2) - rx + 1)];
-          if (p.type) v = sao_one(p, ax, ay, maxv, d);
-        }
-        sm.sL[(y - (Y0 - 3)) * S::SLP + (x - (X0 - 4))] = (uint16_t)v;
-      } else {
-        const int cc = i < ns0 + ns1 ? 0 : 1;
-        const int j = i - ns0 - (cc ? ns1 : 0);
-        slow_pos(j, xc0 - 4, yc0 - 2, S::SCW, S::SCH, fr[1 + cc], x, y);
-        const DPlane &CS = a.src[cc + 1];
-        const int cx0 = max(crx0, 0), cy0 = max(cry0, 0), cx1 = min(crx1, CS.w), cy1 = min(cry1, CS.h);
-        const int ax = clampd(x, cx0, cx1 - 1), ay = clampd(y, cy0, cy1 - 1);
-        const uint16_t *d = sm.dC(cc) + (ay - (yc0 - 3)) * S::DCW + ax - (xc0 - 8);
-        int v = *d;
-        if (sao_on[1 + cc]) {
-          const SaoLocal &p = sm.sao[cc + 1][(((ay * 2) >> log2) - ry + 1) * 3 + (((ax * 2) >> log2) - rx + 1)];
-          if (p.type) v = sao_one(p, ax, ay, maxv, d);
-        }
-        sm.sC[cc][(y - (yc0 - 2)) * S::SCP + (x - (xc0 - 4))] = (uint16_t)v;
+    {
+      const int nc0 = chroma_on[0] ? fr[1].quads() : 0, nc1 = chroma_on[1] ? fr[2].quads() : 0;
+      for (int i = tid; i < nc0 + nc1; i += NT3) {
+        const int cc = i < nc0 ? 0 : 1, j = i - (cc ? nc0 : 0);
+        const FastRect &q = fr[1 + cc];
+        const SaoFast f = sm.fast[1 + cc][4];
+        const int r = q.row_of((uint32_t)j), x = q.x0 + 4 * (j - r * q.nq), y = q.y0 + r;
+        put(&sm.sC[cc][(y - (yc0 - 2)) * S::SCP + (x - (xc0 - 4))],
+            sao_quad(f, sm.dC(cc) + (y - (yc0 - 3)) * S::DCW + (x - (xc0 - 8)), maxv2));
       }
+    }
+    // the rest: quads of neighbouring CTBs with their parameters, and sample by
+    // sample what is clamped or at the edges of the clip rectangle
+    const int ns0 = rest_count(WQL, S::SLH, fr[0]);
+    const int ns1 = chroma_on[0] ? rest_count(WQC, S::SCH, fr[1]) : 0;
+    const int ns2 = chroma_on[1] ? rest_count(WQC, S::SCH, fr[2]) : 0;
+    for (int i = tid; i < ns0 + ns1 + ns2; i += NT3) {
+      const int comp = i < ns0 ? 0 : (i < ns0 + ns1 ? 1 : 2), cc = comp ? comp - 1 : 0;
+      const int j = i - (comp ? ns0 + (comp == 2 ? ns1 : 0) : 0);
+      const int ox = comp ? xc0 - 4 : X0 - 4, oy = comp ? yc0 - 2 : Y0 - 3;  // the window's origin
+      int x, y;
+      if (comp) rest_pos(j, ox, oy, WQC, S::SCH, fr[comp], x, y);
+      else rest_pos(j, ox, oy, WQL, S::SLH, fr[0], x, y);
+      // the component's fetch rectangle
+      const int fx0 = comp ? max(crx0, 0) : rx0, fy0 = comp ? max(cry0, 0) : ry0;
+      const int fx1 = comp ? min(crx1, a.src[comp].w) : rx1, fy1 = comp ? min(cry1, a.src[comp].h) : ry1;
+      const int clog = comp ? log2 - 1 : log2;
+      const int pitch = comp ? S::DCW : S::DLW;
+      const uint16_t *D = comp ? sm.dC(cc) : dL;
+      const int dx0 = comp ? xc0 - 8 : X0 - 8, dy0 = comp ? yc0 - 3 : Y0 - 4;
+      const bool on = sao_on[comp];
+      uint2 v;
+      int n = 4;  // of the 3x3 neighbourhood, the CTB that holds the quad
+      bool fast = x >= fx0 && x + 4 <= fx1 && y >= fy0 && y < fy1;
+      if (fast && on) {
+        n = ((y >> clog) - ry + 1) * 3 + ((x >> clog) - rx + 1);
+        const SaoLocal &p = sm.sao[comp][n];
+        fast = fast_ok[comp] && (p.type != 2 || (x >= p.ex0 && x + 4 <= p.ex1 && y >= p.ey0 && y < p.ey1));
+      }
+      if (fast) {
+        v = sao_quad_any(sm.fast[comp][n], D + (y - dy0) * pitch + (x - dx0), maxv2);
+      } else {
+        const int ay = clampd(y, fy0, fy1 - 1);
+        uint32_t s4[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int ax = clampd(x + k, fx0, fx1 - 1);
+          const uint16_t *d = D + (ay - dy0) * pitch + (ax - dx0);
+          s4[k] = *d;
+          if (on) {
+            const SaoLocal &p = sm.sao[comp][((ay >> clog) - ry + 1) * 3 + ((ax >> clog) - rx + 1)];
+            if (p.type) s4[k] = (uint16_t)sao_one(p, ax, ay, maxv, d);
+          }
+        }
+        v = make_uint2(s4[0] | s4[1] << 16, s4[2] | s4[3] << 16);
+      }
+      uint16_t *w = comp ? &sm.sC[cc][(y - oy) * S::SCP + (x - ox)] : &sm.sL[(y - oy) * S::SLP + (x - ox)];
+      put(w, v);
     }
   }
+  if (DO_ALF && (seen & 0xC000C000u)) sm.big = 1;
   __syncthreads();
+  const bool big = DO_ALF && sm.big != 0;
 
   // ---- (3) luma Laplacian sums per 2x2 cell (into the dead deblocked windows); chroma ALF / CC-ALF
   const bool luma_alf = DO_ALF && me && me->luma_set >= 0;
@@ -487,7 +601,7 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
         load_words<NP + 2, 1, (NP > 1)>(w0, R0, 1, NP + 1);
 #pragma unroll
         for (int q = 0; q < NP; ++q) {
-          const uint32_t cur = w0.w[1 + q];
+          const uint32_t cur = w0.w[1 + q] ^ kBias;
           v[2 * q] = (int)(cur & 0xFFFF);
           v[2 * q + 1] = (int)(cur >> 16);
         }
@@ -497,50 +611,54 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
         int s2 = 7, y1 = 1, y2 = 2;
         if (jr == ctb_c - 2 || jr == ctb_c - 3) { s2 = 10; y1 = y2 = 0; }
         else if (jr == ctb_c - 1 || jr == ctb_c - 4) { y2 = 1; }
-        const uint32_t *ct = a.tables.chroma_packed + min(cf, 7) * 18;
-        uint32_t c2[6], nc2[6], f[6];
+        const uint32_t *ct = a.tables.chroma_packed[min(cf, 7)];
+        if (big) {
+          chroma_run_plain<SPT>(R0, S::SCP, y1, y2, s2, ct, maxv, v);
+        } else {
+          uint32_t c2[6], f[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          c2[k] = ct[3 * k];
-          nc2[k] = ct[3 * k + 1];
-          f[k] = ct[3 * k + 2];
+          for (int k = 0; k < 6; ++k) {
+            c2[k] = clip_of(ct, k);
+            f[k] = coef_of(ct + 3, k);
+          }
+          const int start = (int)ct[5] + (1 << (s2 - 1));
+          int acc[SPT];
+#pragma unroll
+          for (int k = 0; k < SPT; ++k) acc[k] = start;
+          uint32_t m[NP];  // 0x8000 - cur per lane
+          Words<NP + 2, 1> r0, ra, rb;
+          load_words<NP + 2, 1, (NP > 1)>(r0, R0, 0, NP + 2);
+#pragma unroll
+          for (int q = 0; q < NP; ++q) m[q] = kBias - (r0.w[1 + q] ^ kBias);
+          auto tap = [&](const Words<NP + 2, 1> &up, const Words<NP + 2, 1> &dn, auto dx, int k) {
+            constexpr int DX = decltype(dx)::value;
+            const uint32_t c22 = c2[k] + c2[k];
+            static_for<NP>([&](auto qc) {
+              constexpr int q = decltype(qc)::value;
+              const uint32_t b = c2[k] + m[q];
+              const uint32_t s = clip_off(up.template pair<DX + 2 * q>(), b, c22) +
+                                 clip_off(dn.template pair<-DX + 2 * q>(), b, c22);
+              acc[2 * q] = dp2a_ulo(s, f[k], acc[2 * q]);
+              acc[2 * q + 1] = dp2a_uhi(s, f[k], acc[2 * q + 1]);
+            });
+          };
+          using I0 = std::integral_constant<int, 0>;
+          using I1 = std::integral_constant<int, 1>;
+          using Im1 = std::integral_constant<int, -1>;
+          using I2 = std::integral_constant<int, 2>;
+          load_words<NP + 2, 1, (NP > 1)>(ra, R0 + y2 * S::SCP, 1, NP + 1);
+          load_words<NP + 2, 1, (NP > 1)>(rb, R0 - y2 * S::SCP, 1, NP + 1);
+          tap(ra, rb, I0{}, 0);
+          load_words<NP + 2, 1, (NP > 1)>(ra, R0 + y1 * S::SCP, 0, NP + 2);
+          load_words<NP + 2, 1, (NP > 1)>(rb, R0 - y1 * S::SCP, 0, NP + 2);
+          tap(ra, rb, I1{}, 1);
+          tap(ra, rb, I0{}, 2);
+          tap(ra, rb, Im1{}, 3);
+          tap(r0, r0, I2{}, 4);
+          tap(r0, r0, I1{}, 5);
+#pragma unroll
+          for (int k = 0; k < SPT; ++k) v[k] = clampd(v[k] + (acc[k] >> s2), 0, maxv);
         }
-        int acc[SPT];
-#pragma unroll
-        for (int k = 0; k < SPT; ++k) acc[k] = 0;
-        uint32_t ncur[NP];
-        Words<NP + 2, 1> r0, ra, rb;
-        load_words<NP + 2, 1, (NP > 1)>(r0, R0, 0, NP + 2);
-#pragma unroll
-        for (int q = 0; q < NP; ++q) ncur[q] = neg2(r0.w[1 + q]);
-        auto tap = [&](const Words<NP + 2, 1> &up, const Words<NP + 2, 1> &dn, auto dx, int k) {
-          constexpr int DX = decltype(dx)::value;
-          static_for<NP>([&](auto qc) {
-            constexpr int q = decltype(qc)::value;
-            const uint32_t x = clipd(up.template pair<DX + 2 * q>(), ncur[q], c2[k], nc2[k]);
-            const uint32_t y = clipd(dn.template pair<-DX + 2 * q>(), ncur[q], c2[k], nc2[k]);
-            const uint32_t s = add2(x, y);
-            acc[2 * q] = __dp2a_lo((int)s, (int)f[k], acc[2 * q]);
-            acc[2 * q + 1] = __dp2a_hi((int)s, (int)f[k], acc[2 * q + 1]);
-          });
-        };
-        using I0 = std::integral_constant<int, 0>;
-        using I1 = std::integral_constant<int, 1>;
-        using Im1 = std::integral_constant<int, -1>;
-        using I2 = std::integral_constant<int, 2>;
-        load_words<NP + 2, 1, (NP > 1)>(ra, R0 + y2 * S::SCP, 1, NP + 1);
-        load_words<NP + 2, 1, (NP > 1)>(rb, R0 - y2 * S::SCP, 1, NP + 1);
-        tap(ra, rb, I0{}, 0);
-        load_words<NP + 2, 1, (NP > 1)>(ra, R0 + y1 * S::SCP, 0, NP + 2);
-        load_words<NP + 2, 1, (NP > 1)>(rb, R0 - y1 * S::SCP, 0, NP + 2);
-        tap(ra, rb, I1{}, 1);
-        tap(ra, rb, I0{}, 2);
-        tap(ra, rb, Im1{}, 3);
-        tap(r0, r0, I2{}, 4);
-        tap(r0, r0, I1{}, 5);
-        const int round = 1 << (s2 - 1);
-#pragma unroll
-        for (int k = 0; k < SPT; ++k) v[k] = clampd(v[k] + ((acc[k] + round) >> s2), 0, maxv);
       }
       if (ccf >= 0) {  // CC-ALF from post-SAO luma (Table 47, src/alf.rs:447-523)
         const int *cc_k = a.tables.cc_coeff[cc][ccf];
@@ -576,7 +694,7 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
           s = __dp2a_hi((int)wb.w[k], (int)k2, s);
           s = __dp2a_lo((int)wb.w[k + 1], (int)k3, s);
           s = __dp2a_hi((int)w2.w[k + 1], (int)k3, s);
-          const int ctr = (int)(wm.w[k + 1] & 0xFFFF);
+          const int ctr = (int16_t)(wm.w[k + 1] & 0xFFFF);  // biased like the taps: the biases cancel
           s -= ctr * csum;
           v[k] = clampd(v[k] + clampd((s + 64) >> 7, -half, half - 1), 0, maxv);
         }
@@ -609,7 +727,9 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
       const int j = p / (W / 4), i = (p % (W / 4)) * 4;
       const int gx = X0 + i, gy = Y0 + j;
       if (gy >= LD.h || gx >= LD.w) continue;
-      const uint2 v = ld64(&sm.sL[(j + 3) * S::SLP + i + 4]);
+      uint2 v = ld64(&sm.sL[(j + 3) * S::SLP + i + 4]);
+      v.x ^= kBias;
+      v.y ^= kBias;
       uint16_t *out = LD.s + (int64_t)gy * LD.stride + gx;
       if (gx + 4 <= LD.w && ((uintptr_t)out & 7) == 0) {
         *reinterpret_cast<uint2 *>(out) = v;
@@ -624,7 +744,7 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
   __syncthreads();
 
   // ---- (4) classes
-  luma_classes<W, TH, S, NT3>(sm.sL, sm.cell(), sm.cls_f, sm.cls_t, Y0, y_ctb, ctb, ph, bd);
+  luma_classes<W, TH, S, NT3>(sm.sL, sm.cell(), sm.cls_f, sm.cls_t, Y0, y_ctb, ctb, ph, bd, big);
   __syncthreads();
 
   // ---- (5) 7x7 diamond: every thread keeps one block's taps and filters RPT of its 4-sample runs
@@ -633,14 +753,10 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
   constexpr int TPB = 4 / RPT;     // threads per 4x4 block
   const int b = tid / TPB;
   const int bx = b % (W / 4), by = b / (W / 4);
-  const uint32_t *tab = a.tables.luma_packed + ((size_t)me->luma_set * 100 + sm.cls_f[b] * 4 + sm.cls_t[b]) * 36;
-  // clip values and coefficients in registers (the negated clips are formed per use: fewer live registers)
-  uint32_t c2[12], f[12];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) {
-    c2[k] = __ldg(tab + 3 * k);
-    f[k] = __ldg(tab + 3 * k + 2);
-  }
+  const uint32_t *tab =
+      a.tables.luma_packed + ((size_t)me->luma_set * 100 + sm.cls_f[b] * 4 + sm.cls_t[b]) * kLumaEntry;
+  uint32_t c2[12], f[12];  // clip values and coefficients in registers
+  const int start = luma_filter(tab, c2, f);
   const int gx = X0 + 4 * bx;
 #pragma unroll 1
   for (int rr = 0; rr < RPT; ++rr) {
@@ -650,57 +766,58 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
     int shift, y1, y2, y3;
     table45(gy - y_ctb, ctb, shift, y1, y2, y3);
     const uint16_t *R0 = &sm.sL[(j + 3) * S::SLP + 4 * bx + 4];
-    int acc[4] = {0, 0, 0, 0};
-    uint32_t cur[2], ncur[2];
-    // words k of a row: samples (c0 - 4 + 2k, +1), c0 = the run's first sample
-    Words<6, 2> ru, rd;
-    auto tap = [&](const Words<6, 2> &up, const Words<6, 2> &dn, auto dx, int k) {
-      constexpr int DX = decltype(dx)::value;
-      const uint32_t nc = neg2(c2[k]);
-      static_for<2>([&](auto qc) {
-        constexpr int q = decltype(qc)::value;
-        const uint32_t x = clipd(up.template pair<DX + 2 * q>(), ncur[q], c2[k], nc);
-        const uint32_t y = clipd(dn.template pair<-DX + 2 * q>(), ncur[q], c2[k], nc);
-        const uint32_t s = add2(x, y);
-        acc[2 * q] = __dp2a_lo((int)s, (int)f[k], acc[2 * q]);
-        acc[2 * q + 1] = __dp2a_hi((int)s, (int)f[k], acc[2 * q + 1]);
-      });
-    };
-    using I0 = std::integral_constant<int, 0>;
-    using I1 = std::integral_constant<int, 1>;
-    using Im1 = std::integral_constant<int, -1>;
-    using I2 = std::integral_constant<int, 2>;
-    using Im2 = std::integral_constant<int, -2>;
-    using I3 = std::integral_constant<int, 3>;
-    load_words<6, 2, true>(ru, R0, 0, 6);  // the run's own row
-    cur[0] = ru.w[2];
-    cur[1] = ru.w[3];
-    ncur[0] = neg2(cur[0]);
-    ncur[1] = neg2(cur[1]);
-    tap(ru, ru, I3{}, 9);
-    tap(ru, ru, I2{}, 10);
-    tap(ru, ru, I1{}, 11);
-    load_words<6, 2, true>(ru, R0 + y3 * S::SLP, 2, 4);
-    load_words<6, 2, true>(rd, R0 - y3 * S::SLP, 2, 4);
-    tap(ru, rd, I0{}, 0);
-    load_words<6, 2, true>(ru, R0 + y2 * S::SLP, 1, 5);
-    load_words<6, 2, true>(rd, R0 - y2 * S::SLP, 1, 5);
-    tap(ru, rd, I1{}, 1);
-    tap(ru, rd, I0{}, 2);
-    tap(ru, rd, Im1{}, 3);
-    load_words<6, 2, true>(ru, R0 + y1 * S::SLP, 1, 5);
-    load_words<6, 2, true>(rd, R0 - y1 * S::SLP, 1, 5);
-    tap(ru, rd, I2{}, 4);
-    tap(ru, rd, I1{}, 5);
-    tap(ru, rd, I0{}, 6);
-    tap(ru, rd, Im1{}, 7);
-    tap(ru, rd, Im2{}, 8);
-    const int round = 1 << (shift - 1);
     int o[4];
+    if (big) {
+      luma_run_plain(R0, S::SLP, y1, y2, y3, shift, tab, maxv, o);
+    } else {
+      const int st = start + (1 << (shift - 1));
+      int acc[4] = {st, st, st, st};
+      // words k of a row: samples (c0 - 4 + 2k, +1), c0 = the run's first sample
+      Words<6, 2> ru, rd;
+      load_words<6, 2, true>(ru, R0, 0, 6);  // the run's own row
+      const uint32_t cur[2] = {ru.w[2] ^ kBias, ru.w[3] ^ kBias};
+      const uint32_t m[2] = {kBias - cur[0], kBias - cur[1]};  // 0x8000 - cur per lane
+      auto tap = [&](const Words<6, 2> &up, const Words<6, 2> &dn, auto dx, int k) {
+        constexpr int DX = decltype(dx)::value;
+        const uint32_t c22 = c2[k] + c2[k];
+        static_for<2>([&](auto qc) {
+          constexpr int q = decltype(qc)::value;
+          const uint32_t b = c2[k] + m[q];
+          const uint32_t s = clip_off(up.template pair<DX + 2 * q>(), b, c22) +
+                             clip_off(dn.template pair<-DX + 2 * q>(), b, c22);
+          acc[2 * q] = dp2a_ulo(s, f[k], acc[2 * q]);
+          acc[2 * q + 1] = dp2a_uhi(s, f[k], acc[2 * q + 1]);
+        });
+      };
+      using I0 = std::integral_constant<int, 0>;
+      using I1 = std::integral_constant<int, 1>;
+      using Im1 = std::integral_constant<int, -1>;
+      using I2 = std::integral_constant<int, 2>;
+      using Im2 = std::integral_constant<int, -2>;
+      using I3 = std::integral_constant<int, 3>;
+      tap(ru, ru, I3{}, 9);
+      tap(ru, ru, I2{}, 10);
+      tap(ru, ru, I1{}, 11);
+      load_words<6, 2, true>(ru, R0 + y3 * S::SLP, 2, 4);
+      load_words<6, 2, true>(rd, R0 - y3 * S::SLP, 2, 4);
+      tap(ru, rd, I0{}, 0);
+      load_words<6, 2, true>(ru, R0 + y2 * S::SLP, 1, 5);
+      load_words<6, 2, true>(rd, R0 - y2 * S::SLP, 1, 5);
+      tap(ru, rd, I1{}, 1);
+      tap(ru, rd, I0{}, 2);
+      tap(ru, rd, Im1{}, 3);
+      load_words<6, 2, true>(ru, R0 + y1 * S::SLP, 1, 5);
+      load_words<6, 2, true>(rd, R0 - y1 * S::SLP, 1, 5);
+      tap(ru, rd, I2{}, 4);
+      tap(ru, rd, I1{}, 5);
+      tap(ru, rd, I0{}, 6);
+      tap(ru, rd, Im1{}, 7);
+      tap(ru, rd, Im2{}, 8);
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      const int cv = (int)((cur[p >> 1] >> ((p & 1) * 16)) & 0xFFFF);
-      o[p] = clampd(cv + ((acc[p] + round) >> shift), 0, maxv);
+      for (int p = 0; p < 4; ++p) {
+        const int cv = (int)((cur[p >> 1] >> ((p & 1) * 16)) & 0xFFFF);
+        o[p] = clampd(cv + (acc[p] >> shift), 0, maxv);
+      }
     }
     uint16_t *out = LD.s + (int64_t)gy * LD.stride + gx;
     if (gx + 4 <= LD.w && ((uintptr_t)out & 7) == 0) {
