@@ -125,6 +125,7 @@ struct Lane {
   DevBuf side;        // side information
   DevBuf walk;        // CU maps and segment grids of device-built side information
   Staging stage;
+  Staging back;  // pinned landing area of small results (read_back)
   int init(cudaStream_t s) {
     if (!s) {
       H266_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
@@ -152,6 +153,9 @@ struct Lane {
     if (stage.ptr) cudaFreeHost(stage.ptr);
     stage.ptr = nullptr;
     stage.cap = 0;
+    if (back.ptr) cudaFreeHost(back.ptr);
+    back.ptr = nullptr;
+    back.cap = 0;
     if (staged) cudaEventDestroy(staged);
     if (mark) cudaEventDestroy(mark);
     staged = mark = nullptr;
@@ -1281,6 +1285,17 @@ int sync_read(Lane &ln, void *host, const void *dev, size_t n) {
   return H266_OK;
 }
 
+// The lane's work so far, then n device bytes in the lane's pinned landing area
+// (until its next read_back): one copy without the staging a pageable
+// destination costs.
+int read_back(Lane &ln, const void *dev, size_t n, const uint8_t **out) {
+  H266_TRY(ln.back.ensure(n));
+  H266_CUDA(cudaMemcpyAsync(ln.back.ptr, dev, n, cudaMemcpyDeviceToHost, ln.stream));
+  H266_CUDA(cudaStreamSynchronize(ln.stream));
+  *out = ln.back.ptr;
+  return H266_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1642,6 +1657,127 @@ int h266_cc_alf_decide_and_apply_clipped(h266_ctx *ctx, const h266_picture *src,
                        n_col, row_bd, n_row);
 }
 
+// One picture of a chroma SAO merge: its planes on the device and the caller's records.
+struct MergeJob {
+  DPlane src[2], pre[2];
+  const h266_sao_ctb_params *indep;
+  uint32_t wc, hc;
+  h266_sao_ctb_params *merged;
+  uint8_t *map;
+};
+
+// Merges the jobs' pictures on lane `ln`: one upload (records and parameters),
+// the wavefront over every picture, one download; then, for pictures the
+// wavefront left, the anti-diagonal launches.
+static int run_merges(h266_ctx *ctx, Lane &ln, const std::vector<MergeJob> &jobs, uint32_t bd, uint32_t log2) {
+  auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const uint32_t np = (uint32_t)jobs.size();
+  // device work area: every picture's results (status, merged records, map), then its work (zeroed)
+  std::vector<size_t> off_work(np), off_rec(np), off_map(np);
+  size_t total = al(np * sizeof(int32_t)), max_ctbs = 0;  // the statuses first
+  for (uint32_t i = 0; i < np; ++i) {
+    const size_t n = (size_t)jobs[i].wc * jobs[i].hc;
+    max_ctbs = std::max(max_ctbs, n);
+    off_rec[i] = total;
+    total += n * sizeof(h266_sao_ctb_params);
+    off_map[i] = total;
+    total = (total + n + 15) & ~(size_t)15;
+  }
+  const size_t results = total;
+  total = al(total);
+  const size_t work_from = total;
+  for (uint32_t i = 0; i < np; ++i) {
+    off_work[i] = total;
+    total += al(sao_merge_work_bytes((size_t)jobs[i].wc * jobs[i].hc));
+  }
+  H266_TRY(ln.walk.ensure(std::max<size_t>(total, 256)));
+  uint8_t *work = ln.walk.as<uint8_t>();
+  Prep &pr = ctx_prep(ctx, 0);
+  const size_t asz = sao_merge_args_size();
+  auto upload = [&](const std::vector<uint32_t> &which, const std::vector<uint32_t> &first, size_t &off_args,
+                    size_t &off_first, uint8_t *&base) -> int {
+    pr.blob.clear();
+    Blob blob{pr.blob};
+    std::vector<size_t> off_ind(which.size());
+    for (size_t k = 0; k < which.size(); ++k) {
+      const MergeJob &j = jobs[which[k]];
+      off_ind[k] = blob.put(j.indep, (size_t)j.wc * j.hc * sizeof(h266_sao_ctb_params));
+    }
+    off_first = blob.put(first.data(), first.size() * sizeof(uint32_t));
+    blob.alloc(asz * which.size(), off_args);  // filled in below, once the base is known
+    H266_TRY(ln.side.ensure(pr.blob.size()));
+    base = ln.side.as<uint8_t>();
+    for (size_t k = 0; k < which.size(); ++k) {
+      const uint32_t i = which[k];
+      const MergeJob &j = jobs[i];
+      int64_t most = 0;  // the largest |offset| of the parameters SAO applies
+      for (size_t c = 0; c < (size_t)j.wc * j.hc; ++c)
+        for (const h266_sao_ctb *p : {&j.indep[c].cb, &j.indep[c].cr})
+          if (p->sao_type_idx == 1 || p->sao_type_idx == 2)
+            for (int o = 1; o < 5; ++o) most = std::max<int64_t>(most, std::abs((int64_t)p->offset_val[o]));
+      fill_sao_merge_args(pr.blob.data() + off_args + asz * k, j.src, j.pre, (int)bd, (1 << log2) / 2, (int)j.wc,
+                          (int)j.hc, (int)std::min<int64_t>(most, 1 << 20),
+                          reinterpret_cast<const h266_sao_ctb_params *>(base + off_ind[k]),
+                          reinterpret_cast<h266_sao_ctb_params *>(work + off_rec[i]), work + off_map[i],
+                          work + off_work[i], reinterpret_cast<int32_t *>(work) + i);
+    }
+    H266_TRY(upload_blob(ln, pr.blob, &base));
+    ctx->h2d_bytes += pr.blob.size();
+    H266_CUDA(cudaMemsetAsync(work + work_from, 0, total - work_from, ln.stream));
+    return H266_OK;
+  };
+  auto take = [&](const uint8_t *host, uint32_t i) {
+    const MergeJob &j = jobs[i];
+    const size_t n = (size_t)j.wc * j.hc;
+    if (!n) return;
+    std::memcpy(j.merged, host + off_rec[i], n * sizeof(h266_sao_ctb_params));
+    std::memcpy(j.map, host + off_map[i], n);
+    ctx->d2h_bytes += n * (sizeof(h266_sao_ctb_params) + 1);
+  };
+  std::vector<uint32_t> all(np), left;
+  for (uint32_t i = 0; i < np; ++i) all[i] = i;
+  size_t off_args, off_first;
+  uint8_t *base = nullptr;
+  H266_TRY(upload(all, {}, off_args, off_first, base));
+  {
+    Prof pf(ctx, ln.stream, H266_PROF_SAO_ALF);
+    H266_TRY(launch_sao_merge_wave(ln.stream, base + off_args, (int)np, (int)max_ctbs, bd > 14, &ctx->launches));
+  }
+  const uint8_t *host = nullptr;
+  H266_TRY(read_back(ln, work, results, &host));
+  uint32_t n_diags = 0;
+  for (uint32_t i = 0; i < np; ++i) {
+    if (!jobs[i].wc || !jobs[i].hc) continue;
+    if (reinterpret_cast<const int32_t *>(host)[i]) {
+      take(host, i);
+      continue;
+    }
+    left.push_back(i);
+    n_diags = std::max(n_diags, jobs[i].wc + jobs[i].hc - 1);
+  }
+  if (left.empty()) return H266_OK;
+  const uint32_t nl = (uint32_t)left.size();
+  std::vector<uint32_t> first((size_t)n_diags * (nl + 1), 0), totals(n_diags, 0);
+  for (uint32_t d = 0; d < n_diags; ++d)
+    for (uint32_t k = 0; k < nl; ++k) {
+      const int wc = (int)jobs[left[k]].wc, hc = (int)jobs[left[k]].hc;
+      int c = 0;
+      if ((int)d <= wc + hc - 2) c = std::min(hc - 1, (int)d) - std::max(0, (int)d - (wc - 1)) + 1;
+      first[(size_t)d * (nl + 1) + k + 1] = first[(size_t)d * (nl + 1) + k] + (uint32_t)std::max(c, 0);
+      totals[d] = first[(size_t)d * (nl + 1) + k + 1];
+    }
+  H266_TRY(upload(left, first, off_args, off_first, base));
+  {
+    Prof pf(ctx, ln.stream, H266_PROF_SAO_ALF);
+    H266_TRY(launch_sao_chroma_merge_batch(ln.stream, base + off_args,
+                                           reinterpret_cast<const uint32_t *>(base + off_first), (int)nl, (int)n_diags,
+                                           totals.data(), &ctx->launches));
+  }
+  H266_TRY(read_back(ln, work, results, &host));
+  for (uint32_t i : left) take(host, i);
+  return H266_OK;
+}
+
 int h266_sao_chroma_merge(h266_ctx *ctx, const h266_picture *src, const h266_picture *pre,
                           const h266_sao_ctb_params *indep, uint32_t wc, uint32_t hc, uint32_t bd, uint32_t log2,
                           h266_sao_ctb_params *merged, uint8_t *map) {
@@ -1681,28 +1817,8 @@ int h266_sao_chroma_merge(h266_ctx *ctx, const h266_picture *src, const h266_pic
     S[i] = dplane(p, ln.scratch[1 + i].as<uint16_t>(), p.width);
     ctx->h2d_bytes += row * p.height;
   }
-  Prep &pr = ctx_prep(ctx, 0);
-  pr.blob.clear();
-  Blob blob{pr.blob};
-  const size_t off = blob.put(indep, n * sizeof(h266_sao_ctb_params));
-  uint8_t *base = nullptr;
-  H266_TRY(upload_blob(ln, pr.blob, &base));
-  ctx->h2d_bytes += pr.blob.size();
-  const size_t rec_b = n * sizeof(h266_sao_ctb_params), map_b = (n + 255) & ~(uint64_t)255;
-  H266_TRY(ln.walk.ensure(rec_b + map_b + sao_merge_work_bytes(n) + 256));
-  auto *d_merged = ln.walk.as<h266_sao_ctb_params>();
-  auto *d_map = ln.walk.as<uint8_t>() + rec_b;
-  void *d_work = ln.walk.as<uint8_t>() + ((rec_b + map_b + 255) & ~(size_t)255);
-  {
-    Prof pf(ctx, ln.stream, H266_PROF_SAO_ALF);
-    H266_TRY(launch_sao_chroma_merge(ln.stream, S, Q, (int)bd, (1 << log2) / 2, (int)wc, (int)hc,
-                                     reinterpret_cast<const h266_sao_ctb_params *>(base + off), d_merged, d_map,
-                                     d_work, &ctx->launches));
-  }
-  H266_CUDA(cudaMemcpyAsync(merged, d_merged, rec_b, cudaMemcpyDeviceToHost, ln.stream));
-  H266_TRY(sync_read(ln, map, d_map, n));
-  ctx->d2h_bytes += rec_b + n;
-  return H266_OK;
+  MergeJob job{{S[0], S[1]}, {Q[0], Q[1]}, indep, wc, hc, merged, map};
+  return run_merges(ctx, ln, {job}, bd, log2);
 }
 
 int h266_sao_chroma_merge_batch(h266_ctx *ctx, uint32_t np, const h266_picture *const *srcs,
@@ -1714,11 +1830,8 @@ int h266_sao_chroma_merge_batch(h266_ctx *ctx, uint32_t np, const h266_picture *
     return set_error(H266_ERR_INVALID_ARGUMENT, "NULL batch arrays");
   if (bd < 8 || bd > 16) return set_error(H266_ERR_INVALID_ARGUMENT, "bit_depth must be 8..16");
   if (log2 < 1 || log2 > 7) return set_error(H266_ERR_INVALID_ARGUMENT, "ctb_log2_size_y must be 1..7");
-  // layout of the device work area: per picture its merged records, map and work, 256-byte sections
-  auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  std::vector<size_t> off_rec(np), off_map(np), off_work(np);
-  size_t total = 0;
-  uint32_t n_diags = 0;
+  std::vector<MergeJob> jobs(np);
+  bool any = false;
   for (uint32_t i = 0; i < np; ++i) {
     const h266_picture *src = srcs[i], *pre = pres[i];
     H266_TRY(check_picture(src));
@@ -1733,71 +1846,22 @@ int h266_sao_chroma_merge_batch(h266_ctx *ctx, uint32_t np, const h266_picture *
     if (src->cb.width < pre->cb.width || src->cb.height < pre->cb.height || src->cr.width < pre->cb.width ||
         src->cr.height < pre->cb.height)
       return set_error(H266_ERR_INVALID_ARGUMENT, "original chroma planes smaller than the reconstruction's");
-    off_rec[i] = total;
-    total += al(n * sizeof(h266_sao_ctb_params));
-    off_map[i] = total;
-    total += al(n);
-    off_work[i] = total;
-    total += al(sao_merge_work_bytes(n));
-    if (n) n_diags = std::max(n_diags, wcs[i] + hcs[i] - 1);
-  }
-  if (!np || !n_diags) return H266_OK;
-  Guard g(ctx->device);
-  Lane &ln = ctx->main;
-  H266_TRY(ln.walk.ensure(std::max<size_t>(total, 256)));
-  uint8_t *work = ln.walk.as<uint8_t>();
-  H266_CUDA(cudaMemsetAsync(work, 0, total, ln.stream));  // per-CTB arrival counts start at zero
-  // one upload: every picture's independent records, merge parameters and per-diagonal picture tables
-  Prep &pr = ctx_prep(ctx, 0);
-  pr.blob.clear();
-  Blob blob{pr.blob};
-  std::vector<size_t> off_ind(np);
-  for (uint32_t i = 0; i < np; ++i)
-    off_ind[i] = blob.put(indeps[i], (size_t)wcs[i] * hcs[i] * sizeof(h266_sao_ctb_params));
-  std::vector<uint32_t> first((size_t)n_diags * (np + 1), 0), totals(n_diags, 0);
-  for (uint32_t d = 0; d < n_diags; ++d)
-    for (uint32_t i = 0; i < np; ++i) {
-      const int wc = (int)wcs[i], hc = (int)hcs[i];
-      int c = 0;
-      if (wc && hc && (int)d <= wc + hc - 2) c = std::min(hc - 1, (int)d) - std::max(0, (int)d - (wc - 1)) + 1;
-      first[(size_t)d * (np + 1) + i + 1] = first[(size_t)d * (np + 1) + i] + (uint32_t)std::max(c, 0);
-      totals[d] = first[(size_t)d * (np + 1) + i + 1];
+    MergeJob &j = jobs[i];
+    const h266_plane *sp[2] = {&src->cb, &src->cr}, *pp[2] = {&pre->cb, &pre->cr};
+    for (int c = 0; c < 2; ++c) {
+      j.src[c] = dplane(*sp[c], sp[c]->samples, (int64_t)std::max<uint64_t>(sp[c]->stride, 1));
+      j.pre[c] = dplane(*pp[c], pp[c]->samples, (int64_t)std::max<uint64_t>(pp[c]->stride, 1));
     }
-  const size_t off_first = blob.put(first.data(), first.size() * sizeof(uint32_t));
-  const size_t asz = sao_merge_args_size();
-  std::vector<uint8_t> args(asz * np);
-  const size_t off_args = blob.put(args.data(), args.size());  // filled in below, once the base is known
-  uint8_t *base = nullptr;
-  H266_TRY(ln.side.ensure(pr.blob.size()));
-  base = ln.side.as<uint8_t>();
-  for (uint32_t i = 0; i < np; ++i) {
-    const h266_picture &src = *srcs[i], &pre = *pres[i];
-    const DPlane S[2] = {dplane(src.cb, src.cb.samples, (int64_t)std::max<uint64_t>(src.cb.stride, 1)),
-                         dplane(src.cr, src.cr.samples, (int64_t)std::max<uint64_t>(src.cr.stride, 1))};
-    const DPlane Q[2] = {dplane(pre.cb, pre.cb.samples, (int64_t)std::max<uint64_t>(pre.cb.stride, 1)),
-                         dplane(pre.cr, pre.cr.samples, (int64_t)std::max<uint64_t>(pre.cr.stride, 1))};
-    fill_sao_merge_args(pr.blob.data() + off_args + asz * i, S, Q, (int)bd, (1 << log2) / 2, (int)wcs[i], (int)hcs[i],
-                        reinterpret_cast<const h266_sao_ctb_params *>(base + off_ind[i]),
-                        reinterpret_cast<h266_sao_ctb_params *>(work + off_rec[i]), work + off_map[i],
-                        work + off_work[i]);
+    j.indep = indeps[i];
+    j.wc = wcs[i];
+    j.hc = hcs[i];
+    j.merged = merged[i];
+    j.map = maps[i];
+    any = any || n;
   }
-  H266_TRY(upload_blob(ln, pr.blob, &base));
-  ctx->h2d_bytes += pr.blob.size();
-  {
-    Prof pf(ctx, ln.stream, H266_PROF_SAO_ALF);
-    H266_TRY(launch_sao_chroma_merge_batch(ln.stream, base + off_args, reinterpret_cast<const uint32_t *>(base + off_first),
-                                           (int)np, (int)n_diags, totals.data(), &ctx->launches));
-  }
-  for (uint32_t i = 0; i < np; ++i) {
-    const size_t n = (size_t)wcs[i] * hcs[i];
-    if (!n) continue;
-    H266_CUDA(cudaMemcpyAsync(merged[i], work + off_rec[i], n * sizeof(h266_sao_ctb_params), cudaMemcpyDeviceToHost,
-                              ln.stream));
-    H266_CUDA(cudaMemcpyAsync(maps[i], work + off_map[i], n, cudaMemcpyDeviceToHost, ln.stream));
-    ctx->d2h_bytes += n * (sizeof(h266_sao_ctb_params) + 1);
-  }
-  H266_CUDA(cudaStreamSynchronize(ln.stream));
-  return H266_OK;
+  if (!any) return H266_OK;
+  Guard g(ctx->device);
+  return run_merges(ctx, ctx->main, jobs, bd, log2);
 }
 
 int h266_sao_decide_picture(h266_ctx *ctx, const h266_picture *src, const h266_picture *rec, uint32_t log2,
@@ -1834,19 +1898,21 @@ int h266_sao_decide_picture(h266_ctx *ctx, const h266_picture *src, const h266_p
     ctx->h2d_bytes += row * p.height;
   }
   const size_t st_bytes = sao_stats_bytes((int)n), out_bytes = n * sizeof(h266_sao_ctb_params);
-  H266_TRY(ln.walk.ensure(st_bytes + out_bytes + 256));
-  uint8_t *w = ln.walk.as<uint8_t>();
+  // the error word and the statistics (both zeroed by the launch), then the records
+  H266_TRY(ln.walk.ensure(16 + st_bytes + out_bytes + 256));
+  uint8_t *w = ln.walk.as<uint8_t>() + 16;
   auto *d_out = reinterpret_cast<h266_sao_ctb_params *>(w + st_bytes);
-  auto *d_err = reinterpret_cast<uint32_t *>(w + st_bytes + ((out_bytes + 15) & ~(size_t)15));
-  H266_CUDA(cudaMemsetAsync(d_err, 0, 4, ln.stream));
+  auto *d_err = reinterpret_cast<uint32_t *>(w) - 1;
   {
     Prof pf(ctx, ln.stream, H266_PROF_SAO_ALF);
     H266_TRY(launch_sao_decide(ln.stream, S, R, (int)bd, (int)log2, (int)wc, (int)hc, sao_luma != 0, sao_chroma != 0,
                                w, d_err, d_out, &ctx->launches));
   }
-  uint32_t err = 0;
-  H266_CUDA(cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, ln.stream));
-  H266_TRY(sync_read(ln, &err, d_err, 4));
+  const uint8_t *host = nullptr;
+  H266_TRY(read_back(ln, d_out, out_bytes + 4, &host));
+  std::memcpy(out, host, out_bytes);
+  uint32_t err;
+  std::memcpy(&err, host + out_bytes, 4);
   ctx->d2h_bytes += out_bytes;
   if (err) return set_error(H266_ERR_INVALID_ARGUMENT, "SAO decision: a sample above (1 << bit_depth) - 1 has no band");
   return H266_OK;
