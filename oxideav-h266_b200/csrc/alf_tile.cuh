@@ -24,6 +24,8 @@
 #pragma once
 
 #include <initializer_list>
+#include <type_traits>
+#include <utility>
 
 #include "internal.h"
 
@@ -373,6 +375,211 @@ __device__ __forceinline__ void luma_sums(const S &sm, int j, int bx, int yr, in
     sum[q][9] = tap(pair_at<3>(R0, c), pair_at<-3>(R0, c));
     sum[q][10] = tap(pair_at<2>(R0, c), pair_at<-2>(R0, c));
     sum[q][11] = tap(pair_at<1>(R0, c), pair_at<-1>(R0, c));
+  }
+}
+
+// f(integral_constant<int, 0>) ... f(integral_constant<int, N - 1>): indices as constants
+template <class F, int... I>
+__device__ __forceinline__ void static_for_impl(F &&f, std::integer_sequence<int, I...>) {
+  (f(std::integral_constant<int, I>{}), ...);
+}
+template <int N, class F>
+__device__ __forceinline__ void static_for(F &&f) {
+  static_for_impl(f, std::make_integer_sequence<int, N>{});
+}
+
+__device__ __forceinline__ uint32_t ld32(const uint16_t *p) { return *reinterpret_cast<const uint32_t *>(p); }
+__device__ __forceinline__ uint2 ld64(const uint16_t *p) { return *reinterpret_cast<const uint2 *>(p); }
+__device__ __forceinline__ void st64(uint16_t *p, uint2 v) { *reinterpret_cast<uint2 *>(p) = v; }
+
+// Rows of packed words around a run of samples: word k covers samples
+// (c0 - 2B + 2k, c0 - 2B + 2k + 1) of the row at p = &row[c0].
+template <int NW, int B>
+struct Words {
+  uint32_t w[NW];
+  // pair (p[o], p[o + 1])
+  template <int O>
+  __device__ __forceinline__ uint32_t pair() const {
+    static_assert(O + 2 * B >= 0 && O + 2 * B + 1 < 2 * NW, "pair inside the loaded words");
+    if constexpr (((O + 2 * B) & 1) == 0) return w[(O + 2 * B) / 2];
+    else return __byte_perm(w[(O + 2 * B - 1) / 2], w[(O + 2 * B + 1) / 2], 0x5432);
+  }
+};
+
+// Loads words [k0, k1) of a Words<NW, B> at p (p - 2B + 2k0 4-byte aligned;
+// 64-bit loads where the address is 8-byte aligned by construction: A8).
+template <int NW, int B, bool A8>
+__device__ __forceinline__ void load_words(Words<NW, B> &r, const uint16_t *p, int k0, int k1) {
+  const uint16_t *q = p - 2 * B;
+  // word k starts an 8-byte aligned pair of words
+  auto lead = [](int k) { return A8 && (((2 * B) % 4 == 0) == (k % 2 == 0)); };
+#pragma unroll
+  for (int k = 0; k < NW; ++k) {
+    if (k < k0 || k >= k1) continue;
+    if (k > k0 && lead(k - 1)) continue;  // loaded with word k - 1
+    if (lead(k) && k + 1 < k1) {
+      const uint2 v = ld64(q + 2 * k);
+      r.w[k] = v.x;
+      r.w[k + 1 < NW ? k + 1 : k] = v.y;
+    } else {
+      r.w[k] = ld32(q + 2 * k);
+    }
+  }
+}
+
+// The plain form of the clipped taps for tiles that hold a sample of 2^14 or
+// above, tap by tap (out of line: no picture of a supported depth has any).
+__device__ __forceinline__ uint32_t pair_plain(const uint16_t *p) {
+  return ((uint32_t)p[0] | (uint32_t)p[1] << 16) ^ kBias;
+}
+__device__ __forceinline__ void tap_plain(const uint16_t *up, const uint16_t *dn, uint32_t ncur, uint32_t c2,
+                                          uint32_t f, int acc[2]) {
+  const uint32_t nc2 = neg2(c2);
+  const uint32_t s = add2(clipd(pair_plain(up), ncur, c2, nc2), clipd(pair_plain(dn), ncur, c2, nc2));
+  acc[0] = __dp2a_lo((int)s, (int)f, acc[0]);
+  acc[1] = __dp2a_hi((int)s, (int)f, acc[1]);
+}
+// taps (dx, dy) of the 7x7 and 5x5 diamonds in table order, mirrored taps at (-dx, -dy)
+static __constant__ int8_t kLumaTaps[12][2] = {{0, 3}, {1, 2}, {0, 2}, {-1, 2}, {2, 1}, {1, 1},
+                                        {0, 1}, {-1, 1}, {-2, 1}, {3, 0}, {2, 0}, {1, 0}};
+static __constant__ int8_t kChromaTaps[6][2] = {{0, 2}, {1, 1}, {0, 1}, {-1, 1}, {2, 0}, {1, 0}};
+
+static __device__ __noinline__ void luma_run_plain(const uint16_t *R0, int pitch, int y1, int y2, int y3, int shift,
+                                            const uint32_t *tab, int maxv, int out[4]) {
+  const int ys[4] = {0, y1, y2, y3};
+#pragma unroll 1
+  for (int q = 0; q < 2; ++q) {
+    const uint16_t *R = R0 + 2 * q;
+    const uint32_t cur = pair_plain(R), ncur = neg2(cur);
+    int acc[2] = {0, 0};
+#pragma unroll 1
+    for (int k = 0; k < 12; ++k) {
+      const int o = ys[kLumaTaps[k][1]] * pitch + kLumaTaps[k][0];
+      tap_plain(R + o, R - o, ncur, plain_clip(clip_of(tab, k)), coef_of(tab + 6, k), acc);
+    }
+    const int round = 1 << (shift - 1);
+    out[2 * q] = clampd((int)(cur & 0xFFFF) + ((acc[0] + round) >> shift), 0, maxv);
+    out[2 * q + 1] = clampd((int)(cur >> 16) + ((acc[1] + round) >> shift), 0, maxv);
+  }
+}
+
+template <int SPT>
+__device__ __noinline__ void chroma_run_plain(const uint16_t *R0, int pitch, int y1, int y2, int shift,
+                                              const uint32_t *ct, int maxv, int v[SPT]) {
+  const int ys[3] = {0, y1, y2};
+#pragma unroll 1
+  for (int q = 0; q < SPT / 2; ++q) {
+    const uint16_t *R = R0 + 2 * q;
+    const uint32_t cur = pair_plain(R), ncur = neg2(cur);
+    int acc[2] = {0, 0};
+#pragma unroll 1
+    for (int k = 0; k < 6; ++k) {
+      const int o = ys[kChromaTaps[k][1]] * pitch + kChromaTaps[k][0];
+      tap_plain(R + o, R - o, ncur, plain_clip(clip_of(ct, k)), coef_of(ct + 3, k), acc);
+    }
+    const int round = 1 << (shift - 1);
+    v[2 * q] = clampd((int)(cur & 0xFFFF) + ((acc[0] + round) >> shift), 0, maxv);
+    v[2 * q + 1] = clampd((int)(cur >> 16) + ((acc[1] + round) >> shift), 0, maxv);
+  }
+}
+
+// The 5x5 chroma diamond on SPT samples of a row (R0: the first in the biased
+// window; jr: the row inside its CTB of ctb_c rows), added to v[] (src/alf.rs:
+// 1014-1065, Table 46 line-buffer arms always applied).
+template <int SPT>
+__device__ __forceinline__ void chroma_alf_run(const uint16_t *R0, int pitch, int jr, int ctb_c, const uint32_t *ct,
+                                               int maxv, bool big, int v[SPT]) {
+  constexpr int NP = SPT / 2;
+  int s2 = 7, y1 = 1, y2 = 2;
+  if (jr == ctb_c - 2 || jr == ctb_c - 3) { s2 = 10; y1 = y2 = 0; }
+  else if (jr == ctb_c - 1 || jr == ctb_c - 4) { y2 = 1; }
+  if (big) {
+    chroma_run_plain<SPT>(R0, pitch, y1, y2, s2, ct, maxv, v);
+    return;
+  }
+  uint32_t c2[6], f[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    c2[k] = clip_of(ct, k);
+    f[k] = coef_of(ct + 3, k);
+  }
+  const int start = (int)ct[5] + (1 << (s2 - 1));
+  int acc[SPT];
+#pragma unroll
+  for (int k = 0; k < SPT; ++k) acc[k] = start;
+  uint32_t m[NP];  // 0x8000 - cur per lane
+  Words<NP + 2, 1> r0, ra, rb;
+  load_words<NP + 2, 1, (NP > 1)>(r0, R0, 0, NP + 2);
+#pragma unroll
+  for (int q = 0; q < NP; ++q) m[q] = kBias - (r0.w[1 + q] ^ kBias);
+  auto tap = [&](const Words<NP + 2, 1> &up, const Words<NP + 2, 1> &dn, auto dx, int k) {
+    constexpr int DX = decltype(dx)::value;
+    const uint32_t c22 = c2[k] + c2[k];
+    static_for<NP>([&](auto qc) {
+      constexpr int q = decltype(qc)::value;
+      const uint32_t b = c2[k] + m[q];
+      const uint32_t s = clip_off(up.template pair<DX + 2 * q>(), b, c22) +
+                         clip_off(dn.template pair<-DX + 2 * q>(), b, c22);
+      acc[2 * q] = dp2a_ulo(s, f[k], acc[2 * q]);
+      acc[2 * q + 1] = dp2a_uhi(s, f[k], acc[2 * q + 1]);
+    });
+  };
+  using I0 = std::integral_constant<int, 0>;
+  using I1 = std::integral_constant<int, 1>;
+  using Im1 = std::integral_constant<int, -1>;
+  using I2 = std::integral_constant<int, 2>;
+  load_words<NP + 2, 1, (NP > 1)>(ra, R0 + y2 * pitch, 1, NP + 1);
+  load_words<NP + 2, 1, (NP > 1)>(rb, R0 - y2 * pitch, 1, NP + 1);
+  tap(ra, rb, I0{}, 0);
+  load_words<NP + 2, 1, (NP > 1)>(ra, R0 + y1 * pitch, 0, NP + 2);
+  load_words<NP + 2, 1, (NP > 1)>(rb, R0 - y1 * pitch, 0, NP + 2);
+  tap(ra, rb, I1{}, 1);
+  tap(ra, rb, I0{}, 2);
+  tap(ra, rb, Im1{}, 3);
+  tap(r0, r0, I2{}, 4);
+  tap(r0, r0, I1{}, 5);
+#pragma unroll
+  for (int k = 0; k < SPT; ++k) v[k] = clampd(v[k] + (acc[k] >> s2), 0, maxv);
+}
+
+// CC-ALF of SPT chroma samples from the luma window (L0: luma of the first one;
+// yline: its luma row inside the CTB; lbb: the line-buffer arms apply), added to
+// v[] (Table 47, src/alf.rs:447-523).
+template <int SPT>
+__device__ __forceinline__ void cc_alf_run(const uint16_t *L0, int pitch, int yline, int ctb, bool lbb,
+                                           const int32_t *cc_k, int bd, int maxv, int v[SPT]) {
+  auto b8 = [](int x) { return (uint32_t)(x & 0xFF); };
+  // taps 0..6 at (0,-yP1), (-1,0), (+1,0), (-1,yP1), (0,yP1), (+1,yP1), (0,yP2) as dp2a byte pairs
+  const uint32_t k1 = b8(cc_k[0]) | b8(cc_k[1]) << 24;
+  const uint32_t k2 = b8(cc_k[2]) << 8 | b8(cc_k[3]) << 24;
+  const uint32_t k3 = b8(cc_k[4]) | b8(cc_k[5]) << 8 | b8(cc_k[6]) << 16;
+  const int csum = cc_k[0] + cc_k[1] + cc_k[2] + cc_k[3] + cc_k[4] + cc_k[5] + cc_k[6];
+  const int half = 1 << (bd - 1);
+  int yp1 = 1, yp2 = 2;
+  if (lbb) {
+    if (yline == ctb - 5 || yline == ctb - 4) { yp1 = 0; yp2 = 0; }
+    else if (yline == ctb - 6 || yline == ctb - 3) { yp2 = 1; }
+  }
+  // word k of a row: luma samples (2k - 2, 2k - 1) of the run; 8-byte loads for
+  // word pairs (k, k + 1), k odd (L0 is 8-byte aligned when SPT > 2)
+  constexpr int LW = SPT + 1;
+  Words<LW, 1> wt, wm, wb, w2;
+  load_words<LW, 1, (SPT > 2)>(wt, L0 - yp1 * pitch, 0, LW);
+  load_words<LW, 1, (SPT > 2)>(wm, L0, 0, LW);
+  load_words<LW, 1, (SPT > 2)>(wb, L0 + yp1 * pitch, 0, LW);
+  load_words<LW, 1, (SPT > 2)>(w2, L0 + yp2 * pitch, 0, LW);
+#pragma unroll
+  for (int k = 0; k < SPT; ++k) {
+    // chroma sample k: luma (2k - 2, 2k - 1) in word k, (2k, 2k + 1) in word k + 1
+    int s = __dp2a_lo((int)wt.w[k + 1], (int)k1, 0);
+    s = __dp2a_hi((int)wm.w[k], (int)k1, s);
+    s = __dp2a_lo((int)wm.w[k + 1], (int)k2, s);
+    s = __dp2a_hi((int)wb.w[k], (int)k2, s);
+    s = __dp2a_lo((int)wb.w[k + 1], (int)k3, s);
+    s = __dp2a_hi((int)w2.w[k + 1], (int)k3, s);
+    const int ctr = (int16_t)(wm.w[k + 1] & 0xFFFF);  // biased like the taps: the biases cancel
+    s -= ctr * csum;
+    v[k] = clampd(v[k] + clampd((s + 64) >> 7, -half, half - 1), 0, maxv);
   }
 }
 

@@ -1494,10 +1494,8 @@ int h266_apply_alf_clipped(h266_ctx *ctx, h266_picture *pic, const h266_alf_pict
   return pass2_entry(ctx, pic, in);
 }
 
-// The chroma ALF (cc = false) and CC-ALF (cc = true) decisions: one chain
-// SAO/ALF pass per candidate into its own chroma plane (the other chroma
-// plane left out, luma written to a throw-away plane), per-CTB SSE, pick,
-// commit.
+// The chroma ALF (cc = false) and CC-ALF (cc = true) decisions: every
+// candidate's per-CTB SSE in one launch, pick and commit in another.
 static int chroma_trials(h266_ctx *ctx, const h266_picture *src, h266_picture *rec, const uint16_t *pre_luma,
                          h266_alf_ctb *apply, uint64_t n_apply, const h266_alf_aps_data *aps, uint32_t comp, bool cc,
                          uint32_t log2, uint32_t bd, uint32_t cfi, const uint32_t *col_bd, uint64_t n_col,
@@ -1560,71 +1558,66 @@ static int chroma_trials(h266_ctx *ctx, const h266_picture *src, h266_picture *r
       ctx->h2d_bytes += row * rec->luma.height;
     }
   }
-  // scratch: SSE table, picks, one chroma plane per candidate, a throw-away luma plane
-  const int cols = (int)n_cand + 1;
-  const size_t cw = rp.width, chh = rp.height, lw = rec->luma.width, lh = rec->luma.height;
-  const size_t sse_b = (size_t)n * cols * 8, pick_b = ((size_t)n + 255) & ~(size_t)255;
-  const size_t plane_b = ((cw * chh * 2) + 255) & ~(size_t)255, luma_b = lw * lh * 2;
-  H266_TRY(ln.walk.ensure(sse_b + pick_b + plane_b * n_cand + luma_b + 256));
-  uint8_t *w = ln.walk.as<uint8_t>();
-  auto *d_sse = reinterpret_cast<unsigned long long *>(w);
-  auto *d_pick = reinterpret_cast<int8_t *>(w + sse_b);
-  auto *d_trials = reinterpret_cast<uint16_t *>(w + sse_b + pick_b);
-  auto *d_luma = reinterpret_cast<uint16_t *>(w + sse_b + pick_b + plane_b * n_cand);
-  const int cwc = (int)(ctb / 2), chc = (int)(ctb / 2);
-  Prof pf(ctx, ln.stream, H266_PROF_SAO_ALF);
-  H266_TRY(launch_ctb_sse(ln.stream, S, R[comp], cwc, chc, (int)wc, n, d_sse, cols, 0, &ctx->launches));
-  std::vector<h266_alf_ctb> trial((size_t)n);
+  // CTB clip rectangles and packed filters, as the chain takes them (any candidate's parameters)
+  std::vector<h266_alf_ctb> trial((size_t)n, h266_alf_ctb{});
   h266_alf_config cfg{1, comp == 1, comp == 2, comp == 1, comp == 2, bd, log2, cfi};
   h266_alf_aps_binding binding{};
   if (!cc) binding.chroma_aps = aps;
   else if (comp == 1) binding.cc_cb_aps = aps;
   else binding.cc_cr_aps = aps;
-  for (uint32_t k = 0; k < n_cand; ++k) {
-    for (h266_alf_ctb &c : trial) {
-      c = h266_alf_ctb{};
-      if (!cc) {
-        (comp == 1 ? c.cb_on : c.cr_on) = 1;
-        (comp == 1 ? c.cb_alt_idx : c.cr_alt_idx) = (uint8_t)k;
-      } else {
-        (comp == 1 ? c.cc_cb_idc : c.cc_cr_idc) = (uint8_t)(k + 1);
-      }
-    }
-    const h266_alf_picture ap{wc, hc, trial.data()};
-    Pass2Inputs in;
-    in.alf = &ap;
-    in.alf_cfg = &cfg;
-    in.binding = &binding;
-    in.cols = col_bd;
-    in.rows = row_bd;
-    in.n_cols = n_col;
-    in.n_rows = n_row;
-    H266_TRY(build_pass2(*rec, in, h));
-    if (!h.packed) return set_error(H266_ERR_UNSUPPORTED, "chroma ALF trials: coefficients outside [-128, 127]");
-    Staged st;
-    pr.blob.clear();
-    stage_pass2(h, pr.blob, st);
-    H266_TRY(upload_blob(ln, pr.blob, &st.base));
-    ctx->h2d_bytes += pr.blob.size();
-    const DPlane none{nullptr, 1, 0, 0};
-    DPlane SRC[3] = {cc ? PL : R[0], none, none}, DST[3] = {DPlane{d_luma, (int64_t)lw, (int)lw, (int)lh}, none, none};
-    SRC[comp] = R[comp];
-    DST[comp] = DPlane{d_trials + (size_t)k * (plane_b / 2), (int64_t)cw, (int)cw, (int)chh};
-    Pass2Args a = h.args;
-    bind_pass2(a, st.base, st, SRC, DST);
-    H266_TRY(launch_pass2_packed(ln.stream, a, false, true, &ctx->launches));
-    H266_TRY(launch_ctb_sse(ln.stream, S, DST[comp], cwc, chc, (int)wc, n, d_sse, cols, 1 + (int)k, &ctx->launches));
+  const h266_alf_picture ap{wc, hc, trial.data()};
+  Pass2Inputs in;
+  in.alf = &ap;
+  in.alf_cfg = &cfg;
+  in.binding = &binding;
+  in.cols = col_bd;
+  in.rows = row_bd;
+  in.n_cols = n_col;
+  in.n_rows = n_row;
+  H266_TRY(build_pass2(*rec, in, h));
+  if (!h.packed) return set_error(H266_ERR_UNSUPPORTED, "chroma ALF trials: coefficients outside [-128, 127]");
+  Staged st;
+  pr.blob.clear();
+  stage_pass2(h, pr.blob, st);
+  H266_TRY(upload_blob(ln, pr.blob, &st.base));
+  ctx->h2d_bytes += pr.blob.size();
+  // scratch: picks, SSE table, a copy of the component
+  const size_t cw = rp.width, chh = rp.height;
+  const size_t sse_b = (size_t)n * (n_cand + 1) * 8, pick_b = ((size_t)n + 255) & ~(size_t)255;
+  H266_TRY(ln.walk.ensure(pick_b + ((sse_b + 255) & ~(size_t)255) + cw * chh * 2));
+  uint8_t *w = ln.walk.as<uint8_t>();
+  ChromaTrialArgs t{};
+  t.rec = R[comp];
+  t.src = S;
+  t.luma = PL;
+  t.copy = DPlane{reinterpret_cast<uint16_t *>(w + pick_b + ((sse_b + 255) & ~(size_t)255)), (int64_t)cw, (int)cw,
+                  (int)chh};
+  t.bd = (int)bd;
+  t.log2 = (int)log2;
+  t.cc = cc ? 1 : 0;
+  t.n_cand = (int)n_cand;
+  t.w_ctbs = (int)wc;
+  t.h_ctbs = (int)hc;
+  t.pic_w = h.args.pic_w;
+  t.pic_h = h.args.pic_h;
+  t.ctbs = reinterpret_cast<const CtbDev *>(st.base + st.ctb);
+  t.pick = reinterpret_cast<int8_t *>(w);
+  t.sse = reinterpret_cast<unsigned long long *>(w + pick_b);
+  std::memcpy(t.packed, h.args.tables.chroma_packed, sizeof t.packed);
+  std::memcpy(t.cc_coeff, h.args.tables.cc_coeff[comp - 1], sizeof t.cc_coeff);
+  {
+    Prof pf(ctx, ln.stream, H266_PROF_SAO_ALF);
+    H266_CUDA(cudaMemsetAsync(t.sse, 0, sse_b, ln.stream));
+    H266_TRY(launch_chroma_trials(ln.stream, t, &ctx->launches));
   }
-  H266_TRY(launch_trial_pick_commit(ln.stream, d_sse, cols, n, d_pick, R[comp], d_trials, (int64_t)(plane_b / 2),
-                                    (int)cw, cwc, chc, (int)wc, &ctx->launches));
-  std::vector<int8_t> pick((size_t)n);
-  H266_CUDA(cudaMemcpyAsync(pick.data(), d_pick, (size_t)n, cudaMemcpyDeviceToHost, ln.stream));
+  const uint8_t *host = nullptr;
+  H266_TRY(read_back(ln, t.pick, (size_t)n, &host));
+  const int8_t *pick = reinterpret_cast<const int8_t *>(host);
   h266_picture one = *rec;  // copy back only the decided plane
   h266_plane *pl[3] = {&one.luma, &one.cb, &one.cr};
   for (int i = 0; i < 3; ++i)
     if (i != (int)comp) pl[i]->width = pl[i]->height = 0;
   H266_TRY(picture_from_device(ln, one));
-  if (rec->mem == H266_MEM_DEVICE) H266_CUDA(cudaStreamSynchronize(ln.stream));
   ctx->d2h_bytes += host_plane_bytes(one) + (size_t)n;
   for (int i = 0; i < n; ++i) {
     if (pick[i] < 0) continue;
@@ -2306,10 +2299,12 @@ int h266_alf_decide_and_apply_clipped(h266_ctx *ctx, const h266_picture *src, h2
                                     d_dec, &ctx->launches));
   }
   H266_TRY(run_pass2(ctx, ln.stream, h.args, false, true, true, st.base, st, S, P));
-  std::vector<int16_t> dec(n);
-  H266_CUDA(cudaMemcpyAsync(dec.data(), d_dec, n * sizeof(int16_t), cudaMemcpyDeviceToHost, ln.stream));
-  if (sse) H266_CUDA(cudaMemcpyAsync(sse, d_sse, sse_bytes, cudaMemcpyDeviceToHost, ln.stream));
-  H266_TRY(picture_from_device(ln, rl));
+  if (rl.mem == H266_MEM_HOST) H266_TRY(picture_from_device(ln, rl, false));
+  const uint8_t *host = nullptr;  // the decisions lie behind the SSE table
+  const size_t skip = sse ? 0 : sse_bytes;
+  H266_TRY(read_back(ln, ln.walk.as<uint8_t>() + skip, sse_bytes - skip + n * sizeof(int16_t), &host));
+  const int16_t *dec = reinterpret_cast<const int16_t *>(host + sse_bytes - skip);
+  if (sse) std::memcpy(sse, host, sse_bytes);
   ctx->d2h_bytes += host_plane_bytes(rl) + n * sizeof(int16_t) + (sse ? sse_bytes : 0);
   for (size_t i = 0; i < n; ++i) {
     decisions[i] = h266_alf_ctb{};

@@ -442,14 +442,20 @@ int launch_chroma_residual(cudaStream_t st, DPlane cb, DPlane cr, const ResPiece
                            const int32_t *d_res, int bd, uint64_t *launches);
 int launch_output_dump(cudaStream_t st, const OutPlanes &o, uint8_t *d_dst, bool wide, uint64_t *launches);
 
-// Encoder chroma ALF / CC-ALF trials (alf_enc.cu): per-CTB chroma SSE of a
-// against b into d_sse[ctb * cols + col]; then the first-minimum pick per CTB
-// and the copy of the chosen trial plane's CTB region into dst.
-int launch_ctb_sse(cudaStream_t st, DPlane a, DPlane b, int cw, int ch, int w_ctbs, int n, unsigned long long *d_sse,
-                   int cols, int col, uint64_t *launches);
-int launch_trial_pick_commit(cudaStream_t st, const unsigned long long *d_sse, int cols, int n, int8_t *d_pick,
-                             DPlane dst, const uint16_t *d_trials, int64_t trial_samples, int trial_pitch, int cw,
-                             int ch, int w_ctbs, uint64_t *launches);
+// Encoder chroma ALF / CC-ALF trials (alf_enc.cu): the n_cand candidate filters
+// of one chroma component per CTB, the first minimum of {off, candidates} in
+// pick[] (-1: off) and committed to `rec`.
+struct ChromaTrialArgs {
+  DPlane rec, src, copy;  // the component: reconstruction, original, scratch of rec's size (contiguous)
+  DPlane luma;            // CC-ALF: the luma before luma ALF
+  int bd, log2, cc, n_cand, w_ctbs, h_ctbs, pic_w, pic_h, tiles_x;
+  const CtbDev *ctbs;        // the CTBs' clip rectangles
+  unsigned long long *sse;   // [ctb][1 + n_cand], zero at the start
+  int8_t *pick;
+  uint32_t packed[8][8];     // AlfTablesDev::chroma_packed
+  int32_t cc_coeff[4][7];    // AlfTablesDev::cc_coeff of the component
+};
+int launch_chroma_trials(cudaStream_t st, const ChromaTrialArgs &a, uint64_t *launches);
 
 // Encoder SAO decision (sao_enc.cu): statistics per (CTB, component) into
 // d_stats (sao_stats_bytes), then the per-CTB decision into d_out.

@@ -94,21 +94,7 @@ struct Smem3 {
 // TMA and mbarrier helpers (tma.cuh); waits give up after kWaitNs.
 using namespace tile_dev;
 
-// f(integral_constant<int, 0>) ... f(integral_constant<int, N - 1>): indices as constants
-template <class F, int... I>
-__device__ __forceinline__ void static_for_impl(F &&f, std::integer_sequence<int, I...>) {
-  (f(std::integral_constant<int, I>{}), ...);
-}
-template <int N, class F>
-__device__ __forceinline__ void static_for(F &&f) {
-  static_for_impl(f, std::make_integer_sequence<int, N>{});
-}
-
 // ---------------------------------------------------------------- packed helpers
-__device__ __forceinline__ uint32_t ld32(const uint16_t *p) { return *reinterpret_cast<const uint32_t *>(p); }
-__device__ __forceinline__ uint2 ld64(const uint16_t *p) { return *reinterpret_cast<const uint2 *>(p); }
-__device__ __forceinline__ void st64(uint16_t *p, uint2 v) { *reinterpret_cast<uint2 *>(p) = v; }
-
 // Byte permute with sign replication (PTX prmt, default mode: selector bit 3
 // copies the sign bit of the selected byte).
 __device__ __forceinline__ uint32_t prmt(uint32_t lo, uint32_t hi, uint32_t sel) {
@@ -241,97 +227,6 @@ __device__ __forceinline__ void rest_pos(int i, int wx0, int wy0, int WQ, int WH
 }
 
 __device__ __forceinline__ int rest_count(int WQ, int WH, const FastRect &f) { return WQ * WH - f.quads(); }
-
-// Rows of packed words around a run of samples: word k covers samples
-// (c0 - 2B + 2k, c0 - 2B + 2k + 1) of the row at p = &row[c0].
-template <int NW, int B>
-struct Words {
-  uint32_t w[NW];
-  // pair (p[o], p[o + 1])
-  template <int O>
-  __device__ __forceinline__ uint32_t pair() const {
-    static_assert(O + 2 * B >= 0 && O + 2 * B + 1 < 2 * NW, "pair inside the loaded words");
-    if constexpr (((O + 2 * B) & 1) == 0) return w[(O + 2 * B) / 2];
-    else return __byte_perm(w[(O + 2 * B - 1) / 2], w[(O + 2 * B + 1) / 2], 0x5432);
-  }
-};
-
-// Loads words [k0, k1) of a Words<NW, B> at p (p - 2B + 2k0 4-byte aligned;
-// 64-bit loads where the address is 8-byte aligned by construction: A8).
-template <int NW, int B, bool A8>
-__device__ __forceinline__ void load_words(Words<NW, B> &r, const uint16_t *p, int k0, int k1) {
-  const uint16_t *q = p - 2 * B;
-  // word k starts an 8-byte aligned pair of words
-  auto lead = [](int k) { return A8 && (((2 * B) % 4 == 0) == (k % 2 == 0)); };
-#pragma unroll
-  for (int k = 0; k < NW; ++k) {
-    if (k < k0 || k >= k1) continue;
-    if (k > k0 && lead(k - 1)) continue;  // loaded with word k - 1
-    if (lead(k) && k + 1 < k1) {
-      const uint2 v = ld64(q + 2 * k);
-      r.w[k] = v.x;
-      r.w[k + 1 < NW ? k + 1 : k] = v.y;
-    } else {
-      r.w[k] = ld32(q + 2 * k);
-    }
-  }
-}
-
-// The plain form of the clipped taps for tiles that hold a sample of 2^14 or
-// above, tap by tap (out of line: no picture of a supported depth has any).
-__device__ __forceinline__ uint32_t pair_plain(const uint16_t *p) {
-  return ((uint32_t)p[0] | (uint32_t)p[1] << 16) ^ kBias;
-}
-__device__ __forceinline__ void tap_plain(const uint16_t *up, const uint16_t *dn, uint32_t ncur, uint32_t c2,
-                                          uint32_t f, int acc[2]) {
-  const uint32_t nc2 = neg2(c2);
-  const uint32_t s = add2(clipd(pair_plain(up), ncur, c2, nc2), clipd(pair_plain(dn), ncur, c2, nc2));
-  acc[0] = __dp2a_lo((int)s, (int)f, acc[0]);
-  acc[1] = __dp2a_hi((int)s, (int)f, acc[1]);
-}
-// taps (dx, dy) of the 7x7 and 5x5 diamonds in table order, mirrored taps at (-dx, -dy)
-__constant__ int8_t kLumaTaps[12][2] = {{0, 3}, {1, 2}, {0, 2}, {-1, 2}, {2, 1}, {1, 1},
-                                        {0, 1}, {-1, 1}, {-2, 1}, {3, 0}, {2, 0}, {1, 0}};
-__constant__ int8_t kChromaTaps[6][2] = {{0, 2}, {1, 1}, {0, 1}, {-1, 1}, {2, 0}, {1, 0}};
-
-__device__ __noinline__ void luma_run_plain(const uint16_t *R0, int pitch, int y1, int y2, int y3, int shift,
-                                            const uint32_t *tab, int maxv, int out[4]) {
-  const int ys[4] = {0, y1, y2, y3};
-#pragma unroll 1
-  for (int q = 0; q < 2; ++q) {
-    const uint16_t *R = R0 + 2 * q;
-    const uint32_t cur = pair_plain(R), ncur = neg2(cur);
-    int acc[2] = {0, 0};
-#pragma unroll 1
-    for (int k = 0; k < 12; ++k) {
-      const int o = ys[kLumaTaps[k][1]] * pitch + kLumaTaps[k][0];
-      tap_plain(R + o, R - o, ncur, plain_clip(clip_of(tab, k)), coef_of(tab + 6, k), acc);
-    }
-    const int round = 1 << (shift - 1);
-    out[2 * q] = clampd((int)(cur & 0xFFFF) + ((acc[0] + round) >> shift), 0, maxv);
-    out[2 * q + 1] = clampd((int)(cur >> 16) + ((acc[1] + round) >> shift), 0, maxv);
-  }
-}
-
-template <int SPT>
-__device__ __noinline__ void chroma_run_plain(const uint16_t *R0, int pitch, int y1, int y2, int shift,
-                                              const uint32_t *ct, int maxv, int v[SPT]) {
-  const int ys[3] = {0, y1, y2};
-#pragma unroll 1
-  for (int q = 0; q < SPT / 2; ++q) {
-    const uint16_t *R = R0 + 2 * q;
-    const uint32_t cur = pair_plain(R), ncur = neg2(cur);
-    int acc[2] = {0, 0};
-#pragma unroll 1
-    for (int k = 0; k < 6; ++k) {
-      const int o = ys[kChromaTaps[k][1]] * pitch + kChromaTaps[k][0];
-      tap_plain(R + o, R - o, ncur, plain_clip(clip_of(ct, k)), coef_of(ct + 3, k), acc);
-    }
-    const int round = 1 << (shift - 1);
-    v[2 * q] = clampd((int)(cur & 0xFFFF) + ((acc[0] + round) >> shift), 0, maxv);
-    v[2 * q + 1] = clampd((int)(cur >> 16) + ((acc[1] + round) >> shift), 0, maxv);
-  }
-}
 
 // ---------------------------------------------------------------- the tile
 // Tile `tile` of the picture whose parameters are `a` (tensor maps at `maps`).
@@ -593,8 +488,7 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
       const int cf = (DO_ALF && me) ? me->chroma_filt[cc] : -1;
       const int ccf = (DO_ALF && me) ? me->cc_filt[cc] : -1;
       const int ctb_c = ctb / 2, y_ctb_c = y_ctb / 2;
-      const int c0 = i0 + 4;
-      const uint16_t *R0 = &sm.sC[cc][(jj + 2) * S::SCP + c0];
+      const uint16_t *R0 = &sm.sC[cc][(jj + 2) * S::SCP + i0 + 4];
       int v[SPT];
       {
         Words<NP + 2, 1> w0;
@@ -606,99 +500,11 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
           v[2 * q + 1] = (int)(cur >> 16);
         }
       }
-      if (cf >= 0) {  // 5x5 diamond (src/alf.rs:1014-1065, Table 46 line-buffer arms always applied)
-        const int jr = gy - y_ctb_c;
-        int s2 = 7, y1 = 1, y2 = 2;
-        if (jr == ctb_c - 2 || jr == ctb_c - 3) { s2 = 10; y1 = y2 = 0; }
-        else if (jr == ctb_c - 1 || jr == ctb_c - 4) { y2 = 1; }
-        const uint32_t *ct = a.tables.chroma_packed[min(cf, 7)];
-        if (big) {
-          chroma_run_plain<SPT>(R0, S::SCP, y1, y2, s2, ct, maxv, v);
-        } else {
-          uint32_t c2[6], f[6];
-#pragma unroll
-          for (int k = 0; k < 6; ++k) {
-            c2[k] = clip_of(ct, k);
-            f[k] = coef_of(ct + 3, k);
-          }
-          const int start = (int)ct[5] + (1 << (s2 - 1));
-          int acc[SPT];
-#pragma unroll
-          for (int k = 0; k < SPT; ++k) acc[k] = start;
-          uint32_t m[NP];  // 0x8000 - cur per lane
-          Words<NP + 2, 1> r0, ra, rb;
-          load_words<NP + 2, 1, (NP > 1)>(r0, R0, 0, NP + 2);
-#pragma unroll
-          for (int q = 0; q < NP; ++q) m[q] = kBias - (r0.w[1 + q] ^ kBias);
-          auto tap = [&](const Words<NP + 2, 1> &up, const Words<NP + 2, 1> &dn, auto dx, int k) {
-            constexpr int DX = decltype(dx)::value;
-            const uint32_t c22 = c2[k] + c2[k];
-            static_for<NP>([&](auto qc) {
-              constexpr int q = decltype(qc)::value;
-              const uint32_t b = c2[k] + m[q];
-              const uint32_t s = clip_off(up.template pair<DX + 2 * q>(), b, c22) +
-                                 clip_off(dn.template pair<-DX + 2 * q>(), b, c22);
-              acc[2 * q] = dp2a_ulo(s, f[k], acc[2 * q]);
-              acc[2 * q + 1] = dp2a_uhi(s, f[k], acc[2 * q + 1]);
-            });
-          };
-          using I0 = std::integral_constant<int, 0>;
-          using I1 = std::integral_constant<int, 1>;
-          using Im1 = std::integral_constant<int, -1>;
-          using I2 = std::integral_constant<int, 2>;
-          load_words<NP + 2, 1, (NP > 1)>(ra, R0 + y2 * S::SCP, 1, NP + 1);
-          load_words<NP + 2, 1, (NP > 1)>(rb, R0 - y2 * S::SCP, 1, NP + 1);
-          tap(ra, rb, I0{}, 0);
-          load_words<NP + 2, 1, (NP > 1)>(ra, R0 + y1 * S::SCP, 0, NP + 2);
-          load_words<NP + 2, 1, (NP > 1)>(rb, R0 - y1 * S::SCP, 0, NP + 2);
-          tap(ra, rb, I1{}, 1);
-          tap(ra, rb, I0{}, 2);
-          tap(ra, rb, Im1{}, 3);
-          tap(r0, r0, I2{}, 4);
-          tap(r0, r0, I1{}, 5);
-#pragma unroll
-          for (int k = 0; k < SPT; ++k) v[k] = clampd(v[k] + (acc[k] >> s2), 0, maxv);
-        }
-      }
-      if (ccf >= 0) {  // CC-ALF from post-SAO luma (Table 47, src/alf.rs:447-523)
-        const int *cc_k = a.tables.cc_coeff[cc][ccf];
-        auto b8 = [](int x) { return (uint32_t)(x & 0xFF); };
-        // taps 0..6 at (0,-yP1), (-1,0), (+1,0), (-1,yP1), (0,yP1), (+1,yP1), (0,yP2) as dp2a byte pairs
-        const uint32_t k1 = b8(cc_k[0]) | b8(cc_k[1]) << 24;
-        const uint32_t k2 = b8(cc_k[2]) << 8 | b8(cc_k[3]) << 24;
-        const uint32_t k3 = b8(cc_k[4]) | b8(cc_k[5]) << 8 | b8(cc_k[6]) << 16;
-        const int csum = cc_k[0] + cc_k[1] + cc_k[2] + cc_k[3] + cc_k[4] + cc_k[5] + cc_k[6];
-        const int half = 1 << (bd - 1);
-        const int yline = (gy - y_ctb_c) * 2;
-        const bool lbb = !(gy * 2 + ctb >= ph && (ph - y_ctb) <= ctb - 4);
-        int yp1 = 1, yp2 = 2;
-        if (lbb) {
-          if (yline == ctb - 5 || yline == ctb - 4) { yp1 = 0; yp2 = 0; }
-          else if (yline == ctb - 6 || yline == ctb - 3) { yp2 = 1; }
-        }
-        // luma words of the run: word k = samples (2 i0 + 2 + 2k, +1) of a window row (col 2 i0 + 4 = luma x of i0)
-        const uint16_t *L0 = &sm.sL[(2 * jj + 3) * S::SLP + 2 * i0 + 4];
-        // 8-byte loads for word pairs (k, k + 1), k odd (L0 is 8-byte aligned when SPT > 2)
-        constexpr int LW = SPT + 1;
-        Words<LW, 1> wt, wm, wb, w2;
-        load_words<LW, 1, (SPT > 2)>(wt, L0 - yp1 * S::SLP, 0, LW);
-        load_words<LW, 1, (SPT > 2)>(wm, L0, 0, LW);
-        load_words<LW, 1, (SPT > 2)>(wb, L0 + yp1 * S::SLP, 0, LW);
-        load_words<LW, 1, (SPT > 2)>(w2, L0 + yp2 * S::SLP, 0, LW);
-#pragma unroll
-        for (int k = 0; k < SPT; ++k) {
-          // chroma sample k: luma (2k - 1, 2k) in word k, (2k, 2k + 1) in word k + 1
-          int s = __dp2a_lo((int)wt.w[k + 1], (int)k1, 0);
-          s = __dp2a_hi((int)wm.w[k], (int)k1, s);
-          s = __dp2a_lo((int)wm.w[k + 1], (int)k2, s);
-          s = __dp2a_hi((int)wb.w[k], (int)k2, s);
-          s = __dp2a_lo((int)wb.w[k + 1], (int)k3, s);
-          s = __dp2a_hi((int)w2.w[k + 1], (int)k3, s);
-          const int ctr = (int16_t)(wm.w[k + 1] & 0xFFFF);  // biased like the taps: the biases cancel
-          s -= ctr * csum;
-          v[k] = clampd(v[k] + clampd((s + 64) >> 7, -half, half - 1), 0, maxv);
-        }
-      }
+      if (cf >= 0)
+        chroma_alf_run<SPT>(R0, S::SCP, gy - y_ctb_c, ctb_c, a.tables.chroma_packed[min(cf, 7)], maxv, big, v);
+      if (ccf >= 0)  // col 2 i0 + 4 of the luma window = luma x of i0
+        cc_alf_run<SPT>(&sm.sL[(2 * jj + 3) * S::SLP + 2 * i0 + 4], S::SLP, (gy - y_ctb_c) * 2, ctb,
+                        !(gy * 2 + ctb >= ph && (ph - y_ctb) <= ctb - 4), a.tables.cc_coeff[cc][ccf], bd, maxv, v);
       uint16_t *out = CD.s + (int64_t)gy * CD.stride + gx;
       const bool vec = gx + SPT <= CD.w && ((uintptr_t)out & (2 * SPT - 1)) == 0;
       if (vec && SPT == 8) {
