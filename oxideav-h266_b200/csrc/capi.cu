@@ -501,8 +501,8 @@ const int kTranspose[4][12] = {{0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11},
 
 // Builds the packed tables; returns false when an input is outside the packed
 // path's range (then the scalar kernel runs).
-bool build_packed(Pass2Host &h, int bd, uint32_t cfi, const h266_alf_aps_data *caps) {
-  if (bd > 14 || (cfi != 0 && cfi != 1)) return false;
+bool build_packed(Pass2Host &h, int bd, const h266_alf_aps_data *caps) {
+  if (bd > 14) return false;
   auto in8 = [](int v) { return v >= -128 && v <= 127; };
   // an entry of kLumaEntry words: two 16-bit clip values a word, four coefficient bytes a word, the accumulator start
   auto put_tap = [](uint32_t *w, int clip_words, int k, int coef, int clip) {
@@ -730,7 +730,7 @@ int build_pass2(const h266_picture &pic, const Pass2Inputs &in, Pass2Host &h) {
     for (int c = 0; c < 3; ++c)
       for (int k = 0; k < 4; ++k)
         if (d.sao[c].off[k] < -128 || d.sao[c].off[k] > 127) a.sao_i8 = 0;
-  h.packed = build_packed(h, (int)bd, cfi, caps);
+  h.packed = build_packed(h, (int)bd, caps);
   if (!h.packed) h.luma_packed.clear();
   return H266_OK;
 }
@@ -2260,7 +2260,7 @@ int h266_alf_decide_and_apply_clipped(h266_ctx *ctx, const h266_picture *src, h2
         e[c * 12 + j] = t < 16 ? kFixedSetCoeff[(t * 25 + c) * 12 + j] : aps->luma_coeff[c][j];
         e[300 + c * 12 + j] = alf_clip_value((int)bd, t < 16 ? 0 : aps->luma_clip_idx[c][j]);
       }
-  if (!build_packed(h, (int)bd, 0, nullptr))
+  if (!build_packed(h, (int)bd, nullptr))
     return set_error(H266_ERR_UNSUPPORTED, "ALF trials: APS luma coefficients outside [-128, 127]");
   h.packed = true;
   Lane &ln = ctx->main;
@@ -2279,7 +2279,6 @@ int h266_alf_decide_and_apply_clipped(h266_ctx *ctx, const h266_picture *src, h2
   }
   ctx->h2d_bytes += host_plane_bytes(rl);
   H266_TRY(ensure_scratch(ln, P, S));
-  H266_TRY(plane_map(ctx, ln.stream, S[0], P[0], nullptr));  // the pre-ALF snapshot
   Staged st;
   pr.blob.clear();
   stage_pass2(h, pr.blob, st);
@@ -2292,9 +2291,9 @@ int h266_alf_decide_and_apply_clipped(h266_ctx *ctx, const h266_picture *src, h2
   H266_CUDA(cudaMemsetAsync(d_sse, 0, sse_bytes, ln.stream));
   {
     Pass2Args a = h.args;
-    bind_pass2(a, st.base, st, S, P);
+    bind_pass2(a, st.base, st, P, P);
     Prof pf(ctx, ln.stream, H266_PROF_SAO_ALF);
-    H266_TRY(launch_alf_luma_trials(ln.stream, a, O, run, cols, d_sse, &ctx->launches));
+    H266_TRY(launch_alf_luma_trials(ln.stream, a, O, S[0], run, cols, d_sse, &ctx->launches));  // S: the pre-ALF snapshot
     H266_TRY(launch_alf_luma_decide(ln.stream, reinterpret_cast<CtbDev *>(st.base + st.ctb), (int)n, d_sse, cols, run,
                                     d_dec, &ctx->launches));
   }
@@ -2758,15 +2757,21 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
   H266_TRY(bb.init());
   struct Run {
     bool tile, strips, packed;
-    int variant;
   };
   std::vector<Run> runs(n);
   std::vector<uint8_t> tile_params[2], walk_items;  // tiles: by region, [1] for edges on the 8x8 grid
   std::vector<uint32_t> tile_first[2] = {{0}, {0}}, walk_first[3] = {{0}, {0}, {0}};  // clear, CU map, walk CTAs
   WalkBatchCounts walk_total;
   const size_t wis = walk_batch_item_size();
-  std::vector<Pass2Args> p2[kPass2Variants];
-  std::vector<uint32_t> p2_first[kPass2Variants];
+  // SAO/ALF: per tile kernel variant, then per variant of the full-height chroma tiles
+  constexpr int kP2 = kPass2Variants + kPass2ChromaVariants;
+  std::vector<Pass2Args> p2[kP2];
+  std::vector<uint32_t> p2_first[kP2];
+  auto add_p2 = [&](int v, const Pass2Args &a, uint32_t ctas) {
+    if (p2_first[v].empty()) p2_first[v].push_back(0);
+    p2[v].push_back(a);
+    p2_first[v].push_back(p2_first[v].back() + ctas);
+  };
   const size_t tps = deblock_tile_params_size(), sps = strip_params_size();
   std::vector<uint8_t> strip_params[2];  // rows, columns
   std::vector<uint32_t> strip_first[2] = {{0}, {0}};
@@ -2841,16 +2846,17 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
       }
     }
     r.packed = it.pass2 && it.packed && !ctx->force_scalar;
-    r.variant = -1;
     if (r.packed) {
       Pass2Args a = it.args;
       a.tile_h = tn.sao_alf_tile_h;
       bind_pass2(a, base, it.st, it.S, it.P);
+      a.do_sao = it.do_sao;
+      a.do_alf = it.do_alf;
       uint32_t c = 0;
-      r.variant = pass2_packed_variant(a, it.do_sao, it.do_alf, &c);
-      if (p2_first[r.variant].empty()) p2_first[r.variant].push_back(0);
-      p2[r.variant].push_back(a);
-      p2_first[r.variant].push_back(p2_first[r.variant].back() + c);
+      const int cv = pass2_chroma_variant(a, &c);
+      if (cv >= 0) add_p2(kPass2Variants + cv, a, c);
+      const int v = pass2_packed_variant(a, it.do_sao, it.do_alf, &c);
+      add_p2(v, a, c);
     }
   }
   // one upload of every batched launch's parameter table
@@ -2870,10 +2876,10 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
   const size_t off_wi = blob.put(walk_items.data(), walk_items.size());
   size_t off_wf[3];
   for (int k = 0; k < 3; ++k) off_wf[k] = blob.put(walk_first[k].data(), walk_first[k].size() * sizeof(uint32_t));
-  size_t off_p2[kPass2Variants] = {0}, off_p2f[kPass2Variants] = {0};
+  size_t off_p2[kP2] = {0}, off_p2f[kP2] = {0};
   const uint32_t zero_queue[kPass2Variants] = {0};  // the persistent launches' item counters, zero at launch
   const size_t off_q = blob.put(zero_queue, sizeof zero_queue);
-  for (int v = 0; v < kPass2Variants; ++v)
+  for (int v = 0; v < kP2; ++v)
     if (!p2[v].empty()) {
       off_p2[v] = blob.put(p2[v].data(), p2[v].size() * sizeof(Pass2Args));
       off_p2f[v] = blob.put(p2_first[v].data(), p2_first[v].size() * sizeof(uint32_t));
@@ -2925,6 +2931,14 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
     if (!it.pass2 || runs[i].packed) continue;
     H266_TRY(run_pass2(ctx, stream, it.args, it.do_sao, it.do_alf, it.packed, it.st.base, it.st, it.S, it.P));
   }
+  for (int v = kPass2Variants; v < kP2; ++v)
+    if (!p2[v].empty()) {
+      Prof pf(ctx, stream, H266_PROF_SAO_ALF);
+      H266_TRY(launch_pass2_chroma_batch(stream, v - kPass2Variants,
+                                         reinterpret_cast<const Pass2Args *>(dside + off_p2[v]),
+                                         reinterpret_cast<const uint32_t *>(dside + off_p2f[v]), (int)p2[v].size(),
+                                         p2_first[v].back(), &ctx->launches));
+    }
   for (int v = 0; v < kPass2Variants; ++v)
     if (!p2[v].empty()) {
       Prof pf(ctx, stream, H266_PROF_SAO_ALF);

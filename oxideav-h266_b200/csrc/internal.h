@@ -349,6 +349,7 @@ struct Pass2Args {
   CUtensorMap tmap[3];
   int tma;        // windows staged by TMA (else 16-byte vector loads)
   int tile_h;     // tile height for CTBs of 64 and 128: 64 (also 0) or 32
+  int do_sao, do_alf;  // read by the full-height chroma tiles
   int sao_i8;     // every SAO offset of the picture fits a signed byte (the packed offset tables)
   DPlane src[3];  // input planes (post-deblock)
   DPlane dst[3];  // output planes
@@ -383,7 +384,8 @@ int deblock_wait_timeouts(uint32_t *count);
 // Timeouts of the tile kernels' bounded waits since the last call (the
 // kernels leave such a tile unfiltered and count it): 0 when none.
 int pass2_wait_timeouts(uint32_t *count);
-// Packed 16x2 form; requires bit_depth <= 14, 4:2:0 or 4:0:0, coefficients in [-128, 127].
+// Packed 16x2 form; requires bit_depth <= 14 and coefficients in [-128, 127].
+// Chroma of 4:2:2 and 4:4:4 runs in tiles of its own.
 int launch_pass2_packed(cudaStream_t st, const Pass2Args &a, bool do_sao, bool do_alf, uint64_t *launches);
 
 // ---------------------------------------------------------------- recon-side LMCS, output dump (recon.cu)
@@ -482,11 +484,12 @@ int launch_sao_decide(cudaStream_t st, const DPlane src[3], const DPlane rec[3],
 // Encoder luma ALF trials (packed form): `trials` filter-set slots of
 // a.tables.luma_packed evaluated on the pre-ALF luma a.src[0] against the
 // original `orig`; d_sse[ctb * cols + 0] += pre-ALF SSE, [.. + 1 + t] += SSE
-// of trial t (d_sse zeroed by the caller).  Then per CTB the decision, written
+// of trial t (d_sse zeroed by the caller); the luma samples are copied to
+// `copy` on the way, for the pass that commits the choice in place.  Then per CTB the decision, written
 // into d_ctbs[].luma_set (slot or -1) and d_decision[].
 constexpr int kAlfMaxTrials = 17;
-int launch_alf_luma_trials(cudaStream_t st, const Pass2Args &a, const DPlane &orig, int trials, int cols,
-                           unsigned long long *d_sse, uint64_t *launches);
+int launch_alf_luma_trials(cudaStream_t st, const Pass2Args &a, const DPlane &orig, const DPlane &copy, int trials,
+                           int cols, unsigned long long *d_sse, uint64_t *launches);
 int launch_alf_luma_decide(cudaStream_t st, CtbDev *d_ctbs, int n, unsigned long long *d_sse, int cols, int trials_run,
                            int16_t *d_decision, uint64_t *launches);
 int pass2_packed_variant(Pass2Args &a, bool do_sao, bool do_alf, uint32_t *ctas);
@@ -495,7 +498,12 @@ int pass2_packed_variant(Pass2Args &a, bool do_sao, bool do_alf, uint32_t *ctas)
 // picture's CTA count; pictures of one variant share a launch.  With
 // ctas_per_sm > 0 the launch is persistent: that many CTAs per SM drain the
 // variant's (picture, tile) items through the counter *d_queue (zero at launch).
-constexpr int kPass2Variants = 12;
+// pass2_chroma_variant: the batched launch (0..2) and CTA count of a picture's
+// full-height chroma tiles, -1 for none.
+constexpr int kPass2Variants = 12, kPass2ChromaVariants = 3;
+int pass2_chroma_variant(const Pass2Args &a, uint32_t *ctas);
+int launch_pass2_chroma_batch(cudaStream_t st, int variant, const Pass2Args *d_args, const uint32_t *d_first, int n,
+                              uint32_t ctas, uint64_t *launches);
 int launch_pass2_packed_batch(cudaStream_t st, int variant, const Pass2Args *d_args, const uint32_t *d_first, int n,
                               uint32_t ctas, int ctas_per_sm, uint32_t *d_queue, uint64_t *launches);
 

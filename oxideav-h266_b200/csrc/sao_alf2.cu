@@ -32,15 +32,25 @@ struct TrialSmem {
   alignas(8) unsigned long long sse[kAlfMaxTrials + 1];
 };
 
-__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
+// Adds the warp's sum of v to *sum.  NARROW: every lane's v below 2^32, summed
+// as halves by the warp's add reduction (8 squared errors of samples of 14 bits
+// a lane), against five rounds of 64-bit shuffles.
+template <bool NARROW>
+__device__ __forceinline__ void add_errors(unsigned long long v, unsigned long long *sum) {
+  if (NARROW) {
+    const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)v & 0xFFFFu);
+    const unsigned hi = __reduce_add_sync(0xffffffffu, (unsigned)v >> 16);
+    v = (unsigned long long)lo + ((unsigned long long)hi << 16);
+  } else {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  return v;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  }
+  if ((threadIdx.x & 31) == 0) atomicAdd(sum, v);
 }
 
 template <int W>
 __global__ void __launch_bounds__(NT, 2) k_alf_luma_trials(const __grid_constant__ Pass2Args a, const DPlane orig,
-                                                           int trials, int cols, unsigned long long *__restrict__ sse) {
+                                                           const DPlane copy, int trials, int cols, unsigned long long *__restrict__ sse) {
   using S = TrialSmem<W>;
   __shared__ S sm;
   const int tid = threadIdx.x, tile = blockIdx.x;
@@ -88,6 +98,7 @@ __global__ void __launch_bounds__(NT, 2) k_alf_luma_trials(const __grid_constant
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
       const int gx = X0 + 4 * bx + p;
+      if (gx < pw && gy < ph) copy.s[(int64_t)gy * copy.stride + gx] = sm.sL[(j + 3) * S::SLW + 4 * bx + p + 4];
       const bool in = gx < vw && gy < vh;
       org[rr][p] = in ? (int)orig.s[(int64_t)gy * orig.stride + gx] : -1;
       if (in) {
@@ -96,8 +107,13 @@ __global__ void __launch_bounds__(NT, 2) k_alf_luma_trials(const __grid_constant
       }
     }
   }
-  e0 = warp_sum(e0);
-  if ((tid & 31) == 0) atomicAdd(&sm.sse[0], e0);
+  add_errors<false>(e0, &sm.sse[0]);
+  int above = 0;  // an original sample above 2^BitDepth - 1: its squared error may need more than 32 bits
+#pragma unroll
+  for (int rr = 0; rr < RPT; ++rr)
+#pragma unroll
+    for (int p = 0; p < 4; ++p) above |= org[rr][p] > maxv;
+  const bool wide_org = __any_sync(0xffffffffu, above);
   const int cls = sm.cls_f[b] * 4 + sm.cls_t[b];
   int first = 0;  // first trial of the clipped path
   if (!wide) {
@@ -115,41 +131,42 @@ __global__ void __launch_bounds__(NT, 2) k_alf_luma_trials(const __grid_constant
     uint32_t fn[3];  // the next trial's coefficients, loaded while the current trial runs
 #pragma unroll
     for (int k = 0; k < 3; ++k) fn[k] = first > 0 ? __ldg(tab0 + k) : 0u;
-    for (int t = 0; t < first; ++t) {
-      uint32_t f[12];
+    auto fixed_sets = [&](auto narrow) {
+      constexpr bool NARROW = decltype(narrow)::value;
+      using Sum = std::conditional_t<NARROW, uint32_t, unsigned long long>;
+      for (int t = 0; t < first; ++t) {
+        uint32_t f[12];
 #pragma unroll
-      for (int k = 0; k < 12; ++k) f[k] = coef_of(fn, k);
-      if (t + 1 < first) {
+        for (int k = 0; k < 12; ++k) f[k] = coef_of(fn, k);
+        if (t + 1 < first) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) fn[k] = __ldg(tab0 + (size_t)(t + 1) * 100 * kLumaEntry + k);
-      }
-      unsigned long long e = 0;
+          for (int k = 0; k < 3; ++k) fn[k] = __ldg(tab0 + (size_t)(t + 1) * 100 * kLumaEntry + k);
+        }
+        Sum e = 0;
+        auto add = [&](int org_v, int v) {
+          const int d = org_v - v;
+          if (org_v >= 0) e += NARROW ? (Sum)(d * d) : (Sum)((long long)d * d);
+        };
 #pragma unroll
-      for (int rr = 0; rr < RPT; ++rr) {
-        const int round = 1 << (shift[rr] - 1);
+        for (int rr = 0; rr < RPT; ++rr) {
+          const int round = 1 << (shift[rr] - 1);
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          int lo = 0, hi = 0;
+          for (int q = 0; q < 2; ++q) {
+            int lo = round, hi = round;
 #pragma unroll
-          for (int k = 0; k < 12; ++k) {
-            lo = __dp2a_lo((int)sum[rr][q][k], (int)f[k], lo);
-            hi = __dp2a_hi((int)sum[rr][q][k], (int)f[k], hi);
-          }
-          const int v0 = clampd((int)(cur[rr][q] & 0xFFFF) + ((lo + round) >> shift[rr]), 0, maxv);
-          const int v1 = clampd((int)(cur[rr][q] >> 16) + ((hi + round) >> shift[rr]), 0, maxv);
-          if (org[rr][2 * q] >= 0) {
-            const int d = org[rr][2 * q] - v0;
-            e += (unsigned long long)((long long)d * d);
-          }
-          if (org[rr][2 * q + 1] >= 0) {
-            const int d = org[rr][2 * q + 1] - v1;
-            e += (unsigned long long)((long long)d * d);
+            for (int k = 0; k < 12; ++k) {
+              lo = __dp2a_lo((int)sum[rr][q][k], (int)f[k], lo);
+              hi = __dp2a_hi((int)sum[rr][q][k], (int)f[k], hi);
+            }
+            add(org[rr][2 * q], clampd((int)(cur[rr][q] & 0xFFFF) + (lo >> shift[rr]), 0, maxv));
+            add(org[rr][2 * q + 1], clampd((int)(cur[rr][q] >> 16) + (hi >> shift[rr]), 0, maxv));
           }
         }
+        add_errors<NARROW>(e, &sm.sse[1 + t]);
       }
-      e = warp_sum(e);
-      if ((tid & 31) == 0) atomicAdd(&sm.sse[1 + t], e);
-    }
+    };
+    if (wide_org) fixed_sets(std::false_type{});
+    else fixed_sets(std::true_type{});
   }
   for (int t = first; t < trials; ++t) {
     uint32_t c2[12], nc2[12], f[12];
@@ -172,8 +189,7 @@ __global__ void __launch_bounds__(NT, 2) k_alf_luma_trials(const __grid_constant
           e += (unsigned long long)((long long)d * d);
         }
     }
-    e = warp_sum(e);
-    if ((tid & 31) == 0) atomicAdd(&sm.sse[1 + t], e);
+    add_errors<false>(e, &sm.sse[1 + t]);
   }
   __syncthreads();
   if (tid <= trials) atomicAdd(&sse[(size_t)(ry * a.w_ctbs + rx) * cols + tid], sm.sse[tid]);
@@ -202,7 +218,8 @@ __global__ void k_alf_luma_decide(CtbDev *__restrict__ ctbs, int n, unsigned lon
 
 }  // namespace
 
-int launch_alf_luma_trials(cudaStream_t st, const Pass2Args &in, const DPlane &orig, int trials, int cols,
+int launch_alf_luma_trials(cudaStream_t st, const Pass2Args &in, const DPlane &orig, const DPlane &copy, int trials,
+                           int cols,
                            unsigned long long *d_sse, uint64_t *launches) {
   if (in.ext_w <= 0 || in.ext_h <= 0) return H266_OK;
   if (trials < 0 || trials > kAlfMaxTrials || cols < trials + 1)
@@ -212,8 +229,8 @@ int launch_alf_luma_trials(cudaStream_t st, const Pass2Args &in, const DPlane &o
   a.tiles_x = (a.ext_w + W - 1) / W;
   a.tiles_y = (a.ext_h + TH - 1) / TH;
   const unsigned n = (unsigned)(a.tiles_x * a.tiles_y);
-  if (W == 64) k_alf_luma_trials<64><<<n, NT, 0, st>>>(a, orig, trials, cols, d_sse);
-  else k_alf_luma_trials<32><<<n, NT, 0, st>>>(a, orig, trials, cols, d_sse);
+  if (W == 64) k_alf_luma_trials<64><<<n, NT, 0, st>>>(a, orig, copy, trials, cols, d_sse);
+  else k_alf_luma_trials<32><<<n, NT, 0, st>>>(a, orig, copy, trials, cols, d_sse);
   H266_CUDA(cudaGetLastError());
   ++*launches;
   return H266_OK;
