@@ -329,5 +329,8 @@ def u32_array(values):
     if values is None:
         return None, (None, 0)
     vals = list(values)
-    arr = np.ascontiguousarray(np.asarray(vals or [0], dtype=np.uint32))
+    if not vals:
+        one = C.c_uint32(0)
+        return C.pointer(one), (one, 0)
+    arr = np.ascontiguousarray(np.asarray(vals, dtype=np.uint32))
     return arr.ctypes.data_as(C.POINTER(C.c_uint32)), (arr, len(vals))

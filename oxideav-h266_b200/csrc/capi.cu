@@ -805,6 +805,7 @@ void bind_pass2(Pass2Args &a, const uint8_t *base, const Staged &st, const DPlan
 
 int run_pass2(h266_ctx *ctx, cudaStream_t stream, Pass2Args a, bool do_sao, bool do_alf, bool packed,
               const uint8_t *base, const Staged &st, const DPlane src[3], const DPlane dst[3]) {
+  a.small_tiles = pass2_small_tiles(pass2_large_tiles(a));
   bind_pass2(a, base, st, src, dst);
   Prof pf(ctx, stream, H266_PROF_SAO_ALF);
   if (packed && !ctx->force_scalar) return launch_pass2_packed(stream, a, do_sao, do_alf, &ctx->launches);
@@ -891,6 +892,16 @@ int check_lmcs(const h266_lmcs_derived *l, uint32_t mn, uint32_t mx) {
 // Host-side preparation of one chain call: the deblocking plan, the pass-2
 // tables and the side-information blob with its section offsets.  A failed
 // preparation keeps its status and message (it may run on a worker thread).
+namespace h266 {
+// One CU list packed for the device walk: every CU's head (compact when all of
+// the list fit), the tails of CUs with a TU map or a TB split.
+struct CuListStage {
+  bool compact = false;
+  std::vector<uint8_t> heads;
+  std::vector<CuTail> tails;
+};
+constexpr int kMotionParts = 4;  // parts of the CU list whose motion is collected in parallel
+}  // namespace h266
 struct h266::Prep {
   DeblockPlan plan;
   std::vector<uint8_t> blob;
@@ -901,6 +912,10 @@ struct h266::Prep {
   std::string msg;
   // Batch pictures: the blob copied to pinned memory by the worker that built
   // it, uploaded from there; `uploaded` marks the end of the last upload.
+  // The device walk's inputs while they are gathered (stage_cu_list, collect_motion).
+  CuListStage lists[2];
+  std::vector<CuMotionRec> motion[kMotionParts];
+  bool motion_ok[kMotionParts] = {};
   Staging pinned;
   cudaEvent_t uploaded = nullptr;
   bool staged_pinned = false;
@@ -971,6 +986,84 @@ static const h266::Tuning &batch_tuning(const h266_ctx *ctx, uint32_t n, const h
 
 namespace {
 
+// Packs CU list `cus` for the device walk.
+void stage_cu_list(const h266_deblock_cu *cus, uint64_t n, CuListStage &out) {
+  auto fits8 = [](int32_t v) { return v >= -127 && v <= 127; };
+  // compact heads when every CU of the list fits them (QPs and sub-block counts in 8 bits)
+  bool compact = true;
+  for (uint64_t i = 0; i < n && compact; ++i) {
+    const h266_deblock_cu &c = cus[i];
+    const bool legacy = c.qp_c[0] == INT32_MIN;
+    compact = fits8(c.qp_y) && (legacy || (fits8(c.qp_c[0]) && fits8(c.qp_c[1]) && fits8(c.qp_c[2]))) &&
+              c.num_sb_x <= 255 && c.num_sb_y <= 255 && c.x + c.w <= 65535 && c.y + c.h <= 65535;
+  }
+  out.compact = compact;
+  out.heads.resize(n * (compact ? sizeof(CuCompact) : kCuHeadBytes));
+  out.tails.clear();
+  uint8_t *heads = out.heads.data();
+  for (uint64_t i = 0; i < n; ++i) {
+    const h266_deblock_cu &c = cus[i];
+    if (compact) {
+      CuCompact k;
+      k.x = (uint16_t)c.x;
+      k.y = (uint16_t)c.y;
+      k.w = (uint16_t)c.w;
+      k.h = (uint16_t)c.h;
+      const bool legacy = c.qp_c[0] == INT32_MIN;
+      k.qp_y = (int8_t)c.qp_y;
+      k.qp_c[0] = legacy ? (int8_t)-128 : (int8_t)c.qp_c[0];
+      k.qp_c[1] = legacy ? (int8_t)0 : (int8_t)c.qp_c[1];
+      k.qp_c[2] = legacy ? (int8_t)0 : (int8_t)c.qp_c[2];
+      const uint8_t fl[13] = {c.intra,        c.tu_y_coded, c.tu_cb_coded, c.tu_cr_coded, c.bdpcm_luma,
+                              c.bdpcm_chroma, c.plt,        c.joint_cbcr2, c.ciip,        c.ibc,
+                              c.has_num_sb,   c.has_tu64,   c.has_tb_split};
+      k.flags = 0;
+      for (int b = 0; b < 13; ++b) k.flags |= (uint16_t)((fl[b] != 0) << b);
+      k.nsb_x = (uint8_t)c.num_sb_x;
+      k.nsb_y = (uint8_t)c.num_sb_y;
+      std::memcpy(heads + i * sizeof(CuCompact), &k, sizeof k);
+    } else {
+      std::memcpy(heads + i * kCuHeadBytes, &c, kCuHeadBytes);
+    }
+    if (c.has_tu64 || c.has_tb_split) {
+      CuTail t;
+      t.index = (uint32_t)i;
+      std::memcpy(t.tail, reinterpret_cast<const uint8_t *>(&c) + kCuHeadBytes, sizeof t.tail);
+      out.tails.push_back(t);
+    }
+  }
+}
+
+// Motion by CU for luma CUs [i0, i1): true when the grid covers the picture and
+// every CU's cells agree (the walk reads motion only inside CUs), so that one
+// record per CU replaces one per 4x4 cell.  Intra CUs read no motion (bS 2
+// comes first), so only the others' records travel.  False, too, for a CU
+// outside the picture or off the 4x4 grid (the host walk's business).
+bool collect_motion(const h266_picture &pic, const h266_in_loop_filter_args &a, uint64_t i0, uint64_t i1,
+                    std::vector<CuMotionRec> &rec) {
+  rec.clear();
+  const h266_deblock_mv_grid &g = *a.mv_grid;
+  const uint64_t w = pic.luma.width, h = pic.luma.height;
+  if (g.cells_w < (w + 3) / 4 || g.cells_h < (h + 3) / 4) return false;
+  for (uint64_t i = i0; i < i1; ++i) {
+    const h266_deblock_cu &c = a.cus[i];
+    if (c.intra) continue;
+    if ((uint64_t)c.x + c.w > w || (uint64_t)c.y + c.h > h || c.w < 4 || c.h < 4) return false;
+    const h266_deblock_mv_cell *first = &g.cells[(c.y / 4) * g.cells_w + c.x / 4];
+    const size_t w4 = c.w / 4;
+    // every cell of the first row equals its left neighbour, every row the first
+    bool same = w4 < 2 || std::memcmp(first + 1, first, (w4 - 1) * sizeof *first) == 0;
+    for (uint32_t y = c.y / 4 + 1; y < (c.y + c.h) / 4 && same; ++y)
+      same = std::memcmp(&g.cells[y * g.cells_w + c.x / 4], first, w4 * sizeof *first) == 0;
+    if (!same) return false;
+    CuMotionRec r;
+    r.index = (uint32_t)i;
+    r.m = *first;
+    rec.push_back(r);
+  }
+  return true;
+}
+
 // `allow_device`: a picture whose side information the device can build
 // (device_walk_mode non-zero) skips the host walk; its CU lists, motion grid
 // and gate lists are staged instead.  Pictures without chained footprints
@@ -997,11 +1090,31 @@ int prepare_chain(Prep &pr, const h266_picture &pic, const h266_in_loop_filter_a
   in.n_rows = a.n_clip_rows;
   H266_TRY(build_pass2(pic, in, pr.h));
   pr.blob.clear();
+  // The device walk's inputs: large lists are gathered by the pool while this
+  // thread decides whether the device takes the picture (1080p, 5300 CUs with
+  // motion: 70 us for the decision, 50 for the lists, 100 for the motion).
+  const bool sep = a.chroma_cus != nullptr, has_mv = a.mv_grid && a.mv_grid->cells && a.mv_grid->cells_w * a.mv_grid->cells_h;
+  const int n_lists = sep ? 2 : 1, parts = has_mv ? kMotionParts : 0;
+  auto gather = [&](size_t t) {
+    if ((int)t < parts) {
+      const uint64_t i0 = a.n_cus * t / kMotionParts, i1 = a.n_cus * (t + 1) / kMotionParts;
+      pr.motion_ok[t] = collect_motion(pic, a, i0, i1, pr.motion[t]);
+    } else {
+      const int l = (int)t - parts;
+      stage_cu_list(l ? a.chroma_cus : a.cus, l ? a.n_chroma_cus : a.n_cus, pr.lists[l]);
+    }
+  };
+  constexpr uint64_t kParallelCus = 1500;  // fewer take less than waking the workers
+  const bool ahead = allow_device && pool && pool->size() > 1 && a.n_cus >= kParallelCus;
+  if (ahead) pool->start((size_t)(parts + n_lists), gather);
   bool grid8 = false;
   const int mode = allow_device ? device_walk_mode(pic, a.cus, a.n_cus, a.chroma_cus, a.n_chroma_cus, a.deblock,
                                                    a.chroma_format_idc, &grid8)
                                 : 0;
+  if (ahead) pool->wait_all();
   if (mode) {
+    if (!ahead)
+      for (int t = 0; t < parts + n_lists; ++t) gather((size_t)t);
     Blob blob{pr.blob};
     DbSide &db = pr.db;
     db.device_walk = true;
@@ -1009,8 +1122,8 @@ int prepare_chain(Prep &pr, const h266_picture &pic, const h266_in_loop_filter_a
     db.dw.tile_lists = mode == 1;  // the walk lists each tile's cells (within the lists' caps in mode 1)
     db.dw.tiles_consume = db.dw_tiles;
     db.dw.grid8 = grid8;
-    db.dw_sep = a.chroma_cus != nullptr;
-    db.dw_mv = a.mv_grid && a.mv_grid->cells && a.mv_grid->cells_w * a.mv_grid->cells_h;
+    db.dw_sep = sep;
+    db.dw_mv = has_mv;
     DeviceWalkIn &w = db.dw;
     w.n_cus = a.n_cus;
     w.n_chroma = db.dw_sep ? a.n_chroma_cus : 0;
@@ -1025,88 +1138,32 @@ int prepare_chain(Prep &pr, const h266_picture &pic, const h266_in_loop_filter_a
     w.sep = db.dw_sep;
     w.cw = (int)pic.cb.width;
     w.ch = (int)pic.cb.height;
-    // the CU lists packed: every CU's head, the tails of CUs with a TU map or a TB split
-    const h266_deblock_cu *lists[2] = {a.cus, a.chroma_cus};
-    const uint64_t counts[2] = {a.n_cus, db.dw_sep ? a.n_chroma_cus : 0};
-    thread_local std::vector<CuTail> tails;
-    auto fits8 = [](int32_t v) { return v >= -127 && v <= 127; };
-    for (int l = 0; l < (db.dw_sep ? 2 : 1); ++l) {
-      // compact heads when every CU of the list fits them (QPs and sub-block counts in 8 bits)
-      bool compact = true;
-      for (uint64_t i = 0; i < counts[l] && compact; ++i) {
-        const h266_deblock_cu &c = lists[l][i];
-        const bool legacy = c.qp_c[0] == INT32_MIN;
-        compact = fits8(c.qp_y) && (legacy || (fits8(c.qp_c[0]) && fits8(c.qp_c[1]) && fits8(c.qp_c[2]))) &&
-                  c.num_sb_x <= 255 && c.num_sb_y <= 255 && c.x + c.w <= 65535 && c.y + c.h <= 65535;
-      }
-      w.compact[l] = compact;
-      const size_t hb = compact ? sizeof(CuCompact) : kCuHeadBytes;
-      size_t off;
-      uint8_t *heads = blob.alloc(counts[l] * hb, off);
-      (l ? pr.st.dw_ccus : pr.st.dw_cus) = off;
-      tails.clear();
-      for (uint64_t i = 0; i < counts[l]; ++i) {
-        const h266_deblock_cu &c = lists[l][i];
-        if (compact) {
-          CuCompact k;
-          k.x = (uint16_t)c.x;
-          k.y = (uint16_t)c.y;
-          k.w = (uint16_t)c.w;
-          k.h = (uint16_t)c.h;
-          const bool legacy = c.qp_c[0] == INT32_MIN;
-          k.qp_y = (int8_t)c.qp_y;
-          k.qp_c[0] = legacy ? (int8_t)-128 : (int8_t)c.qp_c[0];
-          k.qp_c[1] = legacy ? (int8_t)0 : (int8_t)c.qp_c[1];
-          k.qp_c[2] = legacy ? (int8_t)0 : (int8_t)c.qp_c[2];
-          const uint8_t fl[13] = {c.intra,        c.tu_y_coded, c.tu_cb_coded, c.tu_cr_coded, c.bdpcm_luma,
-                                  c.bdpcm_chroma, c.plt,        c.joint_cbcr2, c.ciip,        c.ibc,
-                                  c.has_num_sb,   c.has_tu64,   c.has_tb_split};
-          k.flags = 0;
-          for (int b = 0; b < 13; ++b) k.flags |= (uint16_t)((fl[b] != 0) << b);
-          k.nsb_x = (uint8_t)c.num_sb_x;
-          k.nsb_y = (uint8_t)c.num_sb_y;
-          std::memcpy(heads + i * sizeof(CuCompact), &k, sizeof k);
-        } else {
-          std::memcpy(heads + i * kCuHeadBytes, &c, kCuHeadBytes);
-        }
-        if (c.has_tu64 || c.has_tb_split) {
-          CuTail t;
-          t.index = (uint32_t)i;
-          std::memcpy(t.tail, reinterpret_cast<const uint8_t *>(&c) + kCuHeadBytes, sizeof t.tail);
-          tails.push_back(t);
-        }
-      }
-      w.n_tails[l] = tails.size();
-      pr.st.dw_tails[l] = blob.put(tails.data(), tails.size() * sizeof(CuTail));
+    for (int l = 0; l < n_lists; ++l) {
+      const CuListStage &c = pr.lists[l];
+      w.compact[l] = c.compact;
+      (l ? pr.st.dw_ccus : pr.st.dw_cus) = blob.put(c.heads.data(), c.heads.size());
+      w.n_tails[l] = c.tails.size();
+      pr.st.dw_tails[l] = blob.put(c.tails.data(), c.tails.size() * sizeof(CuTail));
     }
     if (db.dw_mv) {
-      // Motion by CU when the grid covers the picture and every luma CU's
-      // cells agree (the walk reads motion only inside CUs): one record per
-      // CU instead of one per 4x4 cell.
-      const h266_deblock_mv_grid &g = *a.mv_grid;
-      bool per_cu = g.cells_w >= (uint64_t)(w.w + 3) / 4 && g.cells_h >= (uint64_t)(w.h + 3) / 4;
-      // Intra CUs read no motion (bS 2 comes first), so only the others' records travel.
-      thread_local std::vector<CuMotionRec> rec;
-      rec.clear();
-      for (uint64_t i = 0; i < a.n_cus && per_cu; ++i) {
-        const h266_deblock_cu &c = a.cus[i];
-        if (c.intra) continue;
-        const h266_deblock_mv_cell *first = &g.cells[(c.y / 4) * g.cells_w + c.x / 4];
-        const size_t w4 = c.w / 4;
-        // every cell of the first row equals its left neighbour, every row the first
-        per_cu = w4 < 2 || std::memcmp(first + 1, first, (w4 - 1) * sizeof *first) == 0;
-        for (uint32_t y = c.y / 4 + 1; y < (c.y + c.h) / 4 && per_cu; ++y)
-          per_cu = std::memcmp(&g.cells[y * g.cells_w + c.x / 4], first, w4 * sizeof *first) == 0;
-        CuMotionRec r;
-        r.index = (uint32_t)i;
-        r.m = *first;
-        rec.push_back(r);
+      bool per_cu = true;
+      size_t recs = 0;
+      for (int k = 0; k < kMotionParts; ++k) {
+        per_cu = per_cu && pr.motion_ok[k];
+        recs += pr.motion[k].size();
       }
       db.dw_mv_cu = per_cu;
       w.mv_by_cu = per_cu;
-      w.n_mv_recs = per_cu ? rec.size() : 0;
-      if (per_cu) pr.st.dw_mv = blob.put(rec.data(), rec.size() * sizeof(CuMotionRec));
-      else pr.st.dw_mv = blob.put(a.mv_grid->cells, w.mv_w * w.mv_h * sizeof(h266_deblock_mv_cell));
+      w.n_mv_recs = per_cu ? recs : 0;
+      if (per_cu) {
+        uint8_t *dst = blob.alloc(recs * sizeof(CuMotionRec), pr.st.dw_mv);
+        for (const std::vector<CuMotionRec> &m : pr.motion) {
+          if (!m.empty()) std::memcpy(dst, m.data(), m.size() * sizeof(CuMotionRec));
+          dst += m.size() * sizeof(CuMotionRec);
+        }
+      } else {
+        pr.st.dw_mv = blob.put(a.mv_grid->cells, w.mv_w * w.mv_h * sizeof(h266_deblock_mv_cell));
+      }
     }
     pr.st.dw_cols = blob.put(a.no_filter_cols, a.n_no_filter_cols * sizeof(uint32_t));
     pr.st.dw_rows = blob.put(a.no_filter_rows, a.n_no_filter_rows * sizeof(uint32_t));
@@ -2789,6 +2846,10 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
     strip_first[0].push_back(strip_total.rows);
     strip_first[1].push_back(strip_total.cols);
   };
+  uint32_t large_tiles = 0;
+  for (const BatchItem &it : items)
+    if (it.pass2 && it.packed) large_tiles += pass2_large_tiles(it.args);
+  const bool small_tiles = pass2_small_tiles(large_tiles);
   for (uint32_t i = 0; i < n; ++i) {
     BatchItem &it = items[i];
     Run &r = runs[i];
@@ -2849,6 +2910,7 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
     if (r.packed) {
       Pass2Args a = it.args;
       a.tile_h = tn.sao_alf_tile_h;
+      a.small_tiles = small_tiles;
       bind_pass2(a, base, it.st, it.S, it.P);
       a.do_sao = it.do_sao;
       a.do_alf = it.do_alf;

@@ -2503,7 +2503,7 @@ struct DevCuGrid {  // CuGrid::cu_at on device memory
   int cw, ch;
   __device__ int64_t at(int x, int y) const {
     if (x < 0 || y < 0 || x / 4 >= cw || y / 4 >= ch) return -1;
-    return cells[(size_t)(y / 4) * cw + x / 4];
+    return (int64_t)cells[(size_t)(y / 4) * cw + x / 4] - 1;  // 0: none
   }
 };
 
@@ -2661,7 +2661,7 @@ __device__ __forceinline__ void unpack_item(const WalkParams &a, int list, uint3
     const int x0 = cx / 4, y0 = cy / 4;
     const int x1 = min((int)((cx + cw + 3) / 4), a.cw4), y1 = min((int)((cy + ch + 3) / 4), a.ch4);
     for (int y = y0; y < y1; ++y)
-      for (int x = x0; x < x1; ++x) a.cu_grid[list][(size_t)y * a.cw4 + x] = (int32_t)i;  // CUs never overlap here
+      for (int x = x0; x < x1; ++x) a.cu_grid[list][(size_t)y * a.cw4 + x] = (int32_t)i + 1;  // CUs never overlap here
     return;
   }
   i -= a.n[list];
@@ -2812,12 +2812,12 @@ size_t align_up(size_t n) { return (n + 255) & ~(size_t)255; }
 
 struct WalkLayout {
   size_t cu_grid[2], full[2], mv_full, grid[2][3], tile_count, tile_list[2][3], total;
-  size_t zero_from, zero_end;  // [0, zero_from) is set to all ones (CU maps), [zero_from, zero_end) to zero
+  size_t zero_end;  // [0, zero_end) is set to zero
   uint32_t slots[2][3], bands[2][3];
 };
 
 WalkLayout walk_layout(const DeviceWalkIn &in) {
-  // [CU maps: set to -1][tile counts: 0][segment grids: 0 when the strip
+  // [CU maps: 0, no CU][tile counts: 0][segment grids: 0 when the strip
   // kernels scan them][full CU records, motion, tile lists: written before
   // they are read, not cleared]
   WalkLayout L{};
@@ -2828,7 +2828,6 @@ WalkLayout walk_layout(const DeviceWalkIn &in) {
     if (l == 0 || in.sep) off += align_up(cells * 4);
   }
   if (!in.sep) L.cu_grid[1] = L.cu_grid[0];
-  L.zero_from = off;
   const size_t tiles = in.tile_lists ? (size_t)((in.w + kDeblockTile - 1) / kDeblockTile) *
                                            ((in.h + kDeblockTile - 1) / kDeblockTile)
                                      : 0;
@@ -2939,9 +2938,8 @@ int launch_device_walk(cudaStream_t st, const DeviceWalkIn &in, uint8_t *scratch
   WalkLayout L;
   fill_walk(in, scratch, a, out, L);
   const bool sep = in.sep;
-  // CU maps to -1 (no CU); full CU records, motion and segment grids to 0 (bS 0: no segment)
-  H266_CUDA(cudaMemsetAsync(scratch, 0xFF, L.zero_from, st));
-  H266_CUDA(cudaMemsetAsync(scratch + L.zero_from, 0, L.zero_end - L.zero_from, st));
+  // no CU in the maps, no cells in the tiles' lists, bS 0 (no segment) in grids that are scanned
+  H266_CUDA(cudaMemsetAsync(scratch, 0, L.zero_end, st));
   const int lists = in.cfi != 0 ? 6 : 2;
   for (int l = 0; l < (sep && in.cfi != 0 ? 2 : 1); ++l) {
     const uint32_t items = unpack_items(a, l);
@@ -2963,14 +2961,14 @@ int launch_device_walk(cudaStream_t st, const DeviceWalkIn &in, uint8_t *scratch
 // ---------------------------------------------------------------- batched device walk
 //
 // The walks of many pictures in three launches: the clearing of every
-// picture's CU maps (-1) and segment grids (bS 0), the CU maps, and the edge
+// picture's CU maps (no CU) and segment grids (bS 0), the CU maps, and the edge
 // walk.  Per picture a WalkBatchItem (parameters, clear extents, the walk's
 // list count); CTAs find their picture by binary search over
 // per-launch prefix tables of CTA counts.
 struct WalkBatchItem {
   WalkParams p;
   uint4 *clear;            // the picture's walk scratch
-  uint32_t ff_vec, zero_vec;  // 16-byte words set to all ones, then to zero
+  uint32_t zero_vec;       // 16-byte words set to zero
   uint32_t lists;          // (plane, pass) lists of the walk: 6, or 2 without chroma
   uint32_t cu_lists;       // CU maps built: 1, or 2 for a separate chroma tree
 };
@@ -2993,11 +2991,11 @@ __global__ void __launch_bounds__(256) k_walk_clear_batch(const WalkBatchItem *_
                                                           const uint32_t *__restrict__ first, int n) {
   const int p = batch_pick(first, n, blockIdx.x);
   const WalkBatchItem &it = items[p];
-  const uint32_t base = (blockIdx.x - first[p]) * kClearVecPerCta, total = it.ff_vec + it.zero_vec;
+  const uint32_t base = (blockIdx.x - first[p]) * kClearVecPerCta, total = it.zero_vec;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const uint32_t i = base + k * 256 + threadIdx.x;
-    if (i < total) it.clear[i] = i < it.ff_vec ? make_uint4(~0u, ~0u, ~0u, ~0u) : make_uint4(0, 0, 0, 0);
+    if (i < total) it.clear[i] = make_uint4(0, 0, 0, 0);
   }
 }
 
@@ -3036,11 +3034,10 @@ void fill_walk_batch_item(void *out, const DeviceWalkIn &in, uint8_t *scratch, D
   fill_walk(in, scratch, it.p, g, L);
   const bool sep = in.sep;
   it.clear = reinterpret_cast<uint4 *>(scratch);
-  it.ff_vec = (uint32_t)(L.zero_from / 16);  // the CU maps come first (256-byte sections)
-  it.zero_vec = (uint32_t)((L.zero_end - L.zero_from) / 16);
+  it.zero_vec = (uint32_t)(L.zero_end / 16);  // 256-byte sections
   it.lists = in.cfi != 0 ? 6 : 2;
   it.cu_lists = sep && in.cfi != 0 ? 2 : 1;
-  c.clear_ctas = (it.ff_vec + it.zero_vec + kClearVecPerCta - 1) / kClearVecPerCta;
+  c.clear_ctas = (it.zero_vec + kClearVecPerCta - 1) / kClearVecPerCta;
   c.grid_ctas = (unpack_items(it.p, 0) + 127) / 128 + (it.cu_lists == 2 ? (unpack_items(it.p, 1) + 127) / 128 : 0);
   c.walk_ctas = (std::max(it.p.n[0], it.p.n[1]) + 127) / 128;
   std::memcpy(out, &it, sizeof it);

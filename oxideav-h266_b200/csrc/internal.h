@@ -349,6 +349,7 @@ struct Pass2Args {
   CUtensorMap tmap[3];
   int tma;        // windows staged by TMA (else 16-byte vector loads)
   int tile_h;     // tile height for CTBs of 64 and 128: 64 (also 0) or 32
+  int small_tiles;     // 32 x 32 tiles for every CTB size (set before pass2_tma_maps)
   int do_sao, do_alf;  // read by the full-height chroma tiles
   int sao_i8;     // every SAO offset of the picture fits a signed byte (the packed offset tables)
   DPlane src[3];  // input planes (post-deblock)
@@ -492,6 +493,8 @@ int launch_alf_luma_trials(cudaStream_t st, const Pass2Args &a, const DPlane &or
                            int cols, unsigned long long *d_sse, uint64_t *launches);
 int launch_alf_luma_decide(cudaStream_t st, CtbDev *d_ctbs, int n, unsigned long long *d_sse, int cols, int trials_run,
                            int16_t *d_decision, uint64_t *launches);
+uint32_t pass2_large_tiles(const Pass2Args &a);  // 64 x 64 tiles of the picture
+bool pass2_small_tiles(uint32_t large_tiles);    // whether a launch of so many runs in small tiles
 int pass2_packed_variant(Pass2Args &a, bool do_sao, bool do_alf, uint32_t *ctas);
 // Batched packed pass: fills a's tile grid (a.tile_h chooses the tile height
 // for CTBs of 64 and 128), returns the kernel variant (0..11) and the

@@ -913,9 +913,9 @@ constexpr size_t smem3() {
 }
 
 // W x TH of a picture's tiles: 64 x 64 (or 64 x 32 by tuning) for CTBs of 64
-// and 128, 32 x 32 for 32.
-inline int tile_w(int log2) { return log2 >= 6 ? 64 : 32; }
-inline int tile_h(const Pass2Args &a) { return tile_w(a.ctb_log2) == 64 && a.tile_h == 32 ? 32 : tile_w(a.ctb_log2); }
+// and 128, 32 x 32 for 32 and for launches that would leave SMs without a tile.
+inline int tile_w(const Pass2Args &a) { return a.ctb_log2 >= 6 && !a.small_tiles ? 64 : 32; }
+inline int tile_h(const Pass2Args &a) { return tile_w(a) == 64 && a.tile_h == 32 ? 32 : tile_w(a); }
 
 // Once per kernel and device: the largest shared-memory carveout, so that four
 // CTAs of the tile kernel fit on an SM.
@@ -1000,7 +1000,7 @@ int launch_one(cudaStream_t st, const Pass2Args &in, bool do_sao, bool do_alf) {
 }  // namespace
 
 void pass2_tma_maps(Pass2Args &a) {
-  if (tile_w(a.ctb_log2) == 32) maps_for<32, 32>(a);
+  if (tile_w(a) == 32) maps_for<32, 32>(a);
   else if (tile_h(a) == 32) maps_for<64, 32>(a);
   else maps_for<64, 64>(a);
 }
@@ -1011,14 +1011,6 @@ int pass2_wait_timeouts(uint32_t *count) {
   if (v) H266_CUDA(cudaMemcpyToSymbol(g_wait_timeouts, &zero, sizeof zero));
   *count = v;
   return H266_OK;
-}
-
-int pass2_packed_variant(Pass2Args &a, bool do_sao, bool do_alf, uint32_t *ctas) {
-  const int W = tile_w(a.ctb_log2), TH = tile_h(a);
-  a.tiles_x = (a.ext_w + W - 1) / W;
-  a.tiles_y = (a.ext_h + TH - 1) / TH;
-  *ctas = a.ext_w > 0 && a.ext_h > 0 ? (uint32_t)(a.tiles_x * a.tiles_y) : 0;
-  return (W == 32 ? 0 : (TH == 64 ? 8 : 4)) + (do_sao ? 2 : 0) + (do_alf ? 1 : 0);
 }
 
 namespace {
@@ -1034,6 +1026,27 @@ int sm_count() {
   return v;
 }
 
+}  // namespace
+
+uint32_t pass2_large_tiles(const Pass2Args &a) {
+  return a.ext_w > 0 && a.ext_h > 0 ? (uint32_t)((a.ext_w + 63) / 64) * (uint32_t)((a.ext_h + 63) / 64) : 0;
+}
+
+// One SM works on a 64 x 64 tile for 24 us, on a 32 x 32 one for 13 (a tile
+// alone on its SM, bound by its phases' latencies), so launches of at most one
+// large tile per SM run in small ones (416 x 240: 24 -> 13.6 us); with more, the
+// SMs fill and the small tiles' wider borders cost more than they save.
+bool pass2_small_tiles(uint32_t large_tiles) { return large_tiles <= (uint32_t)sm_count(); }
+
+int pass2_packed_variant(Pass2Args &a, bool do_sao, bool do_alf, uint32_t *ctas) {
+  const int W = tile_w(a), TH = tile_h(a);
+  a.tiles_x = (a.ext_w + W - 1) / W;
+  a.tiles_y = (a.ext_h + TH - 1) / TH;
+  *ctas = a.ext_w > 0 && a.ext_h > 0 ? (uint32_t)(a.tiles_x * a.tiles_y) : 0;
+  return (W == 32 ? 0 : (TH == 64 ? 8 : 4)) + (do_sao ? 2 : 0) + (do_alf ? 1 : 0);
+}
+
+namespace {
 template <int W, int TH, bool DO_SAO, bool DO_ALF>
 int launch_variant(cudaStream_t st, const Pass2Args *d_args, const uint32_t *d_first, int n, uint32_t ctas, int cps,
                    uint32_t *d_queue) {
@@ -1118,7 +1131,7 @@ int launch_pass2_packed(cudaStream_t st, const Pass2Args &in, bool do_sao, bool 
     H266_TRY(launch_pass2_chroma(st, a, launches));
     a.chroma = 0;
   }
-  const int rc = tile_w(a.ctb_log2) == 64 ? (tile_h(a) == 32 ? launch_one<64, 32>(st, a, do_sao, do_alf)
+  const int rc = tile_w(a) == 64 ? (tile_h(a) == 32 ? launch_one<64, 32>(st, a, do_sao, do_alf)
                                                               : launch_one<64, 64>(st, a, do_sao, do_alf))
                                           : launch_one<32, 32>(st, a, do_sao, do_alf);
   if (rc == H266_OK) ++*launches;

@@ -54,3 +54,22 @@ def test_samples_outside_the_depth(bd, value):
     for p in pic.planes():
         p[rng.integers(0, p.shape[0] // 2, 20), rng.integers(0, p.shape[1] // 2, 20)] = value
     check(pic, fa, f"{bd} bit with samples of {value}")
+
+
+@pytest.mark.parametrize("tile_h,cps", [(64, 0), (32, 0), (64, 2)])
+def test_large_tiles_in_a_batch(tile_h, cps):
+    """The same sizes and depths in one batch with more 64 x 64 tiles than SMs, which keeps the large tiles."""
+    items = [W.make_workload(100 * bd + w, w, h, bd, log2, ccalf=True, lmcs=bd <= 12, n_luma_aps=2, n_chroma_alt=2,
+                             alf_fixed_frac=0.3) for bd in (8, 10, 12, 14) for w, h, log2 in SIZES]
+    items += [W.make_workload(5, 832, 480, 10, 7, ccalf=True)]
+    with native.Context(0) as ctx:
+        ctx.set_tuning("sao_alf_tile_h", tile_h)
+        ctx.set_tuning("sao_alf_ctas_per_sm", cps)
+        plans = [ctx.plan(p, f) for p, f in items]
+        devs = [native.DevicePicture.from_host(p) for p, _ in items]
+        ctx.execute_plans(plans, devs)
+        ctx.synchronize()
+    for (p, f), d in zip(items, devs):
+        want = p.copy()
+        oracle.apply_in_loop_filters(want, f)
+        assert d.to_host().equal(want), (p.width, p.height, p.bit_depth)
