@@ -2041,8 +2041,9 @@ int h266_lmcs_forward_map_luma_rects(h266_ctx *ctx, h266_picture *pic, const h26
   }
   H266_TRY(picture_from_device(ln, lv, false));
   ctx->d2h_bytes += host_plane_bytes(lv);
-  uint32_t err = 0;
-  H266_TRY(sync_read(ln, &err, d_err, 4));
+  const uint8_t *host = nullptr;
+  H266_TRY(read_back(ln, d_err, 4, &host));
+  const bool err = *reinterpret_cast<const uint32_t *>(host) != 0;
   ln.fwd_key = *lmcs;
   ln.fwd_ok = true;
   if (!err) ln.fwd_cover.done();  // counters back at zero (a raised error word is cleared by the next call's fill)
@@ -2093,7 +2094,11 @@ int h266_lmcs_chroma_var_scale(h266_ctx *ctx, const h266_picture *pic, const h26
     H266_TRY(launch_lmcs_cvs(ln.stream, P[0], reinterpret_cast<const h266_lmcs_cvs_block *>(base + off), (uint32_t)n,
                              (int)size_y, t, ln.walk.as<uint32_t>(), &ctx->launches));
   }
-  if (n) H266_TRY(sync_read(ln, var_scale, ln.walk.as<uint32_t>(), n * 4));
+  if (n) {
+    const uint8_t *host = nullptr;
+    H266_TRY(read_back(ln, ln.walk.ptr, n * 4, &host));
+    std::memcpy(var_scale, host, n * 4);
+  }
   ctx->d2h_bytes += n * 4;
   return H266_OK;
 }
@@ -2167,8 +2172,9 @@ int h266_lmcs_add_chroma_residual(h266_ctx *ctx, h266_picture *pic, uint32_t bd,
                                           (uint32_t)n, d_res, (int)bd, c, d_overlap, &ctx->launches));
   }
   H266_TRY(picture_from_device(ln, cv, false));
-  uint32_t overlap = 0;
-  H266_TRY(sync_read(ln, &overlap, d_overlap, 4));
+  const uint8_t *host = nullptr;
+  H266_TRY(read_back(ln, d_overlap, 4, &host));
+  const bool overlap = *reinterpret_cast<const uint32_t *>(host) != 0;
   ctx->d2h_bytes += host_plane_bytes(cv);
   if (!overlap) {
     ln.res_cover.done();  // owners cleared by the add pass

@@ -165,9 +165,9 @@ H266_HD inline bool motion_differs(const h266_deblock_mv_cell &p, const h266_deb
 }
 
 struct PlaneCfg {
-  uint32_t comp, sub_w, sub_h;
+  uint32_t comp, sub;  // sub: log2 of the chroma grid's luma step (1 for every format, src/deblock.rs), 0 for luma
   int beta_off, tc_off, qp_off, bd;
-  uint32_t ctb;
+  uint32_t ctb;  // a power of two: the walk takes remainders with masks, as a device division costs 25 instructions
 };
 
 struct Emitted {  // a segment in emission (reference) order: its index in the list
@@ -236,21 +236,21 @@ H266_HD inline CuWalkGeo cu_walk_geo(const h266_deblock_cu &cu, const PlaneCfg &
                                      uint64_t n_nf) {
   CuWalkGeo g;
   g.chroma = pc.comp != 0;
-  g.off_grid = g.chroma && ((vert ? cu.x / pc.sub_w : cu.y / pc.sub_h) % 8) != 0;
+  g.off_grid = g.chroma && (((vert ? cu.x : cu.y) >> pc.sub) & 7) != 0;
   g.n_cb = vert ? cu.w : cu.h;
   g.n_other = vert ? cu.h : cu.w;
   const uint32_t lead = vert ? cu.x : cu.y;
   bool gated = false;
   for (uint64_t i = 0; i < n_nf; ++i) gated |= nf[i] == lead;
   g.filter_edge = lead != 0 && !gated;
-  g.step = g.chroma ? 8 * (vert ? pc.sub_w : pc.sub_h) : 4;
-  g.seg = g.chroma ? 2 * (vert ? pc.sub_h : pc.sub_w) : 4;
+  g.step = g.chroma ? 8u << pc.sub : 4;
+  g.seg = g.chroma ? 2u << pc.sub : 4;
   g.nsb = 1;
   if (!g.chroma && cu.has_num_sb) g.nsb = std::max(vert ? cu.num_sb_x : cu.num_sb_y, 1u);
-  g.sb = std::max(8u, g.n_cb / g.nsb);
+  g.sb = std::max(8u, g.nsb == 1 ? g.n_cb : g.n_cb / g.nsb);
   g.n8 = std::max(g.n_cb / 8, 1u);
   g.last_sb = std::min(g.n8 - 1, g.nsb - 1);
-  g.ctb_h_c = pc.ctb / std::max(pc.sub_h, 1u);
+  g.ctb_h_c = pc.ctb >> pc.sub;
   return g;
 }
 
@@ -285,7 +285,7 @@ H266_HD inline void walk_segment(const h266_deblock_cu *cus_, const Grid &grid, 
     if (bs == 0) return;
     uint32_t mp, mq;
     int qp;
-    const bool ctb_row = !chroma && !vert && off == 0 && pc.ctb > 0 && cu.y % pc.ctb == 0;
+    const bool ctb_row = !chroma && !vert && off == 0 && (cu.y & (pc.ctb - 1)) == 0;
     if (pi == memo.pi) {
       mp = memo.mp;
       mq = memo.mq;
@@ -323,10 +323,9 @@ H266_HD inline void walk_segment(const h266_deblock_cu *cus_, const Grid &grid, 
       }
       qp = (p.qp_y + cu.qp_y + 1) >> 1;  // eq. 1274 (no LADF)
     } else {
-      const uint32_t sub = vert ? pc.sub_w : pc.sub_h;
-      const uint32_t wq = q_geo.tb_len(qx, qy, vert, true) / sub, wp = Cu{p}.tb_len(px, py, vert, true) / sub;
+      const uint32_t wq = q_geo.tb_len(qx, qy, vert, true) >> pc.sub, wp = Cu{p}.tb_len(px, py, vert, true) >> pc.sub;
       if (wp >= 8 && wq >= 8) {
-        const bool row = !vert && off == 0 && ctb_h_c > 0 && (cu.y / pc.sub_h) % ctb_h_c == 0;
+        const bool row = !vert && off == 0 && ctb_h_c > 0 && ((cu.y >> pc.sub) & (ctb_h_c - 1)) == 0;
         mp = row ? 1 : 3;
         mq = 3;
       } else {
@@ -348,8 +347,8 @@ H266_HD inline void walk_segment(const h266_deblock_cu *cus_, const Grid &grid, 
     if (tc == 0) return;  // every filter arm is a no-op at tC = 0
     if (chroma && mp == 1 && mq == 1 && bs != 2) return;  // src/deblock.rs:1823, 1888
     Emitted e;
-    e.s.x = (uint16_t)(chroma ? qx / (int)pc.sub_w : qx);
-    e.s.y = (uint16_t)(chroma ? qy / (int)pc.sub_h : qy);
+    e.s.x = (uint16_t)(qx >> pc.sub);
+    e.s.y = (uint16_t)(qy >> pc.sub);
     e.s.beta = (uint16_t)beta;
     e.s.tc = (uint16_t)tc;
     e.s.plane = (uint8_t)pc.comp;
@@ -699,9 +698,9 @@ int build_deblock_plan(const h266_picture &pic, const h266_deblock_cu *cus, uint
   if (cfi != 0 && sep) cwalk.reset(new Walker(chroma_cus, n_chroma, pw, ph, grid_chroma));
   const Walker &cw = sep && cfi != 0 ? *cwalk : luma;
   const PlaneCfg cfg[3] = {
-      {0, 1, 1, params.luma_beta_offset_div2, params.luma_tc_offset_div2, 0, bd, ctb},
-      {1, 2, 2, params.cb_beta_offset_div2, params.cb_tc_offset_div2, params.chroma_qp_offset_cb, bd, ctb},
-      {2, 2, 2, params.cr_beta_offset_div2, params.cr_tc_offset_div2, params.chroma_qp_offset_cr, bd, ctb}};
+      {0, 0, params.luma_beta_offset_div2, params.luma_tc_offset_div2, 0, bd, ctb},
+      {1, 1, params.cb_beta_offset_div2, params.cb_tc_offset_div2, params.chroma_qp_offset_cb, bd, ctb},
+      {2, 1, params.cr_beta_offset_div2, params.cr_tc_offset_div2, params.chroma_qp_offset_cr, bd, ctb}};
   auto one_list = [&](size_t l) {
     thread_local std::vector<Emitted> em;
     thread_local GroupScratch gs;
@@ -2561,14 +2560,13 @@ struct GridEmit {
   int d, p;
   __device__ void operator()(const EdgeSeg &s) const {
     const bool vert = s.flags & 1;
-    const int unit = p ? 2 : 4, pu = p ? 8 : 4;
-    const uint32_t band = (uint32_t)((vert ? s.y : s.x) / unit), pos = (uint32_t)((vert ? s.x : s.y) / pu);
+    const int us = p ? 1 : 2, ps = p ? 3 : 2, ts = p ? 5 : 6;  // log2 of the band, the cell and the tile
+    const uint32_t band = (uint32_t)(vert ? s.y : s.x) >> us, pos = (uint32_t)(vert ? s.x : s.y) >> ps;
     const uint32_t slots = a->slots[d][p];
     if (band >= a->bands[d][p] || pos >= slots) return;
     const uint32_t cell = band * slots + pos;
     a->grid[d][p][cell] = s;
     if (!a->tile_count) return;
-    const int tp = p ? kDeblockTile / 2 : kDeblockTile;
     const int halo = p ? kTileHaloYC : (a->grid8 ? kTileHaloY8 : kTileHaloY4);
     const int along = vert ? a->pw[p] : a->ph[p], bc = vert ? s.y : s.x;
     const SegSpan f = seg_span(s);
@@ -2576,14 +2574,14 @@ struct GridEmit {
     if (fs >= fe) return;  // touches no sample of the plane
     int x0, x1, y0, y1;    // tile columns and rows
     if (vert) {
-      x0 = fs / tp;
-      x1 = (fe - 1) / tp;
-      y0 = bc - halo < 0 ? 0 : (bc - halo) / tp;
-      y1 = (bc + unit + halo - 1) / tp;
+      x0 = fs >> ts;
+      x1 = (fe - 1) >> ts;
+      y0 = max(bc - halo, 0) >> ts;
+      y1 = (bc + (1 << us) + halo - 1) >> ts;
     } else {
-      x0 = x1 = bc / tp;
-      y0 = fs / tp;
-      y1 = (fe - 1) / tp;
+      x0 = x1 = bc >> ts;
+      y0 = fs >> ts;
+      y1 = (fe - 1) >> ts;
     }
     x1 = min(x1, (int)a->tiles_x - 1);
     y1 = min(y1, (int)a->tiles_y - 1);
@@ -2699,6 +2697,7 @@ __global__ void k_cu_grid(const __grid_constant__ WalkParams a, int list) {
 __device__ __forceinline__ void walk_group(const WalkParams &a, int l, uint32_t base, int part, int split,
                                            uint32_t *pre, uint32_t *mask) {
   const int plane = l / 2, d = l % 2, list = plane ? 1 : 0, lane = threadIdx.x & 31;
+  const int seg_shift = plane ? 1 + a.cfg[plane].sub : 2, step_shift = plane ? 3 + a.cfg[plane].sub : 2;
   const bool vert = d == 0;
   const h266_deblock_cu *cus = a.cus[list];
   const DevCuGrid grid{a.cu_grid[list], a.cw4, a.ch4};
@@ -2717,8 +2716,8 @@ __device__ __forceinline__ void walk_group(const WalkParams &a, int l, uint32_t 
     walks = !mine.off_grid;
     // only sub-block grids, TB splits and 64-sample TU tiling put edges inside a CU
     const bool inner = cu.has_num_sb || cu.has_tb_split || (cu.has_tu64 && mine.n_cb > 64);
-    n_off = !walks ? 0 : (inner ? (mine.n_cb + mine.step - 1) / mine.step : 1);
-    along = (mine.n_other + mine.seg - 1) / mine.seg;
+    n_off = !walks ? 0 : (inner ? (mine.n_cb + mine.step - 1) >> step_shift : 1);
+    along = (mine.n_other + mine.seg - 1) >> seg_shift;
   }
   // f(lane whose CU holds the segment, the segment's index in that CU) for this part's share of the group's segments
   auto each = [&](uint32_t nseg, auto &&f) {
@@ -2767,7 +2766,7 @@ __device__ __forceinline__ void walk_group(const WalkParams &a, int l, uint32_t 
     each((uint32_t)__popc(m) * along, [&](int j, uint32_t r) {
       const size_t idx = base + j;
       const CuWalkGeo g = cu_walk_geo(cus[idx], a.cfg[plane], vert, a.nf[d], a.n_nf[d]);
-      const uint32_t n_along = (g.n_other + g.seg - 1) / g.seg;
+      const uint32_t n_along = (g.n_other + g.seg - 1) >> seg_shift;
       uint32_t e = r / n_along, bits = mask[j];
       const uint32_t k = (r - e * n_along) * g.seg;
       for (; e; --e) bits &= bits - 1;
@@ -2902,9 +2901,9 @@ void fill_walk(const DeviceWalkIn &in, uint8_t *scratch, WalkParams &a, DeviceWa
   const h266_deblock_params &pr = in.params;
   const int bd = (int)pr.bit_depth;
   const uint32_t ctb = 1u << pr.ctb_log2_size_y;
-  a.cfg[0] = PlaneCfg{0, 1, 1, pr.luma_beta_offset_div2, pr.luma_tc_offset_div2, 0, bd, ctb};
-  a.cfg[1] = PlaneCfg{1, 2, 2, pr.cb_beta_offset_div2, pr.cb_tc_offset_div2, pr.chroma_qp_offset_cb, bd, ctb};
-  a.cfg[2] = PlaneCfg{2, 2, 2, pr.cr_beta_offset_div2, pr.cr_tc_offset_div2, pr.chroma_qp_offset_cr, bd, ctb};
+  a.cfg[0] = PlaneCfg{0, 0, pr.luma_beta_offset_div2, pr.luma_tc_offset_div2, 0, bd, ctb};
+  a.cfg[1] = PlaneCfg{1, 1, pr.cb_beta_offset_div2, pr.cb_tc_offset_div2, pr.chroma_qp_offset_cb, bd, ctb};
+  a.cfg[2] = PlaneCfg{2, 1, pr.cr_beta_offset_div2, pr.cr_tc_offset_div2, pr.chroma_qp_offset_cr, bd, ctb};
   for (int d = 0; d < 2; ++d)
     for (int p = 0; p < 3; ++p) {
       a.grid[d][p] = reinterpret_cast<EdgeSeg *>(scratch + L.grid[d][p]);
