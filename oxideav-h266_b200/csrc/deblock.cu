@@ -20,6 +20,7 @@
 #include <cstring>
 #include <memory>
 #include <numeric>
+#include <type_traits>
 
 #include "internal.h"
 #include "tma.cuh"
@@ -1638,12 +1639,7 @@ __global__ void __launch_bounds__(128, 8) k_deblock_cols(const __grid_constant__
 // bands (or strips), whose parameters are params[i].
 __device__ __forceinline__ int strip_picture(const StripParams *__restrict__ params,
                                              const uint32_t *__restrict__ first, int n, StripParams &s) {
-  int lo = 0, hi = n;  // first[lo] <= blockIdx.x < first[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (first[mid] <= blockIdx.x) lo = mid;
-    else hi = mid;
-  }
+  const int lo = tile_dev::batch_picture(first, n, blockIdx.x);
   static_assert(sizeof(StripParams) % 4 == 0, "word copy");
   const uint32_t *src = reinterpret_cast<const uint32_t *>(params + lo);
   uint32_t *dst = reinterpret_cast<uint32_t *>(&s);
@@ -1752,8 +1748,24 @@ __device__ __forceinline__ void load_window(uint16_t *sm, int pitch, const DPlan
 
 // Stores rows [y0, y0 + ih) x columns [x0, x0 + iw) (x0 a multiple of 8) from
 // the window whose origin is (ox, oy).
+// FULL: the width and height of a whole tile, whose index arithmetic is then
+// constant (a division by the run-time vector count was most of the store's
+// instructions).
+template <int FULL>
 __device__ __forceinline__ void store_window(const uint16_t *sm, int pitch, const DPlane &dst, int ox, int oy,
                                              int x0, int y0, int iw, int ih) {
+  if (iw == FULL && ih == FULL && vec_ok(dst)) {
+    const uint16_t *s0 = sm + (y0 - oy) * pitch + (x0 - ox);
+    uint16_t *d0 = dst.s + (int64_t)y0 * dst.stride + x0;
+    constexpr int NV = FULL / 8;
+#pragma unroll
+    for (int i = threadIdx.x; i < FULL * NV; i += kTileThreads) {
+      const int r = i / NV, c = (i % NV) * 8;
+      *reinterpret_cast<uint4 *>(d0 + (int64_t)r * dst.stride + c) =
+          *reinterpret_cast<const uint4 *>(s0 + r * pitch + c);
+    }
+    return;
+  }
   const int nvec = vec_ok(dst) ? iw / 8 : 0, tail = iw - nvec * 8;
   const uint16_t *s0 = sm + (y0 - oy) * pitch + (x0 - ox);
   for (int i = threadIdx.x; i < ih * nvec; i += blockDim.x) {
@@ -2047,11 +2059,13 @@ __device__ __forceinline__ void deblock_tile(const TileParams &a, const TilePara
     __syncthreads();  // the barrier's initialisation and the staged components
     bool ok = tile_dev::mbar_wait_bounded(&ts.bar, 0);
     if (ok && a.lut) {  // luma through the LMCS LUT, in place (the whole region: samples outside the plane are never read)
-      uint32_t *w = reinterpret_cast<uint32_t *>(sm);
-      for (int i = threadIdx.x; i < Geo::RH * (Geo::RW / 2); i += blockDim.x) {
-        const int r = i / (Geo::RW / 2), c = i - r * (Geo::RW / 2) + r * (Geo::PY / 2);
-        const uint32_t u = w[c];
-        w[c] = (uint32_t)a.lut[u & 0xFFFF] | (uint32_t)a.lut[u >> 16] << 16;
+      const uint16_t *lut = a.lut;
+      for (int i = threadIdx.x; i < Geo::RH * (Geo::RW / 4); i += kTileThreads) {
+        const int r = i / (Geo::RW / 4), c = i - r * (Geo::RW / 4);
+        uint2 *w = reinterpret_cast<uint2 *>(sm + r * Geo::PY + 4 * c);
+        const uint2 u = *w;
+        const uint32_t l0 = lut[u.x & 0xFFFF], l1 = lut[u.x >> 16], l2 = lut[u.y & 0xFFFF], l3 = lut[u.y >> 16];
+        *w = make_uint2(l0 | l1 << 16, l2 | l3 << 16);
       }
     }
     ok = __syncthreads_and(ok);
@@ -2068,13 +2082,17 @@ __device__ __forceinline__ void deblock_tile(const TileParams &a, const TilePara
     run_tile_pass<G8>(a, sm, ts, tx, ty, d);
     __syncthreads();
   }
-#pragma unroll
-  for (int p = 0; p < 3; ++p) {
+  auto store = [&](int p, auto full) {
+    constexpr int TP = decltype(full)::value;
     const SharedView v = tile_view<G8>(a, sm, p, tx, ty);
-    const int tp = p ? kDeblockTile / 2 : kDeblockTile, x0 = tx * tp, y0 = ty * tp;
-    const int iw = min(x0 + tp, a.dst[p].w) - x0, ih = min(y0 + tp, a.dst[p].h) - y0;
-    if (iw > 0 && ih > 0 && v.ww > 0 && v.wh > 0) store_window(v.s, v.ld, a.dst[p], v.ox, v.oy, x0, y0, iw, ih);
-  }
+    const int x0 = tx * TP, y0 = ty * TP;
+    const int iw = min(x0 + TP, a.dst[p].w) - x0, ih = min(y0 + TP, a.dst[p].h) - y0;
+    if (iw > 0 && ih > 0 && v.ww > 0 && v.wh > 0)
+      store_window<TP>(v.s, v.ld, a.dst[p], v.ox, v.oy, x0, y0, iw, ih);
+  };
+  store(0, std::integral_constant<int, kDeblockTile>{});
+  store(1, std::integral_constant<int, kDeblockTile / 2>{});
+  store(2, std::integral_constant<int, kDeblockTile / 2>{});
 }
 
 template <bool G8>
@@ -2088,12 +2106,7 @@ template <bool G8>
 __global__ void __launch_bounds__(kTileThreads, 4) k_deblock_tiles_batch(const TileParams *__restrict__ params,
                                                                          const uint32_t *__restrict__ first, int n) {
   __shared__ TileParams s_params;  // the picture's parameters, read once per CTA
-  int lo = 0, hi = n;               // first[lo] <= blockIdx.x < first[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (first[mid] <= blockIdx.x) lo = mid;
-    else hi = mid;
-  }
+  const int lo = tile_dev::batch_picture(first, n, blockIdx.x);
   static_assert(sizeof(TileParams) % 4 == 0, "word copy");
   const uint32_t *src = reinterpret_cast<const uint32_t *>(params + lo);
   uint32_t *dst = reinterpret_cast<uint32_t *>(&s_params);
@@ -2974,21 +2987,11 @@ struct WalkBatchItem {
 
 namespace {
 
-__device__ __forceinline__ int batch_pick(const uint32_t *first, int n, uint32_t b) {
-  int lo = 0, hi = n;  // first[lo] <= b < first[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (first[mid] <= b) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
 constexpr int kClearVecPerCta = 256 * 8;
 
 __global__ void __launch_bounds__(256) k_walk_clear_batch(const WalkBatchItem *__restrict__ items,
                                                           const uint32_t *__restrict__ first, int n) {
-  const int p = batch_pick(first, n, blockIdx.x);
+  const int p = tile_dev::batch_picture(first, n, blockIdx.x);
   const WalkBatchItem &it = items[p];
   const uint32_t base = (blockIdx.x - first[p]) * kClearVecPerCta, total = it.zero_vec;
 #pragma unroll
@@ -3000,7 +3003,7 @@ __global__ void __launch_bounds__(256) k_walk_clear_batch(const WalkBatchItem *_
 
 __global__ void __launch_bounds__(128) k_cu_grid_batch(const WalkBatchItem *__restrict__ items,
                                                        const uint32_t *__restrict__ first, int n) {
-  const int p = batch_pick(first, n, blockIdx.x);
+  const int p = tile_dev::batch_picture(first, n, blockIdx.x);
   const WalkParams &a = items[p].p;
   const uint32_t lb = blockIdx.x - first[p], b0 = (unpack_items(a, 0) + 127) / 128;
   const int list = lb < b0 ? 0 : 1;
@@ -3012,7 +3015,7 @@ __global__ void __launch_bounds__(128) k_cu_grid_batch(const WalkBatchItem *__re
 __global__ void __launch_bounds__(kWalkThreads) k_walk_batch(const WalkBatchItem *__restrict__ items,
                                                              const uint32_t *__restrict__ first, int n) {
   __shared__ WalkParams s;
-  const int p = batch_pick(first, n, blockIdx.x);
+  const int p = tile_dev::batch_picture(first, n, blockIdx.x);
   if (blockIdx.y >= items[p].lists) return;  // uniform per CTA
   static_assert(sizeof(WalkParams) % 4 == 0, "word copy");
   const uint32_t *src = reinterpret_cast<const uint32_t *>(&items[p].p);

@@ -649,12 +649,7 @@ template <int W, int TH, bool DO_SAO, bool DO_ALF>
 __global__ void __launch_bounds__(NT3, 4) k_sao_alf_tiles_batch(const Pass2Args *__restrict__ args,
                                                                 const uint32_t *__restrict__ first, int n) {
   __shared__ Pass2Args s_args;  // the picture's parameters, read once per CTA
-  int lo = 0, hi = n;            // first[lo] <= blockIdx.x < first[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (first[mid] <= blockIdx.x) lo = mid;
-    else hi = mid;
-  }
+  const int lo = tile_dev::batch_picture(first, n, blockIdx.x);
   static_assert(sizeof(Pass2Args) % 16 == 0, "vector copy");
   const uint4 *src = reinterpret_cast<const uint4 *>(args + lo);
   uint4 *dst = reinterpret_cast<uint4 *>(&s_args);
@@ -688,12 +683,7 @@ __global__ void __launch_bounds__(NT3, 4) k_sao_alf_tiles_queue(const Pass2Args 
     __syncthreads();  // s_item; the previous tile's last reads of s_args and the windows
     const uint32_t t = s_item;
     if (t >= total) break;
-    int lo = 0, hi = n;  // first[lo] <= t < first[hi]
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (first[mid] <= t) lo = mid;
-      else hi = mid;
-    }
+    const int lo = tile_dev::batch_picture(first, n, t);
     if (lo != cur) {
       const uint4 *src = reinterpret_cast<const uint4 *>(args + lo);
       uint4 *dst = reinterpret_cast<uint4 *>(&s_args);
@@ -894,12 +884,7 @@ template <int TW, int SW>
 __global__ void __launch_bounds__(SmemC<TW, SW>::NT) k_sao_alf_chroma_batch(const Pass2Args *__restrict__ args,
                                                                             const uint32_t *__restrict__ first, int n) {
   __shared__ Pass2Args s_args;
-  int lo = 0, hi = n;  // first[lo] <= blockIdx.x < first[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (first[mid] <= blockIdx.x) lo = mid;
-    else hi = mid;
-  }
+  const int lo = tile_dev::batch_picture(first, n, blockIdx.x);
   const uint4 *src = reinterpret_cast<const uint4 *>(args + lo);
   uint4 *dst = reinterpret_cast<uint4 *>(&s_args);
   for (int i = threadIdx.x; i < (int)(sizeof(Pass2Args) / 16); i += blockDim.x) dst[i] = src[i];

@@ -61,5 +61,16 @@ __device__ __forceinline__ void tmap_acquire(const CUtensorMap *m) {
   asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(m) : "memory");
 }
 
+// The picture of CTA b in a batched launch: the last i < n with first[i] <= b
+// (first[0] = 0, non-decreasing).  Every warp counts the entries up to b with
+// one load per 32 pictures, where a binary search was a chain of dependent
+// loads in front of everything else a CTA does.
+__device__ __forceinline__ int batch_picture(const uint32_t *__restrict__ first, int n, uint32_t b) {
+  const int lane = threadIdx.x & 31;
+  int c = 0;
+  for (int i = 0; i < n; i += 32) c += __popc(__ballot_sync(0xFFFFFFFFu, i + lane < n && first[i + lane] <= b));
+  return c - 1;
+}
+
 }  // namespace tile_dev
 }  // namespace h266
