@@ -928,7 +928,7 @@ struct h266::Prep {
     staged_pinned = false;
     if (!uploaded) H266_CUDA(cudaEventCreateWithFlags(&uploaded, cudaEventDisableTiming));
     H266_CUDA(cudaEventSynchronize(uploaded));
-    H266_TRY(pinned.ensure(blob.size()));
+    H266_TRY(pinned.ensure(blob.size() + 16));  // a pull copies whole 16-byte words
     std::memcpy(pinned.ptr, blob.data(), blob.size());
     staged_pinned = true;
     return H266_OK;
@@ -964,7 +964,7 @@ struct BatchItem {
   uint8_t *walk = nullptr;
 };
 int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<BatchItem> &items,
-               const Tuning &tn, cudaStream_t upload = nullptr);
+               const Tuning &tn, bool pull = false, cudaEvent_t planes = nullptr);
 }  // namespace h266
 
 // The tuning of a batch: the override for its largest picture's geometry, else the context's.
@@ -2512,6 +2512,8 @@ int h266_apply_in_loop_filters_batch(h266_ctx *ctx, uint32_t n, h266_picture *co
       ctx->h2d_bytes += host_plane_bytes(pic);
     }
     // then each picture's side information once its worker has prepared it
+    PullList pulls;
+    static_assert(PullList::kMax >= 16, "a group's pictures");
     for (uint32_t i = i0; i < i1; ++i) {
       const auto tw = HClock::now();
       pool->wait_item(i);
@@ -2521,9 +2523,8 @@ int h266_apply_in_loop_filters_batch(h266_ctx *ctx, uint32_t n, h266_picture *co
       GroupSlot &sl = L.slots[i - i0];
       const h266_in_loop_filter_args &a = *args[i];
       BatchItem &it = items[i - i0];
-      H266_TRY(sl.side.ensure(pr.blob.size()));
-      H266_CUDA(cudaMemcpyAsync(sl.side.ptr, pr.pinned.ptr, pr.blob.size(), cudaMemcpyHostToDevice, up));
-      H266_CUDA(cudaEventRecord(pr.uploaded, up));
+      H266_TRY(sl.side.ensure(pr.blob.size() + 16));
+      pulls.add(sl.side.ptr, pr.pinned.ptr, pr.blob.size());
       ctx->h2d_bytes += pr.blob.size();
       it.st = pr.st;
       it.st.base = sl.side.as<uint8_t>();
@@ -2552,11 +2553,10 @@ int h266_apply_in_loop_filters_batch(h266_ctx *ctx, uint32_t n, h266_picture *co
         it.walk = sl.walk.as<uint8_t>();
       }
     }
-    if (copy_streams) {
-      H266_CUDA(cudaEventRecord(L.ev_up, up));
-      H266_CUDA(cudaStreamWaitEvent(L.stream, L.ev_up, 0));
-    }
-    H266_TRY(exec_batch(ctx, L.bb, L.stream, items, tn, copy_streams ? up : nullptr));
+    H266_TRY(launch_pull(L.stream, pulls, &ctx->launches));
+    for (uint32_t i = i0; i < i1; ++i) H266_CUDA(cudaEventRecord(ctx->preps[i + 1]->uploaded, L.stream));
+    if (copy_streams) H266_CUDA(cudaEventRecord(L.ev_up, up));
+    H266_TRY(exec_batch(ctx, L.bb, L.stream, items, tn, true, copy_streams ? L.ev_up : nullptr));
     const cudaStream_t down = copy_streams ? ctx->e2e_down : L.stream;
     if (copy_streams) {
       H266_CUDA(cudaEventRecord(L.ev_comp, L.stream));
@@ -2810,11 +2810,11 @@ int check_plan_batch(h266_ctx *ctx, uint32_t n, h266_chain_plan *const *plans, h
 // per region size over every picture's tiles, the strip kernels' two launches
 // over every other picture, one SAO/ALF launch per kernel variant, and per
 // picture whatever the batched kernels do not take.
-// `upload`: the stream that carries the parameter table's upload (the
-// end-to-end pipeline's upload stream, so that the table is copied in issue
-// order with the planes instead of competing with them); `stream` by default.
+// `pull`: the parameter table is read from its staging by a kernel (the
+// end-to-end pipeline, whose planes keep the copy engine busy).  `planes`: the
+// planes' uploads; the edge walk, which reads none, runs before it.
 int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<BatchItem> &items,
-               const Tuning &tn, cudaStream_t upload) {
+               const Tuning &tn, bool pull, cudaEvent_t planes) {
   const uint32_t n = (uint32_t)items.size();
   if (!n) return H266_OK;
   H266_TRY(bb.init());
@@ -2952,17 +2952,22 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
       off_p2[v] = blob.put(p2[v].data(), p2[v].size() * sizeof(Pass2Args));
       off_p2f[v] = blob.put(p2_first[v].data(), p2_first[v].size() * sizeof(uint32_t));
     }
-  H266_TRY(bb.side.ensure(b.size()));
-  const cudaStream_t ups = upload ? upload : stream;
+  const size_t pad = pull ? 16 : 0;  // a pull copies whole 16-byte words
+  H266_TRY(bb.side.ensure(b.size() + pad));
   if (!bb.capturing) {
-    H266_CUDA(cudaStreamWaitEvent(ups, bb.done, 0));  // earlier batches read bb.side (any stream)
+    H266_CUDA(cudaStreamWaitEvent(stream, bb.done, 0));  // earlier batches read bb.side (any stream)
     H266_CUDA(cudaEventSynchronize(bb.staged));      // the previous upload has read the staging buffer
   }
-  H266_TRY(bb.stage.ensure(b.size()));
+  H266_TRY(bb.stage.ensure(b.size() + pad));
   std::memcpy(bb.stage.ptr, b.data(), b.size());
-  H266_CUDA(cudaMemcpyAsync(bb.side.ptr, bb.stage.ptr, b.size(), cudaMemcpyHostToDevice, ups));
-  H266_CUDA(cudaEventRecord(bb.staged, ups));
-  if (ups != stream) H266_CUDA(cudaStreamWaitEvent(stream, bb.staged, 0));
+  if (pull) {
+    PullList l;
+    l.add(bb.side.ptr, bb.stage.ptr, b.size());
+    H266_TRY(launch_pull(stream, l, &ctx->launches));
+  } else {
+    H266_CUDA(cudaMemcpyAsync(bb.side.ptr, bb.stage.ptr, b.size(), cudaMemcpyHostToDevice, stream));
+  }
+  H266_CUDA(cudaEventRecord(bb.staged, stream));
   const uint8_t *dside = bb.side.as<uint8_t>();
   // deblocking: the batched walks, per picture where only global memory takes the planes, then the batched strips and tiles
   if (walk_first[0].size() > 1) {
@@ -2975,6 +2980,7 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
                                reinterpret_cast<const uint32_t *>(dside + off_wf[2]), (int)walk_first[0].size() - 1,
                                walk_total, &ctx->launches));
   }
+  if (planes) H266_CUDA(cudaStreamWaitEvent(stream, planes, 0));
   for (uint32_t i = 0; i < n; ++i) {
     BatchItem &it = items[i];
     if (runs[i].tile || runs[i].strips) continue;

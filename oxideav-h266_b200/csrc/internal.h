@@ -445,6 +445,18 @@ int launch_chroma_residual(cudaStream_t st, DPlane cb, DPlane cr, const ResPiece
                            const int32_t *d_res, int bd, uint64_t *launches);
 int launch_output_dump(cudaStream_t st, const OutPlanes &o, uint8_t *d_dst, bool wide, uint64_t *launches);
 
+// Copies pinned host memory (16-byte aligned) to the device by a kernel, whole
+// 16-byte words: both sides have room for the rounded size.
+struct PullList {
+  static constexpr int kMax = 16;
+  const void *src[kMax];
+  void *dst[kMax];
+  uint32_t vec[kMax], first[kMax + 1] = {0};
+  int n = 0;
+  void add(void *to, const void *from, size_t bytes);
+};
+int launch_pull(cudaStream_t st, const PullList &l, uint64_t *launches);
+
 // Encoder chroma ALF / CC-ALF trials (alf_enc.cu): the n_cand candidate filters
 // of one chroma component per CTB, the first minimum of {off, candidates} in
 // pick[] (-1: off) and committed to `rec`.

@@ -356,4 +356,48 @@ int launch_output_dump(cudaStream_t st, const OutPlanes &o, uint8_t *d_dst, bool
   return H266_OK;
 }
 
+// ---- host staging pulled by a kernel
+//
+// While a picture's planes cross the link in both directions, a small
+// host-to-device copy on the copy engine waits its turn against the downloads:
+// the 0.2 MB of a picture's side information took 50-70 us each (8 alone) and
+// held up the planes behind it.  Threads reading the pinned staging directly
+// share the link instead of the engine's queue, and run on the group's own
+// stream, with the edge walk, before the planes have arrived.  16 1080p pictures
+// end to end: 3.85 -> 3.55 ms.
+namespace {
+constexpr int kPullThreads = 256, kPullVec = 4;  // 16-byte words per thread, loaded before any is stored
+__global__ void __launch_bounds__(kPullThreads) k_pull(const __grid_constant__ PullList l) {
+  int p = 0;
+  while (p + 1 < l.n && blockIdx.x >= l.first[p + 1]) ++p;
+  const uint4 *src = static_cast<const uint4 *>(l.src[p]);
+  uint4 *dst = static_cast<uint4 *>(l.dst[p]);
+  const uint32_t base = (blockIdx.x - l.first[p]) * (kPullThreads * kPullVec) + threadIdx.x;
+  uint4 v[kPullVec];
+#pragma unroll
+  for (int k = 0; k < kPullVec; ++k)
+    if (base + k * kPullThreads < l.vec[p]) v[k] = __ldcv(src + base + k * kPullThreads);  // host memory: read anew
+#pragma unroll
+  for (int k = 0; k < kPullVec; ++k)
+    if (base + k * kPullThreads < l.vec[p]) dst[base + k * kPullThreads] = v[k];
+}
+}  // namespace
+
+void PullList::add(void *to, const void *from, size_t bytes) {
+  constexpr uint32_t per = kPullThreads * kPullVec;
+  dst[n] = to;
+  src[n] = from;
+  vec[n] = (uint32_t)((bytes + 15) / 16);
+  first[n + 1] = first[n] + (vec[n] + per - 1) / per;
+  ++n;
+}
+
+int launch_pull(cudaStream_t st, const PullList &l, uint64_t *launches) {
+  if (!l.n || !l.first[l.n]) return H266_OK;
+  k_pull<<<l.first[l.n], kPullThreads, 0, st>>>(l);
+  H266_CUDA(cudaGetLastError());
+  ++*launches;
+  return H266_OK;
+}
+
 }  // namespace h266
