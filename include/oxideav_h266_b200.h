@@ -291,12 +291,12 @@ int h266_ctx_set_profiling(h266_ctx *ctx, int on);
  *                          (values in between: 64)
  *   "prep_threads"         host threads preparing pictures' side information (0 = half the host
  *                          threads less two, 2..16; 1..64); a context-wide value
- *   "e2e_copy_streams"     1: every upload (planes, side information, batch tables) in issue order
- *                          on one stream and every download on another (default); 0: each group's
- *                          copies on its group's stream
- *   "e2e_ramp"             1: the batch starts and ends with groups of 1, 2, 4 ... pictures, so the
- *                          first kernels start and the last downloads end sooner (default); 0: all
- *                          groups of e2e_group pictures
+ *   "e2e_copy_streams"     1: every plane's upload in issue order on one stream and every download on
+ *                          another (default); 0: each group's copies on its group's stream.  Side
+ *                          information and batch tables are read by a kernel on the group's stream
+ *   "e2e_ramp"             1: a batch of host pictures makes at least three groups, so that uploads,
+ *                          kernels and downloads overlap in a short batch too (default); 0: groups
+ *                          of e2e_group pictures whatever the batch
  * h266_ctx_set_tuning sets the context's value; h266_ctx_set_tuning_for sets
  * it for batches whose largest picture has that luma size and bit depth, which
  * takes precedence.  Unknown keys or out-of-range values: H266_ERR_INVALID_ARGUMENT. */

@@ -212,12 +212,11 @@ struct GroupSlot {
 struct Tuning {
   int e2e_group = 4, e2e_lanes = 4, sao_alf_ctas_per_sm = 0, sao_alf_tile_h = 64;
   int prep_threads = 0;  // 0: the default count
-  // 1: every upload of the end-to-end batch (planes, side information, batch
-  // tables) in issue order on one stream and every download on another, so
-  // small latency-critical copies do not wait behind other lanes' planes in
-  // the copy engine (measured 9.0 against 10.3 ms per 32 x 1080p)
+  // 1: every plane of the end-to-end batch is uploaded in issue order on one
+  // stream and every download runs on another (16 x 1080p: 3.33 ms; a second
+  // stream for chroma uploads 3.72, for chroma downloads 3.48)
   int e2e_copy_streams = 1;
-  int e2e_ramp = 1;  // 1: the end-to-end batch starts and ends with groups of 1, 2, ... pictures
+  int e2e_ramp = 1;  // 1: an end-to-end batch of host pictures has three groups at least
 };
 struct TuningKey {
   const char *name;
@@ -2415,33 +2414,15 @@ int h266_apply_in_loop_filters_batch(h266_ctx *ctx, uint32_t n, h266_picture *co
   Guard g(ctx->device);
   const Tuning &tn = batch_tuning(ctx, n, pics);
   const uint32_t kGroup = (uint32_t)tn.e2e_group, kGroupLanes = (uint32_t)tn.e2e_lanes;
-  // Group boundaries.  With e2e_ramp the batch starts and ends with small
-  // groups (1, 2, ... and ..., 2, 1 pictures): the first kernels and
-  // downloads start after one picture's upload instead of a whole group's,
-  // and the last group's kernels and downloads, which nothing overlaps, are
-  // one picture's.
+  // Group boundaries.  With e2e_ramp pictures in host memory make at least three groups, so that
+  // uploads, kernels and downloads of different groups overlap in a short batch
+  // too.  1080p, groups of 4: 5 pictures 1.52 -> 1.40 ms, 8 2.00 -> 1.91, 9 at
+  // 2160p 7.5 -> 6.9.  Ends of 1, 2, ... pictures cost more launches, and more
+  // turns between the copy directions, than their earlier start gave: 16
+  // pictures 3.54 ms against 3.33.
   std::vector<uint32_t> gb(1, 0);
-  {
-    std::vector<uint32_t> ramp;
-    for (uint32_t g = 1; g < kGroup; g *= 2) ramp.push_back(g);
-    uint32_t ends = 0;
-    for (uint32_t g : ramp) ends += 2 * g;
-    const bool use_ramp = tn.e2e_ramp && n >= ends + 2 * kGroup;
-    uint32_t left = n;
-    if (use_ramp)
-      for (uint32_t g : ramp) {
-        gb.push_back(gb.back() + g);
-        left -= g;
-      }
-    const uint32_t tail = use_ramp ? ends / 2 : 0;
-    while (left > tail) {
-      const uint32_t g = std::min(kGroup, left - tail);
-      gb.push_back(gb.back() + g);
-      left -= g;
-    }
-    if (use_ramp)
-      for (size_t k = ramp.size(); k-- > 0;) gb.push_back(gb.back() + ramp[k]);
-  }
+  const uint32_t per = tn.e2e_ramp && any_host ? std::min(kGroup, (n + 2) / 3) : kGroup;
+  while (gb.back() < n) gb.push_back(std::min(gb.back() + per, n));
   const uint32_t n_groups = (uint32_t)gb.size() - 1, n_lanes = std::min(n_groups, kGroupLanes);
   for (auto &l : ctx->glanes)  // a larger group than the lanes were made for: more slots
     if (l->slots.size() < kGroup) l->slots.resize(kGroup);
