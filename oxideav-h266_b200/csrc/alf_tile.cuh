@@ -583,5 +583,49 @@ __device__ __forceinline__ void cc_alf_run(const uint16_t *L0, int pitch, int yl
   }
 }
 
+// The same of 4 chroma samples of 4:4:4, whose luma samples are adjacent
+// (L0 8-byte aligned): every tap pair is a natural word of a row, with the
+// bytes of the coefficients placed for the even or the odd sample of a word.
+__device__ __forceinline__ void cc_alf_run_444(const uint16_t *L0, int pitch, int yline, int ctb, bool lbb,
+                                               const int32_t *cc_k, int bd, int maxv, int v[4]) {
+  uint32_t b[7];
+  int csum = 0;
+#pragma unroll
+  for (int k = 0; k < 7; ++k) {
+    b[k] = (uint32_t)(cc_k[k] & 0xFF);
+    csum += cc_k[k];
+  }
+  const uint32_t m_even = b[1] << 8 | b[2] << 24, m_odd = b[1] | b[2] << 16;  // low: the earlier word
+  const uint32_t d_even = b[3] << 8 | b[4] << 16 | b[5] << 24, d_odd = b[3] | b[4] << 8 | b[5] << 16;
+  const uint32_t t_k = b[0] | b[0] << 24, u_k = b[6] | b[6] << 24;  // low: even sample, high: odd
+  const int half = 1 << (bd - 1);
+  int yp1 = 1, yp2 = 2;
+  if (lbb) {
+    if (yline == ctb - 5 || yline == ctb - 4) { yp1 = 0; yp2 = 0; }
+    else if (yline == ctb - 6 || yline == ctb - 3) { yp2 = 1; }
+  }
+  Words<4, 1> m, d;  // word k: samples (2k - 2, 2k - 1)
+  load_words<4, 1, true>(m, L0, 0, 4);
+  load_words<4, 1, true>(d, L0 + yp1 * pitch, 0, 4);
+  const uint2 tw = ld64(L0 - yp1 * pitch), uw = ld64(L0 + yp2 * pitch);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int t = (int)(k ? tw.y : tw.x), u = (int)(k ? uw.y : uw.x), c = (int)m.w[k + 1];
+    int e = __dp2a_lo(t, (int)t_k, 0), o = __dp2a_hi(t, (int)t_k, 0);
+    e = __dp2a_lo((int)m.w[k], (int)m_even, e);
+    e = __dp2a_hi(c, (int)m_even, e);
+    o = __dp2a_lo(c, (int)m_odd, o);
+    o = __dp2a_hi((int)m.w[k + 2], (int)m_odd, o);
+    e = __dp2a_lo((int)d.w[k], (int)d_even, e);
+    e = __dp2a_hi((int)d.w[k + 1], (int)d_even, e);
+    o = __dp2a_lo((int)d.w[k + 1], (int)d_odd, o);
+    o = __dp2a_hi((int)d.w[k + 2], (int)d_odd, o);
+    e = __dp2a_lo(u, (int)u_k, e) - (int)(int16_t)c * csum;  // biased like the taps: the biases cancel
+    o = __dp2a_hi(u, (int)u_k, o) - (c >> 16) * csum;
+    v[2 * k] = clampd(v[2 * k] + clampd((e + 64) >> 7, -half, half - 1), 0, maxv);
+    v[2 * k + 1] = clampd(v[2 * k + 1] + clampd((o + 64) >> 7, -half, half - 1), 0, maxv);
+  }
+}
+
 }  // namespace tile
 }  // namespace h266

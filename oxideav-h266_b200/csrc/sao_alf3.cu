@@ -706,20 +706,25 @@ __host__ __device__ inline int chroma_tiles_x(const Pass2Args &a, int tw) {
 //
 // SAO, 5x5 ALF and CC-ALF of both chroma planes of formats with full-height
 // chroma, beside the luma tiles of the packed kernel: one CTA per TW x 32 chroma
-// samples (32 x 32; 16 x 32 for the 16-sample-wide CTBs of 4:2:2 at CTB 32, so
-// that a tile never straddles a CTB) for Cb, then Cr.  The post-SAO luma window
-// that CC-ALF reads is staged once for both planes and only where the CTB has a
-// CC filter; windows go through the branch-free SAO quads, the diamond runs four
-// samples a thread in the packed form.  With the luma tiles 65 us per 1080p
-// 4:4:4 10-bit picture in a batch of four, against 131 us for the scalar pass
-// over all planes.
+// samples of both planes (32 x 32; 16 x 32 for the 16-sample-wide CTBs of 4:2:2 at
+// CTB 32, so that a tile never straddles a CTB).  The windows of both planes, and
+// of luma where the CTB has a CC filter, are loaded side by side while the SAO
+// parameters resolve, then go through the branch-free SAO quads together (each
+// window's leftover quads on other warps): three barriers in all.  The diamond
+// and CC-ALF run four samples a thread, CC-ALF by dp2a on natural words.  Four
+// 1080p 4:4:4 10-bit pictures: 182 -> 149 us against one window after the other,
+// eight barriers, scalar CC taps and four CTAs an SM instead of five (160 us).
+// The ALU pipe and the waits between its instructions bound it.  The tile's own
+// quads in a loop of their own, with one set of parameters, cost more in
+// instruction-cache misses than they saved (165 us).
 template <int TW, int SW>
 struct SmemC {
   static constexpr int NT = TW * 8, TH = 32, LW = TW * SW;
   static constexpr int DW = TW + 16, DH = TH + 6, SCW = TW + 8, SCH = TH + 4, SCP = SCW + 4;  // [x - 8, y - 3), [x - 4, y - 2)
   static constexpr int DLW = LW + 16, DLH = TH + 5, SLW = LW + 8, SLH = TH + 3, SLP = SLW + 4;  // [x - 8, y - 2), [x - 4, y - 1)
-  alignas(16) uint16_t d[DW * DH > DLW * DLH ? DW * DH : DLW * DLH];  // the deblocked window in turn
-  alignas(16) uint16_t sC[SCH * SCP];
+  alignas(16) uint16_t dC[2][DW * DH];
+  alignas(16) uint16_t dL[DLW * DLH];
+  alignas(16) uint16_t sC[2][SCH * SCP];
   alignas(16) uint16_t sL[SLH * SLP];
   SaoLocal sao[3][9];
   SaoFast fast[3][9];
@@ -765,101 +770,102 @@ __device__ __forceinline__ void chroma_tile(const Pass2Args &a, int tile) {
     sm.fast[comp][n] = sao_fast(s, pitch);
   }
   const bool quads = a.sao_i8 && bd <= 12;
-  uint32_t seen = 0;
-  // Post-SAO window of component `comp`: W x H at (wx0, wy0), pitch P, from the
-  // deblocked window DW wide with origin (wx0 - 4, wy0 - 1), clamped into
-  // [fx0, fx1) x [fy0, fy1); lx, ly: log2 of the CTB in the component's samples.
-  auto window = [&](int comp, uint16_t *out, int P, int W, int H, int DWp, int wx0, int wy0, int fx0, int fy0, int fx1,
-                    int fy1, int lx, int ly) {
-    const DPlane &src = a.src[comp];
-    const int dx0 = wx0 - 4, dy0 = wy0 - 1, dw = W + 8, dh = H + 2;
-    __syncthreads();  // the parameters; the previous window's last reads of sm.d
+  const bool cc_any = a.do_alf && me && have_luma && (me->cc_filt[0] >= 0 || me->cc_filt[1] >= 0);
+  bool on[2];
+  for (int cc = 0; cc < 2; ++cc) on[cc] = xc0 < a.src[1 + cc].w && yc0 < a.src[1 + cc].h;  // uniform per CTA
+  // The deblocked window of `src`, dw x dh at (dx0, dy0), clamped into the plane.
+  auto load = [&](const DPlane &src, uint16_t *d, int dx0, int dy0, auto dwc, auto dhc) {
+    constexpr int dw = decltype(dwc)::value, dh = decltype(dhc)::value, nv = dw / 8;
     if (dx0 >= 0 && dx0 + dw <= src.w && ((uintptr_t)src.s & 15) == 0 && (src.stride & 7) == 0) {
-      const int nv = dw / 8;
       for (int i = tid; i < dh * nv; i += NT) {
         const int r = i / nv, c = (i - r * nv) * 8, gy = clampd(dy0 + r, 0, src.h - 1);
-        *reinterpret_cast<uint4 *>(&sm.d[r * DWp + c]) =
+        *reinterpret_cast<uint4 *>(&d[r * dw + c]) =
             *reinterpret_cast<const uint4 *>(src.s + (int64_t)gy * src.stride + dx0 + c);
       }
     } else {
       for (int i = tid; i < dh * dw; i += NT) {
         const int r = i / dw, c = i - r * dw;
-        sm.d[r * DWp + c] =
-            src.s[(int64_t)clampd(dy0 + r, 0, src.h - 1) * src.stride + clampd(dx0 + c, 0, src.w - 1)];
+        d[r * dw + c] = src.s[(int64_t)clampd(dy0 + r, 0, src.h - 1) * src.stride + clampd(dx0 + c, 0, src.w - 1)];
       }
     }
-    __syncthreads();
-    const int wq = W / 4;
-    for (int i = tid; i < wq * H; i += NT) {
-      const int r = i / wq, x = wx0 + 4 * (i - r * wq), y = wy0 + r;
+  };
+  using CDW = std::integral_constant<int, S::DW>;
+  using CDH = std::integral_constant<int, S::DH>;
+  for (int cc = 0; cc < 2; ++cc)
+    if (on[cc]) load(a.src[1 + cc], sm.dC[cc], xc0 - 8, yc0 - 3, CDW{}, CDH{});
+  if (cc_any)
+    load(a.src[0], sm.dL, X0 - 8, Y0 - 2, std::integral_constant<int, S::DLW>{}, std::integral_constant<int, S::DLH>{});
+  __syncthreads();
+  // Post-SAO window of component `comp`: W x H at (wx0, wy0), clamped into
+  // [fx0, fx1) x [fy0, fy1); lx: log2 of the CTB's width in the component's
+  // samples; `rot`: the thread that takes the first quad.
+  uint32_t seen = 0;
+  auto window = [&](int comp, const uint16_t *din, uint16_t *out, int wx0, int wy0, int fx0, int fy0, int fx1, int fy1,
+                    int lx, int rot, auto wc, auto hc) {
+    constexpr int W = decltype(wc)::value, H = decltype(hc)::value, P = W + 4, DP = W + 8, WQ = W / 4;
+    const int dx0 = wx0 - 4, dy0 = wy0 - 1;
+    for (int i = (tid + NT - rot) % NT; i < WQ * H; i += NT) {
+      const int r = i / WQ, x = wx0 + 4 * (i - r * WQ), y = wy0 + r;
       uint2 v;
       bool fast = x >= fx0 && x + 4 <= fx1 && y >= fy0 && y < fy1;
       int n = 4;
       if (fast) {
-        n = ((y >> ly) - ry + 1) * 3 + ((x >> lx) - rx + 1);
+        n = ((y >> log2) - ry + 1) * 3 + ((x >> lx) - rx + 1);
         const SaoLocal &p = sm.sao[comp][n];
         fast = !p.type || (quads && (p.type != 2 || (x >= p.ex0 && x + 4 <= p.ex1 && y >= p.ey0 && y < p.ey1)));
       }
       if (fast) {
-        v = sao_quad_any(sm.fast[comp][n], &sm.d[(y - dy0) * DWp + (x - dx0)], maxv2);
+        v = sao_quad_any(sm.fast[comp][n], &din[(y - dy0) * DP + (x - dx0)], maxv2);
       } else {
         const int ay = clampd(y, fy0, fy1 - 1);
         uint32_t s4[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const int ax = clampd(x + k, fx0, fx1 - 1);
-          const uint16_t *d = &sm.d[(ay - dy0) * DWp + (ax - dx0)];
-          const SaoLocal &p = sm.sao[comp][((ay >> ly) - ry + 1) * 3 + ((ax >> lx) - rx + 1)];
+          const uint16_t *d = &din[(ay - dy0) * DP + (ax - dx0)];
+          const SaoLocal &p = sm.sao[comp][((ay >> log2) - ry + 1) * 3 + ((ax >> lx) - rx + 1)];
           s4[k] = p.type ? (uint32_t)(uint16_t)sao_one(p, ax, ay, maxv, d) : *d;
         }
         v = make_uint2(s4[0] | s4[1] << 16, s4[2] | s4[3] << 16);
       }
-      seen |= v.x | v.y;
+      if (comp) seen |= v.x | v.y;
       st64(&out[r * P + (x - wx0)], make_uint2(v.x ^ kBias, v.y ^ kBias));
     }
   };
-  const int lxc = SW == 2 ? log2 - 1 : log2;
-  const bool cc_any = a.do_alf && me && have_luma && (me->cc_filt[0] >= 0 || me->cc_filt[1] >= 0);
+  constexpr int CQ = S::SCW / 4 * S::SCH % NT;  // a chroma window's leftover quads
   if (cc_any)
-    window(0, sm.sL, S::SLP, S::SLW, S::SLH, S::DLW, X0 - 4, Y0 - 1, max(rect[0], 0), max(rect[1], 0), min(rect[2], pw),
-           min(rect[3], ph), log2, log2);
+    window(0, sm.dL, sm.sL, X0 - 4, Y0 - 1, max(rect[0], 0), max(rect[1], 0), min(rect[2], pw), min(rect[3], ph), log2,
+           2 * CQ % NT, std::integral_constant<int, S::SLW>{}, std::integral_constant<int, S::SLH>{});
+#pragma unroll 1
+  for (int cc = 0; cc < 2; ++cc)
+    if (on[cc])
+      window(1 + cc, sm.dC[cc], sm.sC[cc], xc0 - 4, yc0 - 2, max(rect[0] / SW, 0), max(rect[1], 0),
+             min((rect[2] + SW - 1) / SW, a.src[1 + cc].w), min(rect[3], a.src[1 + cc].h), SW == 2 ? log2 - 1 : log2,
+             cc * CQ, std::integral_constant<int, S::SCW>{}, std::integral_constant<int, S::SCH>{});
+  const bool big = __syncthreads_or((seen & 0xC000C000u) != 0) != 0;
+  const int j = tid / (TW / 4), i0 = (tid % (TW / 4)) * 4, gx = xc0 + i0, gy = yc0 + j, jr = gy - y_ctb;
 #pragma unroll 1
   for (int cc = 0; cc < 2; ++cc) {
-    const DPlane CS = a.src[1 + cc], CD = a.dst[1 + cc];
-    if (CS.w <= 0 || CS.h <= 0 || xc0 >= CS.w || yc0 >= CS.h) continue;  // uniform per CTA
-    seen = 0;
-    window(1 + cc, sm.sC, S::SCP, S::SCW, S::SCH, S::DW, xc0 - 4, yc0 - 2, max(rect[0] / SW, 0), max(rect[1], 0),
-           min((rect[2] + SW - 1) / SW, CS.w), min(rect[3], CS.h), lxc, log2);
-    const bool big = __syncthreads_or((seen & 0xC000C000u) != 0) != 0;
-    const int j = tid / (TW / 4), i0 = (tid % (TW / 4)) * 4, gx = xc0 + i0, gy = yc0 + j;
-    if (gx >= CD.w || gy >= CD.h) continue;
+    const DPlane CD = a.dst[1 + cc];
+    if (!on[cc] || gx >= CD.w || gy >= CD.h) continue;
     const int cf = a.do_alf && me ? me->chroma_filt[cc] : -1;
     const int ccf = a.do_alf && me && have_luma ? me->cc_filt[cc] : -1;
-    const uint16_t *R0 = &sm.sC[(j + 2) * S::SCP + i0 + 4];
+    const uint16_t *R0 = &sm.sC[cc][(j + 2) * S::SCP + i0 + 4];
     const uint2 w = ld64(R0);
     int v[4] = {(int)((w.x ^ kBias) & 0xFFFF), (int)((w.x ^ kBias) >> 16), (int)((w.y ^ kBias) & 0xFFFF),
                 (int)((w.y ^ kBias) >> 16)};
-    const int jr = gy - y_ctb;
     if (cf >= 0) chroma_alf_run<4>(R0, S::SCP, jr, ctb, a.tables.chroma_packed[min(cf, 7)], maxv, big, v);
     if (ccf >= 0) {  // CC-ALF (apply_cc_alf_ctb, src/alf.rs:447-523)
-      const int *k = a.tables.cc_coeff[cc][ccf];
+      const uint16_t *L0 = &sm.sL[(j + 1) * S::SLP + SW * i0 + 4];
       const bool lbb = !(gy + ctb >= ph && (ph - y_ctb) <= ctb - 4);
-      int yp1 = 1, yp2 = 2;  // Table 47
-      if (lbb) {
-        if (jr == ctb - 5 || jr == ctb - 4) { yp1 = 0; yp2 = 0; }
-        else if (jr == ctb - 6 || jr == ctb - 3) { yp2 = 1; }
-      }
-      const bool suppress = jr == ctb - 3 || jr == ctb - 4;
-      const int half = 1 << (bd - 1);
-      const uint16_t *L = &sm.sL[(j + 1) * S::SLP + SW * i0 + 4];
-      const int csum = k[0] + k[1] + k[2] + k[3] + k[4] + k[5] + k[6];
+      const int32_t *k = a.tables.cc_coeff[cc][ccf];
+      if (jr == ctb - 3 || jr == ctb - 4) {  // no correction beside the line buffer
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {  // biased samples: the bias drops out with csum
-        const uint16_t *c = L + SW * q, *d1 = c + yp1 * S::SLP;
-        const int sum = k[0] * c[-yp1 * S::SLP] + k[1] * c[-1] + k[2] * c[1] + k[3] * d1[-1] + k[4] * d1[0] +
-                        k[5] * d1[1] + k[6] * c[yp2 * S::SLP] - csum * c[0];
-        const int scaled = clampd((sum + 64) >> 7, -half, half - 1);
-        v[q] = clampd(suppress ? v[q] : v[q] + scaled, 0, maxv);
+        for (int q = 0; q < 4; ++q) v[q] = clampd(v[q], 0, maxv);
+      } else if constexpr (SW == 1) {
+        cc_alf_run_444(L0, S::SLP, jr, ctb, lbb, k, bd, maxv, v);
+      } else {
+        cc_alf_run<4>(L0, S::SLP, jr, ctb, lbb, k, bd, maxv, v);
       }
     }
     uint16_t *out = CD.s + (int64_t)gy * CD.stride + gx;
@@ -875,13 +881,13 @@ __device__ __forceinline__ void chroma_tile(const Pass2Args &a, int tile) {
 }
 
 template <int TW, int SW>
-__global__ void __launch_bounds__(SmemC<TW, SW>::NT) k_sao_alf_chroma(const __grid_constant__ Pass2Args a) {
+__global__ void __launch_bounds__(SmemC<TW, SW>::NT, 1280 / SmemC<TW, SW>::NT) k_sao_alf_chroma(const __grid_constant__ Pass2Args a) {
   chroma_tile<TW, SW>(a, blockIdx.x);
 }
 
 // Many pictures in one grid, as k_sao_alf_tiles_batch.
 template <int TW, int SW>
-__global__ void __launch_bounds__(SmemC<TW, SW>::NT) k_sao_alf_chroma_batch(const Pass2Args *__restrict__ args,
+__global__ void __launch_bounds__(SmemC<TW, SW>::NT, 1280 / SmemC<TW, SW>::NT) k_sao_alf_chroma_batch(const Pass2Args *__restrict__ args,
                                                                             const uint32_t *__restrict__ first, int n) {
   __shared__ Pass2Args s_args;
   const int lo = tile_dev::batch_picture(first, n, blockIdx.x);
