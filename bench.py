@@ -46,12 +46,13 @@ WIDTH, HEIGHT, BITDEPTH = 1920, 1080, 10
 METRIC = "filter-chain Mpx/s 1080p/2160p 10-bit bit-exact"
 # From one ncu capture of the batched SAO/ALF launch (k_sao_alf_tiles_batch
 # <64, 64, 1, 1>) over 4 pictures of this workload: DRAM bytes read + written
-# (25 679 616 + 1 021 696 B; ncu flushes the caches before the launch, and the
+# (25 031 680 + 2 758 400 B; ncu flushes the caches before the launch, and the
 # output planes retire from L2 after it) and thread instructions per luma pixel
-# (warp instructions x threads per warp instruction); the bench line scales
-# them to its own batch and labels them so.
-SAO_ALF_TRAFFIC_PER_PX = (25679616 + 1021696) / (4 * 1920 * 1080)
-SAO_ALF_THREAD_INST_PER_PX = 332.6  # 87 940 862 warp instructions x 31.37 threads / 4 pictures
+# (warp instructions x 32 lanes: the issue rate they are set against counts the
+# lanes of a partly active warp too); the bench line scales them to its own
+# batch and labels them so.
+SAO_ALF_TRAFFIC_PER_PX = (25031680 + 2758400) / (4 * 1920 * 1080)
+SAO_ALF_THREAD_INST_PER_PX = 266.6  # 69 098 582 warp instructions x 32 lanes / 4 pictures
 
 
 def _import_pkg():
@@ -613,23 +614,27 @@ def run_encoder_trials(ctx, local_rank, stream, steps: int, n_pics: int = 4):
     torch.cuda.synchronize()
     m_total, m_calls = 0.0, 0
     for _ in range(max(1, steps)):
+        m_launches = ctx.kernel_launches
         e0.record(stream)
         native.sao_chroma_merge(ctx, d[0], d[1], indep, 15, 9, bit_depth=10, ctb_log2=7)
+        m_launches = ctx.kernel_launches - m_launches
         e1.record(stream)
         torch.cuda.synchronize()
         m_total += e0.elapsed_time(e1)
         m_calls += 1
     t0 = time.perf_counter()
     oracle.sao_chroma_merge(s_, r_, indep, 15, 9, bit_depth=10, ctb_log2=7)
-    sao["chroma_merge"] = {"ms_per_picture": round(m_total / m_calls, 4), "launches": 23,
+    sao["chroma_merge"] = {"ms_per_picture": round(m_total / m_calls, 4), "launches": m_launches,
                            "cpu_oracle_ms_per_picture": round((time.perf_counter() - t0) * 1e3, 1)}
-    # the same merge batched over the 4 pictures: one launch per anti-diagonal for all of them
+    # the same merge batched over the 4 pictures: the same launches for all of them
     indeps = [native.sao_decide_picture(ctx, d_[0], d_[1], ctb_log2=7, bit_depth=10) for d_ in devs]
     want_b = [native.sao_chroma_merge(ctx, d_[0], d_[1], ind, 15, 9, bit_depth=10, ctb_log2=7)
               for d_, ind in zip(devs, indeps)]
     run_b = lambda: native.sao_chroma_merge_batch(ctx, [d_[0] for d_ in devs], [d_[1] for d_ in devs], indeps,
                                                   [(15, 9)] * len(devs), bit_depth=10, ctb_log2=7)
+    b_launches = ctx.kernel_launches
     got_b = run_b()
+    b_launches = ctx.kernel_launches - b_launches
     same = all(np.array_equal(g[1], w[1]) and g[0].tobytes() == w[0].tobytes() for g, w in zip(got_b, want_b))
     torch.cuda.synchronize()
     t0 = time.perf_counter()
@@ -637,7 +642,7 @@ def run_encoder_trials(ctx, local_rank, stream, steps: int, n_pics: int = 4):
         run_b()
     b_ms = (time.perf_counter() - t0) * 1e3 / max(1, steps) / len(devs)
     sao["chroma_merge_batch"] = {"pictures": len(devs), "ms_per_picture": round(b_ms, 4),
-                                 "launches_per_call": 23, "same_as_per_picture_calls": bool(same),
+                                 "launches_per_call": b_launches, "same_as_per_picture_calls": bool(same),
                                  "path": "h266_sao_chroma_merge_batch on device pictures (host wall time per call, "
                                          "records back in host memory)"}
     del devs

@@ -378,8 +378,9 @@ int h266_sao_chroma_merge(h266_ctx *ctx, const h266_picture *src, const h266_pic
                           uint32_t bit_depth, uint32_t ctb_log2_size_y, h266_sao_ctb_params *merged,
                           uint8_t *merge_map);
 /* The same merge for n pictures at once (device pictures, H266_MEM_DEVICE):
- * each CTB anti-diagonal is one launch over the CTBs of every picture on it,
- * so the diagonals' few CTBs per picture fill the GPU together.  Per picture
+ * the statistics of every picture's CTBs in one launch, then a CTA per
+ * picture that walks its anti-diagonals (pictures that clip widely: one launch
+ * per anti-diagonal over the CTBs of all of them).  Per picture
  * i: srcs[i], pres[i], independent[i] (w_ctbs[i] x h_ctbs[i] records),
  * merged[i] and merge_maps[i] as for h266_sao_chroma_merge; results are the
  * same as n separate calls.  Returns when the results are in host memory. */

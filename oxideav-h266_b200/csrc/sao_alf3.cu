@@ -26,8 +26,9 @@
 //  4. luma classes, one 4x4 block per thread;
 //  5. the 7x7 luma diamond, one block per thread with its 12 taps in
 //     registers and each of the 7 rows held as packed words.
-// The ALU pipe (64 lanes a clock: half the issue rate) bounds phases 2, 3 and
-// 5, so the taps are in the offset form of alf_tile.cuh.  16 1080p 10-bit
+// The ALU pipe (64 lanes a clock: half the issue rate) and the waits between
+// its instructions bound phases 2, 3 and 5 (issue 0.63 and ALU 0.50 busy over the
+// whole launch), so the taps are in the offset form of alf_tile.cuh.  16 1080p 10-bit
 // pictures: 389 us (472 with two clamps a tap, pairs instead of quads, border
 // samples one by one and word-per-value filter tables).
 #include <algorithm>
