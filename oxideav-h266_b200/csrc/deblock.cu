@@ -1357,6 +1357,7 @@ struct StripParams {
   // none), unit 4 luma / 8 chroma samples along the edge normal.
   int grid_mode;
   const EdgeSeg *grid[3];
+  uint32_t scratch;  // byte offset of the RunScratch in dynamic shared memory
   uint32_t grid_slots[3], grid_bands[3];
 };
 
@@ -1419,6 +1420,16 @@ __device__ __forceinline__ void segment_group(const SharedView &v, const EdgeSeg
   }
 }
 
+// A segment record as its three words: the struct alone is 2-byte aligned and
+// would load in eight pieces, the records of lists and grids are 4-byte aligned
+// (4:4:4 columns from host lists 58 -> 54 us).
+__device__ __forceinline__ EdgeSeg load_seg(const uint32_t *p) {
+  const uint32_t w[3] = {p[0], p[1], p[2]};
+  EdgeSeg e;
+  memcpy(&e, w, sizeof e);
+  return e;
+}
+
 // Components [c0, c1) of the window, one lane group per component.  All lanes
 // of a group walk the same segments; after each segment the group
 // synchronises, as the next segment may read samples another lane wrote
@@ -1428,10 +1439,11 @@ __device__ __forceinline__ void run_components(const StripParams &a, const Share
   const int lane = threadIdx.x & 31, k = lane % G, base = lane - k;
   const unsigned mask = ((1u << G) - 1) << base;
   const uint32_t groups = blockDim.x / G;
+  const uint32_t *segs = reinterpret_cast<const uint32_t *>(a.segs);
   for (uint32_t c = c0 + threadIdx.x / G; c < c1; c += groups) {
     const uint32_t e = a.comp[c + 1];
     for (uint32_t i = a.comp[c]; i < e; ++i) {
-      segment_group<G>(v, a.segs[i], a.maxv, k, base, mask);
+      segment_group<G>(v, load_seg(segs + (size_t)i * 3), a.maxv, k, base, mask);
       __syncwarp(mask);
     }
   }
@@ -1441,12 +1453,13 @@ __device__ __forceinline__ void run_components(const StripParams &a, const Share
 // before s write what one from s on uses, nor the other way round?  Cells are 4
 // (luma) or 8 (chroma) samples apart and a segment reaches at most 8, so only
 // the 3 cells before s and the 3 from s on can meet.
-__device__ __forceinline__ bool run_starts(const EdgeSeg *cells, uint32_t s, uint32_t ns) {
+template <class Cells>
+__device__ __forceinline__ bool run_starts(Cells cells, uint32_t s, uint32_t ns) {
   int we = INT_MIN, re = INT_MIN, ws = INT_MAX, rs = INT_MAX;
 #pragma unroll
   for (int k = 1; k <= 3; ++k) {
     if (s < (uint32_t)k) break;
-    const EdgeSeg f = cells[s - k];
+    const EdgeSeg f = cells(s - k);
     if (!f.bs) continue;
     const SegSpan x = seg_span(f);
     we = max(we, x.we);
@@ -1456,7 +1469,7 @@ __device__ __forceinline__ bool run_starts(const EdgeSeg *cells, uint32_t s, uin
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     if (s + k >= ns) break;
-    const EdgeSeg f = cells[s + k];
+    const EdgeSeg f = cells(s + k);
     if (!f.bs) continue;
     const SegSpan x = seg_span(f);
     ws = min(ws, x.ws);
@@ -1470,55 +1483,79 @@ __device__ __forceinline__ bool run_starts(const EdgeSeg *cells, uint32_t s, uin
 // host grouping's components, whose members come in position order when every
 // row and column of the CU map is in decode order (checked on the host before
 // the walk runs on the device).  A cell more than 3 slots after the run's last
-// one starts another.  The CTA lists the run starts of kRunChunk slots with a
-// thread per slot, then a lane group takes a run at a time: most slots are
-// empty, and scanning them by lane groups took most of the kernels' time.
-constexpr uint32_t kRunChunk = 1024;
+// one starts another.  The CTA stages kRunChunk slots and their neighbours in
+// shared memory, marks and lists the run starts with a thread per slot, then a
+// lane group takes a run at a time: most slots are empty, and scanning them by
+// lane groups took most of the kernels' time.  A run that leaves the chunk goes
+// on in global memory.  Reading the records from global memory along the run
+// was a chain of L2 latencies: 8 multi-type-tree 1080p pictures, rows 118 -> 96
+// us, columns 141 -> 122.
+constexpr uint32_t kRunChunk = 640;
+
+struct RunScratch {
+  uint32_t cells[(kRunChunk + 6) * 3];
+  uint32_t start[kRunChunk / 32];
+  uint16_t list[kRunChunk];
+  uint32_t n, next;
+};
+
+// After the planes' part of the dynamic shared memory (grid mode only: host
+// lists keep the room for another CTA).
+__device__ __forceinline__ RunScratch &run_scratch(uint16_t *sm, const StripParams &a) {
+  return *reinterpret_cast<RunScratch *>(reinterpret_cast<uint8_t *>(sm) + a.scratch);
+}
 
 template <int G>
-__device__ __forceinline__ void run_cell_runs(const StripParams &a, const SharedView &v, const EdgeSeg *g, uint32_t ns,
-                                              uint32_t nb) {
-  __shared__ uint16_t s_list[kRunChunk];
-  __shared__ uint32_t s_n, s_next;
+__device__ __forceinline__ void run_cell_runs(RunScratch &sc, const StripParams &a, const SharedView &v,
+                                              const EdgeSeg *grid, uint32_t ns, uint32_t nb) {
   const int lane = threadIdx.x & 31, k = lane % G, base = lane - k;
   const unsigned mask = ((1u << G) - 1) << base;
   const uint32_t total = ns * nb;
+  const uint32_t *g = reinterpret_cast<const uint32_t *>(grid);
   for (uint32_t c0 = 0; c0 < total; c0 += kRunChunk) {
-    if (threadIdx.x == 0) s_n = s_next = 0;
+    const uint32_t lo = c0 >= 3 ? c0 - 3 : 0, c1 = min(total, c0 + kRunChunk), hi = min(total, c1 + 3);
+    if (threadIdx.x == 0) sc.n = sc.next = 0;
+    if (threadIdx.x < kRunChunk / 32) sc.start[threadIdx.x] = 0;
+    for (uint32_t i = threadIdx.x; i < (hi - lo) * 3; i += blockDim.x) sc.cells[i] = g[(size_t)lo * 3 + i];
     __syncthreads();
-    for (uint32_t i = c0 + threadIdx.x; i < min(total, c0 + kRunChunk); i += blockDim.x) {
+    for (uint32_t i = c0 + threadIdx.x; i < c1; i += blockDim.x) {
       const uint32_t b = i / ns, s = i - b * ns;
-      const EdgeSeg *cells = g + (size_t)b * ns;
-      if (cells[s].bs && run_starts(cells, s, ns)) s_list[atomicAdd(&s_n, 1u)] = (uint16_t)(i - c0);
+      auto cells = [&](uint32_t q) { return load_seg(sc.cells + (b * ns + q - lo) * 3); };
+      if (cells(s).bs && run_starts(cells, s, ns)) {
+        sc.list[atomicAdd(&sc.n, 1u)] = (uint16_t)(i - c0);
+        atomicOr(&sc.start[(i - c0) / 32], 1u << (i - c0) % 32);
+      }
     }
     __syncthreads();
-    const uint32_t n = s_n;
+    const uint32_t n = sc.n;
     for (;;) {
       uint32_t t = 0;
-      if (k == 0) t = atomicAdd(&s_next, 1u);
+      if (k == 0) t = atomicAdd(&sc.next, 1u);
       t = __shfl_sync(mask, t, base);
       if (t >= n) break;
-      const uint32_t i = c0 + s_list[t], b = i / ns;
-      const EdgeSeg *cells = g + (size_t)b * ns;
-      uint32_t cur = i - b * ns;
-      EdgeSeg e = cells[cur];
+      uint32_t cur = c0 + sc.list[t];
+      const uint32_t b = cur / ns, end = (b + 1) * ns;
+      EdgeSeg e = load_seg(sc.cells + (cur - lo) * 3);
       for (;;) {
         segment_group<G>(v, e, a.maxv, k, base, mask);
         __syncwarp(mask);
         uint32_t nx = cur + 1;
         bool found = false;
-        for (; nx < ns && nx <= cur + 3; ++nx) {
-          e = cells[nx];
+        for (; nx < end && nx <= cur + 3; ++nx) {
+          e = nx < hi ? load_seg(sc.cells + (nx - lo) * 3) : load_seg(g + (size_t)nx * 3);
           if (e.bs) {
             found = true;
             break;
           }
         }
-        if (!found || run_starts(cells, nx, ns)) break;
+        if (!found) break;
+        if (nx < c1 ? sc.start[(nx - c0) / 32] >> (nx - c0) % 32 & 1
+                    : run_starts([&](uint32_t q) { return load_seg(g + ((size_t)b * ns + q) * 3); }, nx - b * ns, ns))
+          break;
         cur = nx;
       }
     }
-    __syncthreads();  // the list is free again
+    __syncthreads();  // the scratch is free again
   }
 }
 
@@ -1554,8 +1591,8 @@ __device__ __forceinline__ void deblock_rows_cta(const StripParams &a, int band)
   if (a.grid_mode) {
     if ((uint32_t)band < a.grid_bands[plane]) {
       const EdgeSeg *g = a.grid[plane] + (size_t)band * a.grid_slots[plane];
-      if (plane == 0) run_cell_runs<4>(a, view, g, a.grid_slots[plane], 1);
-      else run_cell_runs<2>(a, view, g, a.grid_slots[plane], 1);
+      if (plane == 0) run_cell_runs<4>(run_scratch(sm, a), a, view, g, a.grid_slots[plane], 1);
+      else run_cell_runs<2>(run_scratch(sm, a), a, view, g, a.grid_slots[plane], 1);
     }
   } else {
     const uint32_t *bf = a.band_first + a.band_off[plane];
@@ -1603,8 +1640,8 @@ __device__ __forceinline__ void deblock_cols_cta(const StripParams &a, int strip
     const uint32_t b0 = min((uint32_t)(x0 / unit), nb), b1 = min((uint32_t)((x0 + kStripCols) / unit), nb);
     if (b1 > b0) {
       const EdgeSeg *g = a.grid[plane] + (size_t)b0 * a.grid_slots[plane];
-      if (plane == 0) run_cell_runs<4>(a, view, g, a.grid_slots[plane], b1 - b0);
-      else run_cell_runs<2>(a, view, g, a.grid_slots[plane], b1 - b0);
+      if (plane == 0) run_cell_runs<4>(run_scratch(sm, a), a, view, g, a.grid_slots[plane], b1 - b0);
+      else run_cell_runs<2>(run_scratch(sm, a), a, view, g, a.grid_slots[plane], b1 - b0);
     }
   } else {
     const uint32_t *bf = a.band_first + a.band_off[plane];
@@ -2186,7 +2223,10 @@ int fill_strip_params_grid(void *rows, void *cols, const DPlane src[3], const DP
   strip_geometry(src, dst, lut, bit_depth, bands, p[0], p[1], c);
   if (c.smem_rows > (size_t)kMaxStripSmem || c.smem_cols > (size_t)kMaxStripSmem)
     return set_error(H266_ERR_UNSUPPORTED, "deblock: planes too large for the strip kernels");
+  size_t *const smem[2] = {&c.smem_rows, &c.smem_cols};
   for (int d = 0; d < 2; ++d) {
+    p[d].scratch = (uint32_t)(*smem[d] + 15) & ~15u;
+    *smem[d] = p[d].scratch + sizeof(RunScratch);
     p[d].grid_mode = 1;
     for (int i = 0; i < 3; ++i) {
       p[d].grid[i] = g.grid[d][i];
@@ -2202,7 +2242,7 @@ int fill_strip_params_grid(void *rows, void *cols, const DPlane src[3], const DP
 namespace {
 template <class K>
 int strip_smem(K kern, size_t bytes) {
-  if (bytes > 40 * 1024)  // above the default limit with the kernels' static shared memory
+  if (bytes > 32 * 1024)  // above the default limit with the kernels' static shared memory
     H266_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   return H266_OK;
 }
