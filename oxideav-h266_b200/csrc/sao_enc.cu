@@ -29,7 +29,7 @@ constexpr int kSliceSamples = 4096;
 struct SaoStats {  // one (CTB, component): sums over at most 128 x 128 samples of 16 bits
   int bo_cnt[32], bo_dif[32];
   int eo_cnt[4][5], eo_dif[4][5];  // category 0 is not gathered (the decision never reads it)
-  unsigned vmax, inv_vmin;         // largest sample, and 65535 less the smallest
+  unsigned vmax, inv_vmin;         // largest sample, and 65536 less the smallest (0: no sample)
 };
 
 struct SaoEncArgs {
@@ -191,7 +191,7 @@ __device__ __forceinline__ void stats_cta(const DPlane &R, const DPlane &S, int 
       sp += S.stride;
     }
   }
-  uint32_t vmax = hi2, imin = lo2 > 65535u ? 0u : 65535u - lo2;
+  uint32_t vmax = hi2, imin = lo2 > 65535u ? 0u : 65536u - lo2;
   if (above) atomicOr(err, 1u);
   vmax = __reduce_max_sync(0xFFFFFFFFu, vmax);
   imin = __reduce_max_sync(0xFFFFFFFFu, imin);
@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(kWaveThreads) k_merge_wave(const MergeArgs *__
   for (int i = tid; i < n; i += kWaveThreads)
     for (int c = 0; c < 2; ++c) {
       const SaoStats &s = a.stats[(size_t)i * 2 + c];
-      near += s.inv_vmin && ((int)s.vmax > maxv - a.max_off || 65535 - (int)s.inv_vmin < a.max_off);
+      near += s.inv_vmin && ((int)s.vmax > maxv - a.max_off || 65536 - (int)s.inv_vmin < a.max_off);
     }
   __shared__ int s_near;
   if (tid == 0) s_near = 0;
@@ -600,7 +600,7 @@ __global__ void __launch_bounds__(kWaveThreads) k_merge_wave(const MergeArgs *__
       h.ec[q] = (&s.eo_cnt[0][0])[min(lane, 19)];
       h.ed[q] = (&s.eo_dif[0][0])[min(lane, 19)];
       h.hi[q] = s.inv_vmin ? (int)s.vmax : -1;  // no sample: -1
-      h.lo[q] = 65535 - (int)s.inv_vmin;
+      h.lo[q] = 65536 - (int)s.inv_vmin;
     }
     const h266_sao_ctb &p = c ? a.indep[i].cr : a.indep[i].cb;
     h.type = p.sao_type_idx;
