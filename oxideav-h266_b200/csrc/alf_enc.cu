@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(ChromaWin<TW>::NT) k_chroma_commit(const __gri
       best = row[1 + f];
       p = f;
     }
-  if (threadIdx.x == 0 && xc0 == rx << log2c && yc0 == ry << log2c) a.pick[i] = (int8_t)p;
+  if (threadIdx.x == 0 && xc0 == rx << log2c && yc0 == ry << log2c) a.pick[i] = (uint8_t)(p + 1);
   if (p < 0) return;  // uniform per CTA
   ChromaTile<TW> t;
   t.stage(a, a.copy, w);

@@ -1657,18 +1657,19 @@ static int chroma_trials(h266_ctx *ctx, const h266_picture *src, h266_picture *r
   t.pic_w = h.args.pic_w;
   t.pic_h = h.args.pic_h;
   t.ctbs = reinterpret_cast<const CtbDev *>(st.base + st.ctb);
-  t.pick = reinterpret_cast<int8_t *>(w);
+  t.pick = w;
   t.sse = reinterpret_cast<unsigned long long *>(w + pick_b);
   std::memcpy(t.packed, h.args.tables.chroma_packed, sizeof t.packed);
   std::memcpy(t.cc_coeff, h.args.tables.cc_coeff[comp - 1], sizeof t.cc_coeff);
   {
     Prof pf(ctx, ln.stream, H266_PROF_SAO_ALF);
-    H266_CUDA(cudaMemsetAsync(t.sse, 0, sse_b, ln.stream));
+    // the SSE sums at zero, every choice at "off": a CTB without samples of the
+    // component (halved odd sizes rounded down) has no tile that would write it
+    H266_CUDA(cudaMemsetAsync(w, 0, pick_b + sse_b, ln.stream));
     H266_TRY(launch_chroma_trials(ln.stream, t, &ctx->launches));
   }
-  const uint8_t *host = nullptr;
-  H266_TRY(read_back(ln, t.pick, (size_t)n, &host));
-  const int8_t *pick = reinterpret_cast<const int8_t *>(host);
+  const uint8_t *pick = nullptr;
+  H266_TRY(read_back(ln, t.pick, (size_t)n, &pick));
   h266_picture one = *rec;  // copy back only the decided plane
   h266_plane *pl[3] = {&one.luma, &one.cb, &one.cr};
   for (int i = 0; i < 3; ++i)
@@ -1676,13 +1677,13 @@ static int chroma_trials(h266_ctx *ctx, const h266_picture *src, h266_picture *r
   H266_TRY(picture_from_device(ln, one));
   ctx->d2h_bytes += host_plane_bytes(one) + (size_t)n;
   for (int i = 0; i < n; ++i) {
-    if (pick[i] < 0) continue;
+    if (!pick[i]) continue;
     h266_alf_ctb &e = apply[i];
     if (!cc) {
       (comp == 1 ? e.cb_on : e.cr_on) = 1;
-      (comp == 1 ? e.cb_alt_idx : e.cr_alt_idx) = (uint8_t)pick[i];
+      (comp == 1 ? e.cb_alt_idx : e.cr_alt_idx) = (uint8_t)(pick[i] - 1);
     } else {
-      (comp == 1 ? e.cc_cb_idc : e.cc_cr_idc) = (uint8_t)(pick[i] + 1);
+      (comp == 1 ? e.cc_cb_idc : e.cc_cr_idc) = pick[i];
     }
   }
   return H266_OK;

@@ -459,14 +459,14 @@ int launch_pull(cudaStream_t st, const PullList &l, uint64_t *launches);
 
 // Encoder chroma ALF / CC-ALF trials (alf_enc.cu): the n_cand candidate filters
 // of one chroma component per CTB, the first minimum of {off, candidates} in
-// pick[] (-1: off) and committed to `rec`.
+// pick[] (0: off, 1 + candidate) and committed to `rec`.
 struct ChromaTrialArgs {
   DPlane rec, src, copy;  // the component: reconstruction, original, scratch of rec's size (contiguous)
   DPlane luma;            // CC-ALF: the luma before luma ALF
   int bd, log2, cc, n_cand, w_ctbs, h_ctbs, pic_w, pic_h, tiles_x;
   const CtbDev *ctbs;        // the CTBs' clip rectangles
   unsigned long long *sse;   // [ctb][1 + n_cand], zero at the start
-  int8_t *pick;
+  uint8_t *pick;             // zero at the start
   uint32_t packed[8][8];     // AlfTablesDev::chroma_packed
   int32_t cc_coeff[4][7];    // AlfTablesDev::cc_coeff of the component
 };
