@@ -229,9 +229,11 @@ __device__ __forceinline__ void luma_cells(const uint16_t *sL, uint2 *cell) {
 }
 
 // Class and transposeIdx of every 4x4 block of a W x TH tile (src/alf.rs:750-1008).
+// big: a window sample of 2^14 or above (the cells do not hold its sums); wide: one
+// of 2^12 or above (four cells do not add within their halves).
 template <int W, int TH, class S, int NT>
 __device__ __forceinline__ void luma_classes(const uint16_t *sL, const uint2 *cell, uint8_t *cls_f, uint8_t *cls_t,
-                                             int Y0, int y_ctb, int ctb, int ph, int bd, bool big) {
+                                             int Y0, int y_ctb, int ctb, int ph, int bd, bool big, bool wide) {
   const bool bottom = y_ctb + ctb >= ph;
   const bool carve = !bottom || (ph - y_ctb) > ctb - 4;
   const int vb = y_ctb + ctb - 4;
@@ -271,7 +273,7 @@ __device__ __forceinline__ void luma_classes(const uint16_t *sL, const uint2 *ce
         uint2 g[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) g[c] = q[c];
-        if (bd <= 12) {  // four cells of 4 * 4095 at most add within their halves
+        if (!wide) {  // four cells of 4 * 4095 at most add within their halves
           const uint32_t x = g[0].x + g[1].x + g[2].x + g[3].x, y = g[0].y + g[1].y + g[2].y + g[3].y;
           sh += x & 0xFFFF;
           sv += x >> 16;

@@ -80,7 +80,8 @@ __global__ void __launch_bounds__(NT, 2) k_alf_luma_trials(const __grid_constant
   big = __syncthreads_or(big);
   luma_cells<S, NT>(sm.sL, sm.cell);
   __syncthreads();
-  luma_classes<W, TH, S, NT>(sm.sL, sm.cell, sm.cls_f, sm.cls_t, Y0, y_ctb, ctb, ph, bd, big != 0);
+  luma_classes<W, TH, S, NT>(sm.sL, sm.cell, sm.cls_f, sm.cls_t, Y0, y_ctb, ctb, ph, bd, big != 0,
+                         wide != 0 || bd > 12);
   __syncthreads();
 
   constexpr int RUNS = TH * W / 4;

@@ -86,7 +86,7 @@ struct Smem3 {
   SaoLocal sao[3][9];
   SaoFast fast[3][9];
   alignas(8) unsigned long long bar;
-  int big;  // some window sample is 2^14 or above
+  int big, wide;  // some window sample is 2^14 or above, 2^12 or above
   unsigned any_sao;  // bit comp * 9 + n: neighbour n of the 3x3 CTB neighbourhood has SAO for comp
   __device__ uint16_t *dL() { return reinterpret_cast<uint16_t *>(u); }
   __device__ uint16_t *dC(int c) { return reinterpret_cast<uint16_t *>(u + DC_OFF + c * DC_STRIDE); }
@@ -290,7 +290,7 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
     for (int c = 0; c < 2; ++c)
       if (chroma_on[c]) tma_load_2d(sm.dC(c), &maps->tmap[1 + c], xc0 - 8, yc0 - 3, &sm.bar);
   }
-  if (tid == 32) sm.big = 0;
+  if (tid == 32) sm.big = sm.wide = 0;
   int my_type = 0;
   if (tid < 27) {
     const int comp = tid / 9, n = tid % 9;
@@ -470,7 +470,10 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
       put(w, v);
     }
   }
-  if (DO_ALF && (seen & 0xC000C000u)) sm.big = 1;
+  if (DO_ALF && (seen & 0xF000F000u)) {
+    sm.wide = 1;
+    if (seen & 0xC000C000u) sm.big = 1;
+  }
   __syncthreads();
   const bool big = DO_ALF && sm.big != 0;
 
@@ -552,7 +555,8 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
   __syncthreads();
 
   // ---- (4) classes
-  luma_classes<W, TH, S, NT3>(sm.sL, sm.cell(), sm.cls_f, sm.cls_t, Y0, y_ctb, ctb, ph, bd, big);
+  luma_classes<W, TH, S, NT3>(sm.sL, sm.cell(), sm.cls_f, sm.cls_t, Y0, y_ctb, ctb, ph, bd, big,
+                             sm.wide != 0);
   __syncthreads();
 
   // ---- (5) 7x7 diamond: every thread keeps one block's taps and filters RPT of its 4-sample runs
