@@ -162,7 +162,8 @@ __device__ __forceinline__ uint2 quad_shifted(const uint16_t *r, int h) {
 
 // SAO of the 4 samples at d (8-byte aligned window pointer; all inside one CTB,
 // the clip rectangle and the CTB's edge-offset availability rectangle), samples
-// below 2^12.
+// below 2^14: the 16-bit lanes wrap between samples 32767 apart and where an
+// offset meets a sample near it.
 __device__ __forceinline__ uint2 sao_quad(const SaoFast &f, const uint16_t *d, uint32_t maxv2) {
   const uint2 c = ld64(d);
   if (f.type == 0) return c;
@@ -354,8 +355,8 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
   const bool sao_on[3] = {DO_SAO && (any & 0x1FFu) != 0, DO_SAO && ((any >> 9) & 0x1FFu) != 0,
                           DO_SAO && ((any >> 18) & 0x1FFu) != 0};
   // packed SAO: offsets as signed bytes, samples below 2^12 (a plain copy has no such limit)
-  const bool fast_ok[3] = {!sao_on[0] || (a.sao_i8 && bd <= 12), !sao_on[1] || (a.sao_i8 && bd <= 12),
-                           !sao_on[2] || (a.sao_i8 && bd <= 12)};
+  const bool quads = a.sao_i8 && bd <= 12;
+  bool fast_ok[3] = {!sao_on[0] || quads, !sao_on[1] || quads, !sao_on[2] || quads};
   const int crx0 = rect[0] / 2, cry0 = rect[1] / 2, crx1 = (rect[2] + 1) / 2, cry1 = (rect[3] + 1) / 2;
   FastRect fr[3];
   {
@@ -381,16 +382,36 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
                        : fast_rect(0, 0, 0, 0);
     }
   }
-  if (tma) {
-    bool ok = mbar_wait_bounded(&sm.bar, phase, kWaitNs);
+  bool ok = !tma || mbar_wait_bounded(&sm.bar, phase, kWaitNs);
+  // A tile with a sample of 2^14 or above, outside every depth of the quads, runs
+  // sample by sample.  Looking at the windows first costs 0.3 % (16 1080p pictures
+  // from resident plans 658.6 -> 660.7 us); forming the post-SAO windows a second
+  // time where the first pass met such a sample cost 2 to 4 %, by the registers that
+  // its loop or call holds.
+  uint32_t far = 0;
+  if (DO_SAO && quads && any) {
+    auto look = [&](const uint16_t *w, int n) {
+      const uint4 *q = reinterpret_cast<const uint4 *>(w);
+      for (int i = tid; i < n / 8; i += NT3) far |= q[i].x | q[i].y | q[i].z | q[i].w;
+    };
+    look(sm.dL(), S::DLH * S::DLW);
+    for (int c = 0; c < 2; ++c)
+      if (chroma_on[c]) look(sm.dC(c), S::DCH * S::DCW);
+  }
+  if (__syncthreads_or(!ok || (far & 0xC000C000u))) {
     ok = __syncthreads_and(ok);
     if (!ok) {  // the copies did not land: count the tile, let them finish (bounded), leave it unfiltered
       if (tid == 0) atomicAdd(&g_wait_timeouts, 1u);
       mbar_wait_bounded(&sm.bar, phase, kWaitNs);
       return false;
     }
-    phase ^= 1u;
+    for (int k = 0; k < 3; ++k)
+      if (sao_on[k]) {
+        fast_ok[k] = false;
+        fr[k] = fast_rect(0, 0, 0, 0);
+      }
   }
+  if (tma) phase ^= 1u;
 
   // ---- (2) post-SAO windows (biased), clamped into the fetch rectangle, 4 samples per step
   uint32_t seen = 0;  // every sample or'ed together
@@ -774,7 +795,7 @@ __device__ __forceinline__ void chroma_tile(const Pass2Args &a, int tile) {
     }
     sm.fast[comp][n] = sao_fast(s, pitch);
   }
-  const bool quads = a.sao_i8 && bd <= 12;
+  uint32_t far = 0;  // the deblocked samples or'ed together
   const bool cc_any = a.do_alf && me && have_luma && (me->cc_filt[0] >= 0 || me->cc_filt[1] >= 0);
   bool on[2];
   for (int cc = 0; cc < 2; ++cc) on[cc] = xc0 < a.src[1 + cc].w && yc0 < a.src[1 + cc].h;  // uniform per CTA
@@ -784,13 +805,17 @@ __device__ __forceinline__ void chroma_tile(const Pass2Args &a, int tile) {
     if (dx0 >= 0 && dx0 + dw <= src.w && ((uintptr_t)src.s & 15) == 0 && (src.stride & 7) == 0) {
       for (int i = tid; i < dh * nv; i += NT) {
         const int r = i / nv, c = (i - r * nv) * 8, gy = clampd(dy0 + r, 0, src.h - 1);
-        *reinterpret_cast<uint4 *>(&d[r * dw + c]) =
-            *reinterpret_cast<const uint4 *>(src.s + (int64_t)gy * src.stride + dx0 + c);
+        const uint4 v = *reinterpret_cast<const uint4 *>(src.s + (int64_t)gy * src.stride + dx0 + c);
+        *reinterpret_cast<uint4 *>(&d[r * dw + c]) = v;
+        far |= v.x | v.y | v.z | v.w;
       }
     } else {
       for (int i = tid; i < dh * dw; i += NT) {
         const int r = i / dw, c = i - r * dw;
-        d[r * dw + c] = src.s[(int64_t)clampd(dy0 + r, 0, src.h - 1) * src.stride + clampd(dx0 + c, 0, src.w - 1)];
+        const uint16_t v =
+            src.s[(int64_t)clampd(dy0 + r, 0, src.h - 1) * src.stride + clampd(dx0 + c, 0, src.w - 1)];
+        d[r * dw + c] = v;
+        far |= v;
       }
     }
   };
@@ -800,7 +825,8 @@ __device__ __forceinline__ void chroma_tile(const Pass2Args &a, int tile) {
     if (on[cc]) load(a.src[1 + cc], sm.dC[cc], xc0 - 8, yc0 - 3, CDW{}, CDH{});
   if (cc_any)
     load(a.src[0], sm.dL, X0 - 8, Y0 - 2, std::integral_constant<int, S::DLW>{}, std::integral_constant<int, S::DLH>{});
-  __syncthreads();
+  // the quads of SAO for samples below 2^14, as in the tile kernel (else sample by sample)
+  const bool quads = !__syncthreads_or((far & 0xC000C000u) != 0) && a.sao_i8 && bd <= 12;
   // Post-SAO window of component `comp`: W x H at (wx0, wy0), clamped into
   // [fx0, fx1) x [fy0, fy1); lx: log2 of the CTB's width in the component's
   // samples; `rot`: the thread that takes the first quad.
