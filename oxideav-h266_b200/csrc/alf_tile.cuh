@@ -238,6 +238,8 @@ __device__ __forceinline__ void luma_classes(const uint16_t *sL, const uint2 *ce
   const bool carve = !bottom || (ph - y_ctb) > ctb - 4;
   const int vb = y_ctb + ctb - 4;
   constexpr int NB = (TH / 4) * (W / 4);
+  using Sample = std::conditional_t<S::BIASED, int16_t, uint16_t>;  // biased samples are in order as signed numbers
+  const Sample *win = reinterpret_cast<const Sample *>(sL);
   for (int b = threadIdx.x; b < NB; b += NT) {
     const int bx = b % (W / 4), by = b / (W / 4);
     const int y4 = Y0 + 4 * by - y_ctb;
@@ -254,7 +256,7 @@ __device__ __forceinline__ void luma_classes(const uint16_t *sL, const uint2 *ce
       int sh = 0, sv = 0, sd0 = 0, sd1 = 0;
       for (int j = min_y; j <= max_y; ++j) {
         const int gy = y_ctb + y4 + j;
-        const uint16_t *rc = &sL[pad(gy) * S::SLP], *ru = &sL[pad(gy - 1) * S::SLP], *rd = &sL[pad(gy + 1) * S::SLP];
+        const Sample *rc = &win[pad(gy) * S::SLP], *ru = &win[pad(gy - 1) * S::SLP], *rd = &win[pad(gy + 1) * S::SLP];
         for (int i = (j & 1) ? -1 : -2; i <= 5; i += 2) {
           const int c = 4 * bx + i + 4;
           const int c2 = 2 * rc[c];
@@ -430,16 +432,15 @@ __device__ __forceinline__ void load_words(Words<NW, B> &r, const uint16_t *p, i
 }
 
 // The plain form of the clipped taps for tiles that hold a sample of 2^14 or
-// above, tap by tap (out of line: no picture of a supported depth has any).
-__device__ __forceinline__ uint32_t pair_plain(const uint16_t *p) {
-  return ((uint32_t)p[0] | (uint32_t)p[1] << 16) ^ kBias;
-}
-__device__ __forceinline__ void tap_plain(const uint16_t *up, const uint16_t *dn, uint32_t ncur, uint32_t c2,
-                                          uint32_t f, int acc[2]) {
-  const uint32_t nc2 = neg2(c2);
-  const uint32_t s = add2(clipd(pair_plain(up), ncur, c2, nc2), clipd(pair_plain(dn), ncur, c2, nc2));
-  acc[0] = __dp2a_lo((int)s, (int)f, acc[0]);
-  acc[1] = __dp2a_hi((int)s, (int)f, acc[1]);
+// above, sample by sample and tap by tap in 32 bits, as differences take 17 (out
+// of line: no picture of a supported depth has any).  w: the packed filter's
+// clips, f: its coefficients.
+__device__ __forceinline__ int tap_plain(const uint16_t *R, int o, int cur, const uint32_t *w, const uint32_t *f,
+                                         int k) {
+  int c = (int)(w[k / 2] >> (16 * (k & 1)) & 0xFFFF);
+  if (c == 0x3FFF) c = 0x4000;  // as packed (build_packed)
+  // the windows' biased samples are in order as signed numbers
+  return (clampd((int)(int16_t)R[o] - cur, -c, c) + clampd((int)(int16_t)R[-o] - cur, -c, c)) * (int8_t)(f[k / 4] >> (8 * (k & 3)) & 0xFF);
 }
 // taps (dx, dy) of the 7x7 and 5x5 diamonds in table order, mirrored taps at (-dx, -dy)
 static __constant__ int8_t kLumaTaps[12][2] = {{0, 3}, {1, 2}, {0, 2}, {-1, 2}, {2, 1}, {1, 1},
@@ -450,18 +451,13 @@ static __device__ __noinline__ void luma_run_plain(const uint16_t *R0, int pitch
                                             const uint32_t *tab, int maxv, int out[4]) {
   const int ys[4] = {0, y1, y2, y3};
 #pragma unroll 1
-  for (int q = 0; q < 2; ++q) {
-    const uint16_t *R = R0 + 2 * q;
-    const uint32_t cur = pair_plain(R), ncur = neg2(cur);
-    int acc[2] = {0, 0};
+  for (int p = 0; p < 4; ++p) {
+    const uint16_t *R = R0 + p;
+    int acc = 1 << (shift - 1);
 #pragma unroll 1
-    for (int k = 0; k < 12; ++k) {
-      const int o = ys[kLumaTaps[k][1]] * pitch + kLumaTaps[k][0];
-      tap_plain(R + o, R - o, ncur, plain_clip(clip_of(tab, k)), coef_of(tab + 6, k), acc);
-    }
-    const int round = 1 << (shift - 1);
-    out[2 * q] = clampd((int)(cur & 0xFFFF) + ((acc[0] + round) >> shift), 0, maxv);
-    out[2 * q + 1] = clampd((int)(cur >> 16) + ((acc[1] + round) >> shift), 0, maxv);
+    for (int k = 0; k < 12; ++k)
+      acc += tap_plain(R, ys[kLumaTaps[k][1]] * pitch + kLumaTaps[k][0], (int16_t)R[0], tab, tab + 6, k);
+    out[p] = clampd((R[0] ^ 0x8000) + (acc >> shift), 0, maxv);
   }
 }
 
@@ -470,18 +466,13 @@ __device__ __noinline__ void chroma_run_plain(const uint16_t *R0, int pitch, int
                                               const uint32_t *ct, int maxv, int v[SPT]) {
   const int ys[3] = {0, y1, y2};
 #pragma unroll 1
-  for (int q = 0; q < SPT / 2; ++q) {
-    const uint16_t *R = R0 + 2 * q;
-    const uint32_t cur = pair_plain(R), ncur = neg2(cur);
-    int acc[2] = {0, 0};
+  for (int p = 0; p < SPT; ++p) {
+    const uint16_t *R = R0 + p;
+    int acc = 1 << (shift - 1);
 #pragma unroll 1
-    for (int k = 0; k < 6; ++k) {
-      const int o = ys[kChromaTaps[k][1]] * pitch + kChromaTaps[k][0];
-      tap_plain(R + o, R - o, ncur, plain_clip(clip_of(ct, k)), coef_of(ct + 3, k), acc);
-    }
-    const int round = 1 << (shift - 1);
-    v[2 * q] = clampd((int)(cur & 0xFFFF) + ((acc[0] + round) >> shift), 0, maxv);
-    v[2 * q + 1] = clampd((int)(cur >> 16) + ((acc[1] + round) >> shift), 0, maxv);
+    for (int k = 0; k < 6; ++k)
+      acc += tap_plain(R, ys[kChromaTaps[k][1]] * pitch + kChromaTaps[k][0], (int16_t)R[0], ct, ct + 3, k);
+    v[p] = clampd((R[0] ^ 0x8000) + (acc >> shift), 0, maxv);
   }
 }
 

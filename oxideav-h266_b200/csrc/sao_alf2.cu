@@ -23,6 +23,7 @@ constexpr int NT = 256;
 // CTB's row is the pre-ALF SSE (the "off" option).
 template <int W>
 struct TrialSmem {
+  static constexpr bool BIASED = false;
   static constexpr int SLW = W + 8, SLH = TH + 6;        // pre-ALF luma [X0-4, X1+4) x [Y0-3, Y1+3)
   static constexpr int SLP = SLW;                         // its row pitch
   static constexpr int CW = W / 2 + 2, CH = TH / 2 + 2;  // 2x2 Laplacian cells

@@ -61,6 +61,7 @@ struct alignas(16) SaoFast {
 
 template <int W, int TH>
 struct Smem3 {
+  static constexpr bool BIASED = true;  // the post-SAO windows hold samples + 0x8000
   static constexpr int DLW = W + 16, DLH = TH + 8;          // deblocked luma [X0-8, X1+8) x [Y0-4, Y1+4)
   static constexpr int SLW = W + 8, SLH = TH + 6;           // post-SAO luma [X0-4, X1+4) x [Y0-3, Y1+3)
   static constexpr int CW = W / 2 + 2, CH = TH / 2 + 2;     // 2x2 Laplacian cells
@@ -86,7 +87,6 @@ struct Smem3 {
   SaoLocal sao[3][9];
   SaoFast fast[3][9];
   alignas(8) unsigned long long bar;
-  int big, wide;  // some window sample is 2^14 or above, 2^12 or above
   unsigned any_sao;  // bit comp * 9 + n: neighbour n of the 3x3 CTB neighbourhood has SAO for comp
   __device__ uint16_t *dL() { return reinterpret_cast<uint16_t *>(u); }
   __device__ uint16_t *dC(int c) { return reinterpret_cast<uint16_t *>(u + DC_OFF + c * DC_STRIDE); }
@@ -232,6 +232,229 @@ __device__ __forceinline__ void rest_pos(int i, int wx0, int wy0, int WQ, int WH
 __device__ __forceinline__ int rest_count(int WQ, int WH, const FastRect &f) { return WQ * WH - f.quads(); }
 
 // ---------------------------------------------------------------- the tile
+// Whether the tile with chroma origin (xc0, yc0) has samples of half-height chroma plane c.
+__device__ __forceinline__ bool chroma_tile_on(const Pass2Args &a, int c, int xc0, int yc0) {
+  const DPlane &P = a.src[c + 1];
+  return a.chroma && a.sub_h == 2 && P.w > 0 && P.h > 0 && xc0 < P.w && yc0 < P.h;
+}
+
+// Phases 3 to 5 of tile `tile` on its post-SAO windows.  BIG: they may hold samples
+// of 2^14 and above; wide: of 2^12 and above.
+template <int W, int TH, bool DO_ALF, bool BIG>
+__device__ __forceinline__ void finish_tile(const Pass2Args &a, Smem3<W, TH> &sm, int tile, bool wide) {
+  using S = Smem3<W, TH>;
+  const int tid = threadIdx.x;
+  const int X0 = tile % a.tiles_x * W, Y0 = tile / a.tiles_x * TH;
+  const int bd = a.bit_depth, maxv = (1 << bd) - 1, log2 = a.ctb_log2, ctb = 1 << log2;
+  const int rx = X0 >> log2, ry = Y0 >> log2, y_ctb = ry << log2, ph = a.pic_h;
+  const CtbDev *me = rx < a.w_ctbs && ry < a.h_ctbs ? &a.ctbs[ry * a.w_ctbs + rx] : nullptr;
+  constexpr int TWC = W / 2, THC = TH / 2;
+  const int xc0 = X0 / 2, yc0 = Y0 / 2;
+
+
+  // ---- (3) luma Laplacian sums per 2x2 cell (into the dead deblocked windows); chroma ALF / CC-ALF
+  const bool luma_alf = DO_ALF && me && me->luma_set >= 0;
+  if (luma_alf) luma_cells<S, NT3>(sm.sL, sm.cell());
+  {
+    // thread -> (plane, row, run of SPT samples)
+    constexpr int SPT = TWC * THC / (NT3 / 2);  // 8 (64 x 64 tiles) or 2 (32 x 32)
+    constexpr int NP = SPT / 2;                 // pairs per thread
+    constexpr int RPR = TWC / SPT;              // threads per chroma row
+    const int cc = tid / (NT3 / 2), t = tid % (NT3 / 2);
+    const int jj = t / RPR, i0 = (t % RPR) * SPT;
+    const DPlane &CD = a.dst[cc + 1];
+    const int gy = yc0 + jj, gx = xc0 + i0;
+    if (chroma_tile_on(a, cc, xc0, yc0) && gy < CD.h && gx < CD.w) {
+      const int cf = (DO_ALF && me) ? me->chroma_filt[cc] : -1;
+      const int ccf = (DO_ALF && me) ? me->cc_filt[cc] : -1;
+      const int ctb_c = ctb / 2, y_ctb_c = y_ctb / 2;
+      const uint16_t *R0 = &sm.sC[cc][(jj + 2) * S::SCP + i0 + 4];
+      int v[SPT];
+      {
+        Words<NP + 2, 1> w0;
+        load_words<NP + 2, 1, (NP > 1)>(w0, R0, 1, NP + 1);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+          const uint32_t cur = w0.w[1 + q] ^ kBias;
+          v[2 * q] = (int)(cur & 0xFFFF);
+          v[2 * q + 1] = (int)(cur >> 16);
+        }
+      }
+      if (cf >= 0)
+        chroma_alf_run<SPT>(R0, S::SCP, gy - y_ctb_c, ctb_c, a.tables.chroma_packed[min(cf, 7)], maxv, BIG, v);
+      if (ccf >= 0)  // col 2 i0 + 4 of the luma window = luma x of i0
+        cc_alf_run<SPT>(&sm.sL[(2 * jj + 3) * S::SLP + 2 * i0 + 4], S::SLP, (gy - y_ctb_c) * 2, ctb,
+                        !(gy * 2 + ctb >= ph && (ph - y_ctb) <= ctb - 4), a.tables.cc_coeff[cc][ccf], bd, maxv, v);
+      uint16_t *out = CD.s + (int64_t)gy * CD.stride + gx;
+      const bool vec = gx + SPT <= CD.w && ((uintptr_t)out & (2 * SPT - 1)) == 0;
+      if (vec && SPT == 8) {
+        uint4 o;
+        o.x = (uint32_t)v[0] | (uint32_t)v[1] << 16;
+        o.y = (uint32_t)v[2] | (uint32_t)v[3] << 16;
+        o.z = (uint32_t)v[4] | (uint32_t)v[5] << 16;
+        o.w = (uint32_t)v[6 % SPT] | (uint32_t)v[7 % SPT] << 16;
+        *reinterpret_cast<uint4 *>(out) = o;
+      } else if (vec && SPT == 4) {
+        *reinterpret_cast<uint2 *>(out) = make_uint2((uint32_t)v[0] | (uint32_t)v[1 % SPT] << 16,
+                                                     (uint32_t)v[2 % SPT] | (uint32_t)v[3 % SPT] << 16);
+      } else if (vec && SPT == 2) {
+        *reinterpret_cast<uint32_t *>(out) = (uint32_t)v[0] | (uint32_t)v[1 % SPT] << 16;
+      } else {
+#pragma unroll
+        for (int k = 0; k < SPT; ++k)
+          if (gx + k < CD.w) out[k] = (uint16_t)v[k];
+      }
+    }
+  }
+  const DPlane LD = a.dst[0];
+  if (!luma_alf) {
+    // the post-SAO tile as it is, 4 samples per store
+    for (int p = tid; p < TH * W / 4; p += NT3) {
+      const int j = p / (W / 4), i = (p % (W / 4)) * 4;
+      const int gx = X0 + i, gy = Y0 + j;
+      if (gy >= LD.h || gx >= LD.w) continue;
+      uint2 v = ld64(&sm.sL[(j + 3) * S::SLP + i + 4]);
+      v.x ^= kBias;
+      v.y ^= kBias;
+      uint16_t *out = LD.s + (int64_t)gy * LD.stride + gx;
+      if (gx + 4 <= LD.w && ((uintptr_t)out & 7) == 0) {
+        *reinterpret_cast<uint2 *>(out) = v;
+      } else {
+        const uint16_t s4[4] = {(uint16_t)(v.x & 0xFFFF), (uint16_t)(v.x >> 16), (uint16_t)(v.y & 0xFFFF),
+                                (uint16_t)(v.y >> 16)};
+        for (int k = 0; k < 4 && gx + k < LD.w; ++k) out[k] = s4[k];
+      }
+    }
+    return;
+  }
+  __syncthreads();
+
+  // ---- (4) classes
+  luma_classes<W, TH, S, NT3>(sm.sL, sm.cell(), sm.cls_f, sm.cls_t, Y0, y_ctb, ctb, ph, bd, BIG, wide);
+  __syncthreads();
+
+  // ---- (5) 7x7 diamond: every thread keeps one block's taps and filters RPT of its 4-sample runs
+  constexpr int RUNS = TH * W / 4;
+  constexpr int RPT = RUNS / NT3;  // runs per thread: 4 (64 x 64) or 1 (32 x 32)
+  constexpr int TPB = 4 / RPT;     // threads per 4x4 block
+  const int b = tid / TPB;
+  const int bx = b % (W / 4), by = b / (W / 4);
+  const uint32_t *tab =
+      a.tables.luma_packed + ((size_t)me->luma_set * 100 + sm.cls_f[b] * 4 + sm.cls_t[b]) * kLumaEntry;
+  uint32_t c2[12], f[12];  // clip values and coefficients in registers
+  const int start = luma_filter(tab, c2, f);
+  const int gx = X0 + 4 * bx;
+#pragma unroll 1
+  for (int rr = 0; rr < RPT; ++rr) {
+    const int j = 4 * by + (tid % TPB) * RPT + rr;  // tile row
+    const int gy = Y0 + j;
+    if (gy >= LD.h || gx >= LD.w) continue;
+    int shift, y1, y2, y3;
+    table45(gy - y_ctb, ctb, shift, y1, y2, y3);
+    const uint16_t *R0 = &sm.sL[(j + 3) * S::SLP + 4 * bx + 4];
+    int o[4];
+    if (BIG) {
+      luma_run_plain(R0, S::SLP, y1, y2, y3, shift, tab, maxv, o);
+    } else {
+      const int st = start + (1 << (shift - 1));
+      int acc[4] = {st, st, st, st};
+      // words k of a row: samples (c0 - 4 + 2k, +1), c0 = the run's first sample
+      Words<6, 2> ru, rd;
+      load_words<6, 2, true>(ru, R0, 0, 6);  // the run's own row
+      const uint32_t cur[2] = {ru.w[2] ^ kBias, ru.w[3] ^ kBias};
+      const uint32_t m[2] = {kBias - cur[0], kBias - cur[1]};  // 0x8000 - cur per lane
+      auto tap = [&](const Words<6, 2> &up, const Words<6, 2> &dn, auto dx, int k) {
+        constexpr int DX = decltype(dx)::value;
+        const uint32_t c22 = c2[k] + c2[k];
+        static_for<2>([&](auto qc) {
+          constexpr int q = decltype(qc)::value;
+          const uint32_t b = c2[k] + m[q];
+          const uint32_t s = clip_off(up.template pair<DX + 2 * q>(), b, c22) +
+                             clip_off(dn.template pair<-DX + 2 * q>(), b, c22);
+          acc[2 * q] = dp2a_ulo(s, f[k], acc[2 * q]);
+          acc[2 * q + 1] = dp2a_uhi(s, f[k], acc[2 * q + 1]);
+        });
+      };
+      using I0 = std::integral_constant<int, 0>;
+      using I1 = std::integral_constant<int, 1>;
+      using Im1 = std::integral_constant<int, -1>;
+      using I2 = std::integral_constant<int, 2>;
+      using Im2 = std::integral_constant<int, -2>;
+      using I3 = std::integral_constant<int, 3>;
+      tap(ru, ru, I3{}, 9);
+      tap(ru, ru, I2{}, 10);
+      tap(ru, ru, I1{}, 11);
+      load_words<6, 2, true>(ru, R0 + y3 * S::SLP, 2, 4);
+      load_words<6, 2, true>(rd, R0 - y3 * S::SLP, 2, 4);
+      tap(ru, rd, I0{}, 0);
+      load_words<6, 2, true>(ru, R0 + y2 * S::SLP, 1, 5);
+      load_words<6, 2, true>(rd, R0 - y2 * S::SLP, 1, 5);
+      tap(ru, rd, I1{}, 1);
+      tap(ru, rd, I0{}, 2);
+      tap(ru, rd, Im1{}, 3);
+      load_words<6, 2, true>(ru, R0 + y1 * S::SLP, 1, 5);
+      load_words<6, 2, true>(rd, R0 - y1 * S::SLP, 1, 5);
+      tap(ru, rd, I2{}, 4);
+      tap(ru, rd, I1{}, 5);
+      tap(ru, rd, I0{}, 6);
+      tap(ru, rd, Im1{}, 7);
+      tap(ru, rd, Im2{}, 8);
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const int cv = (int)((cur[p >> 1] >> ((p & 1) * 16)) & 0xFFFF);
+        o[p] = clampd(cv + (acc[p] >> shift), 0, maxv);
+      }
+    }
+    uint16_t *out = LD.s + (int64_t)gy * LD.stride + gx;
+    if (gx + 4 <= LD.w && ((uintptr_t)out & 7) == 0) {
+      *reinterpret_cast<uint2 *>(out) =
+          make_uint2((uint32_t)o[0] | (uint32_t)o[1] << 16, (uint32_t)o[2] | (uint32_t)o[3] << 16);
+    } else {
+      for (int p = 0; p < 4 && gx + p < LD.w; ++p) out[p] = (uint16_t)o[p];
+    }
+  }
+}
+
+// Phases 2 to 5 of a tile that holds a sample of 2^14 or above, outside every depth
+// of the packed lanes, which wrap between samples 32767 apart: its post-SAO windows
+// sample by sample, ALF in the plain forms.  Out of line and decided before phase
+// 2, so that the other tiles hold none of it (16 1080p pictures from resident
+// plans 656 -> 637 us against branches in every phase; the windows formed a second
+// time where phase 2 met such a sample: 669, or 684 by a call that returned).
+template <int W, int TH, bool DO_ALF>
+__device__ __noinline__ void finish_big(const Pass2Args &a, int tile) {
+  using S = Smem3<W, TH>;
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  S &sm = *reinterpret_cast<S *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
+  const int X0 = tile % a.tiles_x * W, Y0 = tile / a.tiles_x * TH, log2 = a.ctb_log2;
+  const int rx = X0 >> log2, ry = Y0 >> log2, maxv = (1 << a.bit_depth) - 1;
+  int rect[4] = {0, 0, a.pic_w, a.pic_h};
+  if (rx < a.w_ctbs && ry < a.h_ctbs)
+    for (int k = 0; k < 4; ++k) rect[k] = a.ctbs[ry * a.w_ctbs + rx].rect[k];
+#pragma unroll 1
+  for (int comp = 0; comp < 3; ++comp) {
+    const DPlane &P = a.src[comp];
+    const int sh = comp ? 1 : 0, x0 = X0 >> sh, y0 = Y0 >> sh;
+    if (comp && !chroma_tile_on(a, comp - 1, x0, y0)) continue;
+    const int fx0 = max(rect[0] >> sh, 0), fx1 = min((rect[2] + sh) >> sh, comp ? P.w : a.pic_w);
+    const int fy0 = max(rect[1] >> sh, 0), fy1 = min((rect[3] + sh) >> sh, comp ? P.h : a.pic_h);
+    const int ww = comp ? S::SCW : S::SLW, wh = comp ? S::SCH : S::SLH, wp = comp ? S::SCP : S::SLP;
+    const int ox = x0 - 4, oy = y0 - (comp ? 2 : 3), dx0 = x0 - 8, dy0 = oy - 1, pitch = comp ? S::DCW : S::DLW;
+    const uint16_t *D = comp ? sm.dC(comp - 1) : sm.dL();
+    uint16_t *out = comp ? sm.sC[comp - 1] : sm.sL;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < ww * wh; i += NT3) {
+      const int r = i / ww, c = i - r * ww;
+      const int ax = clampd(ox + c, fx0, fx1 - 1), ay = clampd(oy + r, fy0, fy1 - 1);
+      const uint16_t *d = D + (ay - dy0) * pitch + (ax - dx0);
+      const SaoLocal &p = sm.sao[comp][((ay >> (log2 - sh)) - ry + 1) * 3 + ((ax >> (log2 - sh)) - rx + 1)];
+      out[r * wp + c] = (uint16_t)((p.type ? sao_one(p, ax, ay, maxv, d) : *d) ^ 0x8000);
+    }
+  }
+  __syncthreads();
+  finish_tile<W, TH, DO_ALF, true>(a, sm, tile, true);
+}
+
 // Tile `tile` of the picture whose parameters are `a` (tensor maps at `maps`).
 // PERSIST: the CTA runs many tiles on one barrier, initialised by the caller;
 // `phase` is the barrier's next phase and flips with every completed copy.
@@ -268,10 +491,7 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
   const int xc0 = X0 / 2, yc0 = Y0 / 2;
   bool chroma_on[2];
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    const DPlane &CS = a.src[c + 1];
-    chroma_on[c] = a.chroma && a.sub_h == 2 && CS.w > 0 && CS.h > 0 && xc0 < CS.w && yc0 < CS.h;
-  }
+  for (int c = 0; c < 2; ++c) chroma_on[c] = chroma_tile_on(a, c, xc0, yc0);
   const bool tma = a.tma != 0;
 
   // ---- (1) deblocked windows (thread 0 starts the copies first, so they
@@ -291,7 +511,6 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
     for (int c = 0; c < 2; ++c)
       if (chroma_on[c]) tma_load_2d(sm.dC(c), &maps->tmap[1 + c], xc0 - 8, yc0 - 3, &sm.bar);
   }
-  if (tid == 32) sm.big = sm.wide = 0;
   int my_type = 0;
   if (tid < 27) {
     const int comp = tid / 9, n = tid % 9;
@@ -356,7 +575,7 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
                           DO_SAO && ((any >> 18) & 0x1FFu) != 0};
   // packed SAO: offsets as signed bytes, samples below 2^12 (a plain copy has no such limit)
   const bool quads = a.sao_i8 && bd <= 12;
-  bool fast_ok[3] = {!sao_on[0] || quads, !sao_on[1] || quads, !sao_on[2] || quads};
+  const bool fast_ok[3] = {!sao_on[0] || quads, !sao_on[1] || quads, !sao_on[2] || quads};
   const int crx0 = rect[0] / 2, cry0 = rect[1] / 2, crx1 = (rect[2] + 1) / 2, cry1 = (rect[3] + 1) / 2;
   FastRect fr[3];
   {
@@ -383,45 +602,41 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
     }
   }
   bool ok = !tma || mbar_wait_bounded(&sm.bar, phase, kWaitNs);
-  // A tile with a sample of 2^14 or above, outside every depth of the quads, runs
-  // sample by sample.  Looking at the windows first costs 0.3 % (16 1080p pictures
-  // from resident plans 658.6 -> 660.7 us); forming the post-SAO windows a second
-  // time where the first pass met such a sample cost 2 to 4 %, by the registers that
-  // its loop or call holds.
-  uint32_t far = 0;
-  if (DO_SAO && quads && any) {
+  // The deblocked samples or'ed together: 2^14 and above is outside every depth of
+  // the packed lanes, 2^12 and above (13 and 14 bits, or outside the depth) of the
+  // class sums.  The look costs 0.3 % (16 1080p pictures 658.6 -> 660.7 us).
+  uint32_t seen = 0;
+  if (DO_SAO || DO_ALF) {
     auto look = [&](const uint16_t *w, int n) {
       const uint4 *q = reinterpret_cast<const uint4 *>(w);
-      for (int i = tid; i < n / 8; i += NT3) far |= q[i].x | q[i].y | q[i].z | q[i].w;
+      for (int i = tid; i < n / 8; i += NT3) seen |= q[i].x | q[i].y | q[i].z | q[i].w;
     };
-    look(sm.dL(), S::DLH * S::DLW);
+    if (a.src[0].w > 0 && a.src[0].h > 0) look(sm.dL(), S::DLH * S::DLW);
     for (int c = 0; c < 2; ++c)
       if (chroma_on[c]) look(sm.dC(c), S::DCH * S::DCW);
   }
-  if (__syncthreads_or(!ok || (far & 0xC000C000u))) {
+  bool wide = false;
+  if (__syncthreads_or(!ok || (seen & 0xF000F000u))) {
     ok = __syncthreads_and(ok);
     if (!ok) {  // the copies did not land: count the tile, let them finish (bounded), leave it unfiltered
       if (tid == 0) atomicAdd(&g_wait_timeouts, 1u);
       mbar_wait_bounded(&sm.bar, phase, kWaitNs);
       return false;
     }
-    for (int k = 0; k < 3; ++k)
-      if (sao_on[k]) {
-        fast_ok[k] = false;
-        fr[k] = fast_rect(0, 0, 0, 0);
-      }
+    wide = true;
+    if (__syncthreads_or((seen & 0xC000C000u) != 0)) {
+      finish_big<W, TH, DO_ALF>(a, tile);
+      if (tma) phase ^= 1u;
+      return true;
+    }
   }
   if (tma) phase ^= 1u;
 
   // ---- (2) post-SAO windows (biased), clamped into the fetch rectangle, 4 samples per step
-  uint32_t seen = 0;  // every sample or'ed together
   {
     constexpr int WQL = S::SLW / 4, WQC = S::SCW / 4;
     const uint16_t *dL = sm.dL();
-    auto put = [&](uint16_t *w, uint2 v) {
-      seen |= v.x | v.y;
-      st64(w, make_uint2(v.x ^ kBias, v.y ^ kBias));
-    };
+    auto put = [&](uint16_t *w, uint2 v) { st64(w, make_uint2(v.x ^ kBias, v.y ^ kBias)); };
     {  // the tile's own CTB inside the clip rectangle: one set of parameters
       const SaoFast f = sm.fast[0][4];
       const FastRect q = fr[0];
@@ -491,175 +706,8 @@ __device__ __forceinline__ bool sao_alf_tile3(const Pass2Args &a, const Pass2Arg
       put(w, v);
     }
   }
-  if (DO_ALF && (seen & 0xF000F000u)) {
-    sm.wide = 1;
-    if (seen & 0xC000C000u) sm.big = 1;
-  }
   __syncthreads();
-  const bool big = DO_ALF && sm.big != 0;
-
-  // ---- (3) luma Laplacian sums per 2x2 cell (into the dead deblocked windows); chroma ALF / CC-ALF
-  const bool luma_alf = DO_ALF && me && me->luma_set >= 0;
-  if (luma_alf) luma_cells<S, NT3>(sm.sL, sm.cell());
-  {
-    // thread -> (plane, row, run of SPT samples)
-    constexpr int SPT = TWC * THC / (NT3 / 2);  // 8 (64 x 64 tiles) or 2 (32 x 32)
-    constexpr int NP = SPT / 2;                 // pairs per thread
-    constexpr int RPR = TWC / SPT;              // threads per chroma row
-    const int cc = tid / (NT3 / 2), t = tid % (NT3 / 2);
-    const int jj = t / RPR, i0 = (t % RPR) * SPT;
-    const DPlane &CD = a.dst[cc + 1];
-    const int gy = yc0 + jj, gx = xc0 + i0;
-    if (chroma_on[cc] && gy < CD.h && gx < CD.w) {
-      const int cf = (DO_ALF && me) ? me->chroma_filt[cc] : -1;
-      const int ccf = (DO_ALF && me) ? me->cc_filt[cc] : -1;
-      const int ctb_c = ctb / 2, y_ctb_c = y_ctb / 2;
-      const uint16_t *R0 = &sm.sC[cc][(jj + 2) * S::SCP + i0 + 4];
-      int v[SPT];
-      {
-        Words<NP + 2, 1> w0;
-        load_words<NP + 2, 1, (NP > 1)>(w0, R0, 1, NP + 1);
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-          const uint32_t cur = w0.w[1 + q] ^ kBias;
-          v[2 * q] = (int)(cur & 0xFFFF);
-          v[2 * q + 1] = (int)(cur >> 16);
-        }
-      }
-      if (cf >= 0)
-        chroma_alf_run<SPT>(R0, S::SCP, gy - y_ctb_c, ctb_c, a.tables.chroma_packed[min(cf, 7)], maxv, big, v);
-      if (ccf >= 0)  // col 2 i0 + 4 of the luma window = luma x of i0
-        cc_alf_run<SPT>(&sm.sL[(2 * jj + 3) * S::SLP + 2 * i0 + 4], S::SLP, (gy - y_ctb_c) * 2, ctb,
-                        !(gy * 2 + ctb >= ph && (ph - y_ctb) <= ctb - 4), a.tables.cc_coeff[cc][ccf], bd, maxv, v);
-      uint16_t *out = CD.s + (int64_t)gy * CD.stride + gx;
-      const bool vec = gx + SPT <= CD.w && ((uintptr_t)out & (2 * SPT - 1)) == 0;
-      if (vec && SPT == 8) {
-        uint4 o;
-        o.x = (uint32_t)v[0] | (uint32_t)v[1] << 16;
-        o.y = (uint32_t)v[2] | (uint32_t)v[3] << 16;
-        o.z = (uint32_t)v[4] | (uint32_t)v[5] << 16;
-        o.w = (uint32_t)v[6 % SPT] | (uint32_t)v[7 % SPT] << 16;
-        *reinterpret_cast<uint4 *>(out) = o;
-      } else if (vec && SPT == 4) {
-        *reinterpret_cast<uint2 *>(out) = make_uint2((uint32_t)v[0] | (uint32_t)v[1 % SPT] << 16,
-                                                     (uint32_t)v[2 % SPT] | (uint32_t)v[3 % SPT] << 16);
-      } else if (vec && SPT == 2) {
-        *reinterpret_cast<uint32_t *>(out) = (uint32_t)v[0] | (uint32_t)v[1 % SPT] << 16;
-      } else {
-#pragma unroll
-        for (int k = 0; k < SPT; ++k)
-          if (gx + k < CD.w) out[k] = (uint16_t)v[k];
-      }
-    }
-  }
-  const DPlane LD = a.dst[0];
-  if (!luma_alf) {
-    // the post-SAO tile as it is, 4 samples per store
-    for (int p = tid; p < TH * W / 4; p += NT3) {
-      const int j = p / (W / 4), i = (p % (W / 4)) * 4;
-      const int gx = X0 + i, gy = Y0 + j;
-      if (gy >= LD.h || gx >= LD.w) continue;
-      uint2 v = ld64(&sm.sL[(j + 3) * S::SLP + i + 4]);
-      v.x ^= kBias;
-      v.y ^= kBias;
-      uint16_t *out = LD.s + (int64_t)gy * LD.stride + gx;
-      if (gx + 4 <= LD.w && ((uintptr_t)out & 7) == 0) {
-        *reinterpret_cast<uint2 *>(out) = v;
-      } else {
-        const uint16_t s4[4] = {(uint16_t)(v.x & 0xFFFF), (uint16_t)(v.x >> 16), (uint16_t)(v.y & 0xFFFF),
-                                (uint16_t)(v.y >> 16)};
-        for (int k = 0; k < 4 && gx + k < LD.w; ++k) out[k] = s4[k];
-      }
-    }
-    return true;
-  }
-  __syncthreads();
-
-  // ---- (4) classes
-  luma_classes<W, TH, S, NT3>(sm.sL, sm.cell(), sm.cls_f, sm.cls_t, Y0, y_ctb, ctb, ph, bd, big,
-                             sm.wide != 0);
-  __syncthreads();
-
-  // ---- (5) 7x7 diamond: every thread keeps one block's taps and filters RPT of its 4-sample runs
-  constexpr int RUNS = TH * W / 4;
-  constexpr int RPT = RUNS / NT3;  // runs per thread: 4 (64 x 64) or 1 (32 x 32)
-  constexpr int TPB = 4 / RPT;     // threads per 4x4 block
-  const int b = tid / TPB;
-  const int bx = b % (W / 4), by = b / (W / 4);
-  const uint32_t *tab =
-      a.tables.luma_packed + ((size_t)me->luma_set * 100 + sm.cls_f[b] * 4 + sm.cls_t[b]) * kLumaEntry;
-  uint32_t c2[12], f[12];  // clip values and coefficients in registers
-  const int start = luma_filter(tab, c2, f);
-  const int gx = X0 + 4 * bx;
-#pragma unroll 1
-  for (int rr = 0; rr < RPT; ++rr) {
-    const int j = 4 * by + (tid % TPB) * RPT + rr;  // tile row
-    const int gy = Y0 + j;
-    if (gy >= LD.h || gx >= LD.w) continue;
-    int shift, y1, y2, y3;
-    table45(gy - y_ctb, ctb, shift, y1, y2, y3);
-    const uint16_t *R0 = &sm.sL[(j + 3) * S::SLP + 4 * bx + 4];
-    int o[4];
-    if (big) {
-      luma_run_plain(R0, S::SLP, y1, y2, y3, shift, tab, maxv, o);
-    } else {
-      const int st = start + (1 << (shift - 1));
-      int acc[4] = {st, st, st, st};
-      // words k of a row: samples (c0 - 4 + 2k, +1), c0 = the run's first sample
-      Words<6, 2> ru, rd;
-      load_words<6, 2, true>(ru, R0, 0, 6);  // the run's own row
-      const uint32_t cur[2] = {ru.w[2] ^ kBias, ru.w[3] ^ kBias};
-      const uint32_t m[2] = {kBias - cur[0], kBias - cur[1]};  // 0x8000 - cur per lane
-      auto tap = [&](const Words<6, 2> &up, const Words<6, 2> &dn, auto dx, int k) {
-        constexpr int DX = decltype(dx)::value;
-        const uint32_t c22 = c2[k] + c2[k];
-        static_for<2>([&](auto qc) {
-          constexpr int q = decltype(qc)::value;
-          const uint32_t b = c2[k] + m[q];
-          const uint32_t s = clip_off(up.template pair<DX + 2 * q>(), b, c22) +
-                             clip_off(dn.template pair<-DX + 2 * q>(), b, c22);
-          acc[2 * q] = dp2a_ulo(s, f[k], acc[2 * q]);
-          acc[2 * q + 1] = dp2a_uhi(s, f[k], acc[2 * q + 1]);
-        });
-      };
-      using I0 = std::integral_constant<int, 0>;
-      using I1 = std::integral_constant<int, 1>;
-      using Im1 = std::integral_constant<int, -1>;
-      using I2 = std::integral_constant<int, 2>;
-      using Im2 = std::integral_constant<int, -2>;
-      using I3 = std::integral_constant<int, 3>;
-      tap(ru, ru, I3{}, 9);
-      tap(ru, ru, I2{}, 10);
-      tap(ru, ru, I1{}, 11);
-      load_words<6, 2, true>(ru, R0 + y3 * S::SLP, 2, 4);
-      load_words<6, 2, true>(rd, R0 - y3 * S::SLP, 2, 4);
-      tap(ru, rd, I0{}, 0);
-      load_words<6, 2, true>(ru, R0 + y2 * S::SLP, 1, 5);
-      load_words<6, 2, true>(rd, R0 - y2 * S::SLP, 1, 5);
-      tap(ru, rd, I1{}, 1);
-      tap(ru, rd, I0{}, 2);
-      tap(ru, rd, Im1{}, 3);
-      load_words<6, 2, true>(ru, R0 + y1 * S::SLP, 1, 5);
-      load_words<6, 2, true>(rd, R0 - y1 * S::SLP, 1, 5);
-      tap(ru, rd, I2{}, 4);
-      tap(ru, rd, I1{}, 5);
-      tap(ru, rd, I0{}, 6);
-      tap(ru, rd, Im1{}, 7);
-      tap(ru, rd, Im2{}, 8);
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        const int cv = (int)((cur[p >> 1] >> ((p & 1) * 16)) & 0xFFFF);
-        o[p] = clampd(cv + (acc[p] >> shift), 0, maxv);
-      }
-    }
-    uint16_t *out = LD.s + (int64_t)gy * LD.stride + gx;
-    if (gx + 4 <= LD.w && ((uintptr_t)out & 7) == 0) {
-      *reinterpret_cast<uint2 *>(out) =
-          make_uint2((uint32_t)o[0] | (uint32_t)o[1] << 16, (uint32_t)o[2] | (uint32_t)o[3] << 16);
-    } else {
-      for (int p = 0; p < 4 && gx + p < LD.w; ++p) out[p] = (uint16_t)o[p];
-    }
-  }
+  finish_tile<W, TH, DO_ALF, false>(a, sm, tile, wide);
   return true;
 }
 
