@@ -2240,23 +2240,33 @@ int fill_strip_params_grid(void *rows, void *cols, const DPlane src[3], const DP
 }
 
 namespace {
-template <class K>
-int strip_smem(K kern, size_t bytes) {
-  if (bytes > 32 * 1024)  // above the default limit with the kernels' static shared memory
-    H266_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+// The strip kernels' largest shared memory, once per device: the limit belongs to
+// the kernel, so a launch that set its own amount could take it from under another
+// thread's launch of taller planes.
+int prepare_strip_kernels() {
+  static std::atomic<uint64_t> done{0};
+  int dev = 0;
+  H266_CUDA(cudaGetDevice(&dev));
+  const uint64_t bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_acquire) & bit) return H266_OK;
+  constexpr size_t most = ((kMaxStripSmem + 15) & ~15) + sizeof(RunScratch);
+  for (const void *k : {reinterpret_cast<const void *>(k_deblock_rows), reinterpret_cast<const void *>(k_deblock_cols),
+                        reinterpret_cast<const void *>(k_deblock_rows_batch),
+                        reinterpret_cast<const void *>(k_deblock_cols_batch)})
+    H266_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  done.fetch_or(bit, std::memory_order_release);
   return H266_OK;
 }
 
 int launch_strips_single(cudaStream_t st, const StripParams &v, const StripParams &h, const StripCounts &c,
                          uint64_t *launches) {
+  H266_TRY(prepare_strip_kernels());
   if (c.rows) {
-    H266_TRY(strip_smem(k_deblock_rows, c.smem_rows));
     k_deblock_rows<<<c.rows, 128, c.smem_rows, st>>>(v);
     H266_CUDA(cudaGetLastError());
     ++*launches;
   }
   if (c.cols) {
-    H266_TRY(strip_smem(k_deblock_cols, c.smem_cols));
     k_deblock_cols<<<c.cols, 128, c.smem_cols, st>>>(h);
     H266_CUDA(cudaGetLastError());
     ++*launches;
@@ -2284,14 +2294,13 @@ int launch_deblock_strips_grid(cudaStream_t st, const DPlane src[3], const DPlan
 
 int launch_strips_batch(cudaStream_t st, const void *d_rows, const uint32_t *d_first_rows, const void *d_cols,
                         const uint32_t *d_first_cols, int n, const StripCounts &c, uint64_t *launches) {
+  H266_TRY(prepare_strip_kernels());
   if (c.rows) {
-    H266_TRY(strip_smem(k_deblock_rows_batch, c.smem_rows));
     k_deblock_rows_batch<<<c.rows, 128, c.smem_rows, st>>>(static_cast<const StripParams *>(d_rows), d_first_rows, n);
     H266_CUDA(cudaGetLastError());
     ++*launches;
   }
   if (c.cols) {
-    H266_TRY(strip_smem(k_deblock_cols_batch, c.smem_cols));
     k_deblock_cols_batch<<<c.cols, 128, c.smem_cols, st>>>(static_cast<const StripParams *>(d_cols), d_first_cols, n);
     H266_CUDA(cudaGetLastError());
     ++*launches;
