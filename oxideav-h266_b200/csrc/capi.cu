@@ -2786,6 +2786,20 @@ int check_plan_batch(h266_ctx *ctx, uint32_t n, h266_chain_plan *const *plans, h
 }
 
 
+// SAO/ALF launches of a batch: per tile kernel variant, then per variant of the full-height chroma tiles.
+constexpr int kP2 = kPass2Variants + kPass2ChromaVariants;
+
+// The most bytes that the parameter table of a batch of n pictures takes (exec_batch):
+// per picture its tile or strip parameters, a device walk's, SAO/ALF parameters for
+// the tiles and the full-height chroma, and its entry in each of their prefix
+// tables; per table a first entry and the alignment of its section.
+size_t batch_table_bytes(size_t n) {
+  const size_t item = std::max(deblock_tile_params_size(), 2 * strip_params_size()) + walk_batch_item_size() +
+                      2 * sizeof(Pass2Args) + (2 + 3 + 2) * sizeof(uint32_t);
+  constexpr size_t sections = 4 + 4 + 1 + 3 + 1 + 2 * kP2;
+  return n * item + sections * (256 + sizeof(uint32_t)) + kPass2Variants * sizeof(uint32_t);
+}
+
 // Queues a batch of chain executions on `stream` with its parameter tables in
 // `bb`: the device walks of the pictures that derive their side information
 // on the device (three launches for all of them), one tile-deblocking launch
@@ -2808,8 +2822,6 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
   std::vector<uint32_t> tile_first[2] = {{0}, {0}}, walk_first[3] = {{0}, {0}, {0}};  // clear, CU map, walk CTAs
   WalkBatchCounts walk_total;
   const size_t wis = walk_batch_item_size();
-  // SAO/ALF: per tile kernel variant, then per variant of the full-height chroma tiles
-  constexpr int kP2 = kPass2Variants + kPass2ChromaVariants;
   std::vector<Pass2Args> p2[kP2];
   std::vector<uint32_t> p2_first[kP2];
   auto add_p2 = [&](int v, const Pass2Args &a, uint32_t ctas) {
@@ -3317,8 +3329,7 @@ int h266_server_create(int device, uint32_t max_batch, uint64_t memory_budget, h
   Guard g(device);
   // Parameter tables sized for a full batch up front: growing them later
   // would synchronise the device (and allocate pinned memory) mid-run.
-  const size_t reserve = std::max<size_t>((size_t)max_batch * (deblock_tile_params_size() + sizeof(Pass2Args) + 64),
-                                          256 * 1024);
+  const size_t reserve = std::max<size_t>(batch_table_bytes(max_batch), 256 * 1024);
   for (ServerSlot &sl : s->slots) {
     cudaError_t e = cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming);
