@@ -2800,6 +2800,42 @@ size_t batch_table_bytes(size_t n) {
   return n * item + sections * (256 + sizeof(uint32_t)) + kPass2Variants * sizeof(uint32_t);
 }
 
+// Whether two planes share samples: exact for planes of one stride (views of one
+// surface), by their address ranges otherwise.
+bool planes_meet(const DPlane &p, const DPlane &q) {
+  const DPlane &a = p.s <= q.s ? p : q, &b = p.s <= q.s ? q : p;  // a starts first
+  if (b.s >= a.s + (a.h - 1) * a.stride + a.w) return false;
+  if (a.stride != b.stride) return true;
+  const int64_t d = b.s - a.s, y = d / a.stride, x = d % a.stride;  // b's first sample in a's rows
+  return (x < a.w && y < a.h) || (x + b.w > a.stride && y + 1 < a.h);
+}
+
+// The items that cannot share the strip kernels' launches: a launch runs its
+// pictures in no order, so an item filtered in place, and every other one that
+// reads the same samples, run one after the other as listed.  Tile items (tile[i])
+// have launches of their own, after the strips'.
+std::vector<uint8_t> items_in_turn(const std::vector<BatchItem> &items, const std::vector<uint8_t> &tile) {
+  std::vector<uint8_t> turn(items.size(), 0);
+  if (std::all_of(items.begin(), items.end(), [](const BatchItem &it) { return it.pass2; })) return turn;
+  struct Span {
+    const uint16_t *end;
+    const DPlane *p;
+    uint32_t item;
+  };
+  std::vector<Span> spans;
+  for (uint32_t i = 0; i < items.size(); ++i)
+    for (const DPlane &p : items[i].P)
+      if (!tile[i] && p.w > 0 && p.h > 0) spans.push_back(Span{p.s + (p.h - 1) * p.stride + p.w, &p, i});
+  std::sort(spans.begin(), spans.end(), [](const Span &a, const Span &b) { return a.p->s < b.p->s; });
+  for (size_t k = 0; k < spans.size(); ++k)
+    for (size_t m = k + 1; m < spans.size() && spans[m].p->s < spans[k].end; ++m) {
+      const uint32_t i = spans[k].item, j = spans[m].item;
+      if (i == j || (items[i].pass2 && items[j].pass2) || !planes_meet(*spans[k].p, *spans[m].p)) continue;
+      turn[i] = turn[j] = 1;
+    }
+  return turn;
+}
+
 // Queues a batch of chain executions on `stream` with its parameter tables in
 // `bb`: the device walks of the pictures that derive their side information
 // on the device (three launches for all of them), one tile-deblocking launch
@@ -2846,6 +2882,13 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
     strip_first[0].push_back(strip_total.rows);
     strip_first[1].push_back(strip_total.cols);
   };
+  std::vector<uint8_t> tile(n);
+  for (uint32_t i = 0; i < n; ++i) {
+    const BatchItem &it = items[i];
+    tile[i] = it.pass2 && (it.db.device_walk ? it.db.dw_tiles : it.db.tiles_ok) && !ctx->force_global_deblock &&
+              !ctx->force_strip_deblock;
+  }
+  const std::vector<uint8_t> in_turn = items_in_turn(items, tile);
   uint32_t large_tiles = 0;
   for (const BatchItem &it : items)
     if (it.pass2 && it.packed) large_tiles += pass2_large_tiles(it.args);
@@ -2854,13 +2897,9 @@ int exec_batch(h266_ctx *ctx, BatchBufs &bb, cudaStream_t stream, std::vector<Ba
     BatchItem &it = items[i];
     Run &r = runs[i];
     const uint8_t *base = it.st.base;
-    r.tile = it.pass2 && (it.db.device_walk ? it.db.dw_tiles : it.db.tiles_ok) && !ctx->force_global_deblock &&
-             !ctx->force_strip_deblock;
+    r.tile = tile[i] != 0;
     const DPlane *dst = it.pass2 ? it.S : it.P;
-    // pictures filtered in place and listed twice run one after the other
-    const bool twice = !it.pass2 && std::count_if(items.begin(), items.end(), [&](const BatchItem &o) {
-                                      return !o.pass2 && o.P[0].s == it.P[0].s;
-                                    }) > 1;
+    const bool twice = in_turn[i] != 0;
     r.strips = !r.tile && !twice && (it.db.device_walk || (!ctx->force_global_deblock && deblock_strips_fit(dst)));
     if (it.db.device_walk && !twice) {  // the side information is derived on the device first, batched
       if (!it.walk) return set_error(H266_ERR_INVALID_ARGUMENT, "device-built side information without walk scratch");
