@@ -1717,8 +1717,8 @@ struct MergeJob {
 };
 
 // Merges the jobs' pictures on lane `ln`: one upload (records and parameters),
-// the wavefront over every picture, one download; then, for pictures the
-// wavefront left, the anti-diagonal launches.
+// the wavefront over every picture it can take, one download; then, for the other
+// pictures and those the wavefront left, the anti-diagonal launches.
 static int run_merges(h266_ctx *ctx, Lane &ln, const std::vector<MergeJob> &jobs, uint32_t bd, uint32_t log2) {
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const uint32_t np = (uint32_t)jobs.size();
@@ -1727,7 +1727,7 @@ static int run_merges(h266_ctx *ctx, Lane &ln, const std::vector<MergeJob> &jobs
   size_t total = al(np * sizeof(int32_t)), max_ctbs = 0;  // the statuses first
   for (uint32_t i = 0; i < np; ++i) {
     const size_t n = (size_t)jobs[i].wc * jobs[i].hc;
-    max_ctbs = std::max(max_ctbs, n);
+    if (sao_merge_waves(jobs[i].hc)) max_ctbs = std::max(max_ctbs, n);
     off_rec[i] = total;
     total += n * sizeof(h266_sao_ctb_params);
     off_map[i] = total;
@@ -1738,7 +1738,7 @@ static int run_merges(h266_ctx *ctx, Lane &ln, const std::vector<MergeJob> &jobs
   const size_t work_from = total;
   for (uint32_t i = 0; i < np; ++i) {
     off_work[i] = total;
-    total += al(sao_merge_work_bytes((size_t)jobs[i].wc * jobs[i].hc));
+    total += al(sao_merge_work_bytes((size_t)jobs[i].wc * jobs[i].hc, sao_merge_waves(jobs[i].hc)));
   }
   H266_TRY(ln.walk.ensure(std::max<size_t>(total, 256)));
   uint8_t *work = ln.walk.as<uint8_t>();
@@ -1784,28 +1784,28 @@ static int run_merges(h266_ctx *ctx, Lane &ln, const std::vector<MergeJob> &jobs
     std::memcpy(j.map, host + off_map[i], n);
     ctx->d2h_bytes += n * (sizeof(h266_sao_ctb_params) + 1);
   };
-  std::vector<uint32_t> all(np), left;
-  for (uint32_t i = 0; i < np; ++i) all[i] = i;
+  std::vector<uint32_t> wave, left;
+  for (uint32_t i = 0; i < np; ++i)
+    if (jobs[i].wc && jobs[i].hc) (sao_merge_waves(jobs[i].hc) ? wave : left).push_back(i);
   size_t off_args, off_first;
   uint8_t *base = nullptr;
-  H266_TRY(upload(all, {}, off_args, off_first, base));
-  {
-    Prof pf(ctx, ln.stream, H266_PROF_SAO_ALF);
-    H266_TRY(launch_sao_merge_wave(ln.stream, base + off_args, (int)np, (int)max_ctbs, bd > 14, &ctx->launches));
-  }
   const uint8_t *host = nullptr;
-  H266_TRY(read_back(ln, work, results, &host));
-  uint32_t n_diags = 0;
-  for (uint32_t i = 0; i < np; ++i) {
-    if (!jobs[i].wc || !jobs[i].hc) continue;
-    if (reinterpret_cast<const int32_t *>(host)[i]) {
-      take(host, i);
-      continue;
+  if (!wave.empty()) {
+    H266_TRY(upload(wave, {}, off_args, off_first, base));
+    {
+      Prof pf(ctx, ln.stream, H266_PROF_SAO_ALF);
+      H266_TRY(launch_sao_merge_wave(ln.stream, base + off_args, (int)wave.size(), (int)max_ctbs, bd > 14,
+                                     &ctx->launches));
     }
-    left.push_back(i);
-    n_diags = std::max(n_diags, jobs[i].wc + jobs[i].hc - 1);
+    H266_TRY(read_back(ln, work, results, &host));
+    for (uint32_t i : wave) {
+      if (reinterpret_cast<const int32_t *>(host)[i]) take(host, i);
+      else left.push_back(i);
+    }
   }
   if (left.empty()) return H266_OK;
+  uint32_t n_diags = 0;
+  for (uint32_t i : left) n_diags = std::max(n_diags, jobs[i].wc + jobs[i].hc - 1);
   const uint32_t nl = (uint32_t)left.size();
   std::vector<uint32_t> first((size_t)n_diags * (nl + 1), 0), totals(n_diags, 0);
   for (uint32_t d = 0; d < n_diags; ++d)

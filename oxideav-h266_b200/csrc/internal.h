@@ -482,7 +482,9 @@ size_t sao_stats_bytes(int n_ctbs);
 // diagonal form: one launch per anti-diagonal, d_first holding per diagonal
 // the n + 1 prefix sums of the pictures' CTB counts on it, h_totals the
 // diagonals' totals.
-size_t sao_merge_work_bytes(size_t n_ctbs);
+constexpr uint32_t kSaoWaveRows = 256;  // CTB rows of the largest picture the wave takes
+inline bool sao_merge_waves(uint32_t h_ctbs) { return h_ctbs <= kSaoWaveRows; }
+size_t sao_merge_work_bytes(size_t n_ctbs, bool wave);  // wave: with the statistics
 size_t sao_merge_args_size();
 void fill_sao_merge_args(void *out, const DPlane src[2], const DPlane pre[2], int bd, int chr_ctb, int w_ctbs,
                          int h_ctbs, int max_off, const h266_sao_ctb_params *d_indep, h266_sao_ctb_params *d_merged,

@@ -516,8 +516,9 @@ __global__ void __launch_bounds__(kMergeThreads) k_sao_merge_diag_batch(const Me
 // That holds where no sample clips.  A candidate that could clip some sample of
 // its CTB (the CTB's extremes against the candidate's offsets) is summed from
 // the samples by its warp; a picture with more than n / 32 + 4 CTBs within the
-// largest offset of the range's ends, or more than kWaveRows CTB rows, is left
-// to the diagonal launches.
+// largest offset of the range's ends is left to the diagonal launches, and one of
+// more than kSaoWaveRows CTB rows never comes here (its choices would not fit, and
+// its statistics take 850 bytes a CTB, more than the CTB where that is small).
 
 // blockIdx: CTB, Cb or Cr, picture.
 template <bool WIDE>
@@ -551,7 +552,6 @@ __device__ long long merge_delta_direct(const MergeArgs &a, int c, int cx, int c
 }
 
 constexpr int kWaveThreads = 512;
-constexpr int kWaveRows = 256;  // CTB rows of the largest picture it takes
 
 // One CTA per picture.
 __global__ void __launch_bounds__(kWaveThreads) k_merge_wave(const MergeArgs *__restrict__ args) {
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(kWaveThreads) k_merge_wave(const MergeArgs *__
   __syncthreads();
   if (near) atomicAdd(&s_near, near);
   __syncthreads();
-  const bool go = s_near <= 2 * (n / 32 + 4) && a.h_ctbs <= kWaveRows;
+  const bool go = s_near <= 2 * (n / 32 + 4);
   if (tid == 0) *a.status = go ? 1 : 0;
   if (!go) return;
   // The last two diagonals' choices by CTB row: what a neighbour's candidate needs.
@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(kWaveThreads) k_merge_wave(const MergeArgs *__
     int type, band, cls, from;
     int off[4];
   };
-  __shared__ Choice ring[2][kWaveRows][2];
+  __shared__ Choice ring[2][kSaoWaveRows][2];
   // lane 8 k + 4 c + j: offset j of component c of candidate k (own, left, above)
   const int k = lane >> 3, c = (lane >> 2) & 1, j = lane & 3;
   // A CTB's statistics and its own parameters, loaded while the diagonal before
@@ -725,17 +725,21 @@ void fill_sao_merge_args(void *out, const DPlane src[2], const DPlane pre[2], in
   std::memcpy(out, &a, sizeof a);
 }
 
-size_t sao_merge_work_bytes(size_t n) { return n * (3 * 8 + 4 + 4 + 2 * sizeof(SaoStats)); }
+size_t sao_merge_work_bytes(size_t n, bool wave) { return n * (3 * 8 + 4 + (wave ? 4 + 2 * sizeof(SaoStats) : 0)); }
 
 int launch_sao_merge_wave(cudaStream_t st, const void *d_args, int n, int max_ctbs, bool wide, uint64_t *launches) {
   if (n <= 0 || max_ctbs <= 0) return H266_OK;
   const MergeArgs *args = static_cast<const MergeArgs *>(d_args);
-  if (wide) k_merge_stats<true><<<dim3(max_ctbs, 2, n), kStatThreads, 0, st>>>(args);
-  else k_merge_stats<false><<<dim3(max_ctbs, 2, n), kStatThreads, 0, st>>>(args);
-  H266_CUDA(cudaGetLastError());
+  for (int i0 = 0; i0 < n; i0 += 65535) {  // the z dimension of a grid
+    const dim3 grid(max_ctbs, 2, std::min(n - i0, 65535));
+    if (wide) k_merge_stats<true><<<grid, kStatThreads, 0, st>>>(args + i0);
+    else k_merge_stats<false><<<grid, kStatThreads, 0, st>>>(args + i0);
+    H266_CUDA(cudaGetLastError());
+    ++*launches;
+  }
   k_merge_wave<<<n, kWaveThreads, 0, st>>>(args);
   H266_CUDA(cudaGetLastError());
-  *launches += 2;
+  ++*launches;
   return H266_OK;
 }
 
