@@ -987,22 +987,7 @@ constexpr size_t smem3() {
 inline int tile_w(const Pass2Args &a) { return a.ctb_log2 >= 6 && !a.small_tiles ? 64 : 32; }
 inline int tile_h(const Pass2Args &a) { return tile_w(a) == 64 && a.tile_h == 32 ? 32 : tile_w(a); }
 
-// Once per kernel and device: the largest shared-memory carveout, so that four
-// CTAs of the tile kernel fit on an SM.
-template <class K>
-int prepare_kernel(K kern, size_t shm) {
-  static_assert(sizeof(Smem3<64, 64>) + 128 + sizeof(Pass2Args) <= 48 * 1024, "default shared-memory limit of a CTA");
-  static std::atomic<uint64_t> done{0};
-  int dev = 0;
-  H266_CUDA(cudaGetDevice(&dev));
-  const uint64_t bit = 1ull << (dev & 63);
-  if (!(done.load(std::memory_order_relaxed) & bit)) {
-    H266_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    done.fetch_or(bit);
-  }
-  (void)shm;
-  return H266_OK;
-}
+static_assert(sizeof(Smem3<64, 64>) + 128 + sizeof(Pass2Args) <= 48 * 1024, "default shared-memory limit of a CTA");
 
 // Host-side driver API entry point for the tensor-map encoder (no libcuda link).
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -1056,7 +1041,6 @@ int launch_one(cudaStream_t st, const Pass2Args &in, bool do_sao, bool do_alf) {
   const unsigned n = (unsigned)(a.tiles_x * a.tiles_y);
   const size_t shm = smem3<W, TH>();
   auto go = [&](auto kern) -> int {
-    H266_TRY(prepare_kernel(kern, shm));
     kern<<<n, NT3, shm, st>>>(a);
     H266_CUDA(cudaGetLastError());
     return H266_OK;
@@ -1123,12 +1107,10 @@ int launch_variant(cudaStream_t st, const Pass2Args *d_args, const uint32_t *d_f
   const size_t shm = smem3<W, TH>();
   if (cps > 0 && d_queue) {
     auto kern = k_sao_alf_tiles_queue<W, TH, DO_SAO, DO_ALF>;
-    H266_TRY(prepare_kernel(kern, shm));
     const uint32_t grid = std::min<uint32_t>(ctas, (uint32_t)(sm_count() * cps));
     kern<<<grid, NT3, shm, st>>>(d_args, d_first, n, ctas, d_queue);
   } else {
     auto kern = k_sao_alf_tiles_batch<W, TH, DO_SAO, DO_ALF>;
-    H266_TRY(prepare_kernel(kern, shm));
     kern<<<ctas, NT3, shm, st>>>(d_args, d_first, n);
   }
   H266_CUDA(cudaGetLastError());
