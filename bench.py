@@ -133,6 +133,18 @@ class ClockSampler:
         self.skip = len(self._lines())
         return self.skip
 
+    def settle(self, step, max_seconds: float = 2.0):
+        """After the timed steps: goes on with untimed ones until a line has come
+        since prime(), as a timed region shorter than the sampling period ends
+        before the next (20 steps of 1.2 ms against 50 ms); gives up after
+        `max_seconds`."""
+        t0 = time.perf_counter()
+        while self.proc and self.proc.poll() is None and time.perf_counter() - t0 < max_seconds:
+            if len(self._lines()) > self.skip:
+                break
+            step()
+            torch_sync()
+
     def summary(self):
         if not self.proc:
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["nvidia-smi unavailable"]}
@@ -807,8 +819,9 @@ def run_ours(args, rank, world, local_rank):
                 fn()
                 end.record(stream)
                 torch.cuda.synchronize()
+                run["launches"] = ctx.kernel_launches - l0
+                cs.settle(step)
             barrier()
-            run["launches"] = ctx.kernel_launches - l0
             run["clocks"] = cs.summary()
             if not bad_clocks(run["clocks"]):
                 break
