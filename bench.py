@@ -46,13 +46,13 @@ WIDTH, HEIGHT, BITDEPTH = 1920, 1080, 10
 METRIC = "filter-chain Mpx/s 1080p/2160p 10-bit bit-exact"
 # From one ncu capture of the batched SAO/ALF launch (k_sao_alf_tiles_batch
 # <64, 64, 1, 1>) over 4 pictures of this workload: DRAM bytes read + written
-# (25 031 680 + 2 758 400 B; ncu flushes the caches before the launch, and the
+# (25 509 120 + 1 189 120 B; ncu flushes the caches before the launch, and the
 # output planes retire from L2 after it) and thread instructions per luma pixel
 # (warp instructions x 32 lanes: the issue rate they are set against counts the
 # lanes of a partly active warp too); the bench line scales them to its own
 # batch and labels them so.
-SAO_ALF_TRAFFIC_PER_PX = (25031680 + 2758400) / (4 * 1920 * 1080)
-SAO_ALF_THREAD_INST_PER_PX = 266.6  # 69 098 582 warp instructions x 32 lanes / 4 pictures
+SAO_ALF_TRAFFIC_PER_PX = (25509120 + 1189120) / (4 * 1920 * 1080)
+SAO_ALF_THREAD_INST_PER_PX = 258.8  # 67 089 580 warp instructions x 32 lanes / 4 pictures
 
 
 def _import_pkg():

@@ -379,8 +379,9 @@ int h266_sao_chroma_merge(h266_ctx *ctx, const h266_picture *src, const h266_pic
                           uint8_t *merge_map);
 /* The same merge for n pictures at once (device pictures, H266_MEM_DEVICE):
  * the statistics of every picture's CTBs in one launch, then a CTA per
- * picture that walks its anti-diagonals (pictures that clip widely: one launch
- * per anti-diagonal over the CTBs of all of them).  Per picture
+ * picture that walks its anti-diagonals (pictures that clip widely or have more
+ * than 256 CTB rows: one launch per anti-diagonal over the CTBs of all of them).
+ * Per picture
  * i: srcs[i], pres[i], independent[i] (w_ctbs[i] x h_ctbs[i] records),
  * merged[i] and merge_maps[i] as for h266_sao_chroma_merge; results are the
  * same as n separate calls.  Returns when the results are in host memory. */

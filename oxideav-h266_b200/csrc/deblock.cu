@@ -3024,8 +3024,8 @@ int launch_device_walk(cudaStream_t st, const DeviceWalkIn &in, uint8_t *scratch
 // The walks of many pictures in three launches: the clearing of every
 // picture's CU maps (no CU) and segment grids (bS 0), the CU maps, and the edge
 // walk.  Per picture a WalkBatchItem (parameters, clear extents, the walk's
-// list count); CTAs find their picture by binary search over
-// per-launch prefix tables of CTA counts.
+// list count); CTAs find their picture in per-launch prefix tables of CTA counts
+// by ballots (batch_picture).
 struct WalkBatchItem {
   WalkParams p;
   uint4 *clear;            // the picture's walk scratch

@@ -163,7 +163,7 @@ int build_deblock_plan(const h266_picture &pic, const h266_deblock_cu *cus, uint
 // the three device planes.  seg/comp point at device copies of the plan.
 // Strip kernels: the vertical pass on row bands read from `src` (luma mapped
 // through `lut` when given) and written to `dst` (which may be `src`), then the
-// horizontal pass on 16-column strips of `dst` in place.
+// horizontal pass on 8-column strips of `dst` in place.
 bool deblock_strips_fit(const DPlane planes[3]);
 struct StripSide {  // device pointers of one pass
   const EdgeSeg *segs;

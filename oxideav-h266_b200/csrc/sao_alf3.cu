@@ -27,10 +27,12 @@
 //  5. the 7x7 luma diamond, one block per thread with its 12 taps in
 //     registers and each of the 7 rows held as packed words.
 // The ALU pipe (64 lanes a clock: half the issue rate) and the waits between
-// its instructions bound phases 2, 3 and 5 (issue 0.63 and ALU 0.50 busy over the
+// its instructions bound phases 2, 3 and 5 (issue 0.64 and ALU 0.51 busy over the
 // whole launch), so the taps are in the offset form of alf_tile.cuh.  16 1080p 10-bit
-// pictures: 389 us (472 with two clamps a tap, pairs instead of quads, border
-// samples one by one and word-per-value filter tables).
+// pictures: 364 us (472 with two clamps a tap, pairs instead of quads, border
+// samples one by one and word-per-value filter tables; 389 with the plain form's
+// branches in every phase).  Tiles with samples outside the packed lanes' range are
+// told apart before phase 2 (finish_big).
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
